@@ -1,22 +1,16 @@
 // Shared device machinery of the graphop kernels for sm_100a.
 //
-// Work decomposition.  Every op sees the graph as a flat stream of CSR positions
-// 0..E-1.  A one-pass "expansion" turns the caller's chunk table (row[c], indptr[c]),
-// in which several consecutive chunks may belong to one node, into erow[j] = owner node
-// of position j (-1 where no chunk covers j).  All other kernels cut the position stream
-// into fixed tiles of `tile` positions, one warp per tile, so the work per warp is the
-// same whatever the degree distribution looks like: a node with a million in-edges is
-// simply spread over thousands of warps, and a thousand one-edge nodes share one warp.
+// Work decomposition.  Every op sees the graph as a flat stream of CSR positions 0..E-1.  A one-pass "expansion" turns the
+// caller's chunk table (row[c], indptr[c]), in which several consecutive chunks may belong to one node, into erow[j] =
+// owner node of position j (-1 where no chunk covers j), and cuts the stream into work tiles of equal cost.  The walker
+// of gk_group.cuh does the work of all row-reducing and per-edge ops; walk_kernel below is the plain form of it that
+// takes any shape (one element per lane and slot, tiles of equal length) and reduces the softmax's open segments.
 //
-// Row-owned reductions without atomics.  Inside a tile a warp walks the positions in
-// order; all 32 lanes work on one edge at a time, each lane owning R vector slots of the
-// node's H*D feature row, and a run of equal erow[] values is one segment.  A segment
-// that lies wholly inside the tile is reduced in registers and stored once.  The first
-// segment of a tile whose node already started in an earlier tile ("open head") and the
-// last segment of a tile whose node continues in the next one ("open tail") are stored
-// as partials in a per-tile carry slot; a second small kernel lets the tile in which the
-// node starts fold the carries of the following tiles in ascending tile order.  The sum
-// order is therefore a function of (E, tile) only: results are bit-reproducible.
+// Row-owned reductions without atomics.  A run of equal erow[] values is one segment.  A segment that lies wholly inside
+// a tile is reduced in registers and stored once.  The first segment of a tile whose node already started in an earlier
+// tile ("open head") and the last segment of a tile whose node continues in the next one ("open tail") are stored as
+// partials in two carry slots per tile, and later launches fold the slots of a node in ascending tile order.  The sum
+// order is a function of the graph and the tile size only: results are bit-reproducible.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -159,10 +153,29 @@ __device__ __forceinline__ void reduce_heads(A (&p)[R], int lph) {
 // ---------------------------------------------------------------------------------------
 constexpr int kExpandTile = 256;  // positions per warp
 
+// Work tiles of equal cost.  A position costs 1 and a node kRowCost (its begin and end cost the walker about as much as
+// that many edges), so that neither a tile of one-edge nodes nor one inside a hub takes much longer than the others.
+// With cost(p) = p + kRowCost * (node of p) the boundary of tile t is the first position whose cost reaches t * tile:
+// every position knows which boundaries fall between its predecessor and itself, and writes them.  Positions before the
+// covered ones count for node 0, those after for the last node.  Boundaries past the last position are E.
+constexpr int kRowCost = 4;
+struct TileCut {
+  int32_t* start;      // (n + 1) boundaries, or null
+  long long n;         // tiles
+  int shift;           // log2 of the cost per tile
+};
+__device__ __forceinline__ void cut_tiles(const TileCut& cut, long long p, long long E, long long node, long long prev_node) {
+  const long long hi = (p + kRowCost * node) >> cut.shift;
+  const long long lo = p > 0 ? (p - 1 + kRowCost * prev_node) >> cut.shift : -1;
+  for (long long t = lo + 1; t <= hi && t <= cut.n; ++t) cut.start[t] = (int32_t)p;
+  if (p == E - 1)
+    for (long long t = hi + 1; t <= cut.n; ++t) cut.start[t] = (int32_t)E;
+}
+
 template <typename I>
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
 expand_rows_kernel(const I* __restrict__ row, const I* __restrict__ indptr, long long C, long long E,
-                   int32_t* __restrict__ erow, PlanHeader* __restrict__ hdr) {
+                   int32_t* __restrict__ erow, PlanHeader* __restrict__ hdr, TileCut cut) {
   const int lane = threadIdx.x & 31;
   const long long t = (long long)blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5);
   const long long p0 = t * kExpandTile;
@@ -177,8 +190,19 @@ expand_rows_kernel(const I* __restrict__ row, const I* __restrict__ indptr, long
   const long long lo = p0 > base ? p0 : base;
   const long long hi = p1 < end ? p1 : end;
   // positions of this tile outside [base, end) belong to no chunk
-  for (long long p = p0 + lane; p < p1; p += 32)
-    if (p < lo || p >= hi) erow[p] = -1;
+  if (p0 < base || p1 > end) {
+    long long tail_node = 0;   // of the last covered position
+    if (cut.start && p1 > end && end > base) {
+      long long c = C - 1;
+      while (c > 0 && (long long)indptr[c] >= end) --c;
+      tail_node = (long long)row[c];
+    }
+    for (long long p = p0 + lane; p < p1; p += 32)
+      if (p < lo || p >= hi) {
+        erow[p] = -1;
+        if (cut.start) cut_tiles(cut, p, E, p < base ? 0 : tail_node, p <= base ? 0 : tail_node);
+      }
+  }
   if (lo >= hi) return;
   // chunk that contains position lo: the last c with indptr[c] <= lo
   // 32-way search: every lane probes one pivot strictly inside (a, b), the ballot picks the sub-range;
@@ -194,6 +218,12 @@ expand_rows_kernel(const I* __restrict__ row, const I* __restrict__ indptr, long
     const long long above = __shfl_sync(kFull, m, cnt < 32 ? cnt : 31);
     if (cnt) a = below;
     if (cnt < 32) b = above;
+  }
+  int prev_row = 0;   // node of the position before the ones at hand
+  if (cut.start && lo > base) {
+    long long c = a;
+    while (c > 0 && (long long)indptr[c] >= lo) --c;
+    prev_row = (int)row[c];
   }
   // 32 chunks at a time: lane l holds chunk a + l; every position of the part of the tile they cover
   // finds its chunk by a 5-step search over the lanes' start positions, so that the stores are
@@ -224,7 +254,13 @@ expand_rows_kernel(const I* __restrict__ row, const I* __restrict__ indptr, long
         if (cand < 32 && start <= p_rel) owner = cand;
       }
       const int rr = __shfl_sync(kFull, r, owner);
-      if (p < to) erow[p] = rr;
+      int before = __shfl_up_sync(kFull, rr, 1);
+      if (lane == 0) before = prev_row;
+      if (p < to) {
+        erow[p] = rr;
+        if (cut.start) cut_tiles(cut, p, E, rr, before);
+      }
+      prev_row = __shfl_sync(kFull, rr, to - q < 32 ? (int)(to - q) - 1 : 31);
     }
     if (__any_sync(kFull, past)) break;
   }
@@ -281,17 +317,14 @@ template <class Op, bool kCarryLevel>
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
 walk_kernel(Op op, const PlanHeader* __restrict__ hdr, const int32_t* __restrict__ erow,
             const int32_t* __restrict__ other, const int32_t* __restrict__ eid, long long E, int tile,
-            long long n_rows, int32_t* __restrict__ rows_next, const int32_t* __restrict__ tile_start) {
+            long long n_rows, int32_t* __restrict__ rows_next) {
   constexpr int U = Op::kUnroll;
   constexpr bool kOut = Op::kRowOut;
   constexpr bool kFill = Op::kRowOut && !kCarryLevel;
   const int lane = threadIdx.x & 31;
   const long long t = (long long)blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5);
-  // tile t covers positions [t * tile, (t + 1) * tile), or, with a plan's row-aligned boundaries,
-  // [tile_start[t], tile_start[t + 1]): the same number of tiles, each boundary moved up to the next row start
   if (t * tile >= E) return;
-  const long long j0 = tile_start ? (long long)__ldg(tile_start + t) : t * tile;
-  const long long j1 = tile_start ? (long long)__ldg(tile_start + t + 1) : (j0 + tile < E ? j0 + tile : E);
+  const long long j0 = t * tile, j1 = j0 + tile < E ? j0 + tile : E;
 
   if constexpr (kFill) {
     if (t == 0 && hdr->cover_hi <= hdr->cover_lo) {  // no covered position at all

@@ -3,6 +3,7 @@
 #pragma once
 #include <atomic>
 #include <cstdio>
+#include <initializer_list>
 #include <mutex>
 #include <type_traits>
 #include <utility>
@@ -10,9 +11,9 @@
 
 #include "../../include/graphop_b200.h"
 #include "gk_common.cuh"
+#include "gk_group.cuh"
 #include "gk_ops.cuh"
 #include "gk_softmax.cuh"
-#include "gk_staged.cuh"
 
 namespace gk {
 
@@ -90,16 +91,35 @@ struct Arena {
 // ---------------------------------------------------------------------------------------
 // tiling
 // ---------------------------------------------------------------------------------------
+constexpr int kMaxLevels = 12;
 constexpr int kCarryTile = 32;  // wider tiles on the short upper levels save a launch but run slower: a warp
                                 // walks its slots one after the other (ER-small 0.27 -> 0.40 ms with 256)
-constexpr int kMaxLevels = 12;
 
-// Positions per warp at level 0: small graphs get small tiles so that every SM has work,
-// large graphs get 256 so that carries stay a fraction of a percent of the traffic.
+// Positions per warp at level 0 of the register-fetch walker and of the softmax carry streams.
 inline int pick_tile(long long n_edges) {
   long long t = 32;
-  while (t < GK_TILE && n_edges / t > 16384) t <<= 1;
+  while (t < 256 && n_edges / t > 16384) t <<= 1;
   return (int)t;
+}
+
+// Cost of a work tile of the gathering walker (see cut_tiles: positions and nodes) and the number of tiles.  Large
+// graphs get tiles of 256, which keeps carries and the fixed part of a tile a fraction of the work; smaller ones get the
+// smallest tile, down to 32, that makes no more than kTilesWanted: enough for every SM to have several rounds of warps
+// (attention step, 4 heads x 32 fp32: R-MAT 15 with tiles of 256 / 128 / 64 / 32 355 / 274 / 265 / 256 us, R-MAT 18
+// 1480 / 1437 / 1462 / 1545 us, R-MAT 21 12.97 / 12.95 / 13.00 / 14.06 ms).
+constexpr long long kTilesWanted = 49152;
+inline int tile_cost(long long E, long long n_nodes) {
+  const long long total = E + kRowCost * n_nodes;
+  int t = 32;
+  while (t < 256 && total / t > kTilesWanted) t <<= 1;
+  return t;
+}
+inline long long tile_count(long long E, long long n_nodes, int tile) { return (E + kRowCost * n_nodes) / tile + 1; }
+// the most tiles any graph of E positions and up to n_nodes nodes gets
+inline long long tile_bound(long long E, long long n_nodes) {
+  const int t = tile_cost(E, n_nodes);
+  const long long n = tile_count(E, n_nodes, t);
+  return t > 32 && n < kTilesWanted + 2 ? kTilesWanted + 2 : n;
 }
 
 struct Levels {
@@ -137,19 +157,28 @@ struct GraphView {
   const int32_t* other;  // may be null (ops without a second endpoint)
   const int32_t* eid;    // may be null: identity
   long long E;
-  // from a plan: boundaries of the level-0 tiles moved up to row starts (for tiles of `start_tile` positions), and
-  // whether no row crosses a boundary any more (then there is nothing for the carry levels to do)
+  // work tiles: their boundaries (null: the op has no use for them), number and cost; whether the boundaries were moved
+  // to row starts already (a plan's), and whether no row crosses one (then the carry levels have nothing to do)
   const int32_t* tile_start = nullptr;
-  int start_tile = 0;
-  bool no_carry = false;
-  const int32_t* starts_for(int tile) const { return tile == start_tile ? tile_start : nullptr; }
+  long long n_tiles = 0;
+  int tile = 0;
+  bool aligned = false, no_carry = false;
 };
 
 template <typename I>
 inline int prepare_graph(Arena& ar, const I* row, const I* indptr, const I* eid, const I* indices, long long C,
-                         long long E, cudaStream_t st, GraphView* g) {
+                         long long E, long long n_nodes, cudaStream_t st, GraphView* g) {
   auto* hdr = (PlanHeader*)ar.take(sizeof(PlanHeader));
   auto* erow = (int32_t*)ar.take((size_t)E * 4);
+  // n_nodes < 0: an op that cuts no tiles
+  TileCut cut{nullptr, 0, 0};
+  if (n_nodes >= 0) {
+    g->tile = tile_cost(E, n_nodes);
+    while ((1 << cut.shift) < g->tile) ++cut.shift;
+    cut.n = tile_count(E, n_nodes, g->tile);
+    cut.start = (int32_t*)ar.take((size_t)(cut.n + 1) * 4);
+    g->tile_start = cut.start; g->n_tiles = cut.n;
+  }
   int32_t* other32 = nullptr;
   int32_t* eid32 = nullptr;
   if (sizeof(I) == 8) {
@@ -159,7 +188,8 @@ inline int prepare_graph(Arena& ar, const I* row, const I* indptr, const I* eid,
   if (!ar.base) return GRAPHOP_OK;
   if (ar.overflow) return GRAPHOP_ERR_WORKSPACE;
   const long long warps = (E + kExpandTile - 1) / kExpandTile;
-  expand_rows_kernel<I><<<grid_for_warps(warps, kWarpsPerCta), kWarpsPerCta * 32, 0, st>>>(row, indptr, C, E, erow, hdr);
+  expand_rows_kernel<I><<<grid_for_warps(warps, kWarpsPerCta), kWarpsPerCta * 32, 0, st>>>(row, indptr, C, E, erow, hdr,
+                                                                                            cut);
   GK_LAUNCHED("expand_rows");
   g->hdr = hdr;
   g->erow = erow;
@@ -189,24 +219,24 @@ template <typename I>
 struct FromChunks {
   const I* row; const I* indptr; const I* eid; const I* indices; long long C, E;
   bool valid(bool need_indices) const { return row && indptr && (!need_indices || indices); }
-  int operator()(Arena& ar, cudaStream_t st, GraphView* g) const {
-    return prepare_graph<I>(ar, row, indptr, eid, indices, C, E, st, g);
+  int operator()(Arena& ar, long long n_nodes, cudaStream_t st, GraphView* g) const {
+    return prepare_graph<I>(ar, row, indptr, eid, indices, C, E, n_nodes, st, g);
   }
 };
 struct FromPlan {
   const graphop_plan_t* p;
   bool valid(bool need_indices) const { return p && p->erow && p->header && (!need_indices || p->other); }
-  int operator()(Arena&, cudaStream_t, GraphView* g) const {
+  int operator()(Arena&, long long, cudaStream_t, GraphView* g) const {
     g->hdr = (const PlanHeader*)p->header;
     g->erow = p->erow;
     g->other = p->other;
     g->eid = p->eid;
     g->E = p->n_edges;
-    if ((p->flags & GRAPHOP_PLAN_ROW_TILES) && p->tile_start) {
-      g->tile_start = p->tile_start;
-      g->start_tile = p->tile;
-      g->no_carry = (p->flags & GRAPHOP_PLAN_NO_CARRY) != 0;
-    }
+    g->tile_start = p->tile_start;
+    g->tile = p->tile;
+    g->n_tiles = tile_count(p->n_edges, p->n_nodes, p->tile);
+    g->aligned = true;
+    g->no_carry = (p->flags & GRAPHOP_PLAN_NO_CARRY) != 0;
     return GRAPHOP_OK;
   }
 };
@@ -228,92 +258,18 @@ template <typename T> struct VecMax { static constexpr int value = 16 / (int)siz
 inline bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 inline bool is_pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
 
-struct VecShape { int V, R, S; };
-// V elements per slot and R slots per lane for an H*D row; R = 0: does not fit 8 slots per lane.
-template <typename T>
-inline VecShape pick_shape(int HD, int D, bool all_aligned) {
-  VecShape s;
-  constexpr int VM = VecMax<T>::value;
-  s.V = (all_aligned && D % VM == 0) ? VM : 1;
-  s.S = HD / s.V;
-  if (s.V == 1) s.R = s.S <= 256 ? 8 : 0;
-  else s.R = s.S <= 32 ? 1 : s.S <= 64 ? 2 : s.S <= 128 ? 4 : s.S <= 256 ? 8 : 0;
-  return s;
-}
-
-// Calls f(integral_constant<int,V>, integral_constant<int,R>) for the instantiated pairs.
-template <typename T, class F>
-inline int dispatch_shape(const VecShape& s, F&& f) {
-  constexpr int VM = VecMax<T>::value;
-  using std::integral_constant;
-  if (s.V == 1 && s.R == 8) return f(integral_constant<int, 1>{}, integral_constant<int, 8>{});
-  if (s.V == VM) {
-    switch (s.R) {
-      case 1: return f(integral_constant<int, VM>{}, integral_constant<int, 1>{});
-      case 2: return f(integral_constant<int, VM>{}, integral_constant<int, 2>{});
-      case 4: return f(integral_constant<int, VM>{}, integral_constant<int, 4>{});
-      case 8: return f(integral_constant<int, VM>{}, integral_constant<int, 8>{});
-    }
-  }
-  return GRAPHOP_ERR_UNSUPPORTED;
-}
-
-// Calls f(integral_constant<int, LPH>) with the compile-time lanes-per-head the staged dot-product
-// ops are specialised for (2 to 32), or 0 for "read it at run time".
-template <class F>
-inline int dispatch_lph(int lph, F&& f) {
-  using std::integral_constant;
-  switch (lph) {
-    case 2: return f(integral_constant<int, 2>{});
-    case 4: return f(integral_constant<int, 4>{});
-    case 8: return f(integral_constant<int, 8>{});
-    case 16: return f(integral_constant<int, 16>{});
-    case 32: return f(integral_constant<int, 32>{});
-    default: return f(integral_constant<int, 0>{});
-  }
-}
+}  // namespace gk
+#include "gk_launch.cuh"
+namespace gk {
 
 // ---------------------------------------------------------------------------------------
-// level-0 + carry-level launch sequence of a row-producing op
+// level-0 + carry-level launch sequence of a row-producing op of the register-fetch walker (gk_common.cuh): the shapes
+// the gathering walker has no slot width for
 // ---------------------------------------------------------------------------------------
-template <class Op>
-inline size_t staged_smem_bytes() {
-  return (size_t)Op::kWarps * staged_warp_bytes<Op>();
-}
-
-// Launches the staged level-0 walker; raises the kernel's dynamic shared memory limit once per device.
-template <class Op>
-inline int launch_staged(const Op& op, const GraphView& g, int tile, long long n_rows, int32_t* rows_next,
-                         cudaStream_t st) {
-  // one flag per device and kernel; several host threads may get here at once (autograd's backward thread):
-  // setting the attribute twice is harmless, the flag only saves the call
-  static std::atomic<bool> configured[64];
-  int dev = 0;
-  GK_CUDA(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 64 || !configured[dev].load(std::memory_order_acquire)) {
-    GK_CUDA(cudaFuncSetAttribute(walk_staged_kernel<Op>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)staged_smem_bytes<Op>()));
-    if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
-  }
-  const long long nt = (g.E + tile - 1) / tile;
-  walk_staged_kernel<Op><<<grid_for_warps(nt, Op::kWarps), Op::kWarps * 32, staged_smem_bytes<Op>(), st>>>(
-      op, g.hdr, g.erow, g.other, g.eid, g.E, tile, n_rows, rows_next, g.starts_for(tile));
-  GK_LAUNCHED(Op::kName);
-  return GRAPHOP_OK;
-}
-
-template <class X> struct TypeTag { using type = X; };
-template <class Op, class = void> struct IsStaged : std::false_type {};
-template <class Op> struct IsStaged<Op, std::void_t<decltype(Op::kEdgeBytes)>> : std::true_type {};
-
-// `make_op(carry_out, carry_in)` returns the op bound to one level's carry buffers; `make_op0`
-// does the same for level 0 when that level runs a different (staged) op that writes the same
-// carry format.
-template <class MakeOp, class MakeOp0>
+template <class MakeOp>
 inline int run_row_levels(Arena& ar, const GraphView& g, int tile0, long long n_rows, size_t carry_elem_bytes,
-                          long long carry_stride, cudaStream_t st, MakeOp&& make_op, MakeOp0&& make_op0) {
+                          long long carry_stride, cudaStream_t st, MakeOp&& make_op) {
   Levels lv = make_levels(g.E, tile0);
-  if (g.no_carry && g.starts_for(tile0)) lv.n = 1;   // row-aligned tiles that no row crosses: level 0 stores every row
   void* carry[kMaxLevels];
   int32_t* rows[kMaxLevels + 1];
   rows[0] = nullptr;
@@ -325,118 +281,69 @@ inline int run_row_levels(Arena& ar, const GraphView& g, int tile0, long long n_
   if (!ar.base) return GRAPHOP_OK;
   if (ar.overflow) return GRAPHOP_ERR_WORKSPACE;
   {
-    auto op = make_op0(carry[0], nullptr);
+    auto op = make_op(carry[0], nullptr);
     using Op = decltype(op);
-    if constexpr (IsStaged<Op>::value) {
-      GK_TRY(launch_staged(op, g, lv.tile[0], n_rows, rows[1], st));
-    } else {
-      walk_kernel<Op, false><<<grid_for_warps(lv.ntiles[0], kWarpsPerCta), kWarpsPerCta * 32, 0, st>>>(
-          op, g.hdr, g.erow, g.other, g.eid, g.E, lv.tile[0], n_rows, rows[1], g.starts_for(lv.tile[0]));
-      GK_LAUNCHED(Op::kName);
-    }
+    walk_kernel<Op, false><<<grid_for_warps(lv.ntiles[0], kWarpsPerCta), kWarpsPerCta * 32, 0, st>>>(
+        op, g.hdr, g.erow, g.other, g.eid, g.E, lv.tile[0], n_rows, rows[1]);
+    GK_LAUNCHED(Op::kName);
   }
   for (int k = 1; k < lv.n; ++k) {
     auto op = make_op(carry[k], carry[k - 1]);
     using Op = decltype(op);
     walk_kernel<Op, true><<<grid_for_warps(lv.ntiles[k], kWarpsPerCta), kWarpsPerCta * 32, 0, st>>>(
-        op, g.hdr, rows[k], nullptr, nullptr, lv.len[k], lv.tile[k], n_rows, rows[k + 1], nullptr);
+        op, g.hdr, rows[k], nullptr, nullptr, lv.len[k], lv.tile[k], n_rows, rows[k + 1]);
     GK_LAUNCHED("carry_level");
   }
   return GRAPHOP_OK;
 }
-template <class MakeOp>
-inline int run_row_levels(Arena& ar, const GraphView& g, int tile0, long long n_rows, size_t carry_elem_bytes,
-                          long long carry_stride, cudaStream_t st, MakeOp&& make_op) {
-  return run_row_levels(ar, g, tile0, n_rows, carry_elem_bytes, carry_stride, st, make_op, make_op);
-}
 
-// out[node] = sum_k w[eid[k]] * feat(k): picks the vector shape, splits very wide rows into
-// feature blocks of 256 slots (each block is an independent aggregation).
+// out[node] = sum_k w[eid[k]] * feat(k)
 template <typename T, bool kEdgeFeat>
 inline int run_aggregate(Arena& ar, const GraphView& g, const T* w, const T* x, T* y, long long n_rows, int H, int D,
                          cudaStream_t st) {
   using A = typename AccOf<T>::type;
-  const int HD = H * D;
-  const bool al = aligned16(x) && aligned16(y);
-  VecShape s = pick_shape<T>(HD, D, al);
-  const int tile0 = pick_tile(g.E);
-  const int block_elems = 256 * s.V;  // widest register-resident block
-  for (int feat0 = 0; feat0 < HD; feat0 += block_elems) {
-    const int elems = HD - feat0 < block_elems ? HD - feat0 : block_elems;
-    VecShape b = s;
-    b.S = elems / s.V;
-    if (s.V == 1) b.R = 8;
-    else b.R = b.S <= 32 ? 1 : b.S <= 64 ? 2 : b.S <= 128 ? 4 : 8;
+  const GeoPick p = pick_geo(H, D, sizeof(T), slot_align_of({x, y}), true);
+  if (p.SB && p.nhb <= kMaxHeadBlocks)
+    return dispatch_geo<T, true>(p, [&](auto tag) -> int {
+      GroupAggregate<typename decltype(tag)::type, kEdgeFeat> op;
+      fill_geo(op, p, H, D);
+      op.w = w; op.x = x; op.y = y;
+      return launch_walk(ar, g, p, op, n_rows, st);
+    });
+  // 2-byte elements with an odd D: one element per slot, feature blocks of 256
+  const int HD = H * D, tile0 = pick_tile(g.E);
+  constexpr int kBlock = 256;
+  for (int feat0 = 0; feat0 < HD; feat0 += kBlock) {
     const size_t mark = ar.used;
-    GK_TRY((dispatch_shape<T>(b, [&](auto Vc, auto Rc) -> int {
-      constexpr int V = decltype(Vc)::value, R = decltype(Rc)::value;
-      using OpT = typename std::conditional<(V > 1 || sizeof(T) == 16), AggregateStaged<T, V, R, kEdgeFeat>,
-                                            AggregateOp<T, V, R, kEdgeFeat>>::type;
-      int wm = 0;
-      if constexpr (IsStaged<OpT>::value) wm = OpT::pick_wmode(w, H, feat0, HD, block_elems);
-      auto run = [&](auto op_type) -> int {
-        using OpM = typename decltype(op_type)::type;
-        return run_row_levels(ar, g, tile0, n_rows, sizeof(A), HD, st, [&](void* cout, void* cin) {
-          OpM op;
-          op.w = w; op.x = x; op.y = y; op.carry = (A*)cout; op.carry_in = (const A*)cin;
-          op.H = H; op.D = D; op.HD = HD; op.S = b.S; op.feat0 = feat0;
-          if constexpr (IsStaged<OpM>::value) { op.wmode = wm; op.set_weight_bounds((long long)g.E * H); }
-          return op;
-        });
-      };
-      if constexpr (IsStaged<OpT>::value) {
-        // the packed modes get their own instantiations; the per-lane mode keeps the run-time test
-        using Pieces = AggregateStaged<T, V, R, kEdgeFeat, OpT::kWeightsPieces>;
-        using Words = AggregateStaged<T, V, R, kEdgeFeat, OpT::kWeightsWords>;
-        if (wm == OpT::kWeightsPieces) return run(TypeTag<Pieces>{});
-        if (wm == OpT::kWeightsWords) return run(TypeTag<Words>{});
-        if constexpr (sizeof(T) == 2) {
-          using Half = AggregateStaged<T, V, R, kEdgeFeat, OpT::kWeightsHalfWords>;
-          if (wm == OpT::kWeightsHalfWords) return run(TypeTag<Half>{});
-        }
-      }
-      return run(TypeTag<OpT>{});
-    })));
-    if (feat0 + block_elems < HD) ar.used = mark;  // blocks run back to back on one stream: reuse the scratch
+    GK_TRY(run_row_levels(ar, g, tile0, n_rows, sizeof(A), HD, st, [&](void* cout, void* cin) {
+      AggregateOp<T, 1, 8, kEdgeFeat> op;
+      op.w = w; op.x = x; op.y = y; op.carry = (A*)cout; op.carry_in = (const A*)cin;
+      op.H = H; op.D = D; op.HD = HD; op.S = HD - feat0 < kBlock ? HD - feat0 : kBlock; op.feat0 = feat0;
+      return op;
+    }));
+    if (feat0 + kBlock < HD) ar.used = mark;  // blocks run back to back on one stream: reuse the scratch
   }
   return GRAPHOP_OK;
 }
 
 // y[eid[k], h] = a[node(k), h, :] . feat(k)[h, :]
 template <typename T, bool kEdgeFeat>
-inline int run_edge_dot(const GraphView& g, const T* a, const T* b, T* y, int H, int D, cudaStream_t st) {
-  const int HD = H * D;
-  const bool al = aligned16(a) && aligned16(b);
-  const VecShape s = pick_shape<T>(HD, D, al);
+inline int run_edge_dot(Arena& ar, const GraphView& g, const T* a, const T* b, T* y, int H, int D, cudaStream_t st) {
+  const GeoPick p = narrow_fix(pick_geo(H, D, sizeof(T), slot_align_of({a, b}), false));
+  if (p.SB && p.nhb <= kMaxHeadBlocks)
+    return dispatch_geo<T, true>(p, [&](auto tag) -> int {
+      GroupEdgeDot<typename decltype(tag)::type, kEdgeFeat> op;
+      fill_geo(op, p, H, D);
+      op.a = a; op.b = b; op.y = y;
+      return launch_walk(ar, g, p, op, 0, st);
+    });
   const int tile0 = pick_tile(g.E);
-  const long long nt = (g.E + tile0 - 1) / tile0;
-  const unsigned grid = grid_for_warps(nt, kWarpsPerCta);
-  const int lph = D / s.V;
-  if (s.R == 0 || !is_pow2(lph)) {
-    EdgeDotAnyOp<T, kEdgeFeat> op;
-    op.a = a; op.b = b; op.y = y; op.H = H; op.D = D; op.HD = HD;
-    walk_kernel<decltype(op), false><<<grid, kWarpsPerCta * 32, 0, st>>>(op, g.hdr, g.erow, g.other, g.eid, g.E, tile0, 0,
-                                                                        nullptr, nullptr);
-    GK_LAUNCHED("edge_dot_any");
-    return GRAPHOP_OK;
-  }
-  return dispatch_shape<T>(s, [&](auto Vc, auto Rc) -> int {
-    constexpr int V = decltype(Vc)::value, R = decltype(Rc)::value;
-    if constexpr (V > 1) {
-      return dispatch_lph(lph, [&](auto Lc) -> int {
-        EdgeDotStaged<T, V, R, kEdgeFeat, decltype(Lc)::value> op;
-        op.a = a; op.b = b; op.y = y; op.H = H; op.D = D; op.HD = HD; op.S = s.S; op.lph = lph;
-        return launch_staged(op, g, tile0, 0, nullptr, st);
-      });
-    } else {
-      EdgeDotOp<T, V, R, kEdgeFeat> op;
-      op.a = a; op.b = b; op.y = y; op.H = H; op.D = D; op.HD = HD; op.S = s.S; op.lph = lph;
-      walk_kernel<decltype(op), false><<<grid, kWarpsPerCta * 32, 0, st>>>(op, g.hdr, g.erow, g.other, g.eid, g.E,
-                                                                          tile0, 0, nullptr, nullptr);
-      GK_LAUNCHED("edge_dot");
-      return (int)GRAPHOP_OK;
-    }
-  });
+  EdgeDotAnyOp<T, kEdgeFeat> op;
+  op.a = a; op.b = b; op.y = y; op.H = H; op.D = D; op.HD = H * D;
+  walk_kernel<decltype(op), false><<<grid_for_warps((g.E + tile0 - 1) / tile0, kWarpsPerCta), kWarpsPerCta * 32, 0, st>>>(
+      op, g.hdr, g.erow, g.other, g.eid, g.E, tile0, 0, nullptr);
+  GK_LAUNCHED("edge_dot_any");
+  return GRAPHOP_OK;
 }
 
 // dB[eid[k], :] = sum_h dy[eid[k], h] * A[node(k), h, :]
@@ -497,7 +404,7 @@ inline int run_softmax_heads(Arena& ar, const GraphView& g, const T* in0, const 
     op.stats = stats; op.carry = (A*)carry[k]; op.carry_in = k ? (const A*)carry[k - 1] : carry0; op.H = H;
     op.n_nodes = n_nodes;
     walk_kernel<decltype(op), true><<<grid_for_warps(lv.ntiles[k], kWarpsPerCta), kWarpsPerCta * 32, 0, st>>>(
-        op, g.hdr, rows[k], nullptr, nullptr, lv.len[k], lv.tile[k], n_nodes, rows[k + 1], nullptr);
+        op, g.hdr, rows[k], nullptr, nullptr, lv.len[k], lv.tile[k], n_nodes, rows[k + 1]);
     GK_LAUNCHED("carry_level");
   }
   softmax_finish_kernel<T, H, kBackward><<<grid0, kSoftmaxWarps * 32, 0, st>>>(g.erow, g.eid, in0, in1, out, stats,
@@ -552,9 +459,9 @@ inline int maskedmm_forward(const GS& gs, const T* A_, const T* B_, T* y, long l
   GK_TRY(check_ws(ws));
   Arena ar(ws, wsb);
   GraphView g;
-  GK_TRY(gs(ar, st, &g));
+  GK_TRY(gs(ar, n_dst, st, &g));
   GK_TRY(zero_uncovered(g, y, (size_t)E * H * sizeof(T), st));
-  return run_edge_dot<T, false>(g, A_, B_, y, H, D, st);
+  return run_edge_dot<T, false>(ar, g, A_, B_, y, H, D, st);
 }
 
 template <typename T, class GS>
@@ -574,12 +481,12 @@ inline int maskedmm_backward(const GS& gs_r, const GS& gs_c, long long Cr, long 
   Arena ar(ws, wsb);
   {
     GraphView g;
-    GK_TRY(gs_r(ar, st, &g));
+    GK_TRY(gs_r(ar, n_dst, st, &g));
     GK_TRY((run_aggregate<T, false>(ar, g, dy, B_, dA, n_dst, H, D, st)));
   }
   ar.used = 0;  // the second pass runs after the first on the same stream: reuse the scratch
   GraphView g;
-  GK_TRY(gs_c(ar, st, &g));
+  GK_TRY(gs_c(ar, n_src, st, &g));
   return run_aggregate<T, false>(ar, g, dy, A_, dB, n_src, H, D, st);
 }
 
@@ -592,9 +499,9 @@ inline int node_mul_edge_forward(const GS& gs, const T* A_, const T* B_, T* y, l
   GK_TRY(check_ws(ws));
   Arena ar(ws, wsb);
   GraphView g;
-  GK_TRY(gs(ar, st, &g));
+  GK_TRY(gs(ar, n_dst, st, &g));
   GK_TRY(zero_uncovered(g, y, (size_t)E * H * sizeof(T), st));
-  return run_edge_dot<T, true>(g, A_, B_, y, H, D, st);
+  return run_edge_dot<T, true>(ar, g, A_, B_, y, H, D, st);
 }
 
 template <typename T, class GS>
@@ -609,7 +516,7 @@ inline int node_mul_edge_backward(const GS& gs, const T* A_, const T* B_, const 
   GK_TRY(check_ws(ws));
   Arena ar(ws, wsb);
   GraphView g;
-  GK_TRY(gs(ar, st, &g));
+  GK_TRY(gs(ar, n_dst, st, &g));
   GK_TRY((run_aggregate<T, true>(ar, g, dy, B_, dA, n_dst, H, D, st)));
   if (!ar.base) return GRAPHOP_OK;
   GK_TRY(zero_uncovered(g, dB, (size_t)E * D * sizeof(T), st));
@@ -625,7 +532,7 @@ inline int sparse_softmax(const GS& gs, const T* in0, const T* in1, T* out, long
   GK_TRY(check_ws(ws));
   Arena ar(ws, wsb);
   GraphView g;
-  GK_TRY(gs(ar, st, &g));
+  GK_TRY(gs(ar, -1, st, &g));
   GK_TRY(zero_uncovered(g, out, (size_t)E * H * sizeof(T), st));
   return run_softmax<T, kBackward>(ar, g, in0, in1, out, n_nodes, H, st);
 }
@@ -643,7 +550,7 @@ inline int spmm_forward(const GS& gs, const T* edata, const T* x, T* y, long lon
   GK_TRY(check_ws(ws));
   Arena ar(ws, wsb);
   GraphView g;
-  GK_TRY(gs(ar, st, &g));
+  GK_TRY(gs(ar, n_dst, st, &g));
   return run_aggregate<T, false>(ar, g, edata, x, y, n_dst, H, D, st);
 }
 
@@ -662,15 +569,15 @@ inline int spmm_backward(const GS& gs_r, const GS& gs_c, long long C, long long 
   Arena ar(ws, wsb);
   {
     GraphView g;
-    GK_TRY(gs_r(ar, st, &g));
+    GK_TRY(gs_r(ar, n_dst, st, &g));
     if (ar.base) {
       GK_TRY(zero_uncovered(g, dedata, (size_t)E * H * sizeof(T), st));
-      GK_TRY((run_edge_dot<T, false>(g, dy, x, dedata, H, D, st)));
+      GK_TRY((run_edge_dot<T, false>(ar, g, dy, x, dedata, H, D, st)));
     }
   }
   ar.used = 0;
   GraphView g;
-  GK_TRY(gs_c(ar, st, &g));
+  GK_TRY(gs_c(ar, n_src, st, &g));
   return run_aggregate<T, false>(ar, g, edata, dy, dx, n_src, H, D, st);
 }
 
@@ -683,10 +590,50 @@ template <typename A> inline A neg_inf_host();
 template <> inline float neg_inf_host<float>() { return -INFINITY; }
 template <> inline double neg_inf_host<double>() { return -(double)INFINITY; }
 
+// The fused kernels take heads of a power-of-two number of 16-byte slots and node rows of at most 4 KB.
 template <typename T>
-inline bool attention_shape_ok(int H, int D, bool al, VecShape* s) {
-  *s = pick_shape<T>(H * D, D, al);
-  return s->V == VecMax<T>::value && s->R != 0 && is_pow2(D / s->V);
+inline bool attention_shape_ok(int H, int D, bool al, GeoPick* p) {
+  constexpr int VM = VecMax<T>::value;
+  if (!al || D % VM || !is_pow2(D / VM) || (long long)H * D / VM > 256) return false;
+  *p = pick_geo(H, D, sizeof(T), 16, false);
+  return p->SB == 16;
+}
+
+template <typename T, bool kBias>
+inline int run_attn_forward(Arena& ar, const GraphView& g, const GeoPick& s, const T* q, const T* k, const T* v,
+                            const T* rel, double scale, T* o, void* lse, long long n_dst, int H, int D,
+                            cudaStream_t st) {
+  return dispatch_geo<T, false>(s, [&](auto tag) -> int {
+    GroupAttnFwd<typename decltype(tag)::type, kBias> op;
+    using A = typename decltype(op)::A;
+    fill_geo(op, s, H, D);
+    op.q = q; op.k = k; op.v = v; op.rel = rel; op.o = o; op.lse = (A*)lse; op.scale = (A)scale;
+    return launch_walk(ar, g, s, op, n_dst, st);
+  });
+}
+template <typename T, bool kBias, class A>
+inline int run_attn_bwd_dst(Arena& ar, const GraphView& g, const GeoPick& s, const T* q, const T* k, const T* v,
+                            const T* rel, const T* o, const T* dout, const void* lse, StatPair<A>* stat,
+                            EdgePair<A>* pd, double scale, T* dq, long long n_dst, int H, int D, cudaStream_t st) {
+  return dispatch_geo<T, false>(s, [&](auto tag) -> int {
+    GroupAttnBwdDst<typename decltype(tag)::type, kBias> op;
+    fill_geo(op, s, H, D);
+    op.q = q; op.k = k; op.v = v; op.rel = rel; op.o = o; op.dout = dout; op.lse = (const A*)lse; op.stat = stat;
+    op.pd = pd; op.dq = dq; op.scale = (A)scale; op.Hp = stat_heads(H, (int)sizeof(A));
+    return launch_walk(ar, g, s, op, n_dst, st);
+  });
+}
+template <typename T, bool kPairs, class A>
+inline int run_attn_bwd_src(Arena& ar, const GraphView& g, const GeoPick& s, const T* q, const T* k, const T* v,
+                            const T* dout, const StatPair<A>* stat, const EdgePair<A>* pd, double scale, T* dk, T* dv,
+                            long long n_src, int H, int D, cudaStream_t st) {
+  return dispatch_geo<T, false>(s, [&](auto tag) -> int {
+    GroupAttnBwdSrc<typename decltype(tag)::type, kPairs> op;
+    fill_geo(op, s, H, D);
+    op.q = q; op.k = k; op.v = v; op.dout = dout; op.stat = stat; op.pd = pd; op.dk = dk; op.dv = dv;
+    op.scale = (A)scale; op.Hp = stat_heads(H, (int)sizeof(A));
+    return launch_walk(ar, g, s, op, n_src, st);
+  });
 }
 
 template <typename T, class GS>
@@ -695,7 +642,7 @@ inline int attention_forward(const GS& gs, long long C, const T* q, const T* k, 
                              size_t wsb, cudaStream_t st) {
   using A = typename AccOf<T>::type;
   GK_TRY(check_sizes(C, E, n_dst, n_src, H, D));
-  VecShape s;
+  GeoPick s;
   if (!attention_shape_ok<T>(H, D, aligned16(q) && aligned16(k) && aligned16(v) && aligned16(o), &s))
     return GRAPHOP_ERR_UNSUPPORTED;
   if (n_dst == 0) return GRAPHOP_OK;
@@ -714,23 +661,8 @@ inline int attention_forward(const GS& gs, long long C, const T* q, const T* k, 
     return GRAPHOP_OK;
   }
   if (!gs.valid(true)) return GRAPHOP_ERR_INVALID_ARGUMENT;
-  GK_TRY(gs(ar, st, &g));
-  const int tile0 = pick_tile(E);
-  return dispatch_shape<T>(s, [&](auto Vc, auto Rc) -> int {
-    constexpr int V = decltype(Vc)::value, R = decltype(Rc)::value;
-    const long long cstride = HD + 2 * s.S;
-    if constexpr (V == 1) return (int)GRAPHOP_ERR_UNSUPPORTED;
-    else return dispatch_lph(D / V, [&](auto Lc) -> int {
-      constexpr int LPH = decltype(Lc)::value;
-      auto generic = [&](void* cout, void* cin) {
-        AttnFwdStaged<T, V, R, LPH> op;
-        op.q = q; op.k = k; op.v = v; op.o = o; op.lse = (A*)lse; op.carry = (A*)cout; op.carry_in = (const A*)cin;
-        op.scale = (A)scale; op.H = H; op.D = D; op.HD = HD; op.S = s.S; op.lph = D / V; op.cstride = cstride;
-        return op;
-      };
-      return run_row_levels(ar, g, tile0, n_dst, sizeof(A), cstride, st, generic);
-    });
-  });
+  GK_TRY(gs(ar, n_dst, st, &g));
+  return run_attn_forward<T, false>(ar, g, s, q, k, v, (const T*)nullptr, scale, o, lse, n_dst, H, D, st);
 }
 
 // Defined in gk_banded.cuh for bfloat16: the tensor-core kernel for dense-band graphs.  Returns
@@ -777,7 +709,7 @@ inline int attention_backward(const GS& gs_r, const GS& gs_c, bool has_eid_t, lo
   using A = typename AccOf<T>::type;
   GK_TRY(check_sizes(C, E, n_dst, n_src, H, D));
   if (Ct < 0) return GRAPHOP_ERR_INVALID_ARGUMENT;
-  VecShape s;
+  GeoPick s;
   const bool al = aligned16(q) && aligned16(k) && aligned16(v) && aligned16(o) && aligned16(dout) && aligned16(dq) &&
                   aligned16(dk) && aligned16(dv);
   if (!attention_shape_ok<T>(H, D, al, &s)) return GRAPHOP_ERR_UNSUPPORTED;
@@ -793,8 +725,6 @@ inline int attention_backward(const GS& gs_r, const GS& gs_c, bool has_eid_t, lo
     return GRAPHOP_ERR_INVALID_ARGUMENT;
   GK_TRY(check_ws(ws));
   Arena ar(ws, wsb);
-  const int HD = H * D;
-  const int tile0 = pick_tile(E);
   const int Hp = stat_heads(H, (int)sizeof(A));
   StatPair<A>* stat = (StatPair<A>*)ar.take((size_t)n_dst * Hp * sizeof(StatPair<A>));  // survives both passes
   // with the transposed CSR's edge ids the destination pass leaves (p, ds) of every edge for the source pass
@@ -802,51 +732,15 @@ inline int attention_backward(const GS& gs_r, const GS& gs_c, bool has_eid_t, lo
   const size_t mark = ar.used;
   {
     GraphView g;
-    GK_TRY(gs_r(ar, st, &g));
-    GK_TRY((dispatch_shape<T>(s, [&](auto Vc, auto Rc) -> int {
-      constexpr int V = decltype(Vc)::value, R = decltype(Rc)::value;
-      if constexpr (V == 1) return (int)GRAPHOP_ERR_UNSUPPORTED;
-      else return dispatch_lph(D / V, [&](auto Lc) -> int {
-        constexpr int LPH = decltype(Lc)::value;
-        auto generic = [&](void* cout, void* cin) {
-          AttnBwdDstStaged<T, V, R, LPH> op;
-          op.q = q; op.k = k; op.v = v; op.o = o; op.dout = dout; op.lse = (const A*)lse; op.stat = stat;
-          op.pd = pd; op.dq = dq; op.carry = (A*)cout; op.carry_in = (const A*)cin; op.scale = (A)scale;
-          op.H = H; op.Hp = Hp; op.D = D; op.HD = HD; op.S = s.S; op.lph = D / V;
-          return op;
-        };
-        return run_row_levels(ar, g, tile0, n_dst, sizeof(A), HD, st, generic);
-      });
-    })));
+    GK_TRY(gs_r(ar, n_dst, st, &g));
+    GK_TRY((run_attn_bwd_dst<T, false>(ar, g, s, q, k, v, (const T*)nullptr, o, dout, lse, stat, pd, scale, dq, n_dst,
+                                       H, D, st)));
   }
   ar.used = mark;
   GraphView g;
-  GK_TRY(gs_c(ar, st, &g));
-  return dispatch_shape<T>(s, [&](auto Vc, auto Rc) -> int {
-    constexpr int V = decltype(Vc)::value, R = decltype(Rc)::value;
-    if constexpr (V == 1) return (int)GRAPHOP_ERR_UNSUPPORTED;
-    else return dispatch_lph(D / V, [&](auto Lc) -> int {
-      constexpr int LPH = decltype(Lc)::value;
-      if (pd) {
-        auto weighted = [&](void* cout, void* cin) {
-          AttnBwdSrcPairsStaged<T, V, R, LPH> op;
-          op.q = q; op.k = k; op.v = v; op.dout = dout; op.stat = stat; op.pd = pd; op.dk = dk;
-          op.dv = dv; op.carry = (A*)cout; op.carry_in = (const A*)cin; op.scale = (A)scale;
-          op.H = H; op.Hp = Hp; op.D = D; op.HD = HD; op.S = s.S; op.lph = D / V;
-          return op;
-        };
-        return run_row_levels(ar, g, tile0, n_src, sizeof(A), 2 * HD, st, weighted);
-      }
-      auto generic = [&](void* cout, void* cin) {
-        AttnBwdSrcStaged<T, V, R, LPH> op;
-        op.q = q; op.k = k; op.v = v; op.dout = dout; op.stat = stat; op.dk = dk;
-        op.dv = dv; op.carry = (A*)cout; op.carry_in = (const A*)cin; op.scale = (A)scale;
-        op.H = H; op.Hp = Hp; op.D = D; op.HD = HD; op.S = s.S; op.lph = D / V;
-        return op;
-      };
-      return run_row_levels(ar, g, tile0, n_src, sizeof(A), 2 * HD, st, generic);
-    });
-  });
+  GK_TRY(gs_c(ar, n_src, st, &g));
+  if (pd) return run_attn_bwd_src<T, true>(ar, g, s, q, k, v, dout, stat, pd, scale, dk, dv, n_src, H, D, st);
+  return run_attn_bwd_src<T, false>(ar, g, s, q, k, v, dout, stat, pd, scale, dk, dv, n_src, H, D, st);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -861,7 +755,7 @@ inline int attention_bias_forward(const GS& gs, long long C, const T* q, const T
                                   int D, void* ws, size_t wsb, cudaStream_t st) {
   using A = typename AccOf<T>::type;
   GK_TRY(check_sizes(C, E, n_dst, n_src, H, D));
-  VecShape s;
+  GeoPick s;
   if (!attention_shape_ok<T>(H, D, aligned16(q) && aligned16(k) && aligned16(v) && aligned16(o) && aligned16(rel), &s))
     return GRAPHOP_ERR_UNSUPPORTED;
   if (E == 0 || n_dst == 0)   // no edge: the edge term has nothing to add
@@ -870,23 +764,8 @@ inline int attention_bias_forward(const GS& gs, long long C, const T* q, const T
   GK_TRY(check_ws(ws));
   Arena ar(ws, wsb);
   GraphView g;
-  GK_TRY(gs(ar, st, &g));
-  const int HD = H * D, tile0 = pick_tile(E);
-  return dispatch_shape<T>(s, [&](auto Vc, auto Rc) -> int {
-    constexpr int V = decltype(Vc)::value, R = decltype(Rc)::value;
-    const long long cstride = HD + 2 * s.S;
-    if constexpr (V == 1) return (int)GRAPHOP_ERR_UNSUPPORTED;
-    else return dispatch_lph(D / V, [&](auto Lc) -> int {
-      constexpr int LPH = decltype(Lc)::value;
-      return run_row_levels(ar, g, tile0, n_dst, sizeof(A), cstride, st, [&](void* cout, void* cin) {
-        AttnFwdStaged<T, V, R, LPH, true> op;
-        op.q = q; op.k = k; op.v = v; op.rel = rel; op.o = o; op.lse = (A*)lse; op.carry = (A*)cout;
-        op.carry_in = (const A*)cin; op.scale = (A)scale; op.H = H; op.D = D; op.HD = HD; op.S = s.S; op.lph = D / V;
-        op.cstride = cstride;
-        return op;
-      });
-    });
-  });
+  GK_TRY(gs(ar, n_dst, st, &g));
+  return run_attn_forward<T, true>(ar, g, s, q, k, v, rel, scale, o, lse, n_dst, H, D, st);
 }
 
 // Gradients of the above.  The transposed CSR must carry eid_t (for each of its positions the row-CSR position of
@@ -901,7 +780,7 @@ inline int attention_bias_backward(const GS& gs_r, const GS& gs_c, bool has_eid_
   using A = typename AccOf<T>::type;
   GK_TRY(check_sizes(C, E, n_dst, n_src, H, D));
   if (Ct < 0) return GRAPHOP_ERR_INVALID_ARGUMENT;
-  VecShape s;
+  GeoPick s;
   const bool al = aligned16(q) && aligned16(k) && aligned16(v) && aligned16(o) && aligned16(dout) && aligned16(dq) &&
                   aligned16(dk) && aligned16(dv) && aligned16(rel);
   if (!attention_shape_ok<T>(H, D, al, &s)) return GRAPHOP_ERR_UNSUPPORTED;
@@ -913,27 +792,14 @@ inline int attention_bias_backward(const GS& gs_r, const GS& gs_c, bool has_eid_
     return GRAPHOP_ERR_INVALID_ARGUMENT;
   GK_TRY(check_ws(ws));
   Arena ar(ws, wsb);
-  const int HD = H * D, tile0 = pick_tile(E), Hp = stat_heads(H, (int)sizeof(A));
+  const int Hp = stat_heads(H, (int)sizeof(A));
   StatPair<A>* stat = (StatPair<A>*)ar.take((size_t)n_dst * Hp * sizeof(StatPair<A>));
   EdgePair<A>* pd = (EdgePair<A>*)ar.take((size_t)E * Hp * sizeof(EdgePair<A>));
   const size_t mark = ar.used;
   {
     GraphView g;
-    GK_TRY(gs_r(ar, st, &g));
-    GK_TRY((dispatch_shape<T>(s, [&](auto Vc, auto Rc) -> int {
-      constexpr int V = decltype(Vc)::value, R = decltype(Rc)::value;
-      if constexpr (V == 1) return (int)GRAPHOP_ERR_UNSUPPORTED;
-      else return dispatch_lph(D / V, [&](auto Lc) -> int {
-        constexpr int LPH = decltype(Lc)::value;
-        return run_row_levels(ar, g, tile0, n_dst, sizeof(A), HD, st, [&](void* cout, void* cin) {
-          AttnBwdDstStaged<T, V, R, LPH, true> op;
-          op.q = q; op.k = k; op.v = v; op.rel = rel; op.o = o; op.dout = dout; op.lse = (const A*)lse;
-          op.stat = stat; op.pd = pd; op.dq = dq; op.carry = (A*)cout; op.carry_in = (const A*)cin;
-          op.scale = (A)scale; op.H = H; op.Hp = Hp; op.D = D; op.HD = HD; op.S = s.S; op.lph = D / V;
-          return op;
-        });
-      });
-    })));
+    GK_TRY(gs_r(ar, n_dst, st, &g));
+    GK_TRY((run_attn_bwd_dst<T, true>(ar, g, s, q, k, v, rel, o, dout, lse, stat, pd, scale, dq, n_dst, H, D, st)));
     {
       constexpr int VM = VecMax<T>::value;
       const bool vec = aligned16(d_rel) && D % VM == 0;   // q is 16-byte aligned (checked above)
@@ -949,21 +815,8 @@ inline int attention_bias_backward(const GS& gs_r, const GS& gs_c, bool has_eid_
   }
   ar.used = mark;
   GraphView g;
-  GK_TRY(gs_c(ar, st, &g));
-  return dispatch_shape<T>(s, [&](auto Vc, auto Rc) -> int {
-    constexpr int V = decltype(Vc)::value, R = decltype(Rc)::value;
-    if constexpr (V == 1) return (int)GRAPHOP_ERR_UNSUPPORTED;
-    else return dispatch_lph(D / V, [&](auto Lc) -> int {
-      constexpr int LPH = decltype(Lc)::value;
-      return run_row_levels(ar, g, tile0, n_src, sizeof(A), 2 * HD, st, [&](void* cout, void* cin) {
-        AttnBwdSrcPairsStaged<T, V, R, LPH> op;
-        op.q = q; op.k = k; op.v = v; op.dout = dout; op.stat = stat; op.pd = pd; op.dk = dk;
-        op.dv = dv; op.carry = (A*)cout; op.carry_in = (const A*)cin; op.scale = (A)scale;
-        op.H = H; op.Hp = Hp; op.D = D; op.HD = HD; op.S = s.S; op.lph = D / V;
-        return op;
-      });
-    });
-  });
+  GK_TRY(gs_c(ar, n_src, st, &g));
+  return run_attn_bwd_src<T, true>(ar, g, s, q, k, v, dout, stat, pd, scale, dk, dv, n_src, H, D, st);
 }
 
 template <typename T>

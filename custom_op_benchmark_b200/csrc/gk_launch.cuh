@@ -1,0 +1,210 @@
+// Launching the gathering walker (gk_group.cuh): which geometry a row shape gets, the carry levels' memory, the launch.
+#pragma once
+#include "gk_group.cuh"
+
+namespace gk {
+
+// ---------------------------------------------------------------------------------------
+// geometry of an (H, D) row
+// ---------------------------------------------------------------------------------------
+struct GeoPick {
+  int SB = 0;      // 0: no slot width fits (2-byte elements with an odd D), or the head is too wide
+  int G = 0, W = 0, LT = 0, L = 0, parts = 1, nhb = 0;
+  int accs(int elem) const { return SB ? W * (SB / elem) * G : 0; }
+};
+
+// slot_align: the largest of 16, 8, 4 that divides every operand's address.  split: a head wider than a block may be
+// walked piece by piece (aggregations; a dot product needs the whole head in one step).
+//
+// Blocks of heads of about 32 slots (512 bytes with 16-byte slots) as 16 lanes x 2 slots, narrower rows 8 x 2, 8 x 1,
+// 4 x 1: two slots per lane halve the shuffles and the address arithmetic per byte.  Narrower blocks of a wide row were
+// measured slower although a head's share of the tensor fits the L2 better (4 x 32 fp32 on R-MAT 21, forward: blocks of
+// 512 / 256 / 128 bytes 3.5 / 3.7 / 5.3 ms): every block walks the nodes again.  Four slots per lane touch 32 bytes of
+// four heads per copy instruction: 6.3 ms.  2-byte elements have twice the accumulators per slot: one slot per lane and
+// blocks of 16 slots (16 lanes x 2 slots spilled and ran half as fast).
+inline GeoPick pick_geo(int H, int D, int elem, int slot_align, bool split) {
+  GeoPick g;
+  const int target = elem == 2 ? 16 : 32;
+  const long long db = (long long)D * elem;
+  int sb = 16;
+  while (sb >= 4 && (db % sb || slot_align % sb)) sb >>= 1;
+  if (sb < 4 || sb < elem) return g;
+  int ds = (int)(db / sb);   // slots per head
+  const auto pow2 = [](int v) { int p = 1; while (p < v) p <<= 1; return p; };
+  bool exact = (ds & (ds - 1)) == 0;
+  const bool two_byte = elem == 2;
+  if (split && ds > target) {
+    g.parts = (ds + target - 1) / target;
+    exact = exact && ds % target == 0;
+    ds = target;
+  }
+  if (ds > 32) {
+    const int w = pow2((ds + 31) / 32);
+    if (w > 8) return g;
+    g.G = 32; g.W = w; g.L = 32;
+  } else {
+    const int dp = pow2(ds);
+    int heads = exact ? pow2(H * g.parts) : 1;
+    if (heads * dp > target) heads = target / dp > 0 ? target / dp : 1;
+    const int ns = heads * dp;
+    if (dp == 1 && ns > 8) { g.G = 32; g.W = 1; }
+    else if (ns == 32) { g.G = two_byte ? 32 : 16; g.W = two_byte ? 1 : 2; }
+    else if (ns == 16) { g.G = two_byte ? 16 : 8; g.W = two_byte ? 1 : 2; }
+    else if (ns == 8) { g.G = 8; g.W = 1; }
+    else { g.G = 4; g.W = 1; }
+    g.L = dp / g.W;
+  }
+  g.SB = sb;
+  const int per = g.G / g.L;
+  g.nhb = (H * g.parts + per - 1) / per;
+  if (exact && ds == g.L * g.W && H * g.parts % per == 0 && sb == 16) g.LT = g.L;
+  return g;
+}
+
+inline int slot_align_of(std::initializer_list<const void*> ptrs) {
+  uintptr_t bits = 16;
+  for (const void* p : ptrs) bits |= (uintptr_t)p;
+  return (bits & 3) ? 1 : (bits & 7) ? 4 : (bits & 15) ? 8 : 16;
+}
+
+constexpr int kMaxHeadBlocks = 65535;   // grid.y
+
+template <class X> struct TypeTag { using type = X; };
+
+// Calls f(TypeTag<Geo<...>>) for the geometry.  kNarrowSlots: slots of 8 and 4 bytes are instantiated too.  The
+// compile-time lane counts cover the heads of 16 to 128 features of the common shapes; every other one reads L.
+template <typename T, bool kNarrowSlots, class F>
+inline int dispatch_geo(const GeoPick& p, F&& f) {
+#define GK_GEO(SB_, G_, W_, LT_) \
+  if (p.SB == SB_ && p.G == G_ && p.W == W_ && (LT_ == 0 || p.LT == LT_)) return f(TypeTag<Geo<T, SB_, G_, W_, LT_>>{});
+  if constexpr (sizeof(T) <= 4) {
+    if constexpr (sizeof(T) == 4) {
+      GK_GEO(16, 16, 2, 2)
+      GK_GEO(16, 16, 2, 4)
+      GK_GEO(16, 16, 2, 8)
+      GK_GEO(16, 16, 2, 16)
+      GK_GEO(16, 8, 2, 2)
+      GK_GEO(16, 8, 2, 4)
+      GK_GEO(16, 8, 2, 8)
+    }
+    GK_GEO(16, 8, 1, 4)
+    GK_GEO(16, 8, 1, 8)
+    if constexpr (sizeof(T) == 2) {
+      GK_GEO(16, 16, 1, 4)
+      GK_GEO(16, 16, 1, 8)
+      GK_GEO(16, 16, 1, 16)
+    }
+  }
+  GK_GEO(16, 32, 1, 0)
+  if constexpr (sizeof(T) == 2) {
+    GK_GEO(16, 16, 1, 0)
+  } else {
+    GK_GEO(16, 16, 2, 0)
+    GK_GEO(16, 8, 2, 0)
+  }
+  GK_GEO(16, 8, 1, 0)
+  GK_GEO(16, 4, 1, 0)
+  GK_GEO(16, 32, 2, 0)
+  GK_GEO(16, 32, 4, 0)
+  GK_GEO(16, 32, 8, 0)
+  if constexpr (kNarrowSlots) {
+    if constexpr (sizeof(T) == 2) {
+      GK_GEO(8, 16, 1, 0)
+    } else {
+      GK_GEO(8, 16, 2, 0)
+      GK_GEO(8, 8, 2, 0)
+    }
+    GK_GEO(8, 8, 1, 0)
+    GK_GEO(8, 4, 1, 0)
+    GK_GEO(8, 32, 1, 0)
+    GK_GEO(8, 32, 2, 0)
+    GK_GEO(8, 32, 8, 0)
+    if constexpr (sizeof(T) <= 4) {
+      if constexpr (sizeof(T) == 2) {
+        GK_GEO(4, 16, 1, 0)
+      } else {
+        GK_GEO(4, 16, 2, 0)
+        GK_GEO(4, 8, 2, 0)
+      }
+      GK_GEO(4, 8, 1, 0)
+      GK_GEO(4, 4, 1, 0)
+      GK_GEO(4, 32, 1, 0)
+      GK_GEO(4, 32, 2, 0)
+      GK_GEO(4, 32, 8, 0)
+    }
+  }
+#undef GK_GEO
+  return GRAPHOP_ERR_UNSUPPORTED;
+}
+// the narrow-slot set has no 32 x 4: such rows take 32 x 8
+inline GeoPick narrow_fix(GeoPick p) {
+  if (p.SB && p.SB < 16 && p.G == 32 && p.W == 4) p.W = 8;
+  return p;
+}
+
+// workspace of the carry slots: records of `carry_elems` accumulators and their ids, two per tile and head block
+inline size_t carry_bytes(long long tiles, int nhb, long long carry_elems, size_t acc) {
+  const size_t slots = (size_t)nhb * 2 * tiles;
+  return align_up(slots * (size_t)carry_elems * acc) + align_up(slots * 4);
+}
+
+template <class GEO>
+inline void fill_geo(GEO& op, const GeoPick& p, int H, int D) {
+  op.H = H; op.D = D; op.HD = H * D; op.L = p.L; op.parts = p.parts;
+  op.drowb = (unsigned)(D * (int)sizeof(typename GEO::T));
+  op.rowb = (unsigned)H * op.drowb;
+}
+
+// Dynamic shared memory above 48 KB is asked for once per device and kernel; several host threads may get here at once
+// (autograd's backward thread): setting the attribute twice is harmless, the flag only saves the call.
+template <class Kernel>
+inline int allow_smem(Kernel kernel, int bytes, std::atomic<bool> (&configured)[64]) {
+  if (bytes <= 48 * 1024) return GRAPHOP_OK;
+  int dev = 0;
+  GK_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64 || !configured[dev].load(std::memory_order_acquire)) {
+    GK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
+  }
+  return GRAPHOP_OK;
+}
+
+// The op over every position and head block, and the merge of the rows that tiles had to cut.
+template <class Op>
+inline int launch_walk(Arena& ar, const GraphView& g, const GeoPick& p, const Op& op, long long n_rows, cudaStream_t st) {
+  WalkArgs a{};
+  a.hdr = g.hdr; a.erow = g.erow; a.other = g.other; a.eid = g.eid;
+  a.tile_start = g.tile_start;
+  a.E = g.E; a.n_rows = n_rows; a.tile = g.tile; a.aligned = g.aligned;
+  a.n_tiles = (unsigned)g.n_tiles;
+  const bool cuts = Op::kRowOut && !g.no_carry;
+  if (cuts) {
+    const size_t slots = (size_t)p.nhb * 2 * g.n_tiles;
+    a.carry = ar.take(slots * Op::kCarryElems * sizeof(typename Op::A));
+    a.rows = (uint32_t*)ar.take(slots * 4);
+  }
+  if (!ar.base) return GRAPHOP_OK;
+  if (ar.overflow) return GRAPHOP_ERR_WORKSPACE;
+  {
+    static std::atomic<bool> configured[64];
+    constexpr int smem = Op::kWarps * Op::kWarpBytes;
+    GK_TRY(allow_smem(group_walk_kernel<Op>, smem, configured));
+    constexpr int per_block = Op::kWarps * Op::NE;   // one tile per lane group
+    const dim3 grid((unsigned)((g.n_tiles + per_block - 1) / per_block), (unsigned)p.nhb);
+    group_walk_kernel<Op><<<grid, Op::kWarps * 32, smem, st>>>(op, a);
+    GK_LAUNCHED(Op::kName);
+  }
+  if constexpr (Op::kRowOut) {
+    if (cuts) {
+      static std::atomic<bool> configured[64];
+      constexpr int threads = kCarryThreads<Op>, smem = threads / Op::G * Op::kCarryElems * (int)sizeof(typename Op::A);
+      GK_TRY(allow_smem(carry_rows_kernel<Op>, smem, configured));
+      const dim3 grid((unsigned)((2 * g.n_tiles + threads - 1) / threads), (unsigned)p.nhb);
+      carry_rows_kernel<Op><<<grid, threads, smem, st>>>(op, a);
+      GK_LAUNCHED("carry_rows");
+    }
+  }
+  return GRAPHOP_OK;
+}
+
+}  // namespace gk

@@ -79,18 +79,15 @@ band_tiles_kernel(const int32_t* __restrict__ other, const int32_t* __restrict__
   }
 }
 
-// Boundaries of the level-0 work tiles, moved up to row starts: tile t nominally begins at position t * tile; if a
-// node starts at one of the positions t * tile .. (t + 1) * tile - 1, the tile begins at the first such position
-// instead, so that no short node is cut in two.  A node longer than a tile still crosses: reported in the verdict.
-__global__ void tile_bounds_kernel(const int32_t* __restrict__ erow, long long E, int tile, long long n_tiles,
+// The boundaries of the work tiles (cut_tiles) moved up to row starts: a boundary inside a node goes to the first position
+// within the next `tile` ones at which another node starts.  A boundary that finds none cuts a node in two: reported.
+__global__ void align_tiles_kernel(const int32_t* __restrict__ erow, long long E, int tile, long long n_tiles,
                                    int32_t* __restrict__ tile_start, BandVerdict* __restrict__ verdict) {
   const long long stride = (long long)gridDim.x * blockDim.x;
   int crosses = 0;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t <= n_tiles; t += stride) {
-    long long b = t * tile;
-    if (t == 0) b = 0;
-    else if (t == n_tiles) b = E;
-    else {
+    long long b = tile_start[t];
+    if (b > 0 && b < E) {
       const long long limit = b + tile < E ? b + tile : E;
       int prev = erow[b - 1];
       long long q = b;
@@ -99,8 +96,8 @@ __global__ void tile_bounds_kernel(const int32_t* __restrict__ erow, long long E
         if (r != prev) break;
         prev = r;
       }
-      if (q < limit) b = q;                       // a row start inside the tile
-      else if (erow[b] >= 0) crosses = 1;         // one node fills the whole tile and began before it
+      if (q < limit) b = q;
+      else if (prev >= 0) crosses = 1;
     }
     tile_start[t] = (int32_t)b;
   }
@@ -110,7 +107,7 @@ __global__ void tile_bounds_kernel(const int32_t* __restrict__ erow, long long E
 inline size_t plan_bytes(long long C, long long E, long long n_nodes, int index_bytes) {
   (void)C;
   size_t b = align_up(sizeof(PlanHeader)) + align_up((size_t)E * 4) + align_up(sizeof(BandVerdict));
-  b += align_up((size_t)((E + 31) / 32 + 2) * 4);   // tile boundaries, sized for the smallest tile
+  b += align_up((size_t)(tile_count(E, n_nodes, tile_cost(E, n_nodes)) + 1) * 4);   // tile boundaries
   if (index_bytes == 8) b += 2 * align_up((size_t)E * 4);
   b += 3 * align_up((size_t)(n_nodes > 0 ? n_nodes : 1) * 4);
   return b + kAlign;
@@ -140,7 +137,7 @@ inline int plan_build(const I* row, const I* indptr, const I* eid, const I* indi
     plan->node_lo = node_lo;
     return GRAPHOP_OK;
   }
-  GK_TRY(prepare_graph<I>(ar, row, indptr, eid, indices, C, E, st, &g));
+  GK_TRY(prepare_graph<I>(ar, row, indptr, eid, indices, C, E, n_nodes, st, &g));
   plan->header = g.hdr;
   plan->erow = g.erow;
   plan->other = g.other;
@@ -157,15 +154,10 @@ inline int plan_build(const I* row, const I* indptr, const I* eid, const I* indi
     node_ranges_kernel<I><<<gc ? gc : 1, 256, 0, st>>>(row, indptr, C, n_nodes, first, deg);
     GK_LAUNCHED("plan_node_ranges");
   }
-  // row-aligned boundaries of the work tiles the ops will use for this many positions
-  const int tile = pick_tile(E);
-  const long long n_tiles = (E + tile - 1) / tile;
-  int32_t* tile_start = (int32_t*)ar.take((size_t)(n_tiles + 1) * 4);
-  if (ar.overflow) return GRAPHOP_ERR_WORKSPACE;
   {
-    const unsigned gb = (unsigned)((n_tiles + 256) / 256 < 4096 ? (n_tiles + 256) / 256 : 4096);
-    tile_bounds_kernel<<<gb, 256, 0, st>>>(g.erow, E, tile, n_tiles, tile_start, verdict);
-    GK_LAUNCHED("plan_tile_bounds");
+    const unsigned gb = (unsigned)((g.n_tiles + 256) / 256 < 4096 ? (g.n_tiles + 256) / 256 : 4096);
+    align_tiles_kernel<<<gb, 256, 0, st>>>(g.erow, E, g.tile, g.n_tiles, const_cast<int32_t*>(g.tile_start), verdict);
+    GK_LAUNCHED("plan_align_tiles");
   }
   BandVerdict host{1, 0, 1};
   if (g.other && n_nodes > 0) {
@@ -182,14 +174,10 @@ inline int plan_build(const I* row, const I* indptr, const I* eid, const I* indi
   plan->band_span = analysed ? host.max_span : 0;
   if (analysed && !host.not_contiguous && host.max_span > 0 && host.max_span <= GRAPHOP_BAND_MAX_SPAN)
     plan->flags |= GRAPHOP_PLAN_DENSE_BAND;
-  // Row-aligned tiles are used only where they remove the carry levels altogether.  Where long rows still cross
-  // (R-MAT 21: hubs of 10^5 positions) the uneven tiles cost the level-0 kernels more than the fewer partial rows
-  // save: the fused step got about 4 % slower, measured.
-  plan->tile = tile;
-  if (!host.row_crosses) {
-    plan->tile_start = tile_start;
-    plan->flags |= GRAPHOP_PLAN_ROW_TILES | GRAPHOP_PLAN_NO_CARRY;
-  }
+  plan->tile = g.tile;
+  plan->tile_start = g.tile_start;
+  plan->flags |= GRAPHOP_PLAN_ROW_TILES;
+  if (!host.row_crosses) plan->flags |= GRAPHOP_PLAN_NO_CARRY;
   return GRAPHOP_OK;
 }
 

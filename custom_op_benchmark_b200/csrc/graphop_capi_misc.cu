@@ -18,8 +18,23 @@ size_t levels_bytes(long long len0, int tile0, size_t stride_bytes) {
   return total;
 }
 
-size_t graph_bytes(long long E, int index_bytes) {
-  size_t b = align_up(sizeof(PlanHeader)) + align_up((size_t)E * 4);
+// Carry levels of one pass of the gathering walker over (H, D) rows, `accs` accumulator rows and `stats` more words per
+// lane each, for whatever slot width the operands' alignment allows; the register-fetch walker's when none fits.
+size_t walk_bytes(long long E, long long n_nodes, int H, int D, int elem, bool split, int accs, int stats) {
+  const size_t acc = elem == 8 ? 8 : 4;
+  const int tile = pick_tile(E);
+  size_t most = split ? levels_bytes(E, tile, (size_t)H * D * acc) : 0;
+  for (int align = 16; align >= 4; align >>= 1) {
+    const GeoPick p = pick_geo(H, D, elem, align, split);
+    if (!p.SB) continue;
+    const size_t b = carry_bytes(tile_bound(E, n_nodes), p.nhb, (long long)accs * p.accs(elem) + stats * p.G, acc);
+    most = b > most ? b : most;
+  }
+  return most;
+}
+
+size_t graph_bytes(long long E, long long n_nodes, int index_bytes) {
+  size_t b = align_up(sizeof(PlanHeader)) + align_up((size_t)E * 4) + align_up((size_t)(tile_bound(E, n_nodes) + 1) * 4);
   if (index_bytes == 8) b += 2 * align_up((size_t)E * 4);
   return b;
 }
@@ -204,9 +219,7 @@ extern "C" size_t graphop_workspace_bytes(int op, int64_t n_edges, int64_t n_nod
   if (n_edges < 0 || n_nodes < 0 || H < 1 || D < 1) return 0;
   const long long E = n_edges;
   const size_t acc = elem_bytes == 8 ? 8 : 4;
-  const size_t HD = (size_t)H * D;
-  const int tile0 = pick_tile(E);
-  const size_t graph = graph_bytes(E, index_bytes);
+  const size_t graph = graph_bytes(E, n_nodes, index_bytes);
   size_t need = graph;
   switch (op) {
     case GRAPHOP_OP_MASKEDMM_FWD:
@@ -216,7 +229,7 @@ extern "C" size_t graphop_workspace_bytes(int op, int64_t n_edges, int64_t n_nod
     case GRAPHOP_OP_NODE_MUL_EDGE_BWD:
     case GRAPHOP_OP_SPMM_FWD:
     case GRAPHOP_OP_SPMM_BWD:
-      need += levels_bytes(E, tile0, HD * acc);
+      need += walk_bytes(E, n_nodes, H, D, elem_bytes, true, 1, 0);
       break;
     case GRAPHOP_OP_SOFTMAX_FWD:
     case GRAPHOP_OP_SOFTMAX_BWD: {
@@ -230,11 +243,11 @@ extern "C" size_t graphop_workspace_bytes(int op, int64_t n_edges, int64_t n_nod
       break;
     }
     case GRAPHOP_OP_ATTENTION_FWD:
-      need += levels_bytes(E, tile0, 3 * HD * acc);
+      need += walk_bytes(E, n_nodes, H, D, elem_bytes, false, 1, 2);
       break;
     case GRAPHOP_OP_ATTENTION_BWD:
     case GRAPHOP_OP_ATTENTION_BWD_PAIRS:
-      need += align_up((size_t)n_nodes * stat_heads(H, (int)acc) * 2 * acc) + levels_bytes(E, tile0, 2 * HD * acc);
+      need += align_up((size_t)n_nodes * stat_heads(H, (int)acc) * 2 * acc) + walk_bytes(E, n_nodes, H, D, elem_bytes, false, 2, 0);
       if (op == GRAPHOP_OP_ATTENTION_BWD_PAIRS) need += align_up((size_t)E * stat_heads(H, (int)acc) * 2 * acc);
       break;
     default:
