@@ -13,8 +13,9 @@
 //     the L2 at a time.
 //   * The gathered rows come through a ring of kDepth steps per warp in shared memory (cp.async; each lane reads back the
 //     bytes it copied itself, so no barriers), and so do the rows of the node that begins at a position: a node's start
-//     waits for nothing.  Per-edge scalars (weights, probabilities, statistics) come through registers, loaded kDepth
-//     steps ahead; node, other endpoint and edge id of the next positions sit in registers, one per lane.
+//     waits for nothing.  Per-edge scalars (weights, probabilities, statistics) come through a table,
+//     copied for a block of G positions at a time, one position per lane; node, other endpoint and edge id of the next
+//     positions sit in registers, one per lane.
 //   * Tiles have equal cost (cut_tiles) and begin at row starts wherever a row is no longer than a tile.  A longer row is
 //     cut: every tile leaves the partials of its open first / last segment in two carry slots, and a second launch
 //     merges each such row's partials in tile order.  Every sum is a function of the graph and the tile cost alone:
@@ -42,6 +43,7 @@ template <int N> __device__ __forceinline__ void cp_async_wait() {
 }
 
 constexpr uint32_t kNoRow = 0xffffffffu;
+constexpr int kMaxBlockHeads = 8;   // heads per block at most
 
 // What a launch of the walker sees of the graph and of the carry levels.
 struct WalkArgs {
@@ -72,6 +74,7 @@ struct Geo {
   using F = Frag<A, V>;
   static constexpr int kAccs = W * V * G;   // accumulators of one row of a head block
   static constexpr int kRow = W * 32 * SB;  // ring bytes of one operand row per group
+  static constexpr int kHeads = LT > 0 ? G / LT : (G < kMaxBlockHeads ? G : kMaxBlockHeads);   // heads (or pieces) per block at most
   int H, D, HD;
   unsigned rowb, drowb;   // bytes of a node row and of a D-vector
   int L;        // lanes per head, a power of two, at most G
@@ -186,20 +189,21 @@ struct Geo {
 
 // Launch shape of an op with kRows operand rows per ring step.  One warp per block: warps are independent and their tiles
 // take different times, a block of several would hold its slot until the slowest is done.
-// A ring step holds kRows operand rows and kScalarBytes per lane of a position's edge and, should a node begin there, kNode
-// rows and kNodeScalar bytes per lane of it; kState fragments of W slots live in a lane's registers.
-template <class GEO, int kRows, int kScalarBytes, int kState, int kNode, int kNodeScalar, int kU>
+// A ring step holds kRows operand rows of a position's edge and, should a node begin there, kNode rows and kNodeScalar bytes
+// per lane of it; kScalar bytes per edge and head wait in a table; kState fragments of W slots live in a lane's registers.
+template <class GEO, int kRows, int kScalar, int kState, int kNode, int kNodeScalar, int kU>
 struct Shape {
   static constexpr int kWarps = 1;
-  static constexpr int kScalarAt = kRows * GEO::kRow;                      // the step's scalars follow its rows
-  static constexpr int kNodeAt = kScalarAt + 32 * kScalarBytes;
+  static constexpr int kNodeAt = kRows * GEO::kRow;
   static constexpr int kNodeScalarAt = kNode * GEO::kRow;                  // from kNodeAt
   static constexpr int kStepBytes = kNodeAt + kNodeScalarAt + 32 * kNodeScalar;
   // Positions folded per iteration: two share the loop, the waits and the checks and give the scheduler two independent
   // chains; one where the step's rows or the registers would leave too few warps.  Two iterations are in flight.
   static constexpr int kUnroll = GEO::W <= 2 ? kU : 1;
   static constexpr int kDepth = 2 * kUnroll;
-  static constexpr int kWarpBytes = kDepth * kStepBytes;
+  static constexpr int kScalarBytes = kScalar;
+  static constexpr int kTable = 32 * GEO::kHeads * kScalar;                // one block of positions
+  static constexpr int kWarpBytes = kDepth * kStepBytes + 2 * kTable;
   static constexpr bool kNodeRows = kNode > 0;
   static constexpr int kFit = 226 * 1024 / (kWarps * kWarpBytes + 1024);   // blocks the shared memory allows
   static constexpr int kWords = GEO::W * GEO::V * (int)sizeof(typename GEO::A) / 4;
@@ -211,8 +215,10 @@ struct Shape {
 // Op interface (all members __device__), on top of its Geo and Shape; `slot` is the ring step's memory at this lane:
 //   kRowOut, kUsesOther, kUsesEid, kFoldsEid; State, Carry
 //   setup(st, gl, hb)
-//   stage(st, slot, lane, id, edge, live)         copy rows and scalars of (other endpoint, edge) into the ring
-//   fold<N>(st, slot, lane, active, pos, edge)    fold N = 1 or 2 positions per group (called by the whole warp)
+//   stage(st, slot, id, edge, live)               copy the rows of (other endpoint, edge) into the ring
+//   scalar_of(h, id, edge)                        where the edge's scalars of head h are
+//   fold<N>(st, slot, tab, active, pos, edge)     fold N = 1 or 2 positions per group (called by the whole warp); tab: the
+//                                                 table's entry of the first position and this lane's head
 //   stage_node(st, buf, lane, node)               copy what begin(node) will read into the node buffer
 //   begin(st, buf, lane)                          a node begins (called by the groups concerned)
 //   began(st, node, mine)                         the part of begin that needs the whole warp
@@ -296,7 +302,7 @@ group_walk_kernel(const __grid_constant__ Op op, const __grid_constant__ WalkArg
     for (int v = 0; v < U; ++v) {
       const int oo = __shfl_sync(kFull, o, i + v, G);
       const int ee = Op::kUsesEid ? __shfl_sync(kFull, e, i + v, G) : 0;
-      op.stage(st, slot + v * STEP, lane, oo < 0 ? 0 : oo, ee, oo >= 0);
+      op.stage(st, slot + v * STEP, oo < 0 ? 0 : oo, ee, oo >= 0);
     }
     if constexpr (Op::kNodeRows) {
       const unsigned m = starts >> i;
@@ -310,8 +316,37 @@ group_walk_kernel(const __grid_constant__ Op op, const __grid_constant__ WalkArg
     }
     cp_async_commit();
   };
+  // The scalars of a block of positions, one position per lane: asked for while the block before it is folded, read
+  // by all lanes of the group afterwards.  cp.async moves 4 bytes at least: 2-byte scalars wait in registers meanwhile.
+  constexpr int SC = Op::kScalarBytes, TB = Op::kTable, ENTRY = Op::kHeads * SC;
+  const unsigned table = ring - lane * Op::SB + DS * STEP;
+  uint16_t held[SC == 2 ? Op::kHeads : 1];
+  auto fetch_scalars = [&](unsigned tab, int o, int e) {
+    if constexpr (SC > 0) {
+      const int per = G / op.lanes_per_head(), pieces = op.parts * op.H - hb * per;   // heads in this block
 #pragma unroll
-  for (int u = 0; u < DS; u += U) stage_some(ring + u * STEP, u, r0, o0, e0, starts0);
+      for (int k = 0; k < Op::kHeads; ++k) {
+        const bool live = o >= 0 && k < per && k < pieces;
+        const int ph = live ? hb * per + k : 0;
+        const void* src = op.scalar_of(op.parts == 1 ? ph : ph / op.parts, live ? o : 0, live ? e : 0);
+        if constexpr (SC == 2) held[k] = live ? __ldg(reinterpret_cast<const uint16_t*>(src)) : (uint16_t)0;
+        else cp_async_slot<SC>(tab + lane * ENTRY + k * SC, src, live);
+      }
+    }
+  };
+  auto publish_scalars = [&](unsigned tab) {
+    if constexpr (SC == 2) {
+#pragma unroll
+      for (int k = 0; k < Op::kHeads; ++k)
+        asm volatile("st.shared.u16 [%0], %1;" ::"r"(tab + lane * ENTRY + k * SC), "h"(held[k]) : "memory");
+    }
+  };
+  fetch_scalars(table, o0, e0);
+  publish_scalars(table);
+  const unsigned my_scalar = table + g * G * ENTRY + (SC > 0 ? gl / op.lanes_per_head() * SC : 0);
+  static_assert(DS == 2 * U, "two iterations in flight");
+  stage_some(ring, 0, r0, o0, e0, starts0);
+  stage_some(ring + U * STEP, U, r0, o0, e0, starts0);
 
   const int first = __shfl_sync(kFull, r0, 0, G);
   const bool head_open = before >= 0 && before == first;
@@ -326,6 +361,12 @@ group_walk_kernel(const __grid_constant__ Op op, const __grid_constant__ WalkArg
   for (int b = 0; b * G < longest; ++b) {
     int r2, o2, e2;
     load_block(b + 2, r2, o2, e2);
+    if constexpr (SC > 0) {
+      cp_async_wait<DS / U - 1>();
+      __syncwarp();   // every lane's part of this block's table has landed, and nobody reads the other table any more
+      fetch_scalars(table + ((b + 1) & 1) * TB, o1, e1);
+    }
+    const unsigned tab0 = my_scalar + (b & 1) * TB;
     const unsigned starts1 = starts_of(r1, __shfl_sync(kFull, r0, G - 1, G));
 #pragma unroll 1
     for (int c = 0; c < CH; ++c) {
@@ -349,7 +390,7 @@ group_walk_kernel(const __grid_constant__ Op op, const __grid_constant__ WalkArg
             act[v] = p + v < lim;
             ed[v] = Op::kFoldsEid ? __shfl_sync(kFull, e0, i + v, G) : 0;
           }
-          op.template fold<U>(st, slot, lane, act, (int)j0 + p, ed);
+          op.template fold<U>(st, slot, tab0 + i * ENTRY, act, (int)j0 + p, ed);
         } else {
 #pragma unroll 1
           for (int v = 0; v < U; ++v) {
@@ -385,12 +426,13 @@ group_walk_kernel(const __grid_constant__ Op op, const __grid_constant__ WalkArg
             }
             const bool act[1] = {p + v < lim};
             const int ed[1] = {Op::kFoldsEid ? __shfl_sync(kFull, e0, i + v, G) : 0};
-            op.template fold<1>(st, slot + v * STEP, lane, act, (int)j0 + p + v, ed);
+            op.template fold<1>(st, slot + v * STEP, tab0 + (i + v) * ENTRY, act, (int)j0 + p + v, ed);
           }
         }
         stage_some(slot, i + ahead, rs, os, es, ss);
       }
     }
+    publish_scalars(table + ((b + 1) & 1) * TB);
     r0 = r1; o0 = o1; e0 = e1;
     r1 = r2; o1 = o2; e1 = e2;
     starts0 = starts1;
@@ -520,48 +562,40 @@ carry_rows_kernel(const __grid_constant__ Op op, const __grid_constant__ WalkArg
 // y[node, h, :] = sum over the node's positions of w[edge, h] * feat: feat = x[other] or, kEdgeFeat, one D-vector per
 // edge shared by the heads (the kernels of graphop_kernel.cu this stands for: see AggregateOp)
 template <class GEO, bool kEdgeFeat>
-struct GroupAggregate : GEO, Shape<GEO, 1, sizeof(typename GEO::T) == 2 ? 4 : sizeof(typename GEO::T), 1, 0, 0, 2> {
+struct GroupAggregate : GEO, Shape<GEO, 1, (int)sizeof(typename GEO::T), 1, 0, 0, 2> {
   using T = typename GEO::T;
   using A = typename GEO::A;
   using F = typename GEO::F;
   static constexpr const char* kName = kEdgeFeat ? "aggregate_edge_feat" : "aggregate";
   static constexpr bool kRowOut = true, kUsesOther = !kEdgeFeat, kUsesEid = true,
-                        kFoldsEid = sizeof(T) == 2;
+                        kFoldsEid = false;
   static constexpr int W = GEO::W;
   const T* __restrict__ w;
   const T* __restrict__ x;
   T* __restrict__ y;
-  struct State { typename GEO::Lane ln; const unsigned char *xb, *wb; F acc[W]; };
+  struct State { typename GEO::Lane ln; const unsigned char* xb; F acc[W]; };
   struct Carry { F x[W]; };
-  static constexpr int kScalar = sizeof(T) == 2 ? 4 : (int)sizeof(T);   // a 2-byte weight travels as the aligned word around it
   __device__ __forceinline__ void setup(State& st, int gl, int hb) const {
     st.ln = this->lane_of(gl, hb);
     st.xb = reinterpret_cast<const unsigned char*>(x + (kEdgeFeat ? st.ln.eoff : st.ln.off));
-    st.wb = reinterpret_cast<const unsigned char*>(w + st.ln.head);
     begin_merge(st);
   }
-  __device__ __forceinline__ const unsigned char* weight(const State& st, int e) const {
-    return st.wb + (unsigned long long)(unsigned)e * (unsigned)(this->H * (int)sizeof(T));
-  }
-  __device__ __forceinline__ void stage(const State& st, unsigned slot, int lane, int id, int e, bool live) const {
+  __device__ __forceinline__ void stage(const State& st, unsigned slot, int id, int e, bool live) const {
     this->stage_row(st.ln, slot, st.xb, kEdgeFeat ? e : id, kEdgeFeat ? this->drowb : this->rowb, live);
-    // the word's other half may lie outside the tensor but never outside an aligned word that holds part of it; it is
-    // not used
-    const unsigned char* p = weight(st, e);
-    if constexpr (sizeof(T) == 2) p = reinterpret_cast<const unsigned char*>(reinterpret_cast<uintptr_t>(p) & ~uintptr_t(3));
-    cp_async_slot<kScalar>(slot + this->kScalarAt + lane * (kScalar - GEO::SB), p, live);
+  }
+  __device__ __forceinline__ const void* scalar_of(int h, int, int e) const {
+    return w + ((unsigned long long)(unsigned)e * (unsigned)this->H + h);
   }
   template <int N>
-  __device__ __forceinline__ void fold(State& st, unsigned slot, int lane, const bool (&)[N], int, const int (&e)[N]) const {
+  __device__ __forceinline__ void fold(State& st, unsigned slot, unsigned tab, const bool (&)[N], int,
+                                       const int (&)[N]) const {
     // positions without an edge have rows and weights of zeros
 #pragma unroll
     for (int v = 0; v < N; ++v) {
       F f[W];
       this->load_staged(f, slot + v * this->kStepBytes);
-      unsigned at = slot + v * this->kStepBytes + this->kScalarAt + lane * (kScalar - GEO::SB);
-      if constexpr (sizeof(T) == 2) at += (unsigned)(reinterpret_cast<uintptr_t>(weight(st, e[v])) & 2);
       T wt;
-      lds(wt, at);
+      lds(wt, tab + v * GEO::kHeads * (int)sizeof(T));
       const A wv = to_acc<T>(wt);
 #pragma unroll
       for (int i = 0; i < W; ++i) st.acc[i].axpy(wv, f[i]);
@@ -608,11 +642,13 @@ struct GroupEdgeDot : GEO, Shape<GEO, 1, 0, 1, 1, 0, 2> {
 #pragma unroll
     for (int i = 0; i < W; ++i) st.a[i].zero();
   }
-  __device__ __forceinline__ void stage(const State& st, unsigned slot, int, int id, int e, bool live) const {
+  __device__ __forceinline__ void stage(const State& st, unsigned slot, int id, int e, bool live) const {
     this->stage_row(st.ln, slot, st.bb, kEdgeFeat ? e : id, kEdgeFeat ? this->drowb : this->rowb, live);
   }
+  __device__ __forceinline__ const void* scalar_of(int, int, int) const { return nullptr; }
   template <int N>
-  __device__ __forceinline__ void fold(State& st, unsigned slot, int, const bool (&active)[N], int, const int (&e)[N]) const {
+  __device__ __forceinline__ void fold(State& st, unsigned slot, unsigned, const bool (&active)[N], int,
+                                       const int (&e)[N]) const {
     A s[N];
 #pragma unroll
     for (int v = 0; v < N; ++v) {
@@ -675,13 +711,15 @@ struct GroupAttnFwd : GEO, Shape<GEO, kBias ? 3 : 2, 0, 2, 1, 0, 2> {
 #pragma unroll
     for (int i = 0; i < W; ++i) st.q[i].zero();
   }
-  __device__ __forceinline__ void stage(const State& st, unsigned slot, int, int id, int e, bool live) const {
+  __device__ __forceinline__ void stage(const State& st, unsigned slot, int id, int e, bool live) const {
     this->stage_row(st.ln, slot, st.kb, id, this->rowb, live);
     this->stage_row(st.ln, slot + kRow, st.vb, id, this->rowb, live);
     if constexpr (kBias) this->stage_row(st.ln, slot + 2 * kRow, st.rb, e, this->drowb, live);
   }
+  __device__ __forceinline__ const void* scalar_of(int, int, int) const { return nullptr; }
   template <int N>
-  __device__ __forceinline__ void fold(State& st, unsigned slot, int, const bool (&active)[N], int, const int (&)[N]) const {
+  __device__ __forceinline__ void fold(State& st, unsigned slot, unsigned, const bool (&active)[N], int,
+                                       const int (&)[N]) const {
     A s[N], p[N];
     A mn = st.m;
 #pragma unroll
@@ -811,13 +849,15 @@ struct GroupAttnBwdDst : GEO, Shape<GEO, kBias ? 3 : 2, 0, 4, 3, (int)sizeof(typ
 #pragma unroll
     for (int i = 0; i < W; ++i) { st.q[i].zero(); st.gr[i].zero(); }
   }
-  __device__ __forceinline__ void stage(const State& st, unsigned slot, int, int id, int e, bool live) const {
+  __device__ __forceinline__ void stage(const State& st, unsigned slot, int id, int e, bool live) const {
     this->stage_row(st.ln, slot, st.kb, id, this->rowb, live);
     this->stage_row(st.ln, slot + kRow, st.vb, id, this->rowb, live);
     if constexpr (kBias) this->stage_row(st.ln, slot + 2 * kRow, st.rb, e, this->drowb, live);
   }
+  __device__ __forceinline__ const void* scalar_of(int, int, int) const { return nullptr; }
   template <int N>
-  __device__ __forceinline__ void fold(State& st, unsigned slot, int, const bool (&active)[N], int pos, const int (&)[N]) const {
+  __device__ __forceinline__ void fold(State& st, unsigned slot, unsigned, const bool (&active)[N], int pos,
+                                       const int (&)[N]) const {
     A s[N], dp[N];
     F f[N][W];
 #pragma unroll
@@ -901,7 +941,7 @@ struct GroupAttnBwdDst : GEO, Shape<GEO, kBias ? 3 : 2, 0, 4, 3, (int)sizeof(typ
 // kPairs: (p, ds) of every edge come from the destination side (by edge id); else they are recomputed from k, v and the
 // destination's (lse, delta).
 template <class GEO, bool kPairs>
-struct GroupAttnBwdSrc : GEO, Shape<GEO, 2, 2 * sizeof(typename GEO::A), kPairs ? 2 : 4, kPairs ? 0 : 2, 0, kPairs ? 2 : 1> {
+struct GroupAttnBwdSrc : GEO, Shape<GEO, 2, 2 * (int)sizeof(typename GEO::A), kPairs ? 2 : 4, kPairs ? 0 : 2, 0, kPairs ? 2 : 1> {
   using T = typename GEO::T;
   using A = typename GEO::A;
   using F = typename GEO::F;
@@ -921,30 +961,30 @@ struct GroupAttnBwdSrc : GEO, Shape<GEO, 2, 2 * sizeof(typename GEO::A), kPairs 
   int Hp;
   struct State {
     typename GEO::Lane ln;
-    const unsigned char *qb, *gb, *sb;
+    const unsigned char *qb, *gb;
     F k[kPairs ? 1 : W], v[kPairs ? 1 : W], ak[W], av[W];
   };
-  struct alignas(2 * sizeof(A)) Pair { A x, y; };   // (p, ds) or (lse, delta)
   struct Carry { F k[W], v[W]; };
   __device__ __forceinline__ void setup(State& st, int gl, int hb) const {
     st.ln = this->lane_of(gl, hb);
     st.qb = reinterpret_cast<const unsigned char*>(q + st.ln.off);
     st.gb = reinterpret_cast<const unsigned char*>(dout + st.ln.off);
-    st.sb = kPairs ? reinterpret_cast<const unsigned char*>(pd + st.ln.head)
-                   : reinterpret_cast<const unsigned char*>(stat + st.ln.head);
     begin_merge(st);
 #pragma unroll
     for (int i = 0; i < (kPairs ? 1 : W); ++i) { st.k[i].zero(); st.v[i].zero(); }
   }
-  __device__ __forceinline__ int pair_at(int lane) const { return this->kScalarAt + lane * ((int)sizeof(Pair) - GEO::SB); }
-  __device__ __forceinline__ void stage(const State& st, unsigned slot, int lane, int id, int e, bool live) const {
+  __device__ __forceinline__ void stage(const State& st, unsigned slot, int id, int, bool live) const {
     this->stage_row(st.ln, slot, st.qb, id, this->rowb, live);
     this->stage_row(st.ln, slot + kRow, st.gb, id, this->rowb, live);
-    cp_async_slot<sizeof(Pair)>(
-        slot + pair_at(lane), st.sb + (unsigned long long)(unsigned)(kPairs ? e : id) * (unsigned)(Hp * (int)sizeof(Pair)), live);
+  }
+  // (p, ds) of the edge or (lse, delta) of its destination
+  __device__ __forceinline__ const void* scalar_of(int h, int id, int e) const {
+    if constexpr (kPairs) return pd + ((unsigned long long)(unsigned)e * (unsigned)Hp + h);
+    else return stat + ((unsigned long long)(unsigned)id * (unsigned)Hp + h);
   }
   template <int N>
-  __device__ __forceinline__ void fold(State& st, unsigned slot, int lane, const bool (&active)[N], int, const int (&)[N]) const {
+  __device__ __forceinline__ void fold(State& st, unsigned slot, unsigned tab, const bool (&active)[N], int,
+                                       const int (&)[N]) const {
     // positions without an edge have rows and pairs of zeros
 #pragma unroll
     for (int v = 0; v < N; ++v) {
@@ -952,7 +992,7 @@ struct GroupAttnBwdSrc : GEO, Shape<GEO, 2, 2 * sizeof(typename GEO::A), kPairs 
       this->load_staged(fq, slot + v * this->kStepBytes);
       this->load_staged(fg, slot + v * this->kStepBytes + kRow);
       A x, y;
-      lds2(x, y, slot + v * this->kStepBytes + pair_at(lane));
+      lds2(x, y, tab + v * GEO::kHeads * 2 * (int)sizeof(A));
       A p = x, ds = y;
       if constexpr (!kPairs) {
         const A s = this->head_sum(frag_dot<V, W>(fq, st.k));

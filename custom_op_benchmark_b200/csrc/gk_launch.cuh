@@ -46,11 +46,11 @@ inline GeoPick pick_geo(int H, int D, int elem, int slot_align, bool split) {
     const int dp = pow2(ds);
     int heads = exact ? pow2(H * g.parts) : 1;
     if (heads * dp > target) heads = target / dp > 0 ? target / dp : 1;
+    if (heads > kMaxBlockHeads) heads = kMaxBlockHeads;
     const int ns = heads * dp;
-    if (dp == 1 && ns > 8) { g.G = 32; g.W = 1; }
-    else if (ns == 32) { g.G = two_byte ? 32 : 16; g.W = two_byte ? 1 : 2; }
+    if (ns == 32) { g.G = two_byte ? 32 : 16; g.W = two_byte ? 1 : 2; }
     else if (ns == 16) { g.G = two_byte ? 16 : 8; g.W = two_byte ? 1 : 2; }
-    else if (ns == 8) { g.G = 8; g.W = 1; }
+    else if (ns == 8) { g.G = 8; g.W = 1; }   // (heads of one slot: at most 8 of them, so never wider)
     else { g.G = 4; g.W = 1; }
     g.L = dp / g.W;
   }
