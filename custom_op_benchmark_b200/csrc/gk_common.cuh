@@ -4,7 +4,7 @@
 // caller's chunk table (row[c], indptr[c]), in which several consecutive chunks may belong to one node, into erow[j] =
 // owner node of position j (-1 where no chunk covers j), and cuts the stream into work tiles of equal cost.  The walker
 // of gk_group.cuh does the work of all row-reducing and per-edge ops; walk_kernel below is the plain form of it that
-// takes any shape (one element per lane and slot, tiles of equal length) and reduces the softmax's open segments.
+// takes any shape (one element per lane and slot, tiles of equal length).
 //
 // Row-owned reductions without atomics.  A run of equal erow[] values is one segment.  A segment that lies wholly inside
 // a tile is reduced in registers and stored once.  The first segment of a tile whose node already started in an earlier
@@ -151,8 +151,6 @@ __device__ __forceinline__ void reduce_heads(A (&p)[R], int lph) {
 // ---------------------------------------------------------------------------------------
 // expansion: chunk table -> erow[], optional int64 -> int32 copies of indices / eid
 // ---------------------------------------------------------------------------------------
-constexpr int kExpandTile = 256;  // positions per warp
-
 // Work tiles of equal cost.  A position costs 1 and a node kRowCost (its begin and end cost the walker about as much as
 // that many edges), so that neither a tile of one-edge nodes nor one inside a hub takes much longer than the others.
 // With cost(p) = p + kRowCost * (node of p) the boundary of tile t is the first position whose cost reaches t * tile:
@@ -164,123 +162,187 @@ struct TileCut {
   long long n;         // tiles
   int shift;           // log2 of the cost per tile
 };
-__device__ __forceinline__ void cut_tiles(const TileCut& cut, long long p, long long E, long long node, long long prev_node) {
-  const long long hi = (p + kRowCost * node) >> cut.shift;
-  const long long lo = p > 0 ? (p - 1 + kRowCost * prev_node) >> cut.shift : -1;
+__device__ __forceinline__ long long tile_at(const TileCut& cut, long long p, long long node) {
+  return p >= 0 ? (p + kRowCost * node) >> cut.shift : -1;
+}
+// position p: lo = tile_at of the position before it, hi = its own
+__device__ __forceinline__ void cut_tiles(const TileCut& cut, long long p, long long E, long long lo, long long hi) {
   for (long long t = lo + 1; t <= hi && t <= cut.n; ++t) cut.start[t] = (int32_t)p;
   if (p == E - 1)
     for (long long t = hi + 1; t <= cut.n; ++t) cut.start[t] = (int32_t)E;
 }
 
+// What an op wants done on the way: 32-bit copies of up to two 64-bit index arrays (a null source is skipped), and an
+// edge output that starts from zero in the reference (at::zeros) cleared when some position belongs to no chunk.
 template <typename I>
-__global__ void __launch_bounds__(kWarpsPerCta * 32)
-expand_rows_kernel(const I* __restrict__ row, const I* __restrict__ indptr, long long C, long long E,
-                   int32_t* __restrict__ erow, PlanHeader* __restrict__ hdr, TileCut cut) {
-  const int lane = threadIdx.x & 31;
-  const long long t = (long long)blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5);
-  const long long p0 = t * kExpandTile;
-  const long long base = (long long)indptr[0];
-  const long long end = (long long)indptr[C];
-  if (t == 0 && lane == 0) {
-    hdr->cover_lo = base;
-    hdr->cover_hi = end < base ? base : end;
-  }
-  if (p0 >= E) return;
-  const long long p1 = p0 + kExpandTile < E ? p0 + kExpandTile : E;
-  const long long lo = p0 > base ? p0 : base;
-  const long long hi = p1 < end ? p1 : end;
-  // positions of this tile outside [base, end) belong to no chunk
-  if (p0 < base || p1 > end) {
-    long long tail_node = 0;   // of the last covered position
-    if (cut.start && p1 > end && end > base) {
-      long long c = C - 1;
-      while (c > 0 && (long long)indptr[c] >= end) --c;
-      tail_node = (long long)row[c];
-    }
-    for (long long p = p0 + lane; p < p1; p += 32)
-      if (p < lo || p >= hi) {
-        erow[p] = -1;
-        if (cut.start) cut_tiles(cut, p, E, p < base ? 0 : tail_node, p <= base ? 0 : tail_node);
-      }
-  }
-  if (lo >= hi) return;
-  // chunk that contains position lo: the last c with indptr[c] <= lo
-  // 32-way search: every lane probes one pivot strictly inside (a, b), the ballot picks the sub-range;
-  // 5 dependent loads for a million chunks instead of 20
-  long long a = 0, b = C;  // invariant: indptr[a] <= lo < indptr[b] (indptr[C] = end > lo)
-  while (b - a > 1) {
-    const long long span = b - a;
-    long long m = a + (span * (lane + 1)) / 33;  // non-decreasing in the lane index
-    m = m <= a ? a + 1 : (m >= b ? b - 1 : m);
-    const unsigned le = __ballot_sync(kFull, (long long)indptr[m] <= lo);  // a prefix of the lanes
-    const int cnt = __popc(le);
-    const long long below = __shfl_sync(kFull, m, cnt ? cnt - 1 : 0);
-    const long long above = __shfl_sync(kFull, m, cnt < 32 ? cnt : 31);
-    if (cnt) a = below;
-    if (cnt < 32) b = above;
-  }
-  int prev_row = 0;   // node of the position before the ones at hand
-  if (cut.start && lo > base) {
-    long long c = a;
-    while (c > 0 && (long long)indptr[c] >= lo) --c;
-    prev_row = (int)row[c];
-  }
-  // 32 chunks at a time: lane l holds chunk a + l; every position of the part of the tile they cover
-  // finds its chunk by a 5-step search over the lanes' start positions, so that the stores are
-  // coalesced whatever the chunk lengths are
-  for (long long c = a; c < C; c += 32) {
-    const long long cc = c + lane;
-    long long s = hi, e = hi;
-    int r = -1;
-    if (cc < C) {
-      s = (long long)indptr[cc];
-      e = (long long)indptr[cc + 1];
-      r = (int)row[cc];
-    }
-    const bool past = s >= hi;  // this chunk starts at or beyond the end of the tile
-    s = s < lo ? lo : (s > hi ? hi : s);
-    e = e < lo ? lo : (e > hi ? hi : e);
-    const int s_rel = (int)(s - lo);  // 0 .. kExpandTile, non-decreasing over the lanes
-    const long long from = __shfl_sync(kFull, s, 0);
-    const long long to = __shfl_sync(kFull, e, 31);
-    for (long long q = from; q < to; q += 32) {
-      const long long p = q + lane;
-      const int p_rel = (int)(p - lo);
-      int owner = 0;  // the last lane whose chunk starts at or before p
-#pragma unroll
-      for (int step = 16; step; step >>= 1) {
-        const int cand = owner + step;
-        const int start = __shfl_sync(kFull, s_rel, cand & 31);
-        if (cand < 32 && start <= p_rel) owner = cand;
-      }
-      const int rr = __shfl_sync(kFull, r, owner);
-      int before = __shfl_up_sync(kFull, rr, 1);
-      if (lane == 0) before = prev_row;
-      if (p < to) {
-        erow[p] = rr;
-        if (cut.start) cut_tiles(cut, p, E, rr, before);
-      }
-      prev_row = __shfl_sync(kFull, rr, to - q < 32 ? (int)(to - q) - 1 : 31);
-    }
-    if (__any_sync(kFull, past)) break;
-  }
-}
+struct ExpandExtra {
+  const I* src[2];
+  int32_t* dst[2];
+  uint16_t* clear;
+  long long clear_n;   // 2-byte words
+};
+
+// A block expands a run of `per_block` chunks (at most one per thread; the launch picks it for about one step of
+// kExpandTile positions), so nothing has to be searched for: its positions are known as soon as its chunks are loaded.
+// Every chunk that is not empty leaves its node at its first position in shared memory, and each thread fills its
+// kExpandPer positions from the last one left at or before them; a chunk of many steps is written straight.  The positions
+// before the first chunk fall to the first block, those after the last to the last one.  Bound by the written table
+// and by how many blocks wait for their chunks at once: with a search per 256 positions 67M positions in chunks of up to
+// 32 took 426 us.
+constexpr int kExpandThreads = 256;
+constexpr int kExpandPer = 8;
+constexpr int kExpandTile = kExpandThreads * kExpandPer;
 
 template <typename I>
-__global__ void narrow_index_kernel(const I* __restrict__ src, int32_t* __restrict__ dst, long long n) {
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) dst[i] = (int32_t)src[i];
+__global__ void __launch_bounds__(kExpandThreads)
+expand_rows_kernel(const I* __restrict__ row, const I* __restrict__ indptr, long long C, long long E, int per_block,
+                   int32_t* __restrict__ erow, PlanHeader* __restrict__ hdr, TileCut cut, ExpandExtra<I> extra) {
+  constexpr int kNone = INT_MIN;
+  __shared__ __align__(16) int s_row[kExpandTile];
+  __shared__ int s_last[kExpandThreads / 32];
+  __shared__ long long s_long_end;   // a chunk of many steps: its end and node
+  __shared__ int s_long_row;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const long long c0 = (long long)blockIdx.x * per_block, c1 = c0 + per_block < C ? c0 + per_block : C;
+  const long long base = (long long)indptr[0], last = (long long)indptr[C], end = last < base ? base : last;
+  const bool first_block = blockIdx.x == 0, last_block = first_block ? c1 >= C : c0 < C && c1 >= C;
+  long long s = 0, e = 0;   // this thread's chunk
+  int r0 = 0;
+  if (c0 + tid < c1) {
+    s = (long long)indptr[c0 + tid];
+    e = (long long)indptr[c0 + tid + 1];
+    r0 = (int)row[c0 + tid];
+  }
+  const bool idle = !first_block && c0 >= C;   // here for the copies alone
+  const long long begin = first_block || idle ? 0 : (long long)indptr[c0];
+  const long long finish = last_block ? E : idle ? 0 : (long long)indptr[c1];
+  if (first_block && tid == 0) {
+    hdr->cover_lo = base;
+    hdr->cover_hi = end;
+  }
+  {
+    // the index copies are dealt out by position
+    const long long share = (E + gridDim.x - 1) / gridDim.x, n0 = blockIdx.x * share, n1 = n0 + share < E ? n0 + share : E;
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+      if (extra.src[a])
+#pragma unroll 8
+        for (long long p = n0 + tid; p < n1; p += kExpandThreads) extra.dst[a][p] = (int32_t)extra.src[a][p];
+  }
+  if (extra.clear && end - base < E)
+    for (long long i = (long long)blockIdx.x * kExpandThreads + tid; i < extra.clear_n;
+         i += (long long)gridDim.x * kExpandThreads)
+      extra.clear[i] = 0;
+
+  // nodes that positions without a chunk count for in the cut: 0 before the covered ones, the last node after them
+  const auto node_before = [&](long long c) {   // of the last chunk before c that is not empty
+    while (c > 0 && (long long)indptr[c - 1] == (long long)indptr[c]) --c;
+    return c > 0 ? (int)row[c - 1] : 0;
+  };
+  int prev = 0, tail = 0;   // node of the position before the step; of the last covered position
+  if (cut.start) {
+    if (tid == 0 && !first_block && !idle) prev = node_before(c0);
+    if (last_block && end < E) tail = node_before(C);
+  }
+  long long q0 = begin & ~(long long)(kExpandPer - 1);   // stores are 16 bytes wide
+  for (long long at = begin; at < finish;) {
+    const long long stop = q0 + kExpandTile < finish ? q0 + kExpandTile : finish;   // of this step
+    *reinterpret_cast<int4*>(s_row + tid * 4) = make_int4(kNone, kNone, kNone, kNone);
+    *reinterpret_cast<int4*>(s_row + tid * 4 + kExpandThreads * 4) = make_int4(kNone, kNone, kNone, kNone);
+    const bool covers = s <= at && e - at >= 4 * kExpandTile;
+    if (covers) { s_long_end = e; s_long_row = r0; }
+    if (__syncthreads_or(covers)) {
+      // one chunk for many steps
+      const long long to = s_long_end;
+      const int r = s_long_row;
+      const long long a0 = (at + 3) & ~3LL, a1 = to & ~3LL;
+      if (tid < a0 - at) erow[at + tid] = r;
+      if (tid < to - a1) erow[a1 + tid] = r;
+      for (long long p = a0 + tid * 4; p < a1; p += kExpandThreads * 4)
+        *reinterpret_cast<int4*>(erow + p) = make_int4(r, r, r, r);
+      if (cut.start) {
+        if (tid == 0) cut_tiles(cut, at, E, tile_at(cut, at - 1, prev), tile_at(cut, at, r));
+        // inside the chunk boundary t lies where the cost reaches it
+        const long long t1 = tile_at(cut, to - 1, r);
+        for (long long t = tile_at(cut, at, r) + 1 + tid; t <= t1 && t <= cut.n; t += kExpandThreads)
+          cut.start[t] = (int32_t)((t << cut.shift) - (long long)kRowCost * r);
+        if (to == E)
+          for (long long t = t1 + 1 + tid; t <= cut.n; t += kExpandThreads) cut.start[t] = (int32_t)E;
+        prev = r;
+      }
+      at = to;
+      q0 = at & ~(long long)(kExpandPer - 1);
+      __syncthreads();
+      continue;
+    }
+    if (e > s && s < stop && e > at) s_row[(s > at ? s : at) - q0] = r0;
+    if (tid == 0) {   // positions that belong to no chunk
+      if (at < base) s_row[at - q0] = -1;
+      if (end < stop) s_row[(end > at ? end : at) - q0] = -1;
+    }
+    __syncthreads();
+    alignas(16) int r[kExpandPer];
+#pragma unroll
+    for (int i = 0; i < kExpandPer; i += 4)
+      *reinterpret_cast<int4*>(r + i) = *reinterpret_cast<const int4*>(s_row + tid * kExpandPer + i);
+#pragma unroll
+    for (int i = 1; i < kExpandPer; ++i) r[i] = r[i] == kNone ? r[i - 1] : r[i];
+    // the node in force before this thread's first position: of the nearest thread before it that met one
+    const unsigned met = __ballot_sync(kFull, r[kExpandPer - 1] != kNone);
+    const unsigned under = met & ((1u << lane) - 1);
+    const int from = __shfl_sync(kFull, r[kExpandPer - 1], under ? 31 - __clz(under) : 0);
+    const int top = __shfl_sync(kFull, r[kExpandPer - 1], met ? 31 - __clz(met) : 0);
+    if (lane == 0) s_last[w] = met ? top : kNone;
+    __syncthreads();
+    int before = under ? from : kNone;
+    for (int k = w - 1; k >= 0 && before == kNone; --k) before = s_last[k];
+#pragma unroll
+    for (int i = 0; i < kExpandPer; ++i) r[i] = r[i] == kNone ? before : r[i];
+    const long long p = q0 + tid * kExpandPer;
+    if (p >= at && p + kExpandPer <= stop) {
+#pragma unroll
+      for (int i = 0; i < kExpandPer; i += 4) *reinterpret_cast<int4*>(erow + p + i) = *reinterpret_cast<int4*>(r + i);
+    } else {
+#pragma unroll
+      for (int i = 0; i < kExpandPer; ++i)
+        if (p + i >= at && p + i < stop) erow[p + i] = r[i];
+    }
+    if (cut.start) {
+      const auto node = [&](int rr, long long pp) { return rr >= 0 ? rr : pp < base ? 0 : tail; };
+      const long long from_p = p > at ? p : at;
+      // the first thread's predecessor lies in the step before
+      long long mine = tile_at(cut, from_p - 1, p <= at ? prev : node(before, p - 1));
+#pragma unroll
+      for (int i = 0; i < kExpandPer; ++i) {
+        const long long q = p + i;
+        if (q >= at && q < stop) {
+          const long long was = mine;
+          mine = tile_at(cut, q, node(r[i], q));
+          if (mine != was || q == E - 1) cut_tiles(cut, q, E, was, mine);
+        }
+      }
+      // the step's last node, for the next one
+      if (stop < finish) {
+        int x = kNone;
+        for (int k = kExpandThreads / 32 - 1; k >= 0 && x == kNone; --k) x = s_last[k];
+        prev = node(x, stop - 1);
+      }
+    }
+    at = stop;
+    q0 = at;
+    __syncthreads();
+  }
 }
 
 // Edge outputs start from zero in the reference (at::zeros); only edge ids that some chunk
 // covers are written by the kernels here, so when the chunk table does not cover all E
-// positions the output is cleared first.  With full coverage this kernel returns at once.
-template <typename W>
-__global__ void zero_uncovered_kernel(const PlanHeader* __restrict__ hdr, long long E, W* __restrict__ out,
-                                      long long n_words) {
+// positions the output is cleared first: by expand_rows_kernel, or, on a plan not known to cover them all, by this
+// kernel.  With full coverage it returns at once.
+inline __global__ void zero_uncovered_kernel(const PlanHeader* __restrict__ hdr, long long E, uint16_t* __restrict__ out,
+                                             long long n) {
   if (hdr->cover_hi - hdr->cover_lo >= E) return;
   const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n_words; i += stride) out[i] = W(0);
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) out[i] = 0;
 }
 
 // ---------------------------------------------------------------------------------------

@@ -95,7 +95,7 @@ constexpr int kMaxLevels = 12;
 constexpr int kCarryTile = 32;  // wider tiles on the short upper levels save a launch but run slower: a warp
                                 // walks its slots one after the other (ER-small 0.27 -> 0.40 ms with 256)
 
-// Positions per warp at level 0 of the register-fetch walker and of the softmax carry streams.
+// Positions per warp at level 0 of the register-fetch walker.
 inline int pick_tile(long long n_edges) {
   long long t = 32;
   while (t < 256 && n_edges / t > 16384) t <<= 1;
@@ -165,10 +165,14 @@ struct GraphView {
   bool aligned = false, no_carry = false;
 };
 
+// an edge output that starts from zero when some position belongs to no chunk
+struct Clear { void* out = nullptr; size_t bytes = 0; };
+
 template <typename I>
 inline int prepare_graph(Arena& ar, const I* row, const I* indptr, const I* eid, const I* indices, long long C,
-                         long long E, long long n_nodes, cudaStream_t st, GraphView* g) {
-  auto* hdr = (PlanHeader*)ar.take(sizeof(PlanHeader));
+                         long long E, long long n_nodes, cudaStream_t st, GraphView* g, Clear clear = {},
+                         PlanHeader* hdr = nullptr) {
+  if (!hdr) hdr = (PlanHeader*)ar.take(sizeof(PlanHeader));
   auto* erow = (int32_t*)ar.take((size_t)E * 4);
   // n_nodes < 0: an op that cuts no tiles
   TileCut cut{nullptr, 0, 0};
@@ -187,23 +191,20 @@ inline int prepare_graph(Arena& ar, const I* row, const I* indptr, const I* eid,
   }
   if (!ar.base) return GRAPHOP_OK;
   if (ar.overflow) return GRAPHOP_ERR_WORKSPACE;
-  const long long warps = (E + kExpandTile - 1) / kExpandTile;
-  expand_rows_kernel<I><<<grid_for_warps(warps, kWarpsPerCta), kWarpsPerCta * 32, 0, st>>>(row, indptr, C, E, erow, hdr,
-                                                                                            cut);
+  const ExpandExtra<I> extra{{other32 ? indices : nullptr, eid32 ? eid : nullptr}, {other32, eid32}, (uint16_t*)clear.out,
+                             (long long)(clear.bytes / 2)};
+  // about one step of positions per block
+  long long per_block = C > 0 ? kExpandTile * C / E : 1;
+  per_block = per_block < 1 ? 1 : per_block > kExpandThreads ? kExpandThreads : per_block;
+  long long blocks = C > 0 ? (C + per_block - 1) / per_block : 1;
+  const long long copies = (other32 || eid32 || clear.out) ? (E + kExpandTile - 1) / kExpandTile : 1;
+  if (blocks < copies && blocks < 1024) blocks = copies < 1024 ? copies : 1024;   // long chunks: blocks for the copies
+  expand_rows_kernel<I><<<(unsigned)blocks, kExpandThreads, 0, st>>>(row, indptr, C, E, (int)per_block, erow, hdr, cut, extra);
   GK_LAUNCHED("expand_rows");
   g->hdr = hdr;
   g->erow = erow;
   g->E = E;
   if (sizeof(I) == 8) {
-    const unsigned grid = (unsigned)((E + 1023) / 1024 < 4096 ? (E + 1023) / 1024 : 4096);
-    if (indices) {
-      narrow_index_kernel<I><<<grid ? grid : 1, 256, 0, st>>>(indices, other32, E);
-      GK_LAUNCHED("narrow_index");
-    }
-    if (eid) {
-      narrow_index_kernel<I><<<grid ? grid : 1, 256, 0, st>>>(eid, eid32, E);
-      GK_LAUNCHED("narrow_index");
-    }
     g->other = other32;
     g->eid = eid32;
   } else {
@@ -219,14 +220,14 @@ template <typename I>
 struct FromChunks {
   const I* row; const I* indptr; const I* eid; const I* indices; long long C, E;
   bool valid(bool need_indices) const { return row && indptr && (!need_indices || indices); }
-  int operator()(Arena& ar, long long n_nodes, cudaStream_t st, GraphView* g) const {
-    return prepare_graph<I>(ar, row, indptr, eid, indices, C, E, n_nodes, st, g);
+  int operator()(Arena& ar, long long n_nodes, cudaStream_t st, GraphView* g, Clear clear = {}) const {
+    return prepare_graph<I>(ar, row, indptr, eid, indices, C, E, n_nodes, st, g, clear);
   }
 };
 struct FromPlan {
   const graphop_plan_t* p;
   bool valid(bool need_indices) const { return p && p->erow && p->header && (!need_indices || p->other); }
-  int operator()(Arena&, long long, cudaStream_t, GraphView* g) const {
+  int operator()(Arena&, long long, cudaStream_t st, GraphView* g, Clear clear = {}) const {
     g->hdr = (const PlanHeader*)p->header;
     g->erow = p->erow;
     g->other = p->other;
@@ -234,21 +235,18 @@ struct FromPlan {
     g->E = p->n_edges;
     g->tile_start = p->tile_start;
     g->tile = p->tile;
-    g->n_tiles = tile_count(p->n_edges, p->n_nodes, p->tile);
-    g->aligned = true;
+    g->n_tiles = p->tile ? tile_count(p->n_edges, p->n_nodes, p->tile) : 0;
+    g->aligned = (p->flags & GRAPHOP_PLAN_ROW_TILES) != 0;
     g->no_carry = (p->flags & GRAPHOP_PLAN_NO_CARRY) != 0;
+    const long long words = (long long)(clear.bytes / 2);
+    if (words && !(p->flags & GRAPHOP_PLAN_COVERED)) {
+      zero_uncovered_kernel<<<(unsigned)((words + 1023) / 1024 < 2048 ? (words + 1023) / 1024 : 2048), 256, 0, st>>>(
+          g->hdr, g->E, (uint16_t*)clear.out, words);
+      GK_LAUNCHED("zero_uncovered");
+    }
     return GRAPHOP_OK;
   }
 };
-
-inline int zero_uncovered(const GraphView& g, void* out, size_t bytes, cudaStream_t st) {
-  const long long words = (long long)(bytes / 4);
-  if (words == 0) return GRAPHOP_OK;
-  const unsigned grid = (unsigned)((words + 1023) / 1024 < 2048 ? (words + 1023) / 1024 : 2048);
-  zero_uncovered_kernel<uint32_t><<<grid, 256, 0, st>>>(g.hdr, g.E, (uint32_t*)out, words);
-  GK_LAUNCHED("zero_uncovered");
-  return GRAPHOP_OK;
-}
 
 // ---------------------------------------------------------------------------------------
 // vector shape selection
@@ -373,61 +371,52 @@ inline int run_edge_mix(const GraphView& g, const T* dy, const T* a, T* db, int 
 // ---------------------------------------------------------------------------------------
 // softmax
 // ---------------------------------------------------------------------------------------
-template <typename T, int H, bool kBackward>
-inline int run_softmax_heads(Arena& ar, const GraphView& g, const T* in0, const T* in1, T* out, long long n_nodes,
-                             int hs, int h0, cudaStream_t st) {
+// Columns h0 .. h0 + H - 1 of (E, hs) tensors.
+template <typename T, int H, bool kBackward, bool kVec>
+inline int run_softmax_heads(Arena& ar, const GraphView& g, const T* in0, const T* in1, T* out, int hs, int h0,
+                             cudaStream_t st) {
   using A = typename AccOf<T>::type;
-  constexpr int kTile = SoftmaxSteps<H>::value * 32;
-  constexpr int kW = kBackward ? H : 2 * H;
-  const long long nt0 = (g.E + kTile - 1) / kTile;
-  // level 0 is the lane-per-edge kernel; levels >= 1 are generic carry levels over 2*nt0 slots
-  Levels lv = make_levels(2 * nt0, kCarryTile);
-  A* carry0 = (A*)ar.take((size_t)(2 * nt0) * kW * sizeof(A));
-  int32_t* rows1 = (int32_t*)ar.take((size_t)(2 * nt0) * 4);
-  A* stats = (A*)ar.take((size_t)n_nodes * kW * sizeof(A));
-  void* carry[kMaxLevels];
-  int32_t* rows[kMaxLevels + 1];
-  for (int k = 0; k < lv.n; ++k) {
-    const bool last = k == lv.n - 1;
-    carry[k] = last ? nullptr : ar.take((size_t)(2 * lv.ntiles[k]) * kW * sizeof(A));
-    rows[k + 1] = last ? nullptr : (int32_t*)ar.take((size_t)(2 * lv.ntiles[k]) * 4);
-  }
+  const long long nt = (g.E + kSoftmaxTile - 1) / kSoftmaxTile;
+  const size_t slot_bytes = (size_t)(2 * nt) * (kBackward ? H : 2 * H) * sizeof(A);
+  A* slots = (A*)ar.take(slot_bytes);
+  int32_t* rows = (int32_t*)ar.take((size_t)(2 * nt) * 4);
+  A* merged = nt > kSoftmaxSelfMerge ? (A*)ar.take(slot_bytes) : nullptr;
   if (!ar.base) return GRAPHOP_OK;
   if (ar.overflow) return GRAPHOP_ERR_WORKSPACE;
-  const unsigned grid0 = grid_for_warps(nt0, kSoftmaxWarps);
-  softmax_tile_kernel<T, H, kBackward><<<grid0, kSoftmaxWarps * 32, 0, st>>>(g.erow, g.eid, in0, in1, out, carry0, rows1,
-                                                                            g.E, hs, h0);
+  softmax_tile_kernel<T, H, kBackward, kVec><<<(unsigned)nt, kSoftmaxThreads, 0, st>>>(g.erow, g.eid, in0, in1, out, slots,
+                                                                                      rows, g.E, hs, h0);
   GK_LAUNCHED(kBackward ? "softmax_bwd_tile" : "softmax_fwd_tile");
-  rows[0] = rows1;
-  for (int k = 0; k < lv.n; ++k) {
-    SegStatOp<A, !kBackward> op;
-    op.stats = stats; op.carry = (A*)carry[k]; op.carry_in = k ? (const A*)carry[k - 1] : carry0; op.H = H;
-    op.n_nodes = n_nodes;
-    walk_kernel<decltype(op), true><<<grid_for_warps(lv.ntiles[k], kWarpsPerCta), kWarpsPerCta * 32, 0, st>>>(
-        op, g.hdr, rows[k], nullptr, nullptr, lv.len[k], lv.tile[k], n_nodes, rows[k + 1]);
-    GK_LAUNCHED("carry_level");
+  if (nt == 1) return GRAPHOP_OK;   // nothing crosses
+  if (merged) {
+    softmax_merge_kernel<A, H, kBackward><<<grid_for_warps(nt, kSoftmaxWarps), kSoftmaxThreads, 0, st>>>(slots, rows, merged,
+                                                                                                         nt);
+    GK_LAUNCHED("softmax_merge");
   }
-  softmax_finish_kernel<T, H, kBackward><<<grid0, kSoftmaxWarps * 32, 0, st>>>(g.erow, g.eid, in0, in1, out, stats,
-                                                                              n_nodes, g.E, hs, h0);
+  softmax_finish_kernel<T, H, kBackward, kVec><<<(unsigned)nt, kSoftmaxThreads, 0, st>>>(g.erow, g.eid, in0, in1, out, slots,
+                                                                                        rows, merged, g.E, nt, hs, h0);
   GK_LAUNCHED(kBackward ? "softmax_bwd_finish" : "softmax_fwd_finish");
   return GRAPHOP_OK;
 }
 
+// Head counts whose edge rows are whole vector moves go in one pass; any other count, and rows at an address that the
+// moves cannot take, in passes of up to four heads read one by one.
 template <typename T, bool kBackward>
-inline int run_softmax(Arena& ar, const GraphView& g, const T* in0, const T* in1, T* out, long long n_nodes, int H,
-                       cudaStream_t st) {
-  const size_t hb = (size_t)H * sizeof(T);
-  const bool vec_ok = ((uintptr_t)in0 % (hb < 16 ? hb : 16)) == 0 && ((uintptr_t)out % (hb < 16 ? hb : 16)) == 0 &&
-                      (!kBackward || ((uintptr_t)in1 % (hb < 16 ? hb : 16)) == 0);
-  if (vec_ok && H == 1) return run_softmax_heads<T, 1, kBackward>(ar, g, in0, in1, out, n_nodes, 1, 0, st);
-  if (vec_ok && H == 2) return run_softmax_heads<T, 2, kBackward>(ar, g, in0, in1, out, n_nodes, 2, 0, st);
-  if (vec_ok && H == 4) return run_softmax_heads<T, 4, kBackward>(ar, g, in0, in1, out, n_nodes, 4, 0, st);
-  if (vec_ok && H == 8) return run_softmax_heads<T, 8, kBackward>(ar, g, in0, in1, out, n_nodes, 8, 0, st);
-  // any other head count: one head at a time through the H = 1 kernels, scratch reused
+inline int run_softmax(Arena& ar, const GraphView& g, const T* in0, const T* in1, T* out, int H, cudaStream_t st) {
+  const size_t hb = (size_t)H * sizeof(T), want = hb < 16 ? hb : 16;
+  const bool vec_ok = (uintptr_t)in0 % want == 0 && (uintptr_t)out % want == 0 && (!kBackward || (uintptr_t)in1 % want == 0);
+  if (vec_ok && H == 1) return run_softmax_heads<T, 1, kBackward, true>(ar, g, in0, in1, out, 1, 0, st);
+  if (vec_ok && H == 2) return run_softmax_heads<T, 2, kBackward, true>(ar, g, in0, in1, out, 2, 0, st);
+  if (vec_ok && H == 4) return run_softmax_heads<T, 4, kBackward, true>(ar, g, in0, in1, out, 4, 0, st);
+  if (vec_ok && H == 8) return run_softmax_heads<T, 8, kBackward, true>(ar, g, in0, in1, out, 8, 0, st);
+  const int passes = (H + 3) / 4, step = (H + passes - 1) / passes;
   const size_t mark = ar.used;
-  for (int h = 0; h < H; ++h) {
-    ar.used = mark;
-    GK_TRY((run_softmax_heads<T, 1, kBackward>(ar, g, in0, in1, out, n_nodes, H, h, st)));
+  for (int h = 0; h < H; h += step) {
+    ar.used = mark;   // the passes run back to back on one stream: scratch reused
+    const int n = H - h < step ? H - h : step;
+    if (n == 1) GK_TRY((run_softmax_heads<T, 1, kBackward, false>(ar, g, in0, in1, out, H, h, st)));
+    if (n == 2) GK_TRY((run_softmax_heads<T, 2, kBackward, false>(ar, g, in0, in1, out, H, h, st)));
+    if (n == 3) GK_TRY((run_softmax_heads<T, 3, kBackward, false>(ar, g, in0, in1, out, H, h, st)));
+    if (n == 4) GK_TRY((run_softmax_heads<T, 4, kBackward, false>(ar, g, in0, in1, out, H, h, st)));
     if (!ar.base) break;
   }
   return GRAPHOP_OK;
@@ -459,8 +448,7 @@ inline int maskedmm_forward(const GS& gs, const T* A_, const T* B_, T* y, long l
   GK_TRY(check_ws(ws));
   Arena ar(ws, wsb);
   GraphView g;
-  GK_TRY(gs(ar, n_dst, st, &g));
-  GK_TRY(zero_uncovered(g, y, (size_t)E * H * sizeof(T), st));
+  GK_TRY(gs(ar, n_dst, st, &g, Clear{y, (size_t)E * H * sizeof(T)}));
   return run_edge_dot<T, false>(ar, g, A_, B_, y, H, D, st);
 }
 
@@ -499,8 +487,7 @@ inline int node_mul_edge_forward(const GS& gs, const T* A_, const T* B_, T* y, l
   GK_TRY(check_ws(ws));
   Arena ar(ws, wsb);
   GraphView g;
-  GK_TRY(gs(ar, n_dst, st, &g));
-  GK_TRY(zero_uncovered(g, y, (size_t)E * H * sizeof(T), st));
+  GK_TRY(gs(ar, n_dst, st, &g, Clear{y, (size_t)E * H * sizeof(T)}));
   return run_edge_dot<T, true>(ar, g, A_, B_, y, H, D, st);
 }
 
@@ -516,10 +503,9 @@ inline int node_mul_edge_backward(const GS& gs, const T* A_, const T* B_, const 
   GK_TRY(check_ws(ws));
   Arena ar(ws, wsb);
   GraphView g;
-  GK_TRY(gs(ar, n_dst, st, &g));
+  GK_TRY(gs(ar, n_dst, st, &g, Clear{dB, (size_t)E * D * sizeof(T)}));
   GK_TRY((run_aggregate<T, true>(ar, g, dy, B_, dA, n_dst, H, D, st)));
   if (!ar.base) return GRAPHOP_OK;
-  GK_TRY(zero_uncovered(g, dB, (size_t)E * D * sizeof(T), st));
   return run_edge_mix<T>(g, dy, A_, dB, H, D, st);
 }
 
@@ -532,9 +518,8 @@ inline int sparse_softmax(const GS& gs, const T* in0, const T* in1, T* out, long
   GK_TRY(check_ws(ws));
   Arena ar(ws, wsb);
   GraphView g;
-  GK_TRY(gs(ar, -1, st, &g));
-  GK_TRY(zero_uncovered(g, out, (size_t)E * H * sizeof(T), st));
-  return run_softmax<T, kBackward>(ar, g, in0, in1, out, n_nodes, H, st);
+  GK_TRY(gs(ar, -1, st, &g, Clear{out, (size_t)E * H * sizeof(T)}));
+  return run_softmax<T, kBackward>(ar, g, in0, in1, out, H, st);
 }
 
 template <typename T, class GS>
@@ -569,11 +554,8 @@ inline int spmm_backward(const GS& gs_r, const GS& gs_c, long long C, long long 
   Arena ar(ws, wsb);
   {
     GraphView g;
-    GK_TRY(gs_r(ar, n_dst, st, &g));
-    if (ar.base) {
-      GK_TRY(zero_uncovered(g, dedata, (size_t)E * H * sizeof(T), st));
-      GK_TRY((run_edge_dot<T, false>(ar, g, dy, x, dedata, H, D, st)));
-    }
+    GK_TRY(gs_r(ar, n_dst, st, &g, Clear{dedata, (size_t)E * H * sizeof(T)}));
+    if (ar.base) GK_TRY((run_edge_dot<T, false>(ar, g, dy, x, dedata, H, D, st)));
   }
   ar.used = 0;
   GraphView g;
@@ -817,6 +799,25 @@ inline int attention_bias_backward(const GS& gs_r, const GS& gs_c, bool has_eid_
   GraphView g;
   GK_TRY(gs_c(ar, n_src, st, &g));
   return run_attn_bwd_src<T, true>(ar, g, s, q, k, v, dout, stat, pd, scale, dk, dv, n_src, H, D, st);
+}
+
+template <typename T>
+inline int attention_bias_forward_planned(const graphop_plan_t* plan, const T* q, const T* k, const T* v, const T* rel,
+                                          double scale, T* o, void* lse, long long n_dst, long long n_src, int H, int D,
+                                          void* ws, size_t wsb, cudaStream_t st) {
+  if (!plan) return GRAPHOP_ERR_INVALID_ARGUMENT;
+  return attention_bias_forward<T>(FromPlan{plan}, plan->n_chunks, q, k, v, rel, scale, o, lse, plan->n_edges, n_dst,
+                                   n_src, H, D, ws, wsb, st);
+}
+template <typename T>
+inline int attention_bias_backward_planned(const graphop_plan_t* plan_r, const graphop_plan_t* plan_t, const T* q,
+                                           const T* k, const T* v, const T* rel, const T* o, const void* lse,
+                                           const T* dout, double scale, T* dq, T* dk, T* dv, T* d_rel, long long n_dst,
+                                           long long n_src, int H, int D, void* ws, size_t wsb, cudaStream_t st) {
+  if (!plan_r || !plan_t) return GRAPHOP_ERR_INVALID_ARGUMENT;
+  return attention_bias_backward<T>(FromPlan{plan_r}, FromPlan{plan_t}, plan_t->eid != nullptr, plan_r->n_chunks,
+                                    plan_t->n_chunks, q, k, v, rel, o, lse, dout, scale, dq, dk, dv, d_rel,
+                                    plan_r->n_edges, n_dst, n_src, H, D, ws, wsb, st);
 }
 
 template <typename T>

@@ -6,6 +6,7 @@
 #include <climits>
 
 #include "gk_host.cuh"
+#include "graphop_internal.h"
 
 namespace gk {
 
@@ -13,6 +14,12 @@ struct BandVerdict {
   int not_contiguous;  // some node's neighbours are not one run of consecutive ids
   int max_span;        // most different neighbours any 128 consecutive nodes reach
   int row_crosses;     // some node's positions cross a row-aligned tile boundary
+  int unused;
+};
+// what a plan finds out on the device, in one piece for one copy back
+struct PlanFacts {
+  PlanHeader cover;
+  BandVerdict verdict;
 };
 
 constexpr int kBandTileRows = 128;
@@ -106,7 +113,7 @@ __global__ void align_tiles_kernel(const int32_t* __restrict__ erow, long long E
 
 inline size_t plan_bytes(long long C, long long E, long long n_nodes, int index_bytes) {
   (void)C;
-  size_t b = align_up(sizeof(PlanHeader)) + align_up((size_t)E * 4) + align_up(sizeof(BandVerdict));
+  size_t b = align_up((size_t)E * 4) + align_up(sizeof(PlanFacts));
   b += align_up((size_t)(tile_count(E, n_nodes, tile_cost(E, n_nodes)) + 1) * 4);   // tile boundaries
   if (index_bytes == 8) b += 2 * align_up((size_t)E * 4);
   b += 3 * align_up((size_t)(n_nodes > 0 ? n_nodes : 1) * 4);
@@ -122,7 +129,8 @@ inline int plan_build(const I* row, const I* indptr, const I* eid, const I* indi
   if (!indptr || (C > 0 && !row)) return GRAPHOP_ERR_INVALID_ARGUMENT;
   GK_TRY(check_ws(memory));
   Arena ar(memory, bytes);
-  auto* verdict = (BandVerdict*)ar.take(sizeof(BandVerdict));
+  auto* facts = (PlanFacts*)ar.take(sizeof(PlanFacts));
+  BandVerdict* verdict = &facts->verdict;
   GraphView g{};
   int32_t* first = (int32_t*)ar.take((size_t)(n_nodes > 0 ? n_nodes : 1) * 4);
   int32_t* deg = (int32_t*)ar.take((size_t)(n_nodes > 0 ? n_nodes : 1) * 4);
@@ -137,7 +145,7 @@ inline int plan_build(const I* row, const I* indptr, const I* eid, const I* indi
     plan->node_lo = node_lo;
     return GRAPHOP_OK;
   }
-  GK_TRY(prepare_graph<I>(ar, row, indptr, eid, indices, C, E, n_nodes, st, &g));
+  GK_TRY(prepare_graph<I>(ar, row, indptr, eid, indices, C, E, n_nodes, st, &g, Clear{}, &facts->cover));
   plan->header = g.hdr;
   plan->erow = g.erow;
   plan->other = g.other;
@@ -159,7 +167,6 @@ inline int plan_build(const I* row, const I* indptr, const I* eid, const I* indi
     align_tiles_kernel<<<gb, 256, 0, st>>>(g.erow, E, g.tile, g.n_tiles, const_cast<int32_t*>(g.tile_start), verdict);
     GK_LAUNCHED("plan_align_tiles");
   }
-  BandVerdict host{1, 0, 1};
   if (g.other && n_nodes > 0) {
     const unsigned ge = (unsigned)((E + 255) / 256 < 8192 ? (E + 255) / 256 : 8192);
     band_positions_kernel<<<ge, 256, 0, st>>>(g.erow, g.other, E, first, verdict);
@@ -169,8 +176,10 @@ inline int plan_build(const I* row, const I* indptr, const I* eid, const I* indi
     GK_LAUNCHED("plan_band_tiles");
   }
   const bool analysed = g.other && n_nodes > 0;
-  GK_CUDA(cudaMemcpyAsync(&host, verdict, sizeof(host), cudaMemcpyDeviceToHost, st));
+  PlanFacts back{};
+  GK_CUDA(cudaMemcpyAsync(&back, facts, sizeof(back), cudaMemcpyDeviceToHost, st));
   GK_CUDA(cudaStreamSynchronize(st));
+  const BandVerdict& host = back.verdict;
   plan->band_span = analysed ? host.max_span : 0;
   if (analysed && !host.not_contiguous && host.max_span > 0 && host.max_span <= GRAPHOP_BAND_MAX_SPAN)
     plan->flags |= GRAPHOP_PLAN_DENSE_BAND;
@@ -178,6 +187,36 @@ inline int plan_build(const I* row, const I* indptr, const I* eid, const I* indi
   plan->tile_start = g.tile_start;
   plan->flags |= GRAPHOP_PLAN_ROW_TILES;
   if (!host.row_crosses) plan->flags |= GRAPHOP_PLAN_NO_CARRY;
+  if (back.cover.cover_hi - back.cover.cover_lo >= E) plan->flags |= GRAPHOP_PLAN_COVERED;
+  return GRAPHOP_OK;
+}
+
+// A plan without the shape analysis, built without waiting (graphop_internal.h).
+inline size_t view_bytes(long long E, long long n_nodes, int index_bytes) {
+  size_t b = align_up((size_t)E * 4) + align_up(sizeof(PlanHeader));
+  if (n_nodes >= 0) b += align_up((size_t)(tile_count(E, n_nodes, tile_cost(E, n_nodes)) + 1) * 4);
+  if (index_bytes == 8) b += 2 * align_up((size_t)E * 4);
+  return b + kAlign;
+}
+template <typename I>
+inline int view_build(const I* row, const I* indptr, const I* eid, const I* indices, long long C, long long E,
+                      long long n_nodes, void* memory, size_t bytes, graphop_plan_t* plan, cudaStream_t st) {
+  *plan = graphop_plan_t{};
+  if (C < 0 || E < 1 || E >= (1LL << 31) || n_nodes >= (1LL << 31)) return GRAPHOP_ERR_INVALID_ARGUMENT;
+  if (!indptr || (C > 0 && !row)) return GRAPHOP_ERR_INVALID_ARGUMENT;
+  GK_TRY(check_ws(memory));
+  Arena ar(memory, bytes);
+  GraphView g{};
+  GK_TRY(prepare_graph<I>(ar, row, indptr, eid, indices, C, E, n_nodes, st, &g));
+  plan->n_chunks = C;
+  plan->n_edges = E;
+  plan->n_nodes = n_nodes > 0 ? n_nodes : 0;
+  plan->header = g.hdr;
+  plan->erow = g.erow;
+  plan->other = g.other;
+  plan->eid = g.eid;
+  plan->tile = g.tile;
+  plan->tile_start = g.tile_start;
   return GRAPHOP_OK;
 }
 

@@ -233,13 +233,10 @@ extern "C" size_t graphop_workspace_bytes(int op, int64_t n_edges, int64_t n_nod
       break;
     case GRAPHOP_OP_SOFTMAX_FWD:
     case GRAPHOP_OP_SOFTMAX_BWD: {
-      // level 0 tiles are 64 or 128 positions; size for 64, and for the widest specialised head count
-      const int hh = H <= 8 ? H : 1;
-      const size_t w = (op == GRAPHOP_OP_SOFTMAX_FWD ? 2 : 1) * (size_t)hh * acc;
-      const long long nt0 = (E + 63) / 64;
-      need += align_up((size_t)(2 * nt0) * w) + align_up((size_t)(2 * nt0) * 4);
-      need += align_up((size_t)n_nodes * w);
-      need += levels_bytes(2 * nt0, kCarryTile, w);
+      const int hh = H <= 8 ? H : 4;   // heads of one pass, at most
+      const long long nt = (E + kSoftmaxTile - 1) / kSoftmaxTile;
+      const size_t slots = align_up((size_t)(2 * nt) * (op == GRAPHOP_OP_SOFTMAX_FWD ? 2 : 1) * (size_t)hh * acc);
+      need += slots * (nt > kSoftmaxSelfMerge ? 2 : 1) + align_up((size_t)(2 * nt) * 4);
       break;
     }
     case GRAPHOP_OP_ATTENTION_FWD:
@@ -286,4 +283,19 @@ extern "C" int graphop_plan_build_i64(const int64_t* row, const int64_t* indptr,
                                       graphop_stream_t stream) {
   return gk::plan_build<int64_t>(row, indptr, eid, indices, n_chunks, n_edges, n_nodes, memory, memory_bytes, plan,
                                  (cudaStream_t)stream);
+}
+
+extern "C" size_t graphop_internal_view_bytes(int64_t n_edges, int64_t n_nodes, int index_bytes) {
+  return gk::view_bytes(n_edges, n_nodes, index_bytes);
+}
+extern "C" int graphop_internal_view_build(const void* row, const void* indptr, const void* eid, const void* indices,
+                                           int index_bytes, int64_t n_chunks, int64_t n_edges, int64_t n_nodes,
+                                           void* memory, size_t memory_bytes, graphop_plan_t* plan,
+                                           graphop_stream_t stream) {
+  const auto st = (cudaStream_t)stream;
+  if (index_bytes == 8)
+    return gk::view_build<int64_t>((const int64_t*)row, (const int64_t*)indptr, (const int64_t*)eid, (const int64_t*)indices,
+                                   n_chunks, n_edges, n_nodes, memory, memory_bytes, plan, st);
+  return gk::view_build<int32_t>((const int32_t*)row, (const int32_t*)indptr, (const int32_t*)eid, (const int32_t*)indices,
+                                 n_chunks, n_edges, n_nodes, memory, memory_bytes, plan, st);
 }

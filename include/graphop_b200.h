@@ -163,7 +163,8 @@ int graphop_check_graph_i64(const int64_t* row, const int64_t* indptr, const int
 enum {
   GRAPHOP_PLAN_DENSE_BAND = 1,
   GRAPHOP_PLAN_ROW_TILES = 2, /* tile_start holds the work tiles' boundaries, moved up to row starts, ... */
-  GRAPHOP_PLAN_NO_CARRY = 4   /* ... and no node's positions cross one: row reductions finish in one launch */
+  GRAPHOP_PLAN_NO_CARRY = 4,  /* ... and no node's positions cross one: row reductions finish in one launch */
+  GRAPHOP_PLAN_COVERED = 8    /* every position belongs to some chunk: no edge output needs clearing first */
 };
 #define GRAPHOP_BAND_MAX_SPAN 384
 
