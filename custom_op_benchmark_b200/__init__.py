@@ -19,19 +19,37 @@ def compiled_graphop():
     reference's graphop/graphop.cpp:216-225, bound with pybind11 on top of the C ABI) and registers it in
     ``sys.modules`` under the reference's name, so that code written against the reference - its wrapper.py does
     ``import graphop`` - runs on it unchanged.  Raises ImportError when the module has not been built."""
+    import sys
+    from . import build as _build
+    loaded = sys.modules.get("graphop")
+    if loaded is not None and getattr(loaded, "__file__", None) == _build.module_path("graphop"):
+        return loaded
+    module = _load_compiled("graphop")
+    sys.modules["graphop"] = module
+    return module
+
+
+def native_functions():
+    """The compiled module with wrapper.py's autograd Functions (csrc/binding/graphop_native.cpp), loaded on first use.
+    Raises ImportError when it has not been built."""
+    global _NATIVE
+    if _NATIVE is None:
+        _NATIVE = _load_compiled("graphop_native")
+    return _NATIVE
+
+
+_NATIVE = None
+
+
+def _load_compiled(name):
     import importlib.util
     import os
-    import sys
     import torch  # noqa: F401  (the module links against torch's libraries: they must be loaded first)
     from . import build as _build
-    path = _build.module_path()
+    path = _build.module_path(name)
     if not os.path.exists(path):
         raise ImportError("%s is missing: build it with `python -m custom_op_benchmark_b200.build`" % path)
-    loaded = sys.modules.get("graphop")
-    if loaded is not None and getattr(loaded, "__file__", None) == path:
-        return loaded
-    spec = importlib.util.spec_from_file_location("graphop", path)
+    spec = importlib.util.spec_from_file_location(name, path)
     module = importlib.util.module_from_spec(spec)
     spec.loader.exec_module(module)
-    sys.modules["graphop"] = module
     return module

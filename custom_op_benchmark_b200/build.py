@@ -1,8 +1,9 @@
 """Builds libgraphop_b200.so (the C ABI of include/graphop_b200.h) in-tree with nvcc for sm_100a,
 libgraphop_b200_bench.so, the instrumented twin bench.py uses to time single kernels (the same sources for
 the element types the benchmark runs, compiled with -DGK_BENCH_HOOKS, plus csrc/bench/graphop_bench.cu), and
-ext/graphop.<abi>.so, the compiled Python module `graphop` (csrc/binding/graphop_module.cpp, g++ against torch's
-headers, linked to libgraphop_b200.so).
+ext/graphop.<abi>.so, the compiled Python module `graphop` (csrc/binding/graphop_module.cpp), and
+ext/graphop_native.<abi>.so, the native autograd Functions (csrc/binding/graphop_native.cpp); g++ against torch's
+headers, linked to libgraphop_b200.so.
 
 ``python -m custom_op_benchmark_b200.build`` compiles the translation units in parallel and
 links them next to this file.  nvcc cross-compiles, so no GPU is needed to build.
@@ -30,39 +31,47 @@ NVCC_FLAGS = ["-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-line
               "-Xcompiler", "-fPIC", "-Xcompiler", "-fno-gnu-unique"]
 
 
-MODULE_SRC = os.path.join(CSRC, "binding", "graphop_module.cpp")
 MODULE_DIR = os.path.join(HERE, "ext")
+BINDING_DIR = os.path.join(CSRC, "binding")
+# module name -> its source
+MODULES = {"graphop": "graphop_module.cpp", "graphop_native": "graphop_native.cpp"}
 
 
-def module_path():
+def module_path(name="graphop"):
     import sysconfig
-    return os.path.join(MODULE_DIR, "graphop" + sysconfig.get_config_var("EXT_SUFFIX"))
+    return os.path.join(MODULE_DIR, name + sysconfig.get_config_var("EXT_SUFFIX"))
 
 
 def build_module(force=False):
-    """Compile the pybind module `graphop` next to the library (needs torch's headers; no GPU).  Returns its path."""
+    """Compile the pybind modules next to the library (needs torch's headers; no GPU): `graphop`, the reference's module
+    by name, and `graphop_native`, the autograd Functions of wrapper.py in native code.  Returns the first one's path."""
+    with ThreadPoolExecutor(max_workers=len(MODULES)) as pool:
+        return list(pool.map(lambda name: _build_one_module(name, force), MODULES))[0]
+
+
+def _build_one_module(name, force):
     import sysconfig
     import torch
     from torch.utils import cpp_extension as ce
-    out = module_path()
-    deps = [MODULE_SRC, LIB, os.path.join(HERE, "..", "include", "graphop_b200.h"),
+    out, src = module_path(name), os.path.join(BINDING_DIR, MODULES[name])
+    deps = [src, LIB, os.path.join(CSRC, "graphop_internal.h"), os.path.join(HERE, "..", "include", "graphop_b200.h"),
             os.path.join(HERE, "..", "include", "graphop_dlpack.h")]
     if not force and not _stale(out, deps):
         return out
     os.makedirs(MODULE_DIR, exist_ok=True)
     cuda_home = os.environ.get("CUDA_HOME", "/usr/local/cuda")
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
-           "-DTORCH_EXTENSION_NAME=graphop", "-DTORCH_API_INCLUDE_EXTENSION_H",
+           "-DTORCH_EXTENSION_NAME=" + name, "-DTORCH_API_INCLUDE_EXTENSION_H",
            "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI)]
     for inc in ce.include_paths() + [sysconfig.get_paths()["include"], os.path.join(cuda_home, "include")]:
         cmd += ["-isystem", inc]
-    cmd += [MODULE_SRC, "-o", out, "-L" + HERE, "-lgraphop_b200", "-Wl,-rpath,$ORIGIN/.."]
+    cmd += [src, "-o", out, "-L" + HERE, "-lgraphop_b200", "-Wl,-rpath,$ORIGIN/.."]
     for lib_dir in ce.library_paths():
         cmd += ["-L" + lib_dir]
     cmd += ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
-        raise RuntimeError("g++ failed for the graphop module:\n" + res.stdout + res.stderr)
+        raise RuntimeError("g++ failed for the %s module:\n" % name + res.stdout + res.stderr)
     return out
 
 

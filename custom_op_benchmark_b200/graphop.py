@@ -164,40 +164,15 @@ def node_mul_edge_backward(row, indptr, eid, A, B, dy):
     return [dA, dB]
 
 
-_NODE_BOUNDS = {}   # id(row tensor) -> (weak reference, version counter, bound)
-
-
-def _softmax_nodes(row, num_nodes=None):
-    """Rows of the per-node statistics the softmax kernels index by node id: largest node id + 1.
-
-    The reference sizes that scratch by the edge count (graphop_kernel.cu:420-427), which wastes memory on
-    dense graphs and is too small for a graph whose node ids exceed its edge count.  ``row`` is non-decreasing,
-    so its last entry is the largest id: it is read back once per chunk table (a small device-to-host copy
-    that waits for the stream) and remembered while the tensor object lives unmodified.  Pass ``num_nodes`` to
-    skip the read."""
-    if num_nodes is not None:
-        return int(num_nodes)
-    if row.numel() == 0:
-        return 0
-    hit = _NODE_BOUNDS.get(id(row))
-    if hit is not None and hit[0]() is row and hit[1] == row._version:
-        return hit[2]
-    bound = int(row[-1].item()) + 1
-    if len(_NODE_BOUNDS) >= 256:
-        _NODE_BOUNDS.clear()
-    _NODE_BOUNDS[id(row)] = (weakref.ref(row), row._version, bound)
-    return bound
-
-
 def sparse_softmax_forward(row, indptr, eid, x, num_nodes=None):
     """Softmax of x over the edges of each node, per head; x is (e,) or (e, h).  ``num_nodes`` (an addition):
-    a bound on node id + 1 when the caller knows it."""
+    a bound on node id + 1 when the caller knows it; the kernels keep no table per node and do without it."""
     _check_all(row=row, indptr=indptr, eid=eid, x=x)
     elem, index = _elem(x), _index(row, indptr, eid)
     h = _heads(x, False)
     e, c = eid.size(0), _chunks(row, indptr)
     y = th.empty_like(x)
-    n = _softmax_nodes(row, num_nodes)
+    n = int(num_nodes or 0)
     with th.cuda.device(x.device):
         _call("sparse_softmax_forward", elem, index, _capi.OP_SOFTMAX_FWD, e, n, h, 1, x.device,
               [_p(row), _p(indptr), _p(eid), _p(x), _p(y), c, e, n, h])
@@ -211,7 +186,7 @@ def sparse_softmax_backward(row, indptr, eid, y, dy, num_nodes=None):
     h = _heads(dy, False)
     e, c = eid.size(0), _chunks(row, indptr)
     dx = th.empty_like(dy)
-    n = _softmax_nodes(row, num_nodes)
+    n = int(num_nodes or 0)
     with th.cuda.device(y.device):
         _call("sparse_softmax_backward", elem, index, _capi.OP_SOFTMAX_BWD, e, n, h, 1, y.device,
               [_p(row), _p(indptr), _p(eid), _p(y), _p(dy), _p(dx), c, e, n, h])
@@ -510,6 +485,7 @@ class GraphPlan:
         self._memory = th.empty(need + 256, dtype=th.uint8, device=self.device)
         base = (self._memory.data_ptr() + 255) // 256 * 256
         self._keep = (row, indptr, eid, indices)
+        self._native = None
         self.c = _capi.Plan()
         fn = getattr(lib, "graphop_plan_build_%s" % index[0])
         with th.cuda.device(self.device):
@@ -535,6 +511,15 @@ class GraphPlan:
     def ref(self):
         import ctypes
         return ctypes.byref(self.c)
+
+    def native(self):
+        """This plan as the native autograd Functions take it."""
+        if self._native is None:
+            import ctypes
+            from . import native_functions
+            keep = [self._memory] + [t for t in self._keep if t is not None]
+            self._native = native_functions().PlanHandle(ctypes.addressof(self.c), keep)
+        return self._native
 
 
 plan_cache_size = 8      # plans kept by cached_plan(); 0 switches the cache off

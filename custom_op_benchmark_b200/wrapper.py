@@ -1,11 +1,17 @@
 """Autograd wiring of the graphop ops: the four `torch.autograd.Function` classes of the
 reference (wrapper.py:8-55) with the same names, the same positional `apply` signatures and
 the same `None` gradients for every index argument, plus `GraphAttention`, the fused chain.
+
+`apply` of these classes runs the same Function in native code (csrc/binding/graphop_native.cpp): on small graphs the
+Python forward and backward below took several times as long as the kernels.  They are what `apply` runs when `_g` is
+another module with the ops of `graphop` (the compiled module of that name, say).
 """
 import torch as th
 from torch.autograd import Function
 
 from . import graphop as _g
+from . import graphop as _graphop
+from . import native_functions as _native
 from .part_csr import partition_csr  # noqa: F401  (the reference wrapper re-exports it, wrapper.py:4)
 
 __all__ = ["SparseSoftmax", "MaskedMMCSR", "NodeMulEdge", "VectorSPMM", "GraphAttention", "GraphAttentionBias", "GraphAttentionPlanned",
@@ -16,6 +22,12 @@ chunk_size = 32  # wrapper.py:6
 
 class SparseSoftmax(Function):
     """wrapper.py:8-18"""
+
+    @staticmethod
+    def apply(row, indptr, eid, x):
+        if _g is not _graphop:
+            return super(SparseSoftmax, SparseSoftmax).apply(row, indptr, eid, x)
+        return _native().sparse_softmax(row, indptr, eid, x)
 
     @staticmethod
     def forward(ctx, row, indptr, eid, x):
@@ -31,6 +43,12 @@ class SparseSoftmax(Function):
 
 class MaskedMMCSR(Function):
     """wrapper.py:20-30"""
+
+    @staticmethod
+    def apply(row, indptr_r, eid_r, indices_r, col, indptr_c, eid_c, indices_c, A, B):
+        if _g is not _graphop:
+            return super(MaskedMMCSR, MaskedMMCSR).apply(row, indptr_r, eid_r, indices_r, col, indptr_c, eid_c, indices_c, A, B)
+        return _native().maskedmm_csr(row, indptr_r, eid_r, indices_r, col, indptr_c, eid_c, indices_c, A, B)
 
     @staticmethod
     def forward(ctx, row, indptr_r, eid_r, indices_r, col, indptr_c, eid_c, indices_c, A, B):
@@ -49,6 +67,12 @@ class NodeMulEdge(Function):
     """wrapper.py:32-42"""
 
     @staticmethod
+    def apply(row, indptr, eid, A, B):
+        if _g is not _graphop:
+            return super(NodeMulEdge, NodeMulEdge).apply(row, indptr, eid, A, B)
+        return _native().node_mul_edge(row, indptr, eid, A, B)
+
+    @staticmethod
     def forward(ctx, row, indptr, eid, A, B):
         ctx.save_for_backward(row, indptr, eid, A, B)
         return _g.node_mul_edge_forward(row, indptr, eid, A, B)
@@ -62,6 +86,12 @@ class NodeMulEdge(Function):
 
 class VectorSPMM(Function):
     """wrapper.py:44-55"""
+
+    @staticmethod
+    def apply(row, indptr, eid, indices, col, ptr_t, eid_t, indices_t, edata, x):
+        if _g is not _graphop:
+            return super(VectorSPMM, VectorSPMM).apply(row, indptr, eid, indices, col, ptr_t, eid_t, indices_t, edata, x)
+        return _native().vector_spmm(row, indptr, eid, indices, col, ptr_t, eid_t, indices_t, edata, x)
 
     @staticmethod
     def forward(ctx, row, indptr, eid, indices, col, ptr_t, eid_t, indices_t, edata, x):
@@ -84,6 +114,19 @@ class GraphAttention(Function):
     materialised and only the (n, h) log-sum-exp is saved.  ``eid_t`` (the transposed CSR's edge ids, valid
     when the row CSR's edge ids are its positions) lets the backward pass each edge's probability from its
     destination-side kernel to its source-side kernel instead of recomputing it."""
+
+    @staticmethod
+    def apply(row, indptr, indices, col, indptr_t, indices_t, Q, K, V, scale, eid_t=None):
+        if _g is not _graphop:
+            return super(GraphAttention, GraphAttention).apply(row, indptr, indices, col, indptr_t, indices_t, Q, K, V, scale, eid_t)
+        # the same graph tensors come back every step: their plans are built once and looked up here, so this per-call
+        # signature runs the planned kernels (and, on a dense band in bfloat16, the tensor-core ones)
+        if _g.plan_cache_size > 0 and indices.numel() > 0:
+            plans = _g.cached_plan(row, indptr, None, indices, Q.size(0)), _g.cached_plan(col, indptr_t, eid_t, indices_t,
+                                                                                         K.size(0))
+            return _native().attention_planned(plans[0].native(), plans[1].native(), Q, K, V, scale)
+        return super(GraphAttention, GraphAttention).apply(row, indptr, indices, col, indptr_t, indices_t, Q, K, V, scale,
+                                                           eid_t)
 
     @staticmethod
     def forward(ctx, row, indptr, indices, col, indptr_t, indices_t, Q, K, V, scale, eid_t=None):
@@ -122,6 +165,12 @@ class GraphAttentionBias(Function):
     row-CSR position of the same edge."""
 
     @staticmethod
+    def apply(row, indptr, indices, col, indptr_t, eid_t, indices_t, Q, K, V, rel, scale):
+        if _g is not _graphop:
+            return super(GraphAttentionBias, GraphAttentionBias).apply(row, indptr, indices, col, indptr_t, eid_t, indices_t, Q, K, V, rel, scale)
+        return _native().attention_bias(row, indptr, indices, col, indptr_t, eid_t, indices_t, Q, K, V, rel, scale)
+
+    @staticmethod
     def forward(ctx, row, indptr, indices, col, indptr_t, eid_t, indices_t, Q, K, V, rel, scale):
         o, lse = _g.attention_bias_forward(row, indptr, indices, Q, K, V, rel, scale)
         ctx.save_for_backward(row, indptr, indices, col, indptr_t, eid_t, indices_t, Q, K, V, rel, o, lse)
@@ -140,6 +189,12 @@ class GraphAttentionPlanned(Function):
     """GraphAttention on graph plans: ``apply(plan_r, plan_t, Q, K, V, scale)`` with ``graphop.GraphPlan`` objects of
     the row CSR and of the transposed CSR (the latter built with its edge ids).  Nothing that depends on the graph
     alone is recomputed per call."""
+
+    @staticmethod
+    def apply(plan_r, plan_t, Q, K, V, scale):
+        if _g is not _graphop:
+            return super(GraphAttentionPlanned, GraphAttentionPlanned).apply(plan_r, plan_t, Q, K, V, scale)
+        return _native().attention_planned(plan_r.native(), plan_t.native(), Q, K, V, scale)
 
     @staticmethod
     def forward(ctx, plan_r, plan_t, Q, K, V, scale):
