@@ -85,16 +85,18 @@ void check_chunks(const Tensor& row, const Tensor& indptr) {
   if (indptr.size(0) != row.size(0) + 1) fail("indptr must hold row.size(0) + 1 entries");
 }
 
-// The view of a chunk table; eid and indices may be undefined.  n_nodes < 0: for an op that walks no node rows.
+// The view of a chunk table; eid and indices may be undefined.  n_nodes < 0: for an op that walks no node rows.  clear: an
+// edge output that is zero where no chunk covers it, done on the way.
 GraphPtr view_of(const Tensor& row, const Tensor& indptr, const Tensor& eid, const Tensor& indices, int64_t n_edges,
-                 int64_t n_nodes, cudaStream_t stream) {
+                 int64_t n_nodes, cudaStream_t stream, const Tensor& clear = Tensor()) {
   const int ib = index_bytes_of({&row, &indptr, &eid, &indices});
   const auto data = [](const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; };
   auto g = std::make_shared<Graph>();
   const size_t bytes = graphop_internal_view_bytes(n_edges, n_nodes, ib);
   const Tensor memory = at::empty({(int64_t)bytes}, row.options().dtype(at::kByte));
   check_status(graphop_internal_view_build(data(row), data(indptr), data(eid), data(indices), ib, row.size(0), n_edges,
-                                           n_nodes, memory.data_ptr(), bytes, &g->plan, (graphop_stream_t)stream),
+                                           n_nodes, data(clear), clear.defined() ? clear.nbytes() : 0, memory.data_ptr(), bytes,
+                                           &g->plan, (graphop_stream_t)stream),
                "view_build");
   g->keep = {memory};
   // 32-bit index arrays are used where they are
@@ -235,9 +237,11 @@ Tensor sparse_softmax(const Tensor& row, const Tensor& indptr, const Tensor& eid
   const int64_t e = eid.size(0);
   Tensor y = at::empty_like(x.detach());
   if (e > 0) {
-    tb->rows = view_of(row, indptr, eid, Tensor(), e, -1, c.stream);
+    tb->rows = view_of(row, indptr, eid, Tensor(), e, -1, c.stream, y);
     c.workspace(GRAPHOP_OP_SOFTMAX_FWD, e, 0, H, 1, x);
-    const graphop_plan_t* p = &tb->rows->plan;
+    graphop_plan_t cleared = tb->rows->plan;   // by the view, for this call's output
+    cleared.flags |= GRAPHOP_PLAN_COVERED;
+    const graphop_plan_t* p = &cleared;
     check_status(by_elem(elem, [&](auto* k) {
       using E = std::remove_pointer_t<decltype(k)>;
       return sparse_softmax_forward_planned(k, p, (const E*)ptr<E>(x), ptr<E>(y), H, c.ws, c.bytes, raw(c.stream));
@@ -298,9 +302,11 @@ Tensor maskedmm_csr(const Tensor& row, const Tensor& indptr_r, const Tensor& eid
   const int64_t e = eid_r.size(0), nb = B.size(0);
   Tensor y = edge_out(A, e, s.H);
   if (e > 0) {
-    tb->rows = view_of(row, indptr_r, eid_r, indices_r, e, s.n, c.stream);
+    tb->rows = view_of(row, indptr_r, eid_r, indices_r, e, s.n, c.stream, y);
     c.workspace(GRAPHOP_OP_MASKEDMM_FWD, e, std::max(s.n, nb), s.H, s.D, A);
-    const graphop_plan_t* p = &tb->rows->plan;
+    graphop_plan_t cleared = tb->rows->plan;   // by the view, for this call's output
+    cleared.flags |= GRAPHOP_PLAN_COVERED;
+    const graphop_plan_t* p = &cleared;
     check_status(by_elem(elem, [&](auto* k) {
       using E = std::remove_pointer_t<decltype(k)>;
       return maskedmm_csr_forward_planned(k, p, (const E*)ptr<E>(A), (const E*)ptr<E>(B), ptr<E>(y), s.n, nb, s.H, s.D, c.ws,
@@ -351,9 +357,11 @@ Tensor node_mul_edge(const Tensor& row, const Tensor& indptr, const Tensor& eid,
   const int64_t e = eid.size(0);
   Tensor y = edge_out(A, e, s.H);
   if (e > 0) {
-    tb->rows = view_of(row, indptr, eid, Tensor(), e, s.n, c.stream);
+    tb->rows = view_of(row, indptr, eid, Tensor(), e, s.n, c.stream, y);
     c.workspace(GRAPHOP_OP_NODE_MUL_EDGE_FWD, e, s.n, s.H, s.D, A);
-    const graphop_plan_t* p = &tb->rows->plan;
+    graphop_plan_t cleared = tb->rows->plan;   // by the view, for this call's output
+    cleared.flags |= GRAPHOP_PLAN_COVERED;
+    const graphop_plan_t* p = &cleared;
     check_status(by_elem(elem, [&](auto* k) {
       using E = std::remove_pointer_t<decltype(k)>;
       return node_mul_edge_forward_planned(k, p, (const E*)ptr<E>(A), (const E*)ptr<E>(B), ptr<E>(y), s.n, s.H, s.D, c.ws,

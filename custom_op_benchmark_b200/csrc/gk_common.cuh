@@ -195,34 +195,35 @@ constexpr int kExpandTile = kExpandThreads * kExpandPer;
 
 template <typename I>
 __global__ void __launch_bounds__(kExpandThreads)
-expand_rows_kernel(const I* __restrict__ row, const I* __restrict__ indptr, long long C, long long E, int per_block,
+expand_rows_kernel(const I* __restrict__ row, const I* __restrict__ indptr, long long C, int E, int per_block,
                    int32_t* __restrict__ erow, PlanHeader* __restrict__ hdr, TileCut cut, ExpandExtra<I> extra) {
   constexpr int kNone = INT_MIN;
   __shared__ __align__(16) int s_row[kExpandTile];
   __shared__ int s_last[kExpandThreads / 32];
-  __shared__ long long s_long_end;   // a chunk of many steps: its end and node
-  __shared__ int s_long_row;
+  __shared__ int s_long_end, s_long_row;   // a chunk of many steps: its end and node
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const long long c0 = (long long)blockIdx.x * per_block, c1 = c0 + per_block < C ? c0 + per_block : C;
-  const long long base = (long long)indptr[0], last = (long long)indptr[C], end = last < base ? base : last;
+  const int base = (int)indptr[0], last = (int)indptr[C], end = last < base ? base : last;
   const bool first_block = blockIdx.x == 0, last_block = first_block ? c1 >= C : c0 < C && c1 >= C;
-  long long s = 0, e = 0;   // this thread's chunk
-  int r0 = 0;
+  int s = 0, e = 0, r0 = 0;   // this thread's chunk
   if (c0 + tid < c1) {
-    s = (long long)indptr[c0 + tid];
-    e = (long long)indptr[c0 + tid + 1];
+    s = (int)indptr[c0 + tid];
+    e = (int)indptr[c0 + tid + 1];
     r0 = (int)row[c0 + tid];
   }
   const bool idle = !first_block && c0 >= C;   // here for the copies alone
-  const long long begin = first_block || idle ? 0 : (long long)indptr[c0];
-  const long long finish = last_block ? E : idle ? 0 : (long long)indptr[c1];
+  const int begin = first_block || idle ? 0 : (int)indptr[c0];
+  // the chunk before the block's, loaded with it
+  const int ahead = first_block || idle ? 0 : (int)indptr[c0 - 1], ahead_row = first_block || idle ? 0 : (int)row[c0 - 1];
+  const int finish = last_block ? E : idle ? 0 : (int)indptr[c1];
   if (first_block && tid == 0) {
     hdr->cover_lo = base;
     hdr->cover_hi = end;
   }
-  {
+  if (extra.src[0] || extra.src[1]) {
     // the index copies are dealt out by position
-    const long long share = (E + gridDim.x - 1) / gridDim.x, n0 = blockIdx.x * share, n1 = n0 + share < E ? n0 + share : E;
+    const long long share = ((long long)E + gridDim.x - 1) / gridDim.x, n0 = blockIdx.x * share;
+    const long long n1 = n0 + share < E ? n0 + share : E;
 #pragma unroll
     for (int a = 0; a < 2; ++a)
       if (extra.src[a])
@@ -236,26 +237,28 @@ expand_rows_kernel(const I* __restrict__ row, const I* __restrict__ indptr, long
 
   // nodes that positions without a chunk count for in the cut: 0 before the covered ones, the last node after them
   const auto node_before = [&](long long c) {   // of the last chunk before c that is not empty
-    while (c > 0 && (long long)indptr[c - 1] == (long long)indptr[c]) --c;
+    while (c > 0 && indptr[c - 1] == indptr[c]) --c;
     return c > 0 ? (int)row[c - 1] : 0;
   };
   int prev = 0, tail = 0;   // node of the position before the step; of the last covered position
   if (cut.start) {
-    if (tid == 0 && !first_block && !idle) prev = node_before(c0);
+    prev = ahead_row;
+    if (tid == 0 && !first_block && ahead == begin) prev = node_before(c0 - 1);   // that chunk is empty
     if (last_block && end < E) tail = node_before(C);
   }
-  long long q0 = begin & ~(long long)(kExpandPer - 1);   // stores are 16 bytes wide
-  for (long long at = begin; at < finish;) {
-    const long long stop = q0 + kExpandTile < finish ? q0 + kExpandTile : finish;   // of this step
-    *reinterpret_cast<int4*>(s_row + tid * 4) = make_int4(kNone, kNone, kNone, kNone);
-    *reinterpret_cast<int4*>(s_row + tid * 4 + kExpandThreads * 4) = make_int4(kNone, kNone, kNone, kNone);
+  int q0 = begin & ~(kExpandPer - 1);   // stores are 16 bytes wide
+  for (int at = begin; at < finish;) {
+    const int stop = finish - q0 > kExpandTile ? q0 + kExpandTile : finish;   // of this step
+#pragma unroll
+    for (int i = 0; i < kExpandPer; i += 4)
+      *reinterpret_cast<int4*>(s_row + (i * kExpandThreads + tid * 4)) = make_int4(kNone, kNone, kNone, kNone);
     const bool covers = s <= at && e - at >= 4 * kExpandTile;
     if (covers) { s_long_end = e; s_long_row = r0; }
     if (__syncthreads_or(covers)) {
       // one chunk for many steps
-      const long long to = s_long_end;
+      const int to = s_long_end;
       const int r = s_long_row;
-      const long long a0 = (at + 3) & ~3LL, a1 = to & ~3LL;
+      const int a0 = (at + 3) & ~3, a1 = to & ~3;
       if (tid < a0 - at) erow[at + tid] = r;
       if (tid < to - a1) erow[a1 + tid] = r;
       for (long long p = a0 + tid * 4; p < a1; p += kExpandThreads * 4)
@@ -271,12 +274,13 @@ expand_rows_kernel(const I* __restrict__ row, const I* __restrict__ indptr, long
         prev = r;
       }
       at = to;
-      q0 = at & ~(long long)(kExpandPer - 1);
+      q0 = at & ~(kExpandPer - 1);
       __syncthreads();
       continue;
     }
     if (e > s && s < stop && e > at) s_row[(s > at ? s : at) - q0] = r0;
-    if (tid == 0) {   // positions that belong to no chunk
+    const bool bare = at < base || end < stop;   // some positions of the step belong to no chunk
+    if (bare && tid == 0) {
       if (at < base) s_row[at - q0] = -1;
       if (end < stop) s_row[(end > at ? end : at) - q0] = -1;
     }
@@ -298,8 +302,9 @@ expand_rows_kernel(const I* __restrict__ row, const I* __restrict__ indptr, long
     for (int k = w - 1; k >= 0 && before == kNone; --k) before = s_last[k];
 #pragma unroll
     for (int i = 0; i < kExpandPer; ++i) r[i] = r[i] == kNone ? before : r[i];
-    const long long p = q0 + tid * kExpandPer;
-    if (p >= at && p + kExpandPer <= stop) {
+    const int p = q0 + tid * kExpandPer;
+    const bool whole = p >= at && p + kExpandPer <= stop;
+    if (whole) {
 #pragma unroll
       for (int i = 0; i < kExpandPer; i += 4) *reinterpret_cast<int4*>(erow + p + i) = *reinterpret_cast<int4*>(r + i);
     } else {
@@ -308,17 +313,32 @@ expand_rows_kernel(const I* __restrict__ row, const I* __restrict__ indptr, long
         if (p + i >= at && p + i < stop) erow[p + i] = r[i];
     }
     if (cut.start) {
-      const auto node = [&](int rr, long long pp) { return rr >= 0 ? rr : pp < base ? 0 : tail; };
-      const long long from_p = p > at ? p : at;
+      const auto node = [&](int rr, int pp) { return rr >= 0 ? rr : pp < base ? 0 : tail; };
       // the first thread's predecessor lies in the step before
-      long long mine = tile_at(cut, from_p - 1, p <= at ? prev : node(before, p - 1));
+      const int was_node = p <= at ? prev : node(before, p - 1);
+      long long was = tile_at(cut, (p > at ? p : at) - 1, was_node);
+      const long long mine = tile_at(cut, p + kExpandPer - 1, r[kExpandPer - 1]);
+      if (whole && !bare && was <= mine && p + kExpandPer < E) {
+        // nodes do not decrease: boundary t lies at the first of these positions whose cost reaches it
+        for (long long t = was + 1; t <= mine && t <= cut.n; ++t) {
+          const long long reach = t << cut.shift;
+          int below = 0;
 #pragma unroll
-      for (int i = 0; i < kExpandPer; ++i) {
-        const long long q = p + i;
-        if (q >= at && q < stop) {
-          const long long was = mine;
-          mine = tile_at(cut, q, node(r[i], q));
-          if (mine != was || q == E - 1) cut_tiles(cut, q, E, was, mine);
+          for (int i = 0; i < kExpandPer; ++i) below += p + i + (long long)kRowCost * r[i] < reach;
+          cut.start[t] = p + (below < kExpandPer ? below : kExpandPer - 1);
+        }
+      } else {
+#pragma unroll 1
+        for (int i = 0; i < kExpandPer; ++i) {
+          const int q = p + i;
+          int rr = r[0];   // selected, not indexed: r stays in registers
+#pragma unroll
+          for (int k = 1; k < kExpandPer; ++k) rr = k == i ? r[k] : rr;
+          if (q >= at && q < stop) {
+            const long long mine = tile_at(cut, q, node(rr, q));
+            if (mine != was || q == E - 1) cut_tiles(cut, q, E, was, mine);
+            was = mine;
+          }
         }
       }
       // the step's last node, for the next one
@@ -338,11 +358,12 @@ expand_rows_kernel(const I* __restrict__ row, const I* __restrict__ indptr, long
 // covers are written by the kernels here, so when the chunk table does not cover all E
 // positions the output is cleared first: by expand_rows_kernel, or, on a plan not known to cover them all, by this
 // kernel.  With full coverage it returns at once.
-inline __global__ void zero_uncovered_kernel(const PlanHeader* __restrict__ hdr, long long E, uint16_t* __restrict__ out,
-                                             long long n) {
+template <typename W>
+__global__ void zero_uncovered_kernel(const PlanHeader* __restrict__ hdr, long long E, W* __restrict__ out,
+                                      long long n) {
   if (hdr->cover_hi - hdr->cover_lo >= E) return;
   const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) out[i] = 0;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) out[i] = W(0);
 }
 
 // ---------------------------------------------------------------------------------------

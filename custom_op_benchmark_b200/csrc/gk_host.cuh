@@ -199,7 +199,8 @@ inline int prepare_graph(Arena& ar, const I* row, const I* indptr, const I* eid,
   long long blocks = C > 0 ? (C + per_block - 1) / per_block : 1;
   const long long copies = (other32 || eid32 || clear.out) ? (E + kExpandTile - 1) / kExpandTile : 1;
   if (blocks < copies && blocks < 1024) blocks = copies < 1024 ? copies : 1024;   // long chunks: blocks for the copies
-  expand_rows_kernel<I><<<(unsigned)blocks, kExpandThreads, 0, st>>>(row, indptr, C, E, (int)per_block, erow, hdr, cut, extra);
+  expand_rows_kernel<I><<<(unsigned)blocks, kExpandThreads, 0, st>>>(row, indptr, C, (int)E, (int)per_block, erow, hdr, cut,
+                                                                  extra);
   GK_LAUNCHED("expand_rows");
   g->hdr = hdr;
   g->erow = erow;
@@ -240,7 +241,7 @@ struct FromPlan {
     g->no_carry = (p->flags & GRAPHOP_PLAN_NO_CARRY) != 0;
     const long long words = (long long)(clear.bytes / 2);
     if (words && !(p->flags & GRAPHOP_PLAN_COVERED)) {
-      zero_uncovered_kernel<<<(unsigned)((words + 1023) / 1024 < 2048 ? (words + 1023) / 1024 : 2048), 256, 0, st>>>(
+      zero_uncovered_kernel<uint16_t><<<(unsigned)((words + 1023) / 1024 < 2048 ? (words + 1023) / 1024 : 2048), 256, 0, st>>>(
           g->hdr, g->E, (uint16_t*)clear.out, words);
       GK_LAUNCHED("zero_uncovered");
     }

@@ -44,7 +44,7 @@ inline GeoPick pick_geo(int H, int D, int elem, int slot_align, bool split) {
     g.G = 32; g.W = w; g.L = 32;
   } else {
     const int dp = pow2(ds);
-    int heads = exact ? pow2(H * g.parts) : 1;
+    int heads = pow2(H * g.parts);
     if (heads * dp > target) heads = target / dp > 0 ? target / dp : 1;
     if (heads > kMaxBlockHeads) heads = kMaxBlockHeads;
     const int ns = heads * dp;

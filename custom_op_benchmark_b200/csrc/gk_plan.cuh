@@ -200,14 +200,14 @@ inline size_t view_bytes(long long E, long long n_nodes, int index_bytes) {
 }
 template <typename I>
 inline int view_build(const I* row, const I* indptr, const I* eid, const I* indices, long long C, long long E,
-                      long long n_nodes, void* memory, size_t bytes, graphop_plan_t* plan, cudaStream_t st) {
+                      long long n_nodes, Clear clear, void* memory, size_t bytes, graphop_plan_t* plan, cudaStream_t st) {
   *plan = graphop_plan_t{};
   if (C < 0 || E < 1 || E >= (1LL << 31) || n_nodes >= (1LL << 31)) return GRAPHOP_ERR_INVALID_ARGUMENT;
   if (!indptr || (C > 0 && !row)) return GRAPHOP_ERR_INVALID_ARGUMENT;
   GK_TRY(check_ws(memory));
   Arena ar(memory, bytes);
   GraphView g{};
-  GK_TRY(prepare_graph<I>(ar, row, indptr, eid, indices, C, E, n_nodes, st, &g));
+  GK_TRY(prepare_graph<I>(ar, row, indptr, eid, indices, C, E, n_nodes, st, &g, clear));
   plan->n_chunks = C;
   plan->n_edges = E;
   plan->n_nodes = n_nodes > 0 ? n_nodes : 0;

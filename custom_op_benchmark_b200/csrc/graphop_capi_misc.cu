@@ -290,12 +290,12 @@ extern "C" size_t graphop_internal_view_bytes(int64_t n_edges, int64_t n_nodes, 
 }
 extern "C" int graphop_internal_view_build(const void* row, const void* indptr, const void* eid, const void* indices,
                                            int index_bytes, int64_t n_chunks, int64_t n_edges, int64_t n_nodes,
-                                           void* memory, size_t memory_bytes, graphop_plan_t* plan,
+                                           void* clear, size_t clear_bytes, void* memory, size_t memory_bytes, graphop_plan_t* plan,
                                            graphop_stream_t stream) {
   const auto st = (cudaStream_t)stream;
   if (index_bytes == 8)
     return gk::view_build<int64_t>((const int64_t*)row, (const int64_t*)indptr, (const int64_t*)eid, (const int64_t*)indices,
-                                   n_chunks, n_edges, n_nodes, memory, memory_bytes, plan, st);
+                                   n_chunks, n_edges, n_nodes, gk::Clear{clear, clear_bytes}, memory, memory_bytes, plan, st);
   return gk::view_build<int32_t>((const int32_t*)row, (const int32_t*)indptr, (const int32_t*)eid, (const int32_t*)indices,
-                                 n_chunks, n_edges, n_nodes, memory, memory_bytes, plan, st);
+                                 n_chunks, n_edges, n_nodes, gk::Clear{clear, clear_bytes}, memory, memory_bytes, plan, st);
 }

@@ -8,11 +8,12 @@ extern "C" {
 #endif
 
 /* A view is a plan without the shape analysis: owner table, 32-bit index copies and work tiles of a chunk table, built
- * without waiting for the device.  n_nodes < 0: no work tiles (the softmax has no use for them). */
+ * without waiting for the device.  n_nodes < 0: no work tiles (the softmax has no use for them).  `clear` (may be null):
+ * an edge output set to zero if some position belongs to no chunk. */
 size_t graphop_internal_view_bytes(int64_t n_edges, int64_t n_nodes, int index_bytes);
 int graphop_internal_view_build(const void* row, const void* indptr, const void* eid, const void* indices,
-                                int index_bytes, int64_t n_chunks, int64_t n_edges, int64_t n_nodes, void* memory,
-                                size_t memory_bytes, graphop_plan_t* plan, graphop_stream_t stream);
+                                int index_bytes, int64_t n_chunks, int64_t n_edges, int64_t n_nodes, void* clear,
+                                size_t clear_bytes, void* memory, size_t memory_bytes, graphop_plan_t* plan, graphop_stream_t stream);
 
 #define GRAPHOP_DECLARE_INTERNAL(SUF)                                                                                \
   int graphop_internal_attention_bias_forward_##SUF(                                                                 \
