@@ -296,11 +296,50 @@ inline int run_row_levels(Arena& ar, const GraphView& g, int tile0, long long n_
   return GRAPHOP_OK;
 }
 
+// Whether an op with an edge feature row shared by the heads can take all heads in a lane: slots of 16 bytes, a power of
+// two of them per row, 4 to 32, and 2, 4 or 8 heads (8 heads of 8-byte accumulators would not fit the registers; one head
+// gains nothing: 1 x 64 fp32 1.43 against 1.40 ms).  Returns the slots per row or 0.  R-MAT 18, NodeMulEdge and VectorSPMM
+// forward and backward, against the walker with a copy of the row per head: 2 x 32 fp32 1.28 -> 1.19, 4 x 32 1.78 -> 1.60,
+// 8 x 32 3.21 -> 2.74 ms, bf16 1.04 -> 0.97, 1.44 -> 1.31, 2.63 -> 2.37 ms.
+template <typename T>
+inline int feat_slots(int H, int D, std::initializer_list<const void*> rows16) {
+  constexpr int VM = VecMax<T>::value;
+  for (const void* p : rows16) if (!aligned16(p)) return 0;
+  if (D % VM || !(H == 2 || H == 4 || (H == 8 && sizeof(T) <= 4))) return 0;
+  const int ds = D / VM;
+  return ds == 4 || ds == 8 || ds == 16 || ds == 32 ? ds : 0;
+}
+// f(TypeTag<integral_constant heads>, TypeTag<integral_constant slots>)
+template <typename T, class F>
+inline int dispatch_feat(int H, int ds, F&& f) {
+  const auto heads = [&](auto slots) -> int {
+    if (H == 2) return f(std::integral_constant<int, 2>{}, slots);
+    if (H == 4) return f(std::integral_constant<int, 4>{}, slots);
+    if constexpr (sizeof(T) <= 4) return f(std::integral_constant<int, 8>{}, slots);
+    else return GRAPHOP_ERR_UNSUPPORTED;
+  };
+  if (ds == 4) return heads(std::integral_constant<int, 4>{});
+  if (ds == 8) return heads(std::integral_constant<int, 8>{});
+  if (ds == 16) return heads(std::integral_constant<int, 16>{});
+  return heads(std::integral_constant<int, 32>{});
+}
+
 // out[node] = sum_k w[eid[k]] * feat(k)
 template <typename T, bool kEdgeFeat>
 inline int run_aggregate(Arena& ar, const GraphView& g, const T* w, const T* x, T* y, long long n_rows, int H, int D,
                          cudaStream_t st) {
   using A = typename AccOf<T>::type;
+  if constexpr (kEdgeFeat) {
+    if (const int ds = feat_slots<T>(H, D, {x, y}))
+      return dispatch_feat<T>(H, ds, [&](auto heads, auto slots) -> int {
+        GeoPick p;
+        p.SB = 16; p.G = p.L = decltype(slots)::value; p.W = decltype(heads)::value; p.nhb = 1;
+        GroupFeatAggregate<FeatGeo<T, decltype(slots)::value, decltype(heads)::value>> op;
+        fill_geo(op, p, H, D);
+        op.w = w; op.x = x; op.y = y;
+        return launch_walk(ar, g, p, op, n_rows, st);
+      });
+  }
   const GeoPick p = pick_geo(H, D, sizeof(T), slot_align_of({x, y}), true);
   if (p.SB && p.nhb <= kMaxHeadBlocks)
     return dispatch_geo<T, true>(p, [&](auto tag) -> int {
@@ -328,6 +367,20 @@ inline int run_aggregate(Arena& ar, const GraphView& g, const T* w, const T* x, 
 // y[eid[k], h] = a[node(k), h, :] . feat(k)[h, :]
 template <typename T, bool kEdgeFeat>
 inline int run_edge_dot(Arena& ar, const GraphView& g, const T* a, const T* b, T* y, int H, int D, cudaStream_t st) {
+  if constexpr (kEdgeFeat) {
+    const size_t row = (size_t)H * sizeof(T);
+    const int ds = (uintptr_t)y % (row < 16 ? row : 16) == 0 ? feat_slots<T>(H, D, {a, b}) : 0;
+    if (ds) {
+      if (!ar.base) return GRAPHOP_OK;
+      return dispatch_feat<T>(H, ds, [&](auto heads, auto slots) -> int {
+        const long long blocks = ((g.E + kMixPer - 1) / kMixPer * ds + 255) / 256;
+        edge_feat_dot_kernel<T, VecMax<T>::value, decltype(heads)::value, decltype(slots)::value>
+            <<<(unsigned)blocks, 256, 0, st>>>(g.erow, g.eid, a, b, y, g.E, D);
+        GK_LAUNCHED("edge_dot");
+        return GRAPHOP_OK;
+      });
+    }
+  }
   const GeoPick p = narrow_fix(pick_geo(H, D, sizeof(T), slot_align_of({a, b}), false));
   if (p.SB && p.nhb <= kMaxHeadBlocks)
     return dispatch_geo<T, true>(p, [&](auto tag) -> int {
@@ -345,27 +398,29 @@ inline int run_edge_dot(Arena& ar, const GraphView& g, const T* a, const T* b, T
   return GRAPHOP_OK;
 }
 
-// dB[eid[k], :] = sum_h dy[eid[k], h] * A[node(k), h, :]
-template <typename T>
-inline int run_edge_mix(const GraphView& g, const T* dy, const T* a, T* db, int H, int D, cudaStream_t st) {
+// db[edge, :] = sum_h g[edge, h] * a[node, h, :]; g = dy by edge id or, kPairs, the score gradients by position.
+template <typename T, bool kPairs>
+inline int run_edge_mix(const GraphView& g, const T* dy, const EdgePair<typename AccOf<T>::type>* pairs, int Hp, const T* a,
+                        T* db, int H, int D, cudaStream_t st) {
   constexpr int VM = VecMax<T>::value;
   const bool vec = aligned16(a) && aligned16(db) && D % VM == 0;
-  const long long total = g.E * (vec ? D / VM : D);
-  const unsigned grid = (unsigned)((total + 255) / 256 < (1 << 20) ? (total + 255) / 256 : (1 << 20));
+  const size_t row = (size_t)H * sizeof(T);
+  // the head counts whose row of g is whole aligned moves
+  const int hh = vec && (H == 1 || H == 2 || H == 4 || H == 8) && (kPairs || (uintptr_t)dy % (row < 16 ? row : 16) == 0) ? H : 0;
   const int ds = vec ? D / VM : D;
   int shift = -1;
   if (is_pow2(ds)) for (shift = 0; (1 << shift) < ds; ++shift) {}
-  const unsigned blocks = grid ? grid : 1;
-#define GK_MIX(VV, HH) \
-  edge_mix_heads_kernel<T, VV, HH><<<blocks, 256, 0, st>>>(g.erow, g.eid, dy, a, db, g.E, H, D, shift)
-  if (vec) {
-    if (H == 1) GK_MIX(VM, 1); else if (H == 2) GK_MIX(VM, 2); else if (H == 4) GK_MIX(VM, 4);
-    else if (H == 8) GK_MIX(VM, 8); else GK_MIX(VM, 0);
-  } else {
-    GK_MIX(1, 0);
-  }
+  const long long blocks = ((g.E + kMixPer - 1) / kMixPer * ds + 255) / 256;
+#define GK_MIX(VV, HH)                                                                                                \
+  edge_mix_kernel<T, VV, HH, kPairs><<<(unsigned)blocks, 256, 0, st>>>(g.erow, g.eid, dy, pairs, a, db, g.E, H, Hp, D, shift)
+  if (!vec) GK_MIX(1, 0);
+  else if (hh == 1) GK_MIX(VM, 1);
+  else if (hh == 2) GK_MIX(VM, 2);
+  else if (hh == 4) GK_MIX(VM, 4);
+  else if (hh == 8) GK_MIX(VM, 8);
+  else GK_MIX(VM, 0);
 #undef GK_MIX
-  GK_LAUNCHED("edge_mix_heads");
+  GK_LAUNCHED(kPairs ? "attention_bias_grad" : "edge_mix_heads");
   return GRAPHOP_OK;
 }
 
@@ -507,7 +562,7 @@ inline int node_mul_edge_backward(const GS& gs, const T* A_, const T* B_, const 
   GK_TRY(gs(ar, n_dst, st, &g, Clear{dB, (size_t)E * D * sizeof(T)}));
   GK_TRY((run_aggregate<T, true>(ar, g, dy, B_, dA, n_dst, H, D, st)));
   if (!ar.base) return GRAPHOP_OK;
-  return run_edge_mix<T>(g, dy, A_, dB, H, D, st);
+  return run_edge_mix<T, false>(g, dy, nullptr, 0, A_, dB, H, D, st);
 }
 
 template <typename T, bool kBackward, class GS>
@@ -783,18 +838,7 @@ inline int attention_bias_backward(const GS& gs_r, const GS& gs_c, bool has_eid_
     GraphView g;
     GK_TRY(gs_r(ar, n_dst, st, &g));
     GK_TRY((run_attn_bwd_dst<T, true>(ar, g, s, q, k, v, rel, o, dout, lse, stat, pd, scale, dq, n_dst, H, D, st)));
-    {
-      constexpr int VM = VecMax<T>::value;
-      const bool vec = aligned16(d_rel) && D % VM == 0;   // q is 16-byte aligned (checked above)
-      const int slots = vec ? D / VM : D;
-      int shift = -1;
-      if (is_pow2(slots)) for (shift = 0; (1 << shift) < slots; ++shift) {}
-      const long long total = E * slots;
-      const unsigned grid = (unsigned)((total + 255) / 256 < (1 << 20) ? (total + 255) / 256 : (1 << 20));
-      if (vec) bias_grad_kernel<T, VM><<<grid ? grid : 1, 256, 0, st>>>(g.erow, pd, q, d_rel, E, H, Hp, D, shift);
-      else bias_grad_kernel<T, 1><<<grid ? grid : 1, 256, 0, st>>>(g.erow, pd, q, d_rel, E, H, Hp, D, shift);
-    }
-    GK_LAUNCHED("attention_bias_grad");
+    GK_TRY((run_edge_mix<T, true>(g, nullptr, pd, Hp, q, d_rel, H, D, st)));
   }
   ar.used = mark;
   GraphView g;

@@ -139,56 +139,6 @@ struct EdgeDotAnyOp {
   }
 };
 
-// ---------------------------------------------------------------------------------------
-// node_mul_edge backward, edge half:  dB[eid[k], :] = sum_h dy[eid[k], h] * A[node(k), h, :]
-// (graphop_kernel.cu:84-92).  One thread per (position, D-slot); no reduction across edges.
-// ---------------------------------------------------------------------------------------
-// kH: the head count when it is 1, 2, 4 or 8 (all of an edge's loads are then issued before the first use),
-// 0: read it from H.  ds_shift >= 0: D / V is that power of two (no 64-bit division per element).
-template <typename T, int V, int kH>
-__global__ void __launch_bounds__(256)
-edge_mix_heads_kernel(const int32_t* __restrict__ erow, const int32_t* __restrict__ eid, const T* __restrict__ dy,
-                      const T* __restrict__ a, T* __restrict__ db, long long E, int H, int D, int ds_shift) {
-  using A = typename AccOf<T>::type;
-  const int ds = D / V;
-  const int nh = kH ? kH : H;
-  const long long total = E * ds;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += stride) {
-    const long long j = ds_shift >= 0 ? (idx >> ds_shift) : idx / ds;
-    const int s = (int)(idx - j * ds);
-    const int node = __ldg(erow + j);
-    if (node < 0) continue;
-    const long long e = eid ? (long long)__ldg(eid + j) : j;
-    const T* arow = a + (long long)node * nh * D + s * V;
-    const T* grow = dy + e * nh;
-    A acc[V];
-#pragma unroll
-    for (int v = 0; v < V; ++v) acc[v] = A(0);
-    if constexpr (kH != 0) {
-      A g[kH], av[kH][V];
-#pragma unroll
-      for (int h = 0; h < kH; ++h) {
-        g[h] = to_acc<T>(__ldg(grow + h));
-        load_acc<T, V>(av[h], arow + (long long)h * D);
-      }
-#pragma unroll
-      for (int h = 0; h < kH; ++h)
-#pragma unroll
-        for (int v = 0; v < V; ++v) acc[v] += g[h] * av[h][v];
-    } else {
-      for (int h = 0; h < nh; ++h) {
-        const A g = to_acc<T>(__ldg(grow + h));
-        A av[V];
-        load_acc<T, V>(av, arow + (long long)h * D);
-#pragma unroll
-        for (int v = 0; v < V; ++v) acc[v] += g * av[v];
-      }
-    }
-    store_acc<T, V>(db + e * D + s * V, acc);
-  }
-}
-
 // (lse, delta) of one (destination node, head), written side by side by the destination pass so that the
 // source pass fetches both with one load.  Rows hold `stat_heads(H)` pairs: H rounded up so that a row is
 // a whole number of 16-byte pieces.
@@ -198,37 +148,196 @@ template <typename A> struct alignas(2 * sizeof(A)) StatPair { A lse, delta; };
 template <typename A> struct alignas(2 * sizeof(A)) EdgePair { A p, ds; };
 __host__ __device__ constexpr int stat_heads(int H, int acc_bytes) { return acc_bytes >= 8 ? H : ((H + 1) & ~1); }
 
-// Gradient of the edge term of the biased attention:  d_rel[j, :] = sum_h ds[j, h] * q[node(j), h, :]
-// (the dB half of node_mul_edge backward, graphop_kernel.cu:79-93, with the score gradients the destination
-// pass left in `pairs`).  One thread per (position, slot of V features); consecutive threads cover a position's
-// features, consecutive positions of a node re-read its q row from L1 / L2; positions no chunk covers get 0.
-// shift = log2(D / V) when that is a power of two, else -1.
-template <typename T, int V>
+// ---------------------------------------------------------------------------------------
+// node_mul_edge backward, edge half:  db[eid[k], :] = sum_h g[eid[k], h] * a[node(k), h, :]
+// (graphop_kernel.cu:84-92), and the gradient of the edge term of the biased attention, the same sum with the score
+// gradients ds that the destination pass left in the (p, ds) pairs, by position.  No reduction across edges.
+//
+// A thread owns one slot of V features of kMixPer consecutive positions: the positions' nodes, ids and g are loaded
+// together, the node's slots of all heads stay in registers while the node lasts.  Consecutive threads own the slots of a
+// position, so that a store covers whole rows.  Bound by the written tensor; with a thread per position and slot, which
+// reads the H slots of its node again for every edge, 17.8M edges, 4 x 32 fp32, took 1.07 ms.
+// kH: the head count when it is 1, 2, 4 or 8, 0: read it from H, one head at a time.  ds_shift >= 0: D / V is that power
+// of two.
+// ---------------------------------------------------------------------------------------
+constexpr int kMixPer = 8;
+template <typename T, int V, int kH, bool kPairs>
 __global__ void __launch_bounds__(256)
-bias_grad_kernel(const int32_t* __restrict__ erow, const EdgePair<typename AccOf<T>::type>* __restrict__ pairs,
-                 const T* __restrict__ q, T* __restrict__ d_rel, long long E, int H, int Hp, int D, int shift) {
+edge_mix_kernel(const int32_t* __restrict__ erow, const int32_t* __restrict__ eid, const T* __restrict__ dy,
+                const EdgePair<typename AccOf<T>::type>* __restrict__ pairs, const T* __restrict__ a, T* __restrict__ db,
+                long long E, int H, int Hp, int D, int ds_shift) {
   using A = typename AccOf<T>::type;
-  const int slots = D / V;
-  const long long stride = (long long)gridDim.x * blockDim.x, total = E * slots;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-    const long long j = shift >= 0 ? (i >> shift) : i / slots;
-    const int d = (int)(i - j * slots) * V;
-    const int r = __ldg(erow + j);
-    A sum[V];
+  constexpr int P = kMixPer, N = kH ? kH : 1;
+  const unsigned ds = (unsigned)(D / V);
+  const int nh = kH ? kH : H;
+  const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;
+  const long long chunk = ds_shift >= 0 ? idx >> ds_shift : idx <= 0xffffffffLL ? (unsigned)idx / ds : idx / ds;
+  const int s = (int)(idx - chunk * ds);
+  const long long j0 = chunk * P;
+  if (j0 >= E) return;
+  alignas(16) int node[P], edge[P];
+  const bool whole = j0 + P <= E;
+  if (whole) {
 #pragma unroll
-    for (int e = 0; e < V; ++e) sum[e] = A(0);
-    if (r >= 0) {
-      const T* qrow = q + (long long)r * H * D + d;
-      const EdgePair<A>* pr = pairs + j * Hp;
-      for (int h = 0; h < H; ++h) {
-        const A ds = pr[h].ds;
-        A qv[V];
-        load_acc<T, V>(qv, qrow + (long long)h * D);
+    for (int i = 0; i < P; i += 4) *reinterpret_cast<int4*>(node + i) = __ldg(reinterpret_cast<const int4*>(erow + j0 + i));
+  } else {
 #pragma unroll
-        for (int e = 0; e < V; ++e) sum[e] += ds * qv[e];
+    for (int i = 0; i < P; ++i) node[i] = j0 + i < E ? __ldg(erow + j0 + i) : -2;   // -2: nothing to do
+  }
+#pragma unroll
+  for (int i = 0; i < P; ++i) edge[i] = !kPairs && eid && node[i] > -2 ? __ldg(eid + j0 + i) : (int)(j0 + i);
+  const T* base = a + s * V;
+  const auto slot_of = [&](int r, int h) { return base + ((long long)r * nh + h) * D; };
+  const auto g_of = [&](int i, int h) -> A {
+    if constexpr (kPairs) return pairs[(long long)edge[i] * Hp + h].ds;
+    else return to_acc<T>(__ldg(dy + (long long)edge[i] * nh + h));
+  };
+  if constexpr (kH != 0) {
+    A g[P][N];
+#pragma unroll
+    for (int i = 0; i < P; ++i)
+      if (node[i] >= 0) {
+        if constexpr (!kPairs && N * sizeof(T) <= 16 && N > 1) {
+          // rows of g start at multiples of their size wherever the tensor does (checked by the launch)
+          load_acc<T, N>(g[i], dy + (long long)edge[i] * N);
+        } else if constexpr (!kPairs && N > 1) {
+          constexpr int per = 16 / (int)sizeof(T);
+#pragma unroll
+          for (int h = 0; h < N; h += per) load_acc<T, per>(*reinterpret_cast<A(*)[per]>(&g[i][h]), dy + (long long)edge[i] * N + h);
+        } else {
+#pragma unroll
+          for (int h = 0; h < N; ++h) g[i][h] = g_of(i, h);
+        }
+      }
+    A av[N][V];
+    int cur = -1;
+#pragma unroll
+    for (int i = 0; i < P; ++i) {
+      if (node[i] < 0) {
+        if (kPairs && node[i] == -1) {   // a position of no chunk has no gradient
+          A zero[V];
+#pragma unroll
+          for (int v = 0; v < V; ++v) zero[v] = A(0);
+          store_acc<T, V>(db + (long long)edge[i] * D + s * V, zero);
+        }
+        continue;
+      }
+      if (node[i] != cur) {
+        cur = node[i];
+#pragma unroll
+        for (int h = 0; h < N; ++h) load_acc<T, V>(av[h], slot_of(cur, h));
+      }
+      A acc[V];
+#pragma unroll
+      for (int v = 0; v < V; ++v) acc[v] = A(0);
+#pragma unroll
+      for (int h = 0; h < N; ++h)
+#pragma unroll
+        for (int v = 0; v < V; ++v) acc[v] += g[i][h] * av[h][v];
+      store_acc<T, V>(db + (long long)edge[i] * D + s * V, acc);
+    }
+  } else {
+    A acc[P][V];
+#pragma unroll
+    for (int i = 0; i < P; ++i)
+#pragma unroll
+      for (int v = 0; v < V; ++v) acc[i][v] = A(0);
+    for (int h = 0; h < nh; ++h) {
+      A av[V], g[P];
+      int cur = -1;
+#pragma unroll
+      for (int i = 0; i < P; ++i) g[i] = node[i] >= 0 ? g_of(i, h) : A(0);
+#pragma unroll
+      for (int i = 0; i < P; ++i) {
+        if (node[i] < 0) continue;
+        if (node[i] != cur) {
+          cur = node[i];
+          load_acc<T, V>(av, slot_of(cur, h));
+        }
+#pragma unroll
+        for (int v = 0; v < V; ++v) acc[i][v] += g[i] * av[v];
       }
     }
-    store_acc<T, V>(d_rel + j * D + d, sum);
+#pragma unroll
+    for (int i = 0; i < P; ++i)
+      if (node[i] >= 0 || (kPairs && node[i] == -1)) store_acc<T, V>(db + (long long)edge[i] * D + s * V, acc[i]);
+  }
+}
+
+// y[edge, h] = a[node, h, :] . b[edge, :], b an edge tensor shared by the heads (graphop_kernel.cu:16-34): edge_mix_kernel
+// the other way round.  A thread owns one slot of kMixPer consecutive positions and the node's slots of all kH heads, so
+// that an edge's row is read once, whatever the number of heads; the partial sums of DS lanes meet by halves: a lane gives
+// away half of its positions at every step and ends with one position's scores, written together.  The sums are formed in
+// the order of Geo::ordered_dot.  Bound by reading b; on the gathering walker, which copies the row once per head, 17.8M
+// edges, 4 x 32 fp32, took 1.05 ms.
+template <typename T, int V, int kH, int DS>
+__global__ void __launch_bounds__(256)
+edge_feat_dot_kernel(const int32_t* __restrict__ erow, const int32_t* __restrict__ eid, const T* __restrict__ a,
+                     const T* __restrict__ b, T* __restrict__ y, long long E, int D) {
+  using A = typename AccOf<T>::type;
+  constexpr int P = kMixPer, B = DS < P ? DS : P;
+  const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;
+  const int s = threadIdx.x & (DS - 1);
+  const long long j0 = idx / DS * P;
+  alignas(16) int node[P], edge[P];
+  if (j0 + P <= E) {
+#pragma unroll
+    for (int i = 0; i < P; i += 4) *reinterpret_cast<int4*>(node + i) = __ldg(reinterpret_cast<const int4*>(erow + j0 + i));
+  } else {
+#pragma unroll
+    for (int i = 0; i < P; ++i) node[i] = j0 + i < E ? __ldg(erow + j0 + i) : -1;
+  }
+#pragma unroll
+  for (int i = 0; i < P; ++i) edge[i] = eid && node[i] >= 0 ? __ldg(eid + j0 + i) : (int)(j0 + i);
+  using M = typename Mover<sizeof(T) * V>::type;
+  union { M m; T t[V]; } feat[P];
+#pragma unroll
+  for (int i = 0; i < P; ++i)
+    if (node[i] >= 0) feat[i].m = __ldg(reinterpret_cast<const M*>(b + (long long)edge[i] * D + s * V));
+  A av[kH][V], part[P][kH];
+  int cur = -1;
+#pragma unroll
+  for (int i = 0; i < P; ++i) {
+#pragma unroll
+    for (int h = 0; h < kH; ++h) part[i][h] = A(0);
+    if (node[i] < 0) continue;
+    if (node[i] != cur) {
+      cur = node[i];
+#pragma unroll
+      for (int h = 0; h < kH; ++h) load_acc<T, V>(av[h], a + ((long long)cur * kH + h) * D + s * V);
+    }
+#pragma unroll
+    for (int h = 0; h < kH; ++h) {
+      part[i][h] = av[h][0] * to_acc<T>(feat[i].t[0]);
+#pragma unroll
+      for (int v = 1; v < V; ++v) part[i][h] = fma(av[h][v], to_acc<T>(feat[i].t[v]), part[i][h]);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < P; k += B) {
+#pragma unroll
+    for (int d = 1; d < B; d <<= 1) {
+      const bool up = (s & d) != 0;
+#pragma unroll
+      for (int j = 0; j < B / 2 / d; ++j)
+#pragma unroll
+        for (int h = 0; h < kH; ++h) {
+          const A keep = up ? part[k + 2 * j + 1][h] : part[k + 2 * j][h];
+          const A give = up ? part[k + 2 * j][h] : part[k + 2 * j + 1][h];
+          part[k + j][h] = keep + __shfl_xor_sync(kFull, give, d);
+        }
+    }
+#pragma unroll
+    for (int d = B; d < DS; d <<= 1)
+#pragma unroll
+      for (int h = 0; h < kH; ++h) part[k][h] += __shfl_xor_sync(kFull, part[k][h], d);
+    const long long j = j0 + k + (s & (B - 1));   // the position whose sums ended here
+    if (s < B && j < E && __ldg(erow + j) >= 0) {
+      const long long e = eid ? (long long)__ldg(eid + j) : j;
+      constexpr int per = kH * (int)sizeof(T) <= 16 ? kH : 16 / (int)sizeof(T);
+#pragma unroll
+      for (int h = 0; h < kH; h += per) store_acc<T, per>(y + e * kH + h, *reinterpret_cast<const A(*)[per]>(&part[k][h]));
+    }
   }
 }
 
