@@ -557,10 +557,76 @@ Tensor attention_bias(const Tensor& row, const Tensor& indptr, const Tensor& ind
   return attention_common(rows, nullptr, tb, c, q, k, v, rel, scale);
 }
 
+// ---- graph preparation: graphop.py's functions of the same names ---------------------------
+Tensor scratch_of(size_t bytes, const Tensor& like, void** base) {
+  Tensor t = at::empty({(int64_t)bytes + 256}, like.options().dtype(at::kByte));
+  *base = reinterpret_cast<void*>((reinterpret_cast<uintptr_t>(t.data_ptr()) + 255) / 256 * 256);
+  return t;
+}
+template <class I> I* as(const Tensor& t) { return t.defined() ? reinterpret_cast<I*>(t.data_ptr()) : nullptr; }
+
+std::tuple<Tensor, Tensor> partition_csr(const Tensor& indptr, int64_t chunk_size) {
+  const Tensor ip = indptr.contiguous();
+  Call c(ip);
+  const int64_t n = ip.numel() - 1;
+  const bool wide = ip.scalar_type() == at::kLong;
+  const size_t bytes = graphop_partition_csr_workspace_bytes(n);
+  void* ws = nullptr;
+  const Tensor scratch = scratch_of(bytes, ip, &ws);
+  int64_t count = 0;
+  check_status(wide ? graphop_partition_csr_count_i64(as<int64_t>(ip), n, chunk_size, ws, bytes, &count, raw(c.stream))
+                    : graphop_partition_csr_count_i32(as<int32_t>(ip), n, chunk_size, ws, bytes, &count, raw(c.stream)),
+               "partition_csr_count");
+  Tensor row = at::empty({count}, ip.options().dtype(at::kLong)), ptr = at::empty({count + 1}, ip.options().dtype(at::kLong));
+  check_status(wide ? graphop_partition_csr_fill_i64(as<int64_t>(ip), n, chunk_size, ws, count, as<int64_t>(row),
+                                                     as<int64_t>(ptr), raw(c.stream))
+                    : graphop_partition_csr_fill_i32(as<int32_t>(ip), n, chunk_size, ws, count, as<int64_t>(row),
+                                                     as<int64_t>(ptr), raw(c.stream)),
+               "partition_csr_fill");
+  return {row, ptr};
+}
+
+std::tuple<Tensor, Tensor, Tensor> transpose_csr(const Tensor& indptr, const Tensor& indices, int64_t n_src) {
+  const Tensor ip = indptr.contiguous(), idx = indices.contiguous();
+  Call c(ip);
+  const int64_t n_dst = ip.numel() - 1, e = idx.numel();
+  const bool wide = ip.scalar_type() == at::kLong;
+  const size_t bytes = graphop_transpose_csr_workspace_bytes(e, wide ? 8 : 4);
+  void* ws = nullptr;
+  const Tensor scratch = scratch_of(bytes, ip, &ws);
+  Tensor ptr_t = at::empty({n_src + 1}, ip.options()), idx_t = at::empty_like(idx), eid_t = at::empty_like(idx);
+  check_status(wide ? graphop_transpose_csr_i64(as<int64_t>(ip), as<int64_t>(idx), n_dst, n_src, e, as<int64_t>(ptr_t),
+                                                as<int64_t>(idx_t), as<int64_t>(eid_t), ws, bytes, raw(c.stream))
+                    : graphop_transpose_csr_i32(as<int32_t>(ip), as<int32_t>(idx), n_dst, n_src, e, as<int32_t>(ptr_t),
+                                                as<int32_t>(idx_t), as<int32_t>(eid_t), ws, bytes, raw(c.stream)),
+               "transpose_csr");
+  return {ptr_t, idx_t, eid_t};
+}
+
+// Fills the graphop_plan_t at `address`; returns the memory it refers to.
+Tensor plan_build(const Tensor& row, const Tensor& indptr, const c10::optional<Tensor>& eid_in,
+                  const c10::optional<Tensor>& indices_in, int64_t n_edges, int64_t n_nodes, uintptr_t address) {
+  const Tensor eid = eid_in.value_or(Tensor()), indices = indices_in.value_or(Tensor());
+  const int ib = index_bytes_of({&row, &indptr, &eid, &indices});
+  Call c(row);
+  const size_t bytes = graphop_plan_bytes(row.size(0), n_edges, n_nodes, ib);
+  void* base = nullptr;
+  Tensor memory = scratch_of(bytes, row, &base);
+  auto* plan = reinterpret_cast<graphop_plan_t*>(address);
+  check_status(ib == 8 ? graphop_plan_build_i64(as<int64_t>(row), as<int64_t>(indptr), as<int64_t>(eid),
+                                                as<int64_t>(indices), row.size(0), n_edges, n_nodes, base, bytes, plan,
+                                                raw(c.stream))
+                       : graphop_plan_build_i32(as<int32_t>(row), as<int32_t>(indptr), as<int32_t>(eid),
+                                                as<int32_t>(indices), row.size(0), n_edges, n_nodes, base, bytes, plan,
+                                                raw(c.stream)),
+               "plan_build");
+  return memory;
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
-  m.doc() = "the autograd Functions of custom_op_benchmark_b200.wrapper in native code";
+  m.doc() = "the autograd Functions of custom_op_benchmark_b200.wrapper and the graph preparation in native code";
   using free_gil = py::call_guard<py::gil_scoped_release>;
   py::class_<PlanHandle>(m, "PlanHandle").def(py::init<uintptr_t, std::vector<Tensor>>());
   m.def("sparse_softmax", &sparse_softmax, free_gil());
@@ -569,4 +635,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("vector_spmm", &vector_spmm, free_gil());
   m.def("attention_planned", &attention_planned, free_gil());
   m.def("attention_bias", &attention_bias, free_gil());
+  m.def("partition_csr", &partition_csr, free_gil());
+  m.def("transpose_csr", &transpose_csr, free_gil());
+  m.def("plan_build", &plan_build, free_gil());
 }

@@ -180,6 +180,9 @@ struct ExpandExtra {
   int32_t* dst[2];
   uint16_t* clear;
   long long clear_n;   // 2-byte words
+  int32_t* fill[3];    // arrays a plan's next kernels count on (null: none), with their lengths and values
+  long long fill_n[3];
+  int32_t fill_with[3];
 };
 
 // A block expands a run of `per_block` chunks (at most one per thread; the launch picks it for about one step of
@@ -234,6 +237,13 @@ expand_rows_kernel(const I* __restrict__ row, const I* __restrict__ indptr, long
     for (long long i = (long long)blockIdx.x * kExpandThreads + tid; i < extra.clear_n;
          i += (long long)gridDim.x * kExpandThreads)
       extra.clear[i] = 0;
+
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+    if (extra.fill[a])
+      for (long long i = (long long)blockIdx.x * kExpandThreads + tid; i < extra.fill_n[a];
+           i += (long long)gridDim.x * kExpandThreads)
+        extra.fill[a][i] = extra.fill_with[a];
 
   // nodes that positions without a chunk count for in the cut: 0 before the covered ones, the last node after them
   const auto node_before = [&](long long c) {   // of the last chunk before c that is not empty

@@ -167,11 +167,13 @@ struct GraphView {
 
 // an edge output that starts from zero when some position belongs to no chunk
 struct Clear { void* out = nullptr; size_t bytes = 0; };
+// arrays of 32-bit words set on the way
+struct Fill { int32_t* out[3]; long long n[3]; int32_t with[3]; };
 
 template <typename I>
 inline int prepare_graph(Arena& ar, const I* row, const I* indptr, const I* eid, const I* indices, long long C,
                          long long E, long long n_nodes, cudaStream_t st, GraphView* g, Clear clear = {},
-                         PlanHeader* hdr = nullptr) {
+                         PlanHeader* hdr = nullptr, const Fill& fill = {}) {
   if (!hdr) hdr = (PlanHeader*)ar.take(sizeof(PlanHeader));
   auto* erow = (int32_t*)ar.take((size_t)E * 4);
   // n_nodes < 0: an op that cuts no tiles
@@ -192,12 +194,13 @@ inline int prepare_graph(Arena& ar, const I* row, const I* indptr, const I* eid,
   if (!ar.base) return GRAPHOP_OK;
   if (ar.overflow) return GRAPHOP_ERR_WORKSPACE;
   const ExpandExtra<I> extra{{other32 ? indices : nullptr, eid32 ? eid : nullptr}, {other32, eid32}, (uint16_t*)clear.out,
-                             (long long)(clear.bytes / 2)};
+                             (long long)(clear.bytes / 2), {fill.out[0], fill.out[1], fill.out[2]},
+                             {fill.n[0], fill.n[1], fill.n[2]}, {fill.with[0], fill.with[1], fill.with[2]}};
   // about one step of positions per block
   long long per_block = C > 0 ? kExpandTile * C / E : 1;
   per_block = per_block < 1 ? 1 : per_block > kExpandThreads ? kExpandThreads : per_block;
   long long blocks = C > 0 ? (C + per_block - 1) / per_block : 1;
-  const long long copies = (other32 || eid32 || clear.out) ? (E + kExpandTile - 1) / kExpandTile : 1;
+  const long long copies = (other32 || eid32 || clear.out || fill.out[0]) ? (E + kExpandTile - 1) / kExpandTile : 1;
   if (blocks < copies && blocks < 1024) blocks = copies < 1024 ? copies : 1024;   // long chunks: blocks for the copies
   expand_rows_kernel<I><<<(unsigned)blocks, kExpandThreads, 0, st>>>(row, indptr, C, (int)E, (int)per_block, erow, hdr, cut,
                                                                   extra);

@@ -13,27 +13,30 @@
 // transpose_csr: a stable sort of the positions by source id (CUB DeviceRadixSort over just the bits a source id
 // needs; stable, so within one source the destinations ascend and the result is the same on every run, which an
 // atomic counting sort would not give) yields eid_t; one pass over the sorted keys writes indptr_t at every key
-// change (no histogram, no atomics) and looks every position's destination row up in indptr by binary search.
+// change (no histogram, no atomics) and takes every position's destination row from a table made before the sort.
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
+#include <thrust/iterator/counting_iterator.h>
+#include <thrust/iterator/transform_iterator.h>
 
 #include "gk_host.cuh"
 
 namespace gk {
 namespace {
 
+// Chunks of row r (r = n: none, so that the exclusive scan ends with the total), formed while the scan reads them.
 template <typename I>
-__global__ void chunk_counts_kernel(const I* __restrict__ indptr, long long n, long long cs, long long* __restrict__ out) {
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r <= n; r += stride) {
-    long long c = 0;
-    if (r < n) {
-      const long long deg = (long long)indptr[r + 1] - (long long)indptr[r];
-      c = deg > 0 ? (deg + cs - 1) / cs : 0;   // range(a, b, cs) is empty when b <= a
-    }
-    out[r] = c;   // out[n] = 0: after the exclusive scan it holds the total
+struct ChunkCount {
+  const I* indptr;
+  long long n, cs;
+  __host__ __device__ long long operator()(long long r) const {
+    if (r >= n) return 0;
+    const long long deg = (long long)indptr[r + 1] - (long long)indptr[r];
+    return deg > 0 ? (deg + cs - 1) / cs : 0;   // range(a, b, cs) is empty when b <= a
   }
-}
+};
+template <typename I>
+using ChunkCounts = thrust::transform_iterator<ChunkCount<I>, thrust::counting_iterator<long long>>;
 
 template <typename I>
 __global__ void chunk_fill_kernel(const I* __restrict__ indptr, const long long* __restrict__ first, long long n,
@@ -58,7 +61,8 @@ __global__ void chunk_fill_kernel(const I* __restrict__ indptr, const long long*
 
 size_t scan_temp_bytes(long long items) {
   size_t bytes = 0;
-  cub::DeviceScan::ExclusiveSum(nullptr, bytes, (long long*)nullptr, (long long*)nullptr, (int)(items > 0 ? items : 1));
+  const ChunkCounts<int64_t> counts(thrust::counting_iterator<long long>(0), ChunkCount<int64_t>{nullptr, 0, 1});
+  cub::DeviceScan::ExclusiveSum(nullptr, bytes, counts, (long long*)nullptr, (int)(items > 0 ? items : 1));
   return bytes;
 }
 
@@ -76,10 +80,8 @@ int partition_count(const I* indptr, long long n, long long cs, void* ws, size_t
   size_t temp_bytes = scan_temp_bytes(n + 1);
   void* temp = ar.take(temp_bytes);
   if (ar.overflow) return GRAPHOP_ERR_WORKSPACE;
-  const unsigned grid = (unsigned)((n + 256) / 256 < 8192 ? (n + 256) / 256 : 8192);
-  chunk_counts_kernel<I><<<grid, 256, 0, st>>>(indptr, n, cs, first);
-  GK_LAUNCHED("partition_counts");
-  GK_CUDA(cub::DeviceScan::ExclusiveSum(temp, temp_bytes, first, first, (int)(n + 1), st));
+  const ChunkCounts<I> counts(thrust::counting_iterator<long long>(0), ChunkCount<I>{indptr, n, cs});
+  GK_CUDA(cub::DeviceScan::ExclusiveSum(temp, temp_bytes, counts, first, (int)(n + 1), st));
   GK_CUDA(cudaMemcpyAsync(n_chunks, first + n, 8, cudaMemcpyDeviceToHost, st));
   GK_CUDA(cudaStreamSynchronize(st));
   return GRAPHOP_OK;
@@ -104,16 +106,27 @@ int partition_fill(const I* indptr, long long n, long long cs, const void* ws, l
   return GRAPHOP_OK;
 }
 
+// Every position and the row that owns it: the last r with indptr[r] <= position (rows without edges are skipped by it).
+// In position order neighbouring searches read the same entries; after the sort they would not.
 template <typename I>
-__global__ void iota_kernel(I* __restrict__ out, long long n) {
+__global__ void position_rows_kernel(const I* __restrict__ indptr, long long n_dst, long long E, I* __restrict__ position,
+                                     I* __restrict__ rows) {
   const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) out[i] = (I)i;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < E; i += stride) {
+    long long lo = 0, hi = n_dst;
+    while (hi - lo > 1) {
+      const long long mid = (lo + hi) >> 1;
+      if ((long long)indptr[mid] <= i) lo = mid; else hi = mid;
+    }
+    position[i] = (I)i;
+    rows[i] = (I)lo;
+  }
 }
 
 // keys: the source ids in transposed order; eid_t: the row-CSR position of every transposed position.
 template <typename I>
 __global__ void transposed_fill_kernel(const I* __restrict__ keys, const I* __restrict__ eid_t,
-                                       const I* __restrict__ indptr, long long n_dst, long long n_src, long long E,
+                                       const I* __restrict__ rows, long long n_src, long long E,
                                        I* __restrict__ indptr_t, I* __restrict__ indices_t) {
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j <= E; j += stride) {
@@ -125,14 +138,7 @@ __global__ void transposed_fill_kernel(const I* __restrict__ keys, const I* __re
     cur = cur > n_src ? n_src : cur;
     for (long long k = prev + 1; k <= cur; ++k) indptr_t[k] = (I)j;
     if (j == E) continue;
-    // the row that owns position e: the last r with indptr[r] <= e (rows without edges are skipped by it)
-    const long long e = (long long)eid_t[j];
-    long long lo = 0, hi = n_dst;
-    while (hi - lo > 1) {
-      const long long mid = (lo + hi) >> 1;
-      if ((long long)indptr[mid] <= e) lo = mid; else hi = mid;
-    }
-    indices_t[j] = (I)lo;
+    indices_t[j] = rows[eid_t[j]];
   }
 }
 
@@ -151,24 +157,26 @@ int transpose(const I* indptr, const I* indices, long long n_dst, long long n_sr
   if (sizeof(I) == 4 && (n_src >= (1LL << 31) || n_dst >= (1LL << 31))) return GRAPHOP_ERR_INVALID_ARGUMENT;
   if (E > 0 && (!indptr || !indices || !indices_t || !eid_t || n_dst == 0 || n_src == 0))
     return GRAPHOP_ERR_INVALID_ARGUMENT;
-  I* keys = nullptr;
+  I *keys = nullptr, *rows = nullptr;
   if (E > 0) {
     GK_TRY(check_ws(ws));
     Arena ar(ws, wsb);
     keys = (I*)ar.take((size_t)E * sizeof(I));
+    rows = (I*)ar.take((size_t)E * sizeof(I));
     size_t temp_bytes = sort_temp_bytes<I>(E);
     void* temp = ar.take(temp_bytes);
     if (ar.overflow) return GRAPHOP_ERR_WORKSPACE;
     const unsigned grid = (unsigned)((E + 255) / 256 < 16384 ? (E + 255) / 256 : 16384);
-    iota_kernel<I><<<grid, 256, 0, st>>>(indices_t, E);   // the output buffer doubles as the sort's value input
-    GK_LAUNCHED("transpose_iota");
+    // the output buffer doubles as the sort's value input
+    position_rows_kernel<I><<<grid, 256, 0, st>>>(indptr, n_dst, E, indices_t, rows);
+    GK_LAUNCHED("transpose_positions");
     int bits = 1;
     while (bits < (int)sizeof(I) * 8 && ((n_src - 1) >> bits) != 0) ++bits;
     GK_CUDA(cub::DeviceRadixSort::SortPairs(temp, temp_bytes, indices, keys, (const I*)indices_t, eid_t, (int)E, 0, bits,
                                             st));
   }
   const unsigned grid = (unsigned)((E + 256) / 256 < 16384 ? (E + 256) / 256 : 16384);
-  transposed_fill_kernel<I><<<grid, 256, 0, st>>>(keys, eid_t, indptr, n_dst, n_src, E, indptr_t, indices_t);
+  transposed_fill_kernel<I><<<grid, 256, 0, st>>>(keys, eid_t, rows, n_src, E, indptr_t, indices_t);
   GK_LAUNCHED("transpose_fill");
   return GRAPHOP_OK;
 }
@@ -210,7 +218,7 @@ extern "C" int graphop_partition_csr_fill_i64(const int64_t* indptr, int64_t n_r
 extern "C" size_t graphop_transpose_csr_workspace_bytes(int64_t n_edges, int index_bytes) {
   if (n_edges <= 0) return gk::kAlign;
   const size_t temp = index_bytes == 8 ? gk::sort_temp_bytes<int64_t>(n_edges) : gk::sort_temp_bytes<int32_t>(n_edges);
-  return gk::align_up((size_t)n_edges * (size_t)(index_bytes == 8 ? 8 : 4)) + gk::align_up(temp) + gk::kAlign;
+  return 2 * gk::align_up((size_t)n_edges * (size_t)(index_bytes == 8 ? 8 : 4)) + gk::align_up(temp) + gk::kAlign;
 }
 extern "C" int graphop_transpose_csr_i32(const int32_t* indptr, const int32_t* indices, int64_t n_dst, int64_t n_src,
                                          int64_t n_edges, int32_t* indptr_t, int32_t* indices_t, int32_t* eid_t,

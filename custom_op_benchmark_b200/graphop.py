@@ -18,7 +18,7 @@ import weakref
 
 import torch as th
 
-from . import _capi
+from . import _capi, native_functions
 
 __all__ = [
     "maskedmm_csr_forward", "maskedmm_csr_backward", "node_mul_edge_forward", "node_mul_edge_backward",
@@ -382,32 +382,13 @@ def pull_rows(tables, seg, idx, row_bytes, out):
 def partition_csr(indptr, chunk_size=32):
     """partition_csr of the reference (part_csr.py:13-27) for an int32 / int64 indptr on a CUDA device, by the
     library's kernels (graphop_partition_csr_count / _fill): (row, indptr_) as int64 tensors on that device."""
-    import ctypes
     if chunk_size <= 0:
         raise ValueError("chunk_size must be positive")
     if not indptr.is_cuda or indptr.dtype not in (th.int32, th.int64) or indptr.dim() != 1:
         raise RuntimeError("indptr must be a one-dimensional int32 or int64 CUDA tensor")
     if indptr.numel() < 1:
         raise IndexError("indptr must hold at least one element")
-    ip = indptr.contiguous()
-    n = ip.numel() - 1
-    suffix = "i32" if ip.dtype == th.int32 else "i64"
-    lib = _capi.lib()
-    with th.cuda.device(ip.device):
-        stream = th.cuda.current_stream(ip.device).cuda_stream
-        ws = th.empty(lib.graphop_partition_csr_workspace_bytes(n), dtype=th.uint8, device=ip.device)
-        count = ctypes.c_int64(0)
-        rc = getattr(lib, "graphop_partition_csr_count_" + suffix)(
-            _p(ip), n, int(chunk_size), _p(ws), ws.numel(), ctypes.byref(count), stream)
-        if rc != _capi.OK:
-            raise RuntimeError("graphop_partition_csr_count: %s" % _capi.error_message(rc))
-        row = th.empty(count.value, dtype=th.int64, device=ip.device)
-        ptr = th.empty(count.value + 1, dtype=th.int64, device=ip.device)
-        rc = getattr(lib, "graphop_partition_csr_fill_" + suffix)(
-            _p(ip), n, int(chunk_size), _p(ws), count.value, _p(row), _p(ptr), stream)
-        if rc != _capi.OK:
-            raise RuntimeError("graphop_partition_csr_fill: %s" % _capi.error_message(rc))
-    return row, ptr
+    return native_functions().partition_csr(indptr, int(chunk_size))
 
 
 def transpose_csr(indptr, indices, n_src):
@@ -419,20 +400,7 @@ def transpose_csr(indptr, indices, n_src):
         raise RuntimeError("indptr and indices must be one-dimensional CUDA tensors of the same type, int32 or int64")
     if indptr.numel() < 1:
         raise IndexError("indptr must hold at least one element")
-    ip, idx = indptr.contiguous(), indices.contiguous()
-    n_dst, e, n_src = ip.numel() - 1, idx.numel(), int(n_src)
-    suffix, width = ("i32", 4) if ip.dtype == th.int32 else ("i64", 8)
-    lib = _capi.lib()
-    with th.cuda.device(ip.device):
-        ws = th.empty(lib.graphop_transpose_csr_workspace_bytes(e, width), dtype=th.uint8, device=ip.device)
-        ptr_t = th.empty(n_src + 1, dtype=ip.dtype, device=ip.device)
-        idx_t, eid_t = th.empty_like(idx), th.empty_like(idx)
-        rc = getattr(lib, "graphop_transpose_csr_" + suffix)(
-            _p(ip), _p(idx), n_dst, n_src, e, _p(ptr_t), _p(idx_t), _p(eid_t), _p(ws), ws.numel(),
-            th.cuda.current_stream(ip.device).cuda_stream)
-    if rc != _capi.OK:
-        raise RuntimeError("graphop_transpose_csr: %s" % _capi.error_message(rc))
-    return ptr_t, idx_t, eid_t
+    return native_functions().transpose_csr(indptr, indices, int(n_src))
 
 
 def check_graph(row, indptr, eid, indices, n_nodes, n_other):
@@ -474,25 +442,17 @@ class GraphPlan:
         if indices is not None:
             given["indices"] = indices
         _check_all(**given)
-        index = _index(*given.values())
+        _index(*given.values())
         self.n_chunks, self.n_nodes = _chunks(row, indptr), int(n_nodes)
         self.n_edges = int(indices.size(0) if indices is not None else (eid.size(0) if eid is not None else 0))
         if eid is not None and indices is not None and eid.size(0) != indices.size(0):
             raise RuntimeError("eid and indices disagree on the number of edges")
         self.device = row.device
-        lib = _capi.lib()
-        need = lib.graphop_plan_bytes(self.n_chunks, self.n_edges, self.n_nodes, index[1])
-        self._memory = th.empty(need + 256, dtype=th.uint8, device=self.device)
-        base = (self._memory.data_ptr() + 255) // 256 * 256
         self._keep = (row, indptr, eid, indices)
         self._native = None
         self.c = _capi.Plan()
-        fn = getattr(lib, "graphop_plan_build_%s" % index[0])
-        with th.cuda.device(self.device):
-            rc = fn(_p(row), _p(indptr), _p(eid), _p(indices), self.n_chunks, self.n_edges, self.n_nodes, base, need,
-                    ctypes.byref(self.c), th.cuda.current_stream(self.device).cuda_stream)
-        if rc != _capi.OK:
-            raise RuntimeError("graphop_plan_build: %s" % _capi.error_message(rc))
+        self._memory = native_functions().plan_build(row, indptr, eid, indices, self.n_edges, self.n_nodes,
+                                                     ctypes.addressof(self.c))
 
     @property
     def dense_band(self):
@@ -516,7 +476,6 @@ class GraphPlan:
         """This plan as the native autograd Functions take it."""
         if self._native is None:
             import ctypes
-            from . import native_functions
             keep = [self._memory] + [t for t in self._keep if t is not None]
             self._native = native_functions().PlanHandle(ctypes.addressof(self.c), keep)
         return self._native
