@@ -196,8 +196,11 @@ inline int prepare_graph(Arena& ar, const I* row, const I* indptr, const I* eid,
   const ExpandExtra<I> extra{{other32 ? indices : nullptr, eid32 ? eid : nullptr}, {other32, eid32}, (uint16_t*)clear.out,
                              (long long)(clear.bytes / 2), {fill.out[0], fill.out[1], fill.out[2]},
                              {fill.n[0], fill.n[1], fill.n[2]}, {fill.with[0], fill.with[1], fill.with[2]}};
-  // about one step of positions per block
+  // About one step of positions per block, fewer where that would leave most of the chip idle: below kExpandBlocks blocks
+  // the time is one block's chain of loads, and a shorter block has a shorter one.
+  constexpr long long kExpandBlocks = 3 * 148;
   long long per_block = C > 0 ? kExpandTile * C / E : 1;
+  if (C / kExpandBlocks < per_block) per_block = C / kExpandBlocks;
   per_block = per_block < 1 ? 1 : per_block > kExpandThreads ? kExpandThreads : per_block;
   long long blocks = C > 0 ? (C + per_block - 1) / per_block : 1;
   const long long copies = (other32 || eid32 || clear.out || fill.out[0]) ? (E + kExpandTile - 1) / kExpandTile : 1;

@@ -82,7 +82,7 @@ __device__ __forceinline__ void band_tiles(const int32_t* __restrict__ other, co
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int w = 1; w < kBandTileRows / 32; ++w) { lo = min(lo, s_lo[w]); hi = max(hi, s_hi[w]); }
-    if (hi >= lo) atomicMax(&verdict->max_span, hi - lo + 1);
+    if (hi >= lo && hi - lo + 1 > *(volatile const int*)&verdict->max_span) atomicMax(&verdict->max_span, hi - lo + 1);
   }
 }
 
@@ -185,7 +185,7 @@ inline int plan_build(const I* row, const I* indptr, const I* eid, const I* indi
   if (g.other && n_nodes > 0) {
     const unsigned tiles = (unsigned)((n_nodes + kBandTileRows - 1) / kBandTileRows);
     const long long rounds = (E + kBandTileRows - 1) / kBandTileRows;
-    plan_shape_kernel<kBandTileRows><<<tiles + (unsigned)(rounds < 2368 ? rounds : 2368), kBandTileRows, 0, st>>>(
+    plan_shape_kernel<kBandTileRows><<<tiles + (unsigned)(rounds < 592 ? rounds : 592), kBandTileRows, 0, st>>>(
         g.erow, g.other, E, first, deg, n_nodes, node_lo, verdict, tiles);
     GK_LAUNCHED("plan_shape");
   }

@@ -32,7 +32,9 @@ struct ChunkCount {
   __host__ __device__ long long operator()(long long r) const {
     if (r >= n) return 0;
     const long long deg = (long long)indptr[r + 1] - (long long)indptr[r];
-    return deg > 0 ? (deg + cs - 1) / cs : 0;   // range(a, b, cs) is empty when b <= a
+    if (deg <= 0) return 0;   // range(a, b, cs) is empty when b <= a
+    const long long top = deg + cs - 1;
+    return top <= 0xffffffffLL ? (unsigned)top / (unsigned)cs : top / cs;
   }
 };
 template <typename I>
