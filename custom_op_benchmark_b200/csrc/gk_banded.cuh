@@ -475,24 +475,29 @@ attention_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
 // ---------------------------------------------------------------------------------------------------------
 // Backward.  Two kernels with the forward's structure, one per side, so that every gradient row has one owner
 // (no atomics, as everywhere else):
-//   destination side, a tile of 128 query nodes:  S = Q K^T and dP = dO V^T per block of 128 keys,
+//   destination side, a tile of 128 query nodes:  S = Q K^T and dP = dO V^T per block of 64 keys,
 //       p = exp(scale S - lse), dS = p (dP - delta) scale,  dQ += dS K;   delta = dO . O is formed per row first
 //       and left, with lse, in `stat` for the other side;
-//   source side, a tile of 128 key nodes:  S^T = K Q^T and dP^T = V dO^T per block of 128 queries,
+//   source side, a tile of 128 key nodes:  S^T = K Q^T and dP^T = V dO^T per block of 64 queries,
 //       the same p and dS (transposed: a thread is a key, a column a query),  dV += P^T dO,  dK += dS^T Q.
-// Shared memory per tile: the four operand tiles, one 128 x 128 bf16 staging tile per product (32 KB each),
-// the queries' (lse, delta) pairs; tensor memory: 2 x 128 score columns and 64 per gradient.
+// A tile takes the blocks its band reaches, two of them in shared memory at a time: the next but one is asked for when the
+// gradient products that read its slot are done.  85 KB (destination side) or 101 KB (source side) of shared memory and
+// 256 tensor-memory columns, so that two tiles share an SM and one's products and loads run under the other's
+// element-wise stage: with the whole band and 128 x 128 staging tiles (one tile per SM) the tensor pipe was busy 9 to 13 %
+// of the time and every wait was exposed.
 // ---------------------------------------------------------------------------------------------------------
-constexpr int kBlocks = kSpan / kKeyBlock;   // blocks of 128 along the band
-constexpr int kStageBytes = 2 * kBlockBytes; // a 128 x 128 bf16 tile: two 64-column panels
+constexpr int kBThreads = 256;               // two threads per owned row: warp w works on lanes 32 (w % 4) .. + 31
+constexpr int kBGroups = kBThreads / kTileM; // and columns 32 (w / 4) .. + 31 of a block
+constexpr int kBKeys = 64;                   // rows of the band per block
+constexpr int kBBand = kBKeys * kRowBytes;   // 8 KB
+constexpr int kBSlots = 2;                   // blocks in shared memory
 
-// 32 columns of one 128 x 128 staging tile row: 4 chunks of 16 bytes at chunk (c & 1) * 4 + q of panel c >> 1
-__device__ __forceinline__ void store_stage_row(unsigned char* row_in_panel0, int c, int row, const uint32_t (&packed)[16]) {
-  unsigned char* panel = row_in_panel0 + (c >> 1) * kBlockBytes;
+// 32 columns of one 128 x 64 staging tile row: 4 chunks of 16 bytes at chunk c * 4 + q
+__device__ __forceinline__ void store_stage_row(unsigned char* row_at, int c, int row, const uint32_t (&packed)[16]) {
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    const int chunk = ((c & 1) * 4 + q) ^ (row & 7);
-    *reinterpret_cast<uint4*>(panel + chunk * 16) =
+    const int chunk = (c * 4 + q) ^ (row & 7);
+    *reinterpret_cast<uint4*>(row_at + chunk * 16) =
         make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
   }
 }
@@ -513,32 +518,36 @@ struct BwdParams {
 
 constexpr int kBOffA = 0;                          // owned tile, first operand (q | k)
 constexpr int kBOffB = kBOffA + kBlockBytes;       // owned tile, second operand (dO | v)
-constexpr int kBOffC = kBOffB + kBlockBytes;       // band, first operand (k | q)
-constexpr int kBOffD = kBOffC + kBlocks * kBlockBytes;   // band, second operand (v | dO)
-constexpr int kBOffS0 = kBOffD + kBlocks * kBlockBytes;  // staging tile 0 (dS | P^T)
-constexpr int kBOffS1 = kBOffS0 + kStageBytes;           // staging tile 1 (dS^T, source side)
-constexpr int kBOffStat = kBOffS1 + kStageBytes;         // (lse, delta) of the band's queries (source side)
-constexpr int kBOffBar = kBOffStat + kSpan * 8;
-constexpr int kBSmemBytes = kBOffBar + 128 + 1024;
+constexpr int kBOffC = kBOffB + kBlockBytes;       // band, per slot: first operand (k | q), second operand (v | dO)
+constexpr int kBOffS0 = kBOffC + kBSlots * 2 * kBBand;   // staging tile 0 (dS | P^T)
+constexpr int kBOffS1 = kBOffS0 + kBlockBytes;           // staging tile 1 (dS^T, source side)
+constexpr int kBOffBar = 0, kBOffStat = 128;             // behind the staging tiles: barriers, then the (lse, delta) of the
+                                                         // band's queries (source side) or the parts of delta
+__host__ __device__ constexpr int bwd_tail(bool src) { return kBOffS0 + (src ? 2 : 1) * kBlockBytes; }
+__host__ __device__ constexpr int bwd_smem(bool src) { return bwd_tail(src) + kBOffStat + (src ? kSpan * 8 : kBGroups * kTileM * 4) + 1024; }
+
+constexpr int kBTmemCols = 256;   // 64 columns each: scores, dP, two gradients
 
 // kSrc = false: destination side (owned = queries); true: source side (owned = keys)
 template <bool kSrc>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kBThreads, 2)
 attention_backward_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                           const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_d,
                           const BwdParams p) {
   extern __shared__ unsigned char raw_smem[];
   unsigned char* smem = raw_smem + ((1024u - (smem_u32(raw_smem) & 1023u)) & 1023u);
   const uint32_t s_base = smem_u32(smem);
-  // bar_load: the owned tiles and the band's first block; bar_more + 8 (b - 1): the band's block b
-  const uint32_t bar_load = s_base + kBOffBar, bar_s = bar_load + 8, bar_g = bar_load + 16, bar_more = bar_load + 64;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kBOffBar + 32);
-  int* s_red = reinterpret_cast<int*>(smem + kBOffBar + 40);
-  float2* s_stat = reinterpret_cast<float2*>(smem + kBOffStat);
-  float* s_part = reinterpret_cast<float*>(smem + kBOffStat);   // destination side: [column group][row] parts of delta
+  constexpr int kTail = bwd_tail(kSrc);
+  // bar_load: the owned tiles; bar_full + 8 (b % 2): the band's block b
+  const uint32_t bar_load = s_base + kTail + kBOffBar, bar_s = bar_load + 8, bar_g = bar_load + 16, bar_full = bar_load + 64;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kTail + kBOffBar + 32);
+  int* s_red = reinterpret_cast<int*>(smem + kTail + kBOffBar + 40);    // 4 ints: per-quarter minima of the first neighbour
+  int* s_top = reinterpret_cast<int*>(smem + kTail + kBOffBar + 96);    // 4 ints: and maxima of the last one
+  float2* s_stat = reinterpret_cast<float2*>(smem + kTail + kBOffStat);
+  float* s_part = reinterpret_cast<float*>(smem + kTail + kBOffStat);   // destination side: [column group][row] parts of delta
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int quarter = warp & 3, cg = warp >> 2;   // tensor-memory lane quarter; which 32 of a block's 128 columns
+  const int quarter = warp & 3, cg = warp >> 2;   // tensor-memory lane quarter; which 32 of a block's 64 columns
   const int row = quarter * 32 + lane;
   const int head = blockIdx.y;
   const long long r0 = (long long)blockIdx.x * kTileM;
@@ -548,21 +557,24 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     deg = p.node_deg[r];
     if (deg > 0) lo = p.node_lo[r];
   }
-  int wmin = lo;
+  int wmin = lo, wtop = deg > 0 ? lo + deg - 1 : -1;
 #pragma unroll
-  for (int o = 16; o; o >>= 1) wmin = min(wmin, __shfl_xor_sync(kFull, wmin, o));
-  if (lane == 0 && cg == 0) s_red[quarter] = wmin;
+  for (int o = 16; o; o >>= 1) {
+    wmin = min(wmin, __shfl_xor_sync(kFull, wmin, o));
+    wtop = max(wtop, __shfl_xor_sync(kFull, wtop, o));
+  }
+  if (lane == 0 && cg == 0) { s_red[quarter] = wmin; s_top[quarter] = wtop; }
   if (tid == 0) {
     mbar_init(bar_load, 1);
     mbar_init(bar_s, 1);
     mbar_init(bar_g, 1);
 #pragma unroll
-    for (int b = 1; b < kBlocks; ++b) mbar_init(bar_more + 8 * (b - 1), 1);
+    for (int b = 0; b < kBSlots; ++b) mbar_init(bar_full + 8 * b, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(kTmemCols)
+                 "r"(kBTmemCols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -572,32 +584,40 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
   const uint32_t tmem = *tmem_slot;
   const int bmin = min(min(s_red[0], s_red[1]), min(s_red[2], s_red[3]));   // first node of the band
   bool ok = true;
-  constexpr int kColS = 0, kColP = kKeyBlock, kColG0 = 2 * kKeyBlock, kColG1 = 2 * kKeyBlock + kD;
+  constexpr int kColS = 0, kColP = kBKeys, kColG0 = 2 * kBKeys, kColG1 = 2 * kBKeys + kD;
 
   if (bmin != INT_MAX) {
+    const int btop = max(max(s_top[0], s_top[1]), max(s_top[2], s_top[3]));
+    int nb = (btop - bmin) / kBKeys + 1;                    // blocks the tile's band reaches
+    nb = nb < kSpan / kBKeys ? nb : kSpan / kBKeys;
+    auto issue_band = [&](int b) {   // one thread
+      const uint32_t bar = bar_full + 8 * (b & 1), at = s_base + kBOffC + (b & 1) * 2 * kBBand;
+      mbar_expect_tx(bar, (uint32_t)(2 * kBBand));
+      tma_load_3d(at, &map_c, bar, 0, head, bmin + b * kBKeys);
+      tma_load_3d(at + kBBand, &map_d, bar, 0, head, bmin + b * kBKeys);
+    };
     if (tid == 0) {
-      mbar_expect_tx(bar_load, (uint32_t)(kBlockBytes * 4));
-      tma_load_3d(s_base + kBOffA, &map_a, bar_load, 0, head, (int)r0);
-      tma_load_3d(s_base + kBOffB, &map_b, bar_load, 0, head, (int)r0);
+      mbar_expect_tx(bar_load, (uint32_t)(kBlockBytes * 2));
 #pragma unroll
-      for (int b = 0; b < kBlocks; ++b) {   // later blocks land while the first is worked on
-        const uint32_t bar = b == 0 ? bar_load : bar_more + 8 * (b - 1);
-        if (b > 0) mbar_expect_tx(bar, (uint32_t)(kBlockBytes * 2));
-        tma_load_3d(s_base + kBOffC + b * kBlockBytes, &map_c, bar, 0, head, bmin + b * kKeyBlock);
-        tma_load_3d(s_base + kBOffD + b * kBlockBytes, &map_d, bar, 0, head, bmin + b * kKeyBlock);
+      for (int half = 0; half < 2; ++half) {
+        tma_load_3d(s_base + kBOffA + half * kBBand, &map_a, bar_load, 0, head, (int)r0 + half * kBKeys);
+        tma_load_3d(s_base + kBOffB + half * kBBand, &map_b, bar_load, 0, head, (int)r0 + half * kBKeys);
       }
+      issue_band(0);
+      if (nb > 1) issue_band(1);
     }
+    int issued = nb < kBSlots ? nb : kBSlots;
     // per-row scalars while the tiles travel
     float lse2 = 0.f, delta = 0.f, lrow = 0.f;
     const float kL2e = 1.4426950408889634f;
     if constexpr (!kSrc) {
-      // delta = <o, dO> of the row: each of its four threads takes 16 of the 64 features
+      // delta = <o, dO> of the row: each of its two threads takes 32 of the 64 features
       float part = 0.f;
       if (r < p.n_own) {
-        const uint4* orow = reinterpret_cast<const uint4*>(p.o + ((long long)r * p.H + head) * kD) + cg * 2;
-        const uint4* grow = reinterpret_cast<const uint4*>(p.d_o + ((long long)r * p.H + head) * kD) + cg * 2;
+        const uint4* orow = reinterpret_cast<const uint4*>(p.o + ((long long)r * p.H + head) * kD) + cg * 4;
+        const uint4* grow = reinterpret_cast<const uint4*>(p.d_o + ((long long)r * p.H + head) * kD) + cg * 4;
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
+        for (int q = 0; q < 4; ++q) {
           const uint4 ov = __ldg(orow + q), gv = __ldg(grow + q);
           const __nv_bfloat162* o2 = reinterpret_cast<const __nv_bfloat162*>(&ov);
           const __nv_bfloat162* g2 = reinterpret_cast<const __nv_bfloat162*>(&gv);
@@ -613,15 +633,15 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
       s_part[cg * kTileM + row] = part;
     } else {
       // (lse, delta) of the band's queries: column j of the scores is query bmin + j
-      for (int i = tid; i < kSpan; i += kThreads) {
+      for (int i = tid; i < nb * kBKeys; i += kBThreads) {
         const long long qn = (long long)bmin + i;
         s_stat[i] = qn < p.n_other ? p.stat[qn * p.H + head] : make_float2(0.f, 0.f);
       }
     }
-    ok = __syncthreads_and(mbar_wait(bar_load, 0));
+    ok = __syncthreads_and(mbar_wait(bar_load, 0) && mbar_wait(bar_full, 0));
     if constexpr (!kSrc) {
 #pragma unroll
-      for (int g = 0; g < kColGroups; ++g) delta += s_part[g * kTileM + row];   // the same order in all four threads
+      for (int g = 0; g < kBGroups; ++g) delta += s_part[g * kTileM + row];   // the same order in both threads
       if (cg == 0 && r < p.n_own) p.stat[(long long)r * p.H + head] = make_float2(lrow, delta);
     }
 
@@ -639,17 +659,15 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
 
     // scores and dP of one block of the band: owned operands x the band's block (issued by one thread)
     auto issue_scores = [&](int b) {
-      constexpr uint32_t idesc = umma_idesc(kTileM, kKeyBlock, false);
+      constexpr uint32_t idesc = umma_idesc(kTileM, kBKeys, false);
+      const uint32_t at = s_base + kBOffC + (b & 1) * 2 * kBBand;
 #pragma unroll
-      for (int kk = 0; kk < kD / 16; ++kk) {   // scores: owned first operand x band first operand
-        umma_f16(tmem + kColS, umma_desc(s_base + kBOffA + kk * 32, 16, 1024),
-                 umma_desc(s_base + kBOffC + b * kBlockBytes + kk * 32, 16, 1024), idesc, kk > 0);
-      }
+      for (int kk = 0; kk < kD / 16; ++kk)   // scores: owned first operand x band first operand
+        umma_f16(tmem + kColS, umma_desc(s_base + kBOffA + kk * 32, 16, 1024), umma_desc(at + kk * 32, 16, 1024), idesc, kk > 0);
 #pragma unroll
-      for (int kk = 0; kk < kD / 16; ++kk) {   // dP: owned second operand x band second operand
-        umma_f16(tmem + kColP, umma_desc(s_base + kBOffB + kk * 32, 16, 1024),
-                 umma_desc(s_base + kBOffD + b * kBlockBytes + kk * 32, 16, 1024), idesc, kk > 0);
-      }
+      for (int kk = 0; kk < kD / 16; ++kk)   // dP: owned second operand x band second operand
+        umma_f16(tmem + kColP, umma_desc(s_base + kBOffB + kk * 32, 16, 1024), umma_desc(at + kBBand + kk * 32, 16, 1024),
+                 idesc, kk > 0);
     };
     if (ok && tid == 0) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -659,13 +677,17 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     // Per block one wait: the gradient products of block b and the score products of block b + 1 are issued back to
     // back behind one commit (every thread has read block b's scores by then, and the tensor core runs them in
     // order), so when block b + 1's scores are there the staging tiles are free as well.
-    for (int b = 0; b < kBlocks; ++b) {
+    for (int b = 0; b < nb; ++b) {
       ok = __syncthreads_and(ok && mbar_wait(bar_s, b & 1));
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (ok && b > 0 && b + 1 < nb) {   // block b - 1's slot is free: its gradient products were before block b's scores
+        if (tid == 0) issue_band(b + 1);
+        issued = b + 2;
+      }
 
       {
-        const int c = cg;   // this thread's 32 of the block's 128 columns
-        const int col0 = b * kKeyBlock + c * 32;
+        const int c = cg;   // this thread's 32 of the block's 64 columns
+        const int col0 = b * kBKeys + c * 32;
         const bool live = ok && col0 <= whi && col0 + 31 >= wlo;   // warp-uniform
         uint32_t pk0[16], pk1[16];
         if (live) {
@@ -704,24 +726,22 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       // the staging tiles are written by all, and the next block of the band has landed
-      ok = __syncthreads_and(ok && (b + 1 >= kBlocks || mbar_wait(bar_more + 8 * b, 0)));
+      ok = __syncthreads_and(ok && (b + 1 >= nb || mbar_wait(bar_full + 8 * ((b + 1) & 1), ((b + 1) >> 1) & 1)));
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (ok && tid == 0) {
         constexpr uint32_t idesc = umma_idesc(kTileM, kD, true);
+        const uint32_t at = s_base + kBOffC + (b & 1) * 2 * kBBand;
 #pragma unroll
-        for (int ks = 0; ks < kKeyBlock / 16; ++ks) {
-          const uint32_t a_off = (ks >> 2) * kBlockBytes + (ks & 3) * 32;
+        for (int ks = 0; ks < kBKeys / 16; ++ks) {
+          const uint64_t a0 = umma_desc(s_base + kBOffS0 + ks * 32, 16, 1024), c0 = umma_desc(at + ks * 16 * kRowBytes, 16, 1024);
           if constexpr (!kSrc) {   // dQ += dS K_b
-            umma_f16(tmem + kColG0, umma_desc(s_base + kBOffS0 + a_off, 16, 1024),
-                     umma_desc(s_base + kBOffC + b * kBlockBytes + ks * 16 * kRowBytes, 16, 1024), idesc, (b | ks) != 0);
+            umma_f16(tmem + kColG0, a0, c0, idesc, (b | ks) != 0);
           } else {                 // dV += P^T dO_b,  dK += dS^T Q_b
-            umma_f16(tmem + kColG1, umma_desc(s_base + kBOffS0 + a_off, 16, 1024),
-                     umma_desc(s_base + kBOffD + b * kBlockBytes + ks * 16 * kRowBytes, 16, 1024), idesc, (b | ks) != 0);
-            umma_f16(tmem + kColG0, umma_desc(s_base + kBOffS1 + a_off, 16, 1024),
-                     umma_desc(s_base + kBOffC + b * kBlockBytes + ks * 16 * kRowBytes, 16, 1024), idesc, (b | ks) != 0);
+            umma_f16(tmem + kColG1, a0, umma_desc(at + kBBand + ks * 16 * kRowBytes, 16, 1024), idesc, (b | ks) != 0);
+            umma_f16(tmem + kColG0, umma_desc(s_base + kBOffS1 + ks * 32, 16, 1024), c0, idesc, (b | ks) != 0);
           }
         }
-        if (b + 1 < kBlocks) {
+        if (b + 1 < nb) {
           issue_scores(b + 1);
           umma_commit(bar_s);
         } else {
@@ -732,15 +752,17 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     ok = __syncthreads_and(ok && mbar_wait(bar_g, 0));   // the last block's gradient products
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
-    // gradients of the owned rows: this thread's 16 of the 64 features
-    {
+    // gradients of the owned rows: this thread's 32 of the 64 features
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int f0 = cg * 32 + half * 16;
       float g0[16], g1[16];
       if (ok) {
-        tmem_ld16(row_taddr + kColG0 + cg * 16, g0);
-        if constexpr (kSrc) tmem_ld16(row_taddr + kColG1 + cg * 16, g1);
+        tmem_ld16(row_taddr + kColG0 + f0, g0);
+        if constexpr (kSrc) tmem_ld16(row_taddr + kColG1 + f0, g1);
       }
       if (r < p.n_own) {
-        const long long at = ((long long)r * p.H + head) * kD + cg * 16;
+        const long long at = ((long long)r * p.H + head) * kD + f0;
         const float keep = deg > 0 ? 1.f : 0.f;
         if (ok && deg == 0) {
 #pragma unroll
@@ -749,6 +771,10 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
         store_out16(p.out0 + at, g0, keep, ok);
         if constexpr (kSrc) store_out16(p.out1 + at, g1, keep, ok);
       }
+    }
+    if (!ok) {   // a wait ran out: loads asked for are given (bounded) time to land before the shared memory is handed back
+      mbar_wait(bar_load, 0);
+      for (int b = issued > kBSlots ? issued - kBSlots : 0; b < issued; ++b) mbar_wait(bar_full + 8 * (b & 1), (b >> 1) & 1);
     }
   } else if (r < p.n_own && cg == 0) {  // no owned node of the tile has a neighbour: zero gradients
     const long long at = ((long long)r * p.H + head) * kD;
@@ -763,7 +789,7 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kBTmemCols) : "memory");
   }
 }
 
@@ -780,13 +806,13 @@ inline PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   return fn;
 }
 
-// (n, H, 64) bf16 node tensor as a 3-D map (feature, head, node), boxes of 128 nodes of one head, 128-byte swizzle
-inline bool make_map(CUtensorMap* map, const void* base, long long n, int H) {
+// (n, H, 64) bf16 node tensor as a 3-D map (feature, head, node), boxes of `nodes` nodes of one head, 128-byte swizzle
+inline bool make_map(CUtensorMap* map, const void* base, long long n, int H, int nodes) {
   auto fn = encode_fn();
   if (!fn) return false;
   const cuuint64_t dims[3] = {(cuuint64_t)kD, (cuuint64_t)H, (cuuint64_t)n};
   const cuuint64_t strides[2] = {(cuuint64_t)kRowBytes, (cuuint64_t)H * kRowBytes};
-  const cuuint32_t box[3] = {(cuuint32_t)kD, 1u, (cuuint32_t)kKeyBlock};
+  const cuuint32_t box[3] = {(cuuint32_t)kD, 1u, (cuuint32_t)nodes};
   const cuuint32_t estr[3] = {1u, 1u, 1u};
   return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -806,7 +832,7 @@ inline int banded_attention_forward<__nv_bfloat16>(const graphop_plan_t* plan, c
     return GRAPHOP_ERR_UNSUPPORTED;
   if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)o) & 15) return GRAPHOP_ERR_UNSUPPORTED;
   CUtensorMap mq, mk, mv;
-  if (!make_map(&mq, q, n_dst, H) || !make_map(&mk, k, n_src, H) || !make_map(&mv, v, n_src, H))
+  if (!make_map(&mq, q, n_dst, H, kTileM) || !make_map(&mk, k, n_src, H, kKeyBlock) || !make_map(&mv, v, n_src, H, kKeyBlock))
     return GRAPHOP_ERR_UNSUPPORTED;
   static std::atomic<bool> configured[64];
   int dev = 0;
@@ -850,27 +876,27 @@ inline int banded_attention_backward<__nv_bfloat16>(const graphop_plan_t* plan_r
   GK_TRY(check_ws(ws));
   if (wsb < (size_t)n_dst * H * sizeof(float2)) return GRAPHOP_ERR_WORKSPACE;
   CUtensorMap mq, mk, mv, mg;
-  if (!make_map(&mq, q, n_dst, H) || !make_map(&mk, k, n_src, H) || !make_map(&mv, v, n_src, H) ||
-      !make_map(&mg, d_o, n_dst, H))
+  if (!make_map(&mq, q, n_dst, H, kBKeys) || !make_map(&mk, k, n_src, H, kBKeys) || !make_map(&mv, v, n_src, H, kBKeys) ||
+      !make_map(&mg, d_o, n_dst, H, kBKeys))
     return GRAPHOP_ERR_UNSUPPORTED;
   static std::atomic<bool> configured[64];
   int dev = 0;
   GK_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64 || !configured[dev].load(std::memory_order_acquire)) {
-    GK_CUDA(cudaFuncSetAttribute(attention_backward_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBSmemBytes));
-    GK_CUDA(cudaFuncSetAttribute(attention_backward_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBSmemBytes));
+    GK_CUDA(cudaFuncSetAttribute(attention_backward_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bwd_smem(false)));
+    GK_CUDA(cudaFuncSetAttribute(attention_backward_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bwd_smem(true)));
     if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
   }
   BwdParams p;
   p.o = o; p.d_o = d_o; p.lse = (const float*)lse; p.stat = (float2*)ws; p.H = H; p.scale = (float)scale;
   p.out0 = dq; p.out1 = nullptr; p.node_lo = plan_r->node_lo; p.node_deg = plan_r->node_deg; p.n_own = n_dst;
   p.n_other = n_src;
-  attention_backward_kernel<false><<<dim3((unsigned)((n_dst + kTileM - 1) / kTileM), (unsigned)H), kThreads, kBSmemBytes,
+  attention_backward_kernel<false><<<dim3((unsigned)((n_dst + kTileM - 1) / kTileM), (unsigned)H), kBThreads, bwd_smem(false),
                                      st>>>(mq, mg, mk, mv, p);
   GK_LAUNCHED("attention_bwd_dst_banded");
   p.out0 = dk; p.out1 = dv; p.node_lo = plan_t->node_lo; p.node_deg = plan_t->node_deg; p.n_own = n_src;
   p.n_other = n_dst;
-  attention_backward_kernel<true><<<dim3((unsigned)((n_src + kTileM - 1) / kTileM), (unsigned)H), kThreads, kBSmemBytes,
+  attention_backward_kernel<true><<<dim3((unsigned)((n_src + kTileM - 1) / kTileM), (unsigned)H), kBThreads, bwd_smem(true),
                                     st>>>(mk, mv, mq, mg, p);
   GK_LAUNCHED("attention_bwd_src_banded");
   return GRAPHOP_OK;
