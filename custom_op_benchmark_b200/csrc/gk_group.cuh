@@ -224,20 +224,26 @@ struct FeatGeo : Geo<T_, 16, G_, W_, G_> {
 // Launch shape of an op with kRows operand rows per ring step.  One warp per block: warps are independent and their tiles
 // take different times, a block of several would hold its slot until the slowest is done.
 // A ring step holds kRows operand rows of a position's edge and, should a node begin there, kNode rows and kNodeScalar bytes
-// per lane of it; kScalar bytes per edge and head wait in a table; kState fragments of W slots live in a lane's registers.
-template <class GEO, int kRows, int kScalar, int kState, int kNode, int kNodeScalar, int kU>
+// per lane of it.  kShare: the kUnroll steps of an iteration have room for one node together (a second one, after a node of
+// one edge, is fetched when its turn comes), where a room per step would leave too few warps.  kScalar bytes per edge and head wait in a table; kState fragments of W slots live in a lane's registers.
+template <class GEO, int kRows, int kScalar, int kState, int kNode, int kNodeScalar, int kU, bool kShare = false>
 struct Shape {
   static constexpr int kWarps = 1;
-  static constexpr int kNodeAt = kRows * GEO::kRow;
-  static constexpr int kNodeScalarAt = kNode * GEO::kRow;                  // from kNodeAt
-  static constexpr int kStepBytes = kNodeAt + kNodeScalarAt + 32 * kNodeScalar;
+  static constexpr int kStepBytes = kRows * GEO::kRow;
+  static constexpr int kNodeScalarAt = kNode * GEO::kRow;                  // from the node's room
   // Positions folded per iteration: two share the loop, the waits and the checks and give the scheduler two independent
   // chains; one where the step's rows or the registers would leave too few warps.  Two iterations are in flight.
   static constexpr int kUnroll = GEO::W <= 2 || GEO::kAllHeads ? kU : 1;
   static constexpr int kDepth = 2 * kUnroll;
+  static constexpr int kNodeAt = kUnroll * kStepBytes;                     // from the iteration's first step
+  static constexpr int kNodeBytes = kNodeScalarAt + 32 * kNodeScalar;
+  static constexpr bool kShareNode = kShare && kUnroll > 1;
+  static constexpr int kIterBytes = kNodeAt + (kShareNode ? 1 : kUnroll) * kNodeBytes;
+  // where the node that begins at step v waits
+  __device__ __forceinline__ static constexpr unsigned node_at(int v) { return kNodeAt + (kShareNode ? 0 : v * kNodeBytes); }
   static constexpr int kScalarBytes = kScalar;
   static constexpr int kTable = 32 * GEO::kHeads * kScalar;                // one block of positions
-  static constexpr int kWarpBytes = kDepth * kStepBytes + 2 * kTable;
+  static constexpr int kWarpBytes = 2 * kIterBytes + 2 * kTable;
   static constexpr bool kNodeRows = kNode > 0;
   static constexpr int kFit = 226 * 1024 / (kWarps * kWarpBytes + 1024);   // blocks the shared memory allows
   static constexpr int kWords = GEO::W * GEO::V * (int)sizeof(typename GEO::A) / 4;
@@ -261,7 +267,7 @@ struct Shape {
 template <class Op>
 __global__ void __launch_bounds__(Op::kWarps * 32, Op::kMinCtas)
 group_walk_kernel(const __grid_constant__ Op op, const __grid_constant__ WalkArgs a) {
-  constexpr int NE = Op::NE, G = Op::G, DS = Op::kDepth, CH = G / DS, STEP = Op::kStepBytes, U = Op::kUnroll;   // CH ring turns per G positions
+  constexpr int NE = Op::NE, G = Op::G, DS = Op::kDepth, CH = G / DS, STEP = Op::kStepBytes, ITER = Op::kIterBytes, U = Op::kUnroll;   // CH ring turns per G positions
   static_assert(CH * DS == G, "whole ring turns per block of positions");
   constexpr unsigned kOneLane = NE == 1 ? 1u : NE == 2 ? 0x00010001u : NE == 4 ? 0x01010101u : 0x11111111u;
   constexpr bool kOut = Op::kRowOut;
@@ -341,10 +347,13 @@ group_walk_kernel(const __grid_constant__ Op op, const __grid_constant__ WalkArg
     if constexpr (Op::kNodeRows) {
       const unsigned m = starts >> i;
       if (m & (((1u << U) - 1u) * kOneLane)) {
+        bool taken = false;
 #pragma unroll
         for (int v = 0; v < U; ++v) {
           const int rr = __shfl_sync(kFull, r, i + v, G);
-          if (((m >> (g * G + v)) & 1u) && rr >= 0) op.stage_node(st, slot + v * STEP + Op::kNodeAt, lane, rr);
+          const bool begins = ((m >> (g * G + v)) & 1u) && rr >= 0;
+          if (begins && !(Op::kShareNode && taken)) op.stage_node(st, slot + Op::node_at(v), lane, rr);
+          taken = taken || begins;
         }
       }
     }
@@ -353,7 +362,7 @@ group_walk_kernel(const __grid_constant__ Op op, const __grid_constant__ WalkArg
   // The scalars of a block of positions, one position per lane: asked for while the block before it is folded, read
   // by all lanes of the group afterwards.  cp.async moves 4 bytes at least: 2-byte scalars wait in registers meanwhile.
   constexpr int SC = Op::kScalarBytes, TB = Op::kTable, ENTRY = Op::kHeads * SC;
-  const unsigned table = ring - lane * Op::SB + DS * STEP;
+  const unsigned table = ring - lane * Op::SB + 2 * ITER;
   uint16_t held[SC == 2 ? Op::kHeads : 1];
   auto fetch_scalars = [&](unsigned tab, int o, int e) {
     if constexpr (SC > 0) {
@@ -380,7 +389,7 @@ group_walk_kernel(const __grid_constant__ Op op, const __grid_constant__ WalkArg
   const unsigned my_scalar = table + g * G * ENTRY + (SC > 0 ? op.scalar_at(gl) * SC : 0);
   static_assert(DS == 2 * U, "two iterations in flight");
   stage_some(ring, 0, r0, o0, e0, starts0);
-  stage_some(ring + U * STEP, U, r0, o0, e0, starts0);
+  stage_some(ring + ITER, U, r0, o0, e0, starts0);
 
   const int first = __shfl_sync(kFull, r0, 0, G);
   const bool head_open = before >= 0 && before == first;
@@ -412,7 +421,7 @@ group_walk_kernel(const __grid_constant__ Op op, const __grid_constant__ WalkArg
       // one copy of the code for every two steps: with the ring unrolled the loop missed the instruction cache
       unsigned slot = ring;
 #pragma unroll 1
-      for (int i = c * DS; i < c * DS + DS; i += U, slot += U * STEP) {
+      for (int i = c * DS; i < c * DS + DS; i += U, slot += ITER) {
         const int p = b * G + i;
         cp_async_wait<DS / U - 1>();
         const unsigned m = (starts0 >> i) & (((1u << U) - 1u) * kOneLane);
@@ -426,12 +435,22 @@ group_walk_kernel(const __grid_constant__ Op op, const __grid_constant__ WalkArg
           }
           op.template fold<U>(st, slot, tab0 + i * ENTRY, act, (int)j0 + p, ed);
         } else {
+          [[maybe_unused]] bool taken = false;   // the iteration's room for a node held an earlier one
 #pragma unroll 1
           for (int v = 0; v < U; ++v) {
             const unsigned mv = m >> v;
             if (mv & kOneLane) {   // some group's node ends here and another begins
               const int r = __shfl_sync(kFull, r0, i + v, G);
               const bool mine = ((mv >> (g * G)) & 1u) && r > -2;
+              if constexpr (Op::kShareNode) {
+                const bool late = mine && r >= 0 && taken;
+                if (__any_sync(kFull, late)) {
+                  if (late) op.stage_node(st, slot + Op::node_at(v), lane, r);
+                  cp_async_commit();
+                  cp_async_wait<0>();
+                }
+                taken = taken || (mine && r >= 0);
+              }
               if (mine) {
                 if constexpr (kOut) {
                   if (cur >= 0) {
@@ -451,7 +470,7 @@ group_walk_kernel(const __grid_constant__ Op op, const __grid_constant__ WalkArg
                     last_valid = r;
                   }
                 }
-                if (r >= 0) op.begin(st, slot + v * STEP + Op::kNodeAt, lane);
+                if (r >= 0) op.begin(st, slot + Op::node_at(v), lane);
                 cur = r;
                 lim = r >= 0 ? n : 0;
               }
@@ -910,8 +929,11 @@ struct GroupAttnFwd : GEO, Shape<GEO, kBias ? 3 : 2, 0, 2, 1, 0, 2> {
 
 // Fused attention backward, destination side: dq[node] = sum ds (k + rel), ds = p (dO.v - delta) scale; writes
 // (lse, delta) per node and, pd != null, (p, ds) per position and head for the source side.
+// Two positions per iteration pay for 2-byte elements (R-MAT 18, 4 x 64 bf16 with the edge term: 1.19 -> 1.02 ms); for
+// wider ones they leave fewer warps (R-MAT 21, 4 x 32 fp32: 4.64 -> 4.49 ms, but 4096 nodes, 8 x 64: 35 -> 39 us).
 template <class GEO, bool kBias>
-struct GroupAttnBwdDst : GEO, Shape<GEO, kBias ? 3 : 2, 0, 4, 3, (int)sizeof(typename GEO::A), 1> {
+struct GroupAttnBwdDst : GEO, Shape<GEO, kBias ? 3 : 2, 0, 4, 3, (int)sizeof(typename GEO::A),
+                                (sizeof(typename GEO::T) == 2 ? 2 : 1), true> {
   using T = typename GEO::T;
   using A = typename GEO::A;
   using F = typename GEO::F;

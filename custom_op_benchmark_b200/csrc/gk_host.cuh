@@ -348,7 +348,7 @@ inline int run_aggregate(Arena& ar, const GraphView& g, const T* w, const T* x, 
   }
   const GeoPick p = pick_geo(H, D, sizeof(T), slot_align_of({x, y}), true);
   if (p.SB && p.nhb <= kMaxHeadBlocks)
-    return dispatch_geo<T, true>(p, [&](auto tag) -> int {
+    return dispatch_geo<T, true, false>(p, [&](auto tag) -> int {
       GroupAggregate<typename decltype(tag)::type, kEdgeFeat> op;
       fill_geo(op, p, H, D);
       op.w = w; op.x = x; op.y = y;
@@ -389,7 +389,7 @@ inline int run_edge_dot(Arena& ar, const GraphView& g, const T* a, const T* b, T
   }
   const GeoPick p = narrow_fix(pick_geo(H, D, sizeof(T), slot_align_of({a, b}), false));
   if (p.SB && p.nhb <= kMaxHeadBlocks)
-    return dispatch_geo<T, true>(p, [&](auto tag) -> int {
+    return dispatch_geo<T, true, true>(p, [&](auto tag) -> int {
       GroupEdgeDot<typename decltype(tag)::type, kEdgeFeat> op;
       fill_geo(op, p, H, D);
       op.a = a; op.b = b; op.y = y;
@@ -647,7 +647,7 @@ template <typename T, bool kBias>
 inline int run_attn_forward(Arena& ar, const GraphView& g, const GeoPick& s, const T* q, const T* k, const T* v,
                             const T* rel, double scale, T* o, void* lse, long long n_dst, int H, int D,
                             cudaStream_t st) {
-  return dispatch_geo<T, false>(s, [&](auto tag) -> int {
+  return dispatch_geo<T, false, true>(s, [&](auto tag) -> int {
     GroupAttnFwd<typename decltype(tag)::type, kBias> op;
     using A = typename decltype(op)::A;
     fill_geo(op, s, H, D);
@@ -659,7 +659,7 @@ template <typename T, bool kBias, class A>
 inline int run_attn_bwd_dst(Arena& ar, const GraphView& g, const GeoPick& s, const T* q, const T* k, const T* v,
                             const T* rel, const T* o, const T* dout, const void* lse, StatPair<A>* stat,
                             EdgePair<A>* pd, double scale, T* dq, long long n_dst, int H, int D, cudaStream_t st) {
-  return dispatch_geo<T, false>(s, [&](auto tag) -> int {
+  return dispatch_geo<T, false, true>(s, [&](auto tag) -> int {
     GroupAttnBwdDst<typename decltype(tag)::type, kBias> op;
     fill_geo(op, s, H, D);
     op.q = q; op.k = k; op.v = v; op.rel = rel; op.o = o; op.dout = dout; op.lse = (const A*)lse; op.stat = stat;
@@ -671,7 +671,7 @@ template <typename T, bool kPairs, class A>
 inline int run_attn_bwd_src(Arena& ar, const GraphView& g, const GeoPick& s, const T* q, const T* k, const T* v,
                             const T* dout, const StatPair<A>* stat, const EdgePair<A>* pd, double scale, T* dk, T* dv,
                             long long n_src, int H, int D, cudaStream_t st) {
-  return dispatch_geo<T, false>(s, [&](auto tag) -> int {
+  return dispatch_geo<T, false, true>(s, [&](auto tag) -> int {
     GroupAttnBwdSrc<typename decltype(tag)::type, kPairs> op;
     fill_geo(op, s, H, D);
     op.q = q; op.k = k; op.v = v; op.dout = dout; op.stat = stat; op.pd = pd; op.dk = dk; op.dv = dv;

@@ -71,9 +71,10 @@ constexpr int kMaxHeadBlocks = 65535;   // grid.y
 
 template <class X> struct TypeTag { using type = X; };
 
-// Calls f(TypeTag<Geo<...>>) for the geometry.  kNarrowSlots: slots of 8 and 4 bytes are instantiated too.  The
+// Calls f(TypeTag<Geo<...>>) for the geometry.  kNarrowSlots: slots of 8 and 4 bytes are instantiated too; kWide: heads of more
+// than 32 slots (an op that may split them never has one).  A whole warp with one slot per lane is for 2-byte elements.  The
 // compile-time lane counts cover the heads of 16 to 128 features of the common shapes; every other one reads L.
-template <typename T, bool kNarrowSlots, class F>
+template <typename T, bool kNarrowSlots, bool kWide, class F>
 inline int dispatch_geo(const GeoPick& p, F&& f) {
 #define GK_GEO(SB_, G_, W_, LT_) \
   if (p.SB == SB_ && p.G == G_ && p.W == W_ && (LT_ == 0 || p.LT == LT_)) return f(TypeTag<Geo<T, SB_, G_, W_, LT_>>{});
@@ -95,8 +96,8 @@ inline int dispatch_geo(const GeoPick& p, F&& f) {
       GK_GEO(16, 16, 1, 16)
     }
   }
-  GK_GEO(16, 32, 1, 0)
   if constexpr (sizeof(T) == 2) {
+    GK_GEO(16, 32, 1, 0)
     GK_GEO(16, 16, 1, 0)
   } else {
     GK_GEO(16, 16, 2, 0)
@@ -104,11 +105,14 @@ inline int dispatch_geo(const GeoPick& p, F&& f) {
   }
   GK_GEO(16, 8, 1, 0)
   GK_GEO(16, 4, 1, 0)
-  GK_GEO(16, 32, 2, 0)
-  GK_GEO(16, 32, 4, 0)
-  GK_GEO(16, 32, 8, 0)
+  if constexpr (kWide) {
+    GK_GEO(16, 32, 2, 0)
+    GK_GEO(16, 32, 4, 0)
+    GK_GEO(16, 32, 8, 0)
+  }
   if constexpr (kNarrowSlots) {
     if constexpr (sizeof(T) == 2) {
+      GK_GEO(8, 32, 1, 0)
       GK_GEO(8, 16, 1, 0)
     } else {
       GK_GEO(8, 16, 2, 0)
@@ -116,11 +120,13 @@ inline int dispatch_geo(const GeoPick& p, F&& f) {
     }
     GK_GEO(8, 8, 1, 0)
     GK_GEO(8, 4, 1, 0)
-    GK_GEO(8, 32, 1, 0)
-    GK_GEO(8, 32, 2, 0)
-    GK_GEO(8, 32, 8, 0)
+    if constexpr (kWide) {
+      GK_GEO(8, 32, 2, 0)
+      GK_GEO(8, 32, 8, 0)
+    }
     if constexpr (sizeof(T) <= 4) {
       if constexpr (sizeof(T) == 2) {
+        GK_GEO(4, 32, 1, 0)
         GK_GEO(4, 16, 1, 0)
       } else {
         GK_GEO(4, 16, 2, 0)
@@ -128,9 +134,10 @@ inline int dispatch_geo(const GeoPick& p, F&& f) {
       }
       GK_GEO(4, 8, 1, 0)
       GK_GEO(4, 4, 1, 0)
-      GK_GEO(4, 32, 1, 0)
-      GK_GEO(4, 32, 2, 0)
-      GK_GEO(4, 32, 8, 0)
+      if constexpr (kWide) {
+        GK_GEO(4, 32, 2, 0)
+        GK_GEO(4, 32, 8, 0)
+      }
     }
   }
 #undef GK_GEO
