@@ -7,17 +7,14 @@
 // pair per node, and the chain
 //     scores = Q K^T on the band,  P = softmax(scale * scores),  O = P V
 // is two small dense matrix products per tile of 128 query nodes and head:
-//   * TMA (cp.async.bulk.tensor, 128-byte swizzle, no multicast) brings the tile's 128 q rows and the up to 384 k and v
-//     rows its band reaches into shared memory;
-//   * tcgen05.mma (kind::f16, bf16 in, fp32 out) forms the 128 x 384 scores in tensor memory;
-//   * four threads share a query row (512 threads per tile: enough warps to hide the latency of this stage): each
-//     reads every fourth 32-column chunk of the row from tensor memory (tcgen05.ld), masks the columns outside its
-//     node's range, takes max and sum (combined over the four through shared memory), and writes the probabilities
-//     as bf16 into shared memory;
-//   * a second tcgen05.mma chain multiplies them with V; each thread scales 16 of the row's 64 outputs by 1 / sum
-//     and stores them.
-// Everything a tile needs lives on chip: 208 KB of shared memory and 448 of the 512 tensor-memory columns; one block
-// per SM walks its share of the tiles and loads the next tile's operands while the current tile's softmax runs.
+//   * TMA (cp.async.bulk.tensor, 128-byte swizzle, no multicast) brings the tile's 128 q rows and, block by block of 64,
+//     the k and v rows its band reaches into shared memory;
+//   * tcgen05.mma (kind::f16, bf16 in, fp32 out) forms the block's 128 x 64 scores in tensor memory;
+//   * two threads share a query row: each reads 32 of the block's columns from tensor memory (tcgen05.ld), masks those
+//     outside its node's range and writes the probabilities, relative to a running maximum, as bf16 into shared memory;
+//   * a second tcgen05.mma adds their product with v to the tile's output in tensor memory, which is rescaled where a
+//     row's maximum has grown by more than 2^8; at the end each thread scales 32 of the row's 64 outputs by 1 / sum.
+// Several tiles share an SM, so that one's loads and products run under the others' element-wise stages.
 // Every wait on an mbarrier is bounded; a tile whose wait runs out writes NaN to its rows of O instead of hanging.
 #pragma once
 #include <cuda.h>
@@ -32,24 +29,23 @@ namespace gk {
 namespace banded {
 
 constexpr int kTileM = 128;                 // nodes per block = tensor-memory lanes
-constexpr int kColGroups = 4;               // threads per node row: each takes every fourth 32-column chunk
-constexpr int kThreads = kTileM * kColGroups;   // 16 warps: warp w works on lanes 32 (w % 4) .. + 31, chunks w / 4 + 4 i
+constexpr int kThreads = 256;               // two threads per node row: warp w works on lanes 32 (w % 4) .. + 31 and
+constexpr int kColGroups = kThreads / kTileM;   // columns 32 (w / 4) .. + 31 of a block
 constexpr int kD = 64;                      // features per head: one 128-byte swizzle row of bf16
 constexpr int kSpan = GRAPHOP_BAND_MAX_SPAN;  // key rows a tile reaches at most
-constexpr int kKeyBlock = 128;              // key rows per TMA box and per score MMA
 constexpr int kRowBytes = kD * 2;           // 128
-constexpr int kBlockBytes = kKeyBlock * kRowBytes;          // 16 KB: 128 rows of 128 bytes
-constexpr int kPanelKeys = 64;              // keys per probability panel (one swizzle row)
-constexpr int kPanels = kSpan / kPanelKeys;
+constexpr int kKeys = 64;                   // rows of the band per block
+constexpr int kBandBytes = kKeys * kRowBytes;               // 8 KB
+constexpr int kSlots = 2;                   // blocks of the band in shared memory
+constexpr int kBlockBytes = kTileM * kRowBytes;             // 16 KB: a tile's 128 rows, or a 128 x 64 staging tile
 constexpr int kOffQ = 0;
-constexpr int kOffK = kOffQ + kBlockBytes;
-constexpr int kOffV = kOffK + (kSpan / kKeyBlock) * kBlockBytes;
-constexpr int kOffP = kOffV + (kSpan / kKeyBlock) * kBlockBytes;
-constexpr int kOffBar = kOffP + kPanels * kBlockBytes;
-constexpr int kOffRed = kOffBar + 64;                       // per-row partial maxima and sums of the column groups
-constexpr int kSmemBytes = kOffRed + 2 * kColGroups * kTileM * 4 + 1024;   // + alignment slack
-constexpr int kTmemCols = 512;
-constexpr int kColO = kSpan;                // scores in columns [0, 384), the output in [384, 448)
+constexpr int kOffK = kOffQ + kBlockBytes;                  // per slot: k, v
+constexpr int kOffP = kOffK + kSlots * 2 * kBandBytes;
+constexpr int kOffBar = kOffP + kBlockBytes;
+constexpr int kOffRed = kOffBar + 128;                      // maxima (and at the end sums) of the two column groups
+constexpr int kSmemBytes = kOffRed + kColGroups * kTileM * 4 + 1024;   // + alignment slack: 66 KB, three tiles per SM
+constexpr int kTmemCols = 128;              // scores, output
+constexpr int kColO = kKeys;
 constexpr unsigned kWaitLimit = 400000u;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -170,6 +166,21 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 #pragma unroll
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const float (&v)[32]) {
+  uint32_t r[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(v[i]);
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31};"
+      ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]),
+        "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]),
+        "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]), "r"(taddr)
+      : "memory");
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   __nv_bfloat162 h2 = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&h2);
@@ -203,32 +214,54 @@ struct Params {
   float scale;
 };
 
-// One block per SM walks tiles t = blockIdx.x, blockIdx.x + gridDim.x, ... (t = tile of 128 nodes * H + head).  While
-// a tile's softmax runs, the next tile's Q and K are already on their way into the shared memory the score products
-// have released, and its V follows once the second product chain is done: a tile does not start with an idle load.
-__global__ void __launch_bounds__(kThreads, 1)
+// 32 columns of one 128 x 64 staging tile row: 4 chunks of 16 bytes at chunk c * 4 + q
+__device__ __forceinline__ void store_stage_row(unsigned char* row_at, int c, int row, const uint32_t (&packed)[16]) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int chunk = (c * 4 + q) ^ (row & 7);
+    *reinterpret_cast<uint4*>(row_at + chunk * 16) =
+        make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
+  }
+}
+// One block per (tile of 128 nodes, head).  Bound by the chain load - scores - softmax - output of a block of the band; three
+// tiles per SM overlap theirs.  With one tile of 512 threads per SM and the whole band in shared memory, four sequences of
+// 8192, 8 heads, window 128, took 121 us.
+__global__ void __launch_bounds__(kThreads, 3)
 attention_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                          const __grid_constant__ CUtensorMap map_v, const Params p) {
   extern __shared__ unsigned char raw_smem[];
   // the swizzled tiles want a 1024-byte aligned base
   unsigned char* smem = raw_smem + ((1024u - (smem_u32(raw_smem) & 1023u)) & 1023u);
   const uint32_t s_base = smem_u32(smem);
-  const uint32_t bar_load = s_base + kOffBar, bar_s = bar_load + 8, bar_o = bar_load + 16, bar_v = bar_load + 24;
+  // bar_load: the tile's q; bar_s: scores (and the output before them); bar_full + 8 (b % 2): the band's block b
+  const uint32_t bar_load = s_base + kOffBar, bar_s = bar_load + 8, bar_full = bar_load + 64;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kOffBar + 32);
   int* s_red = reinterpret_cast<int*>(smem + kOffBar + 40);   // 4 ints: per-quarter minima of the first neighbour
-  float* s_max = reinterpret_cast<float*>(smem + kOffRed);     // [column group][row]
-  float* s_sum = s_max + kColGroups * kTileM;
+  int* s_top = reinterpret_cast<int*>(smem + kOffBar + 96);   // 4 ints: and maxima of the last one
+  float* s_row = reinterpret_cast<float*>(smem + kOffRed);    // [column group][row]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int quarter = warp & 3, cg = warp >> 2;                // tensor-memory lane quarter, column group
-  const int row = quarter * 32 + lane;                         // row of the tile = tensor-memory lane
-  const long long n_tiles = (p.n_dst + kTileM - 1) / kTileM * p.H;
-
+  const int quarter = warp & 3, cg = warp >> 2;
+  const int row = quarter * 32 + lane;                        // row of the tile = tensor-memory lane
+  const int head = blockIdx.y;
+  const long long r0 = (long long)blockIdx.x * kTileM, r = r0 + row;
+  int lo = INT_MAX, deg = 0;
+  if (r < p.n_dst) {
+    deg = p.node_deg[r];
+    if (deg > 0) lo = p.node_lo[r];
+  }
+  int wmin = lo, wtop = deg > 0 ? lo + deg - 1 : -1;
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    wmin = min(wmin, __shfl_xor_sync(kFull, wmin, o));
+    wtop = max(wtop, __shfl_xor_sync(kFull, wtop, o));
+  }
+  if (lane == 0 && cg == 0) { s_red[quarter] = wmin; s_top[quarter] = wtop; }
   if (tid == 0) {
     mbar_init(bar_load, 1);
     mbar_init(bar_s, 1);
-    mbar_init(bar_o, 1);
-    mbar_init(bar_v, 1);
+#pragma unroll
+    for (int b = 0; b < kSlots; ++b) mbar_init(bar_full + 8 * b, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
@@ -237,231 +270,165 @@ attention_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-
-  // a tile's node range and first key: every thread its own row, the minimum over the tile through shared memory
-  auto tile_rows = [&](long long t, int& lo, int& deg) {
-    lo = INT_MAX;
-    deg = 0;
-    const long long r = t / p.H * kTileM + row;
-    if (t < n_tiles && r < p.n_dst) {
-      deg = p.node_deg[r];
-      if (deg > 0) lo = p.node_lo[r];
-    }
-    int wmin = lo;
-#pragma unroll
-    for (int o = 16; o; o >>= 1) wmin = min(wmin, __shfl_xor_sync(kFull, wmin, o));
-    if (lane == 0 && cg == 0) s_red[quarter] = wmin;
-  };
-  auto issue_qk = [&](long long t, int kmin) {   // one thread
-    mbar_expect_tx(bar_load, (uint32_t)(kBlockBytes * (1 + kSpan / kKeyBlock)));
-    tma_load_3d(s_base + kOffQ, &map_q, bar_load, 0, (int)(t % p.H), (int)(t / p.H * kTileM));
-#pragma unroll
-    for (int b = 0; b < kSpan / kKeyBlock; ++b)
-      tma_load_3d(s_base + kOffK + b * kBlockBytes, &map_k, bar_load, 0, (int)(t % p.H), kmin + b * kKeyBlock);
-  };
-  auto issue_v = [&](long long t, int kmin) {    // one thread
-    mbar_expect_tx(bar_v, (uint32_t)(kBlockBytes * (kSpan / kKeyBlock)));
-#pragma unroll
-    for (int b = 0; b < kSpan / kKeyBlock; ++b)
-      tma_load_3d(s_base + kOffV + b * kBlockBytes, &map_v, bar_v, 0, (int)(t % p.H), kmin + b * kKeyBlock);
-  };
-
-  long long t = blockIdx.x;
-  int lo, deg;
-  tile_rows(t, lo, deg);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
-  int kmin = min(min(s_red[0], s_red[1]), min(s_red[2], s_red[3]));
-  __syncthreads();   // s_red is rewritten for the next tile below
-  if (tid == 0 && t < n_tiles && kmin != INT_MAX) {
-    issue_qk(t, kmin);
-    issue_v(t, kmin);
-  }
-  bool ok = true;
-  uint32_t phase = 0;          // tiles this block has loaded so far, mod 2: the parity of all four barriers
-  bool pending_qk = false, pending_v = false;   // loads issued for the next tile (what to wait for if this one fails)
-  const uint32_t row_taddr = tmem + ((uint32_t)(quarter * 32) << 16);
-  const float sl2 = p.scale * 1.4426950408889634f;
+  const int kmin = min(min(s_red[0], s_red[1]), min(s_red[2], s_red[3]));
 
-  for (; t < n_tiles; t += gridDim.x) {
-    const int head = (int)(t % p.H);
-    const long long r = t / p.H * kTileM + row;
-    const long long t_next = t + gridDim.x;
-    int lo_n, deg_n;
-    tile_rows(t_next, lo_n, deg_n);      // s_red: the next tile's minima, read after the next block-wide barrier
-    pending_qk = pending_v = false;
+  if (kmin != INT_MAX) {
+    const int ktop = max(max(s_top[0], s_top[1]), max(s_top[2], s_top[3]));
+    int nb = (ktop - kmin) / kKeys + 1;   // blocks the tile's band reaches
+    nb = nb < kSpan / kKeys ? nb : kSpan / kKeys;
+    auto issue_band = [&](int b) {   // one thread
+      const uint32_t bar = bar_full + 8 * (b & 1), at = s_base + kOffK + (b & 1) * 2 * kBandBytes;
+      mbar_expect_tx(bar, (uint32_t)(2 * kBandBytes));
+      tma_load_3d(at, &map_k, bar, 0, head, kmin + b * kKeys);
+      tma_load_3d(at + kBandBytes, &map_v, bar, 0, head, kmin + b * kKeys);
+    };
+    auto issue_scores = [&](int b) {   // one thread: 4 steps of 16 features
+      constexpr uint32_t idesc = umma_idesc(kTileM, kKeys, false);
+      const uint32_t at = s_base + kOffK + (b & 1) * 2 * kBandBytes;
+#pragma unroll
+      for (int kk = 0; kk < kD / 16; ++kk)
+        umma_f16(tmem, umma_desc(s_base + kOffQ + kk * 32, 16, 1024), umma_desc(at + kk * 32, 16, 1024), idesc, kk > 0);
+    };
+    if (tid == 0) {
+      mbar_expect_tx(bar_load, (uint32_t)kBlockBytes);
+      tma_load_3d(s_base + kOffQ, &map_q, bar_load, 0, head, (int)r0);
+      tma_load_3d(s_base + kOffQ + kBandBytes, &map_q, bar_load, 0, head, (int)r0 + kKeys);
+      issue_band(0);
+      if (nb > 1) issue_band(1);
+    }
+    int issued = nb < kSlots ? nb : kSlots;
+    bool ok = __syncthreads_and(mbar_wait(bar_load, 0) && mbar_wait(bar_full, 0));
 
-    if (kmin != INT_MAX) {  // some node of the tile has neighbours: its Q, K (and V) are on their way
-      ok = __syncthreads_and(mbar_wait(bar_load, phase));   // the same verdict in every thread
-      const int kmin_n = min(min(s_red[0], s_red[1]), min(s_red[2], s_red[3]));
-      if (ok && tid == 0) {
-        // scores: for each block of 128 keys, 4 steps of 16 features
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        constexpr uint32_t idesc = umma_idesc(kTileM, kKeyBlock, false);
+    const int jlo = deg > 0 ? lo - kmin : 1, jhi = deg > 0 ? lo - kmin + deg - 1 : 0;   // this row's columns of the band
+    int wlo = deg > 0 ? jlo : INT_MAX, whi = deg > 0 ? jhi : -1;
 #pragma unroll
-        for (int b = 0; b < kSpan / kKeyBlock; ++b) {
-#pragma unroll
-          for (int kk = 0; kk < kD / 16; ++kk) {
-            const uint64_t a = umma_desc(s_base + kOffQ + kk * 32, 16, 1024);
-            const uint64_t bd = umma_desc(s_base + kOffK + b * kBlockBytes + kk * 32, 16, 1024);
-            umma_f16(tmem + b * kKeyBlock, a, bd, idesc, kk > 0);
-          }
-        }
-        umma_commit(bar_s);
-      }
-      ok = __syncthreads_and(ok && mbar_wait(bar_s, phase));
+    for (int o = 16; o; o >>= 1) {
+      wlo = min(wlo, __shfl_xor_sync(kFull, wlo, o));
+      whi = max(whi, __shfl_xor_sync(kFull, whi, o));
+    }
+    const uint32_t row_taddr = tmem + ((uint32_t)(quarter * 32) << 16);
+    const float sl2 = p.scale * 1.4426950408889634f;
+    unsigned char* prow = smem + kOffP + row * kRowBytes;
+    float m = -INFINITY, l = 0.f;   // the row's reference maximum, in both of its threads; this thread's part of the sum
+
+    if (ok && tid == 0) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      // the score products are done with Q and K: the next tile's may land there while this tile's softmax runs
-      const bool more = ok && t_next < n_tiles && kmin_n != INT_MAX;
-      if (more && tid == 0) issue_qk(t_next, kmin_n);
-      pending_qk = more;
-
-      // this thread's row: columns [jlo, jhi] are its node's neighbours; it handles chunks cg, cg + 4, cg + 8
-      const int jlo = deg > 0 ? lo - kmin : 1, jhi = deg > 0 ? lo - kmin + deg - 1 : 0;
-      int wlo = deg > 0 ? jlo : INT_MAX, whi = deg > 0 ? jhi : -1;
-#pragma unroll
-      for (int o = 16; o; o >>= 1) {
-        wlo = min(wlo, __shfl_xor_sync(kFull, wlo, o));
-        whi = max(whi, __shfl_xor_sync(kFull, whi, o));
+      issue_scores(0);
+      umma_commit(bar_s);
+    }
+    // Per block one wait: block b's output product and block b + 1's scores are issued back to back behind one commit, so
+    // when the scores are there the staging tile is free and the output is complete as well.
+    for (int b = 0; b < nb; ++b) {
+      ok = __syncthreads_and(ok && mbar_wait(bar_s, b & 1));
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (ok && b > 0 && b + 1 < nb) {   // block b - 1's slot is free
+        if (tid == 0) issue_band(b + 1);
+        issued = b + 2;
       }
-      const int c_first = wlo == INT_MAX ? 0 : wlo / 32, c_last = whi < 0 ? -1 : whi / 32;   // warp-uniform chunk range
-      float m = -INFINITY;
-      for (int c = cg; c < kSpan / 32; c += kColGroups) {
-        if (ok && c >= c_first && c <= c_last) {
-          float v[32];
-          tmem_ld32(row_taddr + c * 32, v);
-          if (c * 32 >= jlo && c * 32 + 31 <= jhi) {   // the whole chunk belongs to the row: no column tests
+      const int col0 = b * kKeys + cg * 32;
+      const bool live = ok && col0 <= whi && col0 + 31 >= wlo;   // warp-uniform
+      const bool whole = col0 >= jlo && col0 + 31 <= jhi;        // the whole chunk belongs to the row: no column tests
+      float v[32], top = -INFINITY;
+      if (live) {
+        tmem_ld32(row_taddr + cg * 32, v);
+        if (whole) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) m = fmaxf(m, v[j]);
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const int col = c * 32 + j;
-              if (col >= jlo && col <= jhi) m = fmaxf(m, v[j]);
-            }
-          }
-        }
-      }
-      s_max[cg * kTileM + row] = m;
-      __syncthreads();
-#pragma unroll
-      for (int g = 0; g < kColGroups; ++g) m = fmaxf(m, s_max[g * kTileM + row]);
-      const float msl2 = deg > 0 ? m * sl2 : 0.f;
-      float l = 0.f;
-      unsigned char* prow = smem + kOffP + row * kRowBytes;   // this row inside each 64-key panel
-      for (int c = cg; c < kSpan / 32; c += kColGroups) {
-        float v[32];
-        const bool live = ok && c >= c_first && c <= c_last;
-        if (live) tmem_ld32(row_taddr + c * 32, v);
-        uint32_t packed[16];
-        if (live && c * 32 >= jlo && c * 32 + 31 <= jhi) {   // the whole chunk belongs to the row
-#pragma unroll
-          for (int j = 0; j < 32; j += 2) {
-            const float p0 = exp2_fast(fmaf(v[j], sl2, -msl2)), p1 = exp2_fast(fmaf(v[j + 1], sl2, -msl2));
-            l += p0 + p1;
-            packed[j / 2] = pack_bf16(p0, p1);
-          }
+          for (int j = 0; j < 32; ++j) top = fmaxf(top, v[j]);
         } else {
 #pragma unroll
-          for (int j = 0; j < 32; j += 2) {
-            float p0 = 0.f, p1 = 0.f;
-            if (live) {
-              const int col = c * 32 + j;
-              if (col >= jlo && col <= jhi) p0 = exp2_fast(fmaf(v[j], sl2, -msl2));
-              if (col + 1 >= jlo && col + 1 <= jhi) p1 = exp2_fast(fmaf(v[j + 1], sl2, -msl2));
-            }
-            l += p0 + p1;
-            packed[j / 2] = pack_bf16(p0, p1);
-          }
-        }
-        // 32 keys = 4 chunks of 16 bytes in panel c / 2, at chunk index (c & 1) * 4 + q, swizzled by the row
-        unsigned char* panel = prow + (c >> 1) * kBlockBytes;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int chunk = ((c & 1) * 4 + q) ^ (row & 7);
-          *reinterpret_cast<uint4*>(panel + chunk * 16) =
-              make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
+          for (int j = 0; j < 32; ++j)
+            if (col0 + j >= jlo && col0 + j <= jhi) top = fmaxf(top, v[j]);
         }
       }
-      s_sum[cg * kTileM + row] = l;
+      s_row[cg * kTileM + row] = top;
+      asm volatile("bar.sync %0, 64;" ::"r"(1 + quarter) : "memory");   // the two warps of these rows
+      top = fmaxf(top, s_row[(cg ^ 1) * kTileM + row]);
+      // A reference that lags behind the maximum by up to 2^8 serves as well: the rounding is relative.
+      const bool grows = top * sl2 > m * sl2 + 8.f || (m == -INFINITY && top > -INFINITY);
+      const float corr = !grows ? 1.f : m == -INFINITY ? 0.f : exp2_fast((m - top) * sl2);
+      if (grows) {
+        m = top;
+        l *= corr;
+      }
+      if (b > 0 && __any_sync(kFull, grows)) {
+        float o[32];
+        tmem_ld32(row_taddr + kColO + cg * 32, o);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) o[j] *= corr;
+        tmem_st32(row_taddr + kColO + cg * 32, o);
+      }
+      const float msl2 = m == -INFINITY ? 0.f : m * sl2;
+      uint32_t packed[16];
+      if (live && whole) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) {
+          const float p0 = exp2_fast(fmaf(v[j], sl2, -msl2)), p1 = exp2_fast(fmaf(v[j + 1], sl2, -msl2));
+          l += p0 + p1;
+          packed[j / 2] = pack_bf16(p0, p1);
+        }
+      } else if (live) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) {
+          const int col = col0 + j;
+          float p0 = 0.f, p1 = 0.f;
+          if (col >= jlo && col <= jhi) p0 = exp2_fast(fmaf(v[j], sl2, -msl2));
+          if (col + 1 >= jlo && col + 1 <= jhi) p1 = exp2_fast(fmaf(v[j + 1], sl2, -msl2));
+          l += p0 + p1;
+          packed[j / 2] = pack_bf16(p0, p1);
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) packed[j] = 0u;
+      }
+      store_stage_row(prow, cg, row, packed);
       // the probabilities were written through the generic proxy; the tensor core reads through the async proxy
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      ok = __syncthreads_and(ok && mbar_wait(bar_v, phase));   // probabilities written by all, values landed
+      ok = __syncthreads_and(ok && (b + 1 >= nb || mbar_wait(bar_full + 8 * ((b + 1) & 1), ((b + 1) >> 1) & 1)));
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      l = 0.f;
-#pragma unroll
-      for (int g = 0; g < kColGroups; ++g) l += s_sum[g * kTileM + row];
       if (ok && tid == 0) {
         constexpr uint32_t idesc = umma_idesc(kTileM, kD, true);
+        const uint32_t at = s_base + kOffK + (b & 1) * 2 * kBandBytes + kBandBytes;
 #pragma unroll
-        for (int ks = 0; ks < kSpan / 16; ++ks) {
-          const uint64_t a = umma_desc(s_base + kOffP + (ks >> 2) * kBlockBytes + (ks & 3) * 32, 16, 1024);
-          const uint64_t bd = umma_desc(s_base + kOffV + ks * 16 * kRowBytes, 16, 1024);
-          umma_f16(tmem + kColO, a, bd, idesc, ks > 0);
-        }
-        umma_commit(bar_o);
+        for (int ks = 0; ks < kKeys / 16; ++ks)
+          umma_f16(tmem + kColO, umma_desc(s_base + kOffP + ks * 32, 16, 1024), umma_desc(at + ks * 16 * kRowBytes, 16, 1024),
+                   idesc, (b | ks) != 0);
+        if (b + 1 < nb) issue_scores(b + 1);
+        umma_commit(bar_s);
       }
-      ok = __syncthreads_and(ok && mbar_wait(bar_o, phase));
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      // the second product chain is done with V: the next tile's may land
-      if (ok && pending_qk && tid == 0) issue_v(t_next, kmin_n);
-      pending_v = ok && pending_qk;
-
-      // this thread's 16 of the row's 64 output features
-      float v[16];
-      if (ok) tmem_ld16(row_taddr + kColO + cg * 16, v);   // warp-wide, whether or not the lane's row exists
+    }
+    s_row[cg * kTileM + row] = l;
+    ok = __syncthreads_and(ok && mbar_wait(bar_s, nb & 1));   // the last block's output product
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    l = s_row[row] + s_row[kTileM + row];
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {   // this thread's 32 of the row's 64 output features
+      const int f0 = cg * 32 + half * 16;
+      float o[16];
+      if (ok) tmem_ld16(row_taddr + kColO + f0, o);   // warp-wide, whether or not the lane's row exists
       if (r < p.n_dst) {
         if (ok && deg == 0) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = 0.f;
+          for (int j = 0; j < 16; ++j) o[j] = 0.f;
         }
-        store_out16(p.o + ((long long)r * p.H + head) * kD + cg * 16, v, deg > 0 ? 1.f / l : 0.f, ok);
-        if (cg == 0) p.lse[(long long)r * p.H + head] = !ok ? NAN : (deg > 0 ? m * p.scale + logf(l) : -INFINITY);
-      }
-      phase ^= 1u;
-      kmin = kmin_n;
-      // tensor memory is read (scores, output) before the next tile's products overwrite it
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      if (!ok) break;
-    } else {
-      // no node of the tile has a neighbour: nothing was loaded; zeros, and the next tile's loads start here
-      __syncthreads();
-      const int kmin_n = min(min(s_red[0], s_red[1]), min(s_red[2], s_red[3]));
-      if (r < p.n_dst && cg == 0) {
-        __nv_bfloat16* orow = p.o + ((long long)r * p.H + head) * kD;
-#pragma unroll
-        for (int q = 0; q < kD / 8; ++q) *reinterpret_cast<uint4*>(orow + q * 8) = make_uint4(0, 0, 0, 0);
-        p.lse[(long long)r * p.H + head] = -INFINITY;
-      }
-      if (tid == 0 && t_next < n_tiles && kmin_n != INT_MAX) {
-        issue_qk(t_next, kmin_n);
-        issue_v(t_next, kmin_n);
-      }
-      kmin = kmin_n;
-    }
-    lo = lo_n;
-    deg = deg_n;
-    __syncthreads();   // s_red and the reduction rows are free for the next tile
-  }
-
-  if (!ok) {
-    // a wait ran out: this tile's rows hold NaN already; so do the rows of the tiles this block will not reach.
-    // Loads issued for the next tile are given (bounded) time to land before the shared memory is handed back.
-    if (pending_qk) mbar_wait(bar_load, phase);
-    if (pending_v) mbar_wait(bar_v, phase);
-    for (long long u = t + gridDim.x; u < n_tiles; u += gridDim.x) {
-      const long long r = u / p.H * kTileM + row;
-      if (r < p.n_dst && cg == 0) {
-        __nv_bfloat16* orow = p.o + ((long long)r * p.H + (int)(u % p.H)) * kD;
-        const uint32_t nan2 = pack_bf16(NAN, NAN);
-#pragma unroll
-        for (int q = 0; q < kD / 8; ++q) *reinterpret_cast<uint4*>(orow + q * 8) = make_uint4(nan2, nan2, nan2, nan2);
-        p.lse[(long long)r * p.H + (int)(u % p.H)] = NAN;
+        store_out16(p.o + ((long long)r * p.H + head) * kD + f0, o, deg > 0 ? 1.f / l : 0.f, ok);
       }
     }
+    if (r < p.n_dst && cg == 0)
+      p.lse[(long long)r * p.H + head] = !ok ? NAN : (deg > 0 ? m * p.scale + logf(l) : -INFINITY);
+    if (!ok) {   // a wait ran out: loads asked for are given (bounded) time to land before the shared memory is handed back
+      mbar_wait(bar_load, 0);
+      for (int b = issued > kSlots ? issued - kSlots : 0; b < issued; ++b) mbar_wait(bar_full + 8 * (b & 1), (b >> 1) & 1);
+    }
+  } else if (r < p.n_dst && cg == 0) {   // no node of the tile has a neighbour
+    __nv_bfloat16* orow = p.o + ((long long)r * p.H + head) * kD;
+#pragma unroll
+    for (int q = 0; q < kD / 8; ++q) *reinterpret_cast<uint4*>(orow + q * 8) = make_uint4(0, 0, 0, 0);
+    p.lse[(long long)r * p.H + head] = -INFINITY;
   }
 
   // every thread is done with tensor memory: hand it back
@@ -486,21 +453,6 @@ attention_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
 // element-wise stage: with the whole band and 128 x 128 staging tiles (one tile per SM) the tensor pipe was busy 9 to 13 %
 // of the time and every wait was exposed.
 // ---------------------------------------------------------------------------------------------------------
-constexpr int kBThreads = 256;               // two threads per owned row: warp w works on lanes 32 (w % 4) .. + 31
-constexpr int kBGroups = kBThreads / kTileM; // and columns 32 (w / 4) .. + 31 of a block
-constexpr int kBKeys = 64;                   // rows of the band per block
-constexpr int kBBand = kBKeys * kRowBytes;   // 8 KB
-constexpr int kBSlots = 2;                   // blocks in shared memory
-
-// 32 columns of one 128 x 64 staging tile row: 4 chunks of 16 bytes at chunk c * 4 + q
-__device__ __forceinline__ void store_stage_row(unsigned char* row_at, int c, int row, const uint32_t (&packed)[16]) {
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int chunk = (c * 4 + q) ^ (row & 7);
-    *reinterpret_cast<uint4*>(row_at + chunk * 16) =
-        make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
-  }
-}
 struct BwdParams {
   const __nv_bfloat16* o;     // (n_dst, H, 64): destination side only
   const __nv_bfloat16* d_o;   // (n_dst, H, 64): destination side only (delta)
@@ -519,18 +471,18 @@ struct BwdParams {
 constexpr int kBOffA = 0;                          // owned tile, first operand (q | k)
 constexpr int kBOffB = kBOffA + kBlockBytes;       // owned tile, second operand (dO | v)
 constexpr int kBOffC = kBOffB + kBlockBytes;       // band, per slot: first operand (k | q), second operand (v | dO)
-constexpr int kBOffS0 = kBOffC + kBSlots * 2 * kBBand;   // staging tile 0 (dS | P^T)
+constexpr int kBOffS0 = kBOffC + kSlots * 2 * kBandBytes;   // staging tile 0 (dS | P^T)
 constexpr int kBOffS1 = kBOffS0 + kBlockBytes;           // staging tile 1 (dS^T, source side)
 constexpr int kBOffBar = 0, kBOffStat = 128;             // behind the staging tiles: barriers, then the (lse, delta) of the
                                                          // band's queries (source side) or the parts of delta
 __host__ __device__ constexpr int bwd_tail(bool src) { return kBOffS0 + (src ? 2 : 1) * kBlockBytes; }
-__host__ __device__ constexpr int bwd_smem(bool src) { return bwd_tail(src) + kBOffStat + (src ? kSpan * 8 : kBGroups * kTileM * 4) + 1024; }
+__host__ __device__ constexpr int bwd_smem(bool src) { return bwd_tail(src) + kBOffStat + (src ? kSpan * 8 : kColGroups * kTileM * 4) + 1024; }
 
 constexpr int kBTmemCols = 256;   // 64 columns each: scores, dP, two gradients
 
 // kSrc = false: destination side (owned = queries); true: source side (owned = keys)
 template <bool kSrc>
-__global__ void __launch_bounds__(kBThreads, 2)
+__global__ void __launch_bounds__(kThreads, 2)
 attention_backward_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                           const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_d,
                           const BwdParams p) {
@@ -569,7 +521,7 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     mbar_init(bar_s, 1);
     mbar_init(bar_g, 1);
 #pragma unroll
-    for (int b = 0; b < kBSlots; ++b) mbar_init(bar_full + 8 * b, 1);
+    for (int b = 0; b < kSlots; ++b) mbar_init(bar_full + 8 * b, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
@@ -584,29 +536,29 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
   const uint32_t tmem = *tmem_slot;
   const int bmin = min(min(s_red[0], s_red[1]), min(s_red[2], s_red[3]));   // first node of the band
   bool ok = true;
-  constexpr int kColS = 0, kColP = kBKeys, kColG0 = 2 * kBKeys, kColG1 = 2 * kBKeys + kD;
+  constexpr int kColS = 0, kColP = kKeys, kColG0 = 2 * kKeys, kColG1 = 2 * kKeys + kD;
 
   if (bmin != INT_MAX) {
     const int btop = max(max(s_top[0], s_top[1]), max(s_top[2], s_top[3]));
-    int nb = (btop - bmin) / kBKeys + 1;                    // blocks the tile's band reaches
-    nb = nb < kSpan / kBKeys ? nb : kSpan / kBKeys;
+    int nb = (btop - bmin) / kKeys + 1;                    // blocks the tile's band reaches
+    nb = nb < kSpan / kKeys ? nb : kSpan / kKeys;
     auto issue_band = [&](int b) {   // one thread
-      const uint32_t bar = bar_full + 8 * (b & 1), at = s_base + kBOffC + (b & 1) * 2 * kBBand;
-      mbar_expect_tx(bar, (uint32_t)(2 * kBBand));
-      tma_load_3d(at, &map_c, bar, 0, head, bmin + b * kBKeys);
-      tma_load_3d(at + kBBand, &map_d, bar, 0, head, bmin + b * kBKeys);
+      const uint32_t bar = bar_full + 8 * (b & 1), at = s_base + kBOffC + (b & 1) * 2 * kBandBytes;
+      mbar_expect_tx(bar, (uint32_t)(2 * kBandBytes));
+      tma_load_3d(at, &map_c, bar, 0, head, bmin + b * kKeys);
+      tma_load_3d(at + kBandBytes, &map_d, bar, 0, head, bmin + b * kKeys);
     };
     if (tid == 0) {
       mbar_expect_tx(bar_load, (uint32_t)(kBlockBytes * 2));
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
-        tma_load_3d(s_base + kBOffA + half * kBBand, &map_a, bar_load, 0, head, (int)r0 + half * kBKeys);
-        tma_load_3d(s_base + kBOffB + half * kBBand, &map_b, bar_load, 0, head, (int)r0 + half * kBKeys);
+        tma_load_3d(s_base + kBOffA + half * kBandBytes, &map_a, bar_load, 0, head, (int)r0 + half * kKeys);
+        tma_load_3d(s_base + kBOffB + half * kBandBytes, &map_b, bar_load, 0, head, (int)r0 + half * kKeys);
       }
       issue_band(0);
       if (nb > 1) issue_band(1);
     }
-    int issued = nb < kBSlots ? nb : kBSlots;
+    int issued = nb < kSlots ? nb : kSlots;
     // per-row scalars while the tiles travel
     float lse2 = 0.f, delta = 0.f, lrow = 0.f;
     const float kL2e = 1.4426950408889634f;
@@ -633,7 +585,7 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
       s_part[cg * kTileM + row] = part;
     } else {
       // (lse, delta) of the band's queries: column j of the scores is query bmin + j
-      for (int i = tid; i < nb * kBKeys; i += kBThreads) {
+      for (int i = tid; i < nb * kKeys; i += kThreads) {
         const long long qn = (long long)bmin + i;
         s_stat[i] = qn < p.n_other ? p.stat[qn * p.H + head] : make_float2(0.f, 0.f);
       }
@@ -641,7 +593,7 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     ok = __syncthreads_and(mbar_wait(bar_load, 0) && mbar_wait(bar_full, 0));
     if constexpr (!kSrc) {
 #pragma unroll
-      for (int g = 0; g < kBGroups; ++g) delta += s_part[g * kTileM + row];   // the same order in both threads
+      for (int g = 0; g < kColGroups; ++g) delta += s_part[g * kTileM + row];   // the same order in both threads
       if (cg == 0 && r < p.n_own) p.stat[(long long)r * p.H + head] = make_float2(lrow, delta);
     }
 
@@ -659,14 +611,14 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
 
     // scores and dP of one block of the band: owned operands x the band's block (issued by one thread)
     auto issue_scores = [&](int b) {
-      constexpr uint32_t idesc = umma_idesc(kTileM, kBKeys, false);
-      const uint32_t at = s_base + kBOffC + (b & 1) * 2 * kBBand;
+      constexpr uint32_t idesc = umma_idesc(kTileM, kKeys, false);
+      const uint32_t at = s_base + kBOffC + (b & 1) * 2 * kBandBytes;
 #pragma unroll
       for (int kk = 0; kk < kD / 16; ++kk)   // scores: owned first operand x band first operand
         umma_f16(tmem + kColS, umma_desc(s_base + kBOffA + kk * 32, 16, 1024), umma_desc(at + kk * 32, 16, 1024), idesc, kk > 0);
 #pragma unroll
       for (int kk = 0; kk < kD / 16; ++kk)   // dP: owned second operand x band second operand
-        umma_f16(tmem + kColP, umma_desc(s_base + kBOffB + kk * 32, 16, 1024), umma_desc(at + kBBand + kk * 32, 16, 1024),
+        umma_f16(tmem + kColP, umma_desc(s_base + kBOffB + kk * 32, 16, 1024), umma_desc(at + kBandBytes + kk * 32, 16, 1024),
                  idesc, kk > 0);
     };
     if (ok && tid == 0) {
@@ -687,7 +639,7 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
 
       {
         const int c = cg;   // this thread's 32 of the block's 64 columns
-        const int col0 = b * kBKeys + c * 32;
+        const int col0 = b * kKeys + c * 32;
         const bool live = ok && col0 <= whi && col0 + 31 >= wlo;   // warp-uniform
         uint32_t pk0[16], pk1[16];
         if (live) {
@@ -730,14 +682,14 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (ok && tid == 0) {
         constexpr uint32_t idesc = umma_idesc(kTileM, kD, true);
-        const uint32_t at = s_base + kBOffC + (b & 1) * 2 * kBBand;
+        const uint32_t at = s_base + kBOffC + (b & 1) * 2 * kBandBytes;
 #pragma unroll
-        for (int ks = 0; ks < kBKeys / 16; ++ks) {
+        for (int ks = 0; ks < kKeys / 16; ++ks) {
           const uint64_t a0 = umma_desc(s_base + kBOffS0 + ks * 32, 16, 1024), c0 = umma_desc(at + ks * 16 * kRowBytes, 16, 1024);
           if constexpr (!kSrc) {   // dQ += dS K_b
             umma_f16(tmem + kColG0, a0, c0, idesc, (b | ks) != 0);
           } else {                 // dV += P^T dO_b,  dK += dS^T Q_b
-            umma_f16(tmem + kColG1, a0, umma_desc(at + kBBand + ks * 16 * kRowBytes, 16, 1024), idesc, (b | ks) != 0);
+            umma_f16(tmem + kColG1, a0, umma_desc(at + kBandBytes + ks * 16 * kRowBytes, 16, 1024), idesc, (b | ks) != 0);
             umma_f16(tmem + kColG0, umma_desc(s_base + kBOffS1 + ks * 32, 16, 1024), c0, idesc, (b | ks) != 0);
           }
         }
@@ -774,7 +726,7 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     }
     if (!ok) {   // a wait ran out: loads asked for are given (bounded) time to land before the shared memory is handed back
       mbar_wait(bar_load, 0);
-      for (int b = issued > kBSlots ? issued - kBSlots : 0; b < issued; ++b) mbar_wait(bar_full + 8 * (b & 1), (b >> 1) & 1);
+      for (int b = issued > kSlots ? issued - kSlots : 0; b < issued; ++b) mbar_wait(bar_full + 8 * (b & 1), (b >> 1) & 1);
     }
   } else if (r < p.n_own && cg == 0) {  // no owned node of the tile has a neighbour: zero gradients
     const long long at = ((long long)r * p.H + head) * kD;
@@ -806,13 +758,13 @@ inline PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   return fn;
 }
 
-// (n, H, 64) bf16 node tensor as a 3-D map (feature, head, node), boxes of `nodes` nodes of one head, 128-byte swizzle
-inline bool make_map(CUtensorMap* map, const void* base, long long n, int H, int nodes) {
+// (n, H, 64) bf16 node tensor as a 3-D map (feature, head, node), boxes of 64 nodes of one head, 128-byte swizzle
+inline bool make_map(CUtensorMap* map, const void* base, long long n, int H) {
   auto fn = encode_fn();
   if (!fn) return false;
   const cuuint64_t dims[3] = {(cuuint64_t)kD, (cuuint64_t)H, (cuuint64_t)n};
   const cuuint64_t strides[2] = {(cuuint64_t)kRowBytes, (cuuint64_t)H * kRowBytes};
-  const cuuint32_t box[3] = {(cuuint32_t)kD, 1u, (cuuint32_t)nodes};
+  const cuuint32_t box[3] = {(cuuint32_t)kD, 1u, (cuuint32_t)kKeys};
   const cuuint32_t estr[3] = {1u, 1u, 1u};
   return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -832,7 +784,7 @@ inline int banded_attention_forward<__nv_bfloat16>(const graphop_plan_t* plan, c
     return GRAPHOP_ERR_UNSUPPORTED;
   if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)o) & 15) return GRAPHOP_ERR_UNSUPPORTED;
   CUtensorMap mq, mk, mv;
-  if (!make_map(&mq, q, n_dst, H, kTileM) || !make_map(&mk, k, n_src, H, kKeyBlock) || !make_map(&mv, v, n_src, H, kKeyBlock))
+  if (!make_map(&mq, q, n_dst, H) || !make_map(&mk, k, n_src, H) || !make_map(&mv, v, n_src, H))
     return GRAPHOP_ERR_UNSUPPORTED;
   static std::atomic<bool> configured[64];
   int dev = 0;
@@ -844,13 +796,8 @@ inline int banded_attention_forward<__nv_bfloat16>(const graphop_plan_t* plan, c
   Params p;
   p.o = o; p.lse = (float*)lse; p.node_lo = plan->node_lo; p.node_deg = plan->node_deg; p.n_dst = n_dst; p.H = H;
   p.scale = (float)scale;
-  // one block per SM (the kernel's shared memory and tensor memory allow no second one), each walking its share of
-  // the (tile, head) pairs
-  int sms = 0;
-  GK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const long long n_tiles = (n_dst + kTileM - 1) / kTileM * H;
-  const unsigned grid = (unsigned)(n_tiles < sms ? n_tiles : sms);
-  attention_forward_kernel<<<grid, kThreads, kSmemBytes, st>>>(mq, mk, mv, p);
+  attention_forward_kernel<<<dim3((unsigned)((n_dst + kTileM - 1) / kTileM), (unsigned)H), kThreads, kSmemBytes, st>>>(mq, mk,
+                                                                                                                mv, p);
   GK_LAUNCHED("attention_fwd_banded");
   return GRAPHOP_OK;
 }
@@ -876,8 +823,8 @@ inline int banded_attention_backward<__nv_bfloat16>(const graphop_plan_t* plan_r
   GK_TRY(check_ws(ws));
   if (wsb < (size_t)n_dst * H * sizeof(float2)) return GRAPHOP_ERR_WORKSPACE;
   CUtensorMap mq, mk, mv, mg;
-  if (!make_map(&mq, q, n_dst, H, kBKeys) || !make_map(&mk, k, n_src, H, kBKeys) || !make_map(&mv, v, n_src, H, kBKeys) ||
-      !make_map(&mg, d_o, n_dst, H, kBKeys))
+  if (!make_map(&mq, q, n_dst, H) || !make_map(&mk, k, n_src, H) || !make_map(&mv, v, n_src, H) ||
+      !make_map(&mg, d_o, n_dst, H))
     return GRAPHOP_ERR_UNSUPPORTED;
   static std::atomic<bool> configured[64];
   int dev = 0;
@@ -891,12 +838,12 @@ inline int banded_attention_backward<__nv_bfloat16>(const graphop_plan_t* plan_r
   p.o = o; p.d_o = d_o; p.lse = (const float*)lse; p.stat = (float2*)ws; p.H = H; p.scale = (float)scale;
   p.out0 = dq; p.out1 = nullptr; p.node_lo = plan_r->node_lo; p.node_deg = plan_r->node_deg; p.n_own = n_dst;
   p.n_other = n_src;
-  attention_backward_kernel<false><<<dim3((unsigned)((n_dst + kTileM - 1) / kTileM), (unsigned)H), kBThreads, bwd_smem(false),
+  attention_backward_kernel<false><<<dim3((unsigned)((n_dst + kTileM - 1) / kTileM), (unsigned)H), kThreads, bwd_smem(false),
                                      st>>>(mq, mg, mk, mv, p);
   GK_LAUNCHED("attention_bwd_dst_banded");
   p.out0 = dk; p.out1 = dv; p.node_lo = plan_t->node_lo; p.node_deg = plan_t->node_deg; p.n_own = n_src;
   p.n_other = n_dst;
-  attention_backward_kernel<true><<<dim3((unsigned)((n_src + kTileM - 1) / kTileM), (unsigned)H), kBThreads, bwd_smem(true),
+  attention_backward_kernel<true><<<dim3((unsigned)((n_src + kTileM - 1) / kTileM), (unsigned)H), kThreads, bwd_smem(true),
                                     st>>>(mk, mv, mq, mg, p);
   GK_LAUNCHED("attention_bwd_src_banded");
   return GRAPHOP_OK;
