@@ -45,7 +45,7 @@ template <int N> __device__ __forceinline__ void cp_async_wait() {
 constexpr uint32_t kNoRow = 0xffffffffu;
 constexpr int kMaxBlockHeads = 8;   // heads per block at most
 
-// What a launch of the walker sees of the graph and of the carry levels.
+// What a launch of the walker sees of the graph and of the carry records.
 struct WalkArgs {
   const PlanHeader* hdr;
   const int32_t* erow;

@@ -158,7 +158,7 @@ struct GraphView {
   const int32_t* eid;    // may be null: identity
   long long E;
   // work tiles: their boundaries (null: the op has no use for them), number and cost; whether the boundaries were moved
-  // to row starts already (a plan's), and whether no row crosses one (then the carry levels have nothing to do)
+  // to row starts already (a plan's), and whether no row crosses one (then there is nothing to merge)
   const int32_t* tile_start = nullptr;
   long long n_tiles = 0;
   int tile = 0;

@@ -1,4 +1,4 @@
-// Launching the gathering walker (gk_group.cuh): which geometry a row shape gets, the carry levels' memory, the launch.
+// Launching the gathering walker (gk_group.cuh): which geometry a row shape gets, the carry records, the launch.
 #pragma once
 #include "gk_group.cuh"
 

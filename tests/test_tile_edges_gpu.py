@@ -7,7 +7,8 @@ import pytest
 import torch as th
 
 from helpers import assert_close, chunked, random_graph
-from custom_op_benchmark_b200 import graphop, wrapper
+from custom_op_benchmark_b200 import graphop, graphs, wrapper
+from oracle import edge_list_f64 as ref
 from oracle import graphop_oracle as orc
 
 pytestmark = pytest.mark.gpu
@@ -136,3 +137,29 @@ def test_functions_from_several_threads(graph):
         t.join()
     assert not errors
     assert all(th.equal(y, want) for y in got)
+
+
+# one block of the band's 64 keys to six of them, tiles that end inside a sequence; scores that grow along the band, so that
+# the forward's running maximum has to move its reference (and ones that fall, and a scale that turns them round)
+@pytest.mark.parametrize("length,window,ramp,scale", [(1, 0, 0, 0.125), (63, 5, 0, 0.125), (128, 31, 0, 0.125),
+                                                      (129, 32, 30, 0.5), (500, 64, 60, 0.5), (700, 128, 100, 1.0),
+                                                      (700, 128, -100, 1.0), (300, 100, 0, -0.125), (300, 100, 0, 0.0)])
+def test_dense_band(length, window, ramp, scale):
+    g = graphs.banded_graph(2, length, window)
+    n, h, d = g.n_dst, 3, 64
+    rc, cc = [t.to(DEV) for t in chunked(g, 32)], [t.to(DEV) for t in chunked(g, 32, transposed=True)]
+    plans = graphop.GraphPlan(*rc, n), graphop.GraphPlan(*cc, n)
+    assert plans[0].dense_band and plans[1].dense_band
+    Q, K, V, dO = (_draw(th.float32, n, h, d, seed=k).to(DEV) for k in range(4))
+    at = th.linspace(0, 1, n, device=DEV).view(-1, 1, 1)
+    K = 0.3 * K + ramp * (at if ramp >= 0 else 1 - at) * Q.mean(0, keepdim=True).sign() / d
+    Q = 0.3 * Q + (1.0 if ramp else 0.0) * Q.mean(0, keepdim=True).sign()
+    Q, K, V, dO = (t.to(th.bfloat16) for t in (Q, K, V, dO))
+    leaves = [t.clone().requires_grad_(True) for t in (Q, K, V)]
+    o = wrapper.GraphAttentionPlanned.apply(*plans, *leaves, scale)
+    got = [o, *th.autograd.grad(o, leaves, dO)]
+    want = ref.attention_f64(g.indptr.to(DEV), g.indices.to(DEV), Q, K, V, scale, dO)
+    for name, a, b in zip(("o", "dq", "dk", "dv"), got, (want[0], *want[2:])):
+        assert_close(a, b, 3e-2, 3e-2 * max(1.0, float(b.abs().max())), name)
+    _, lse = graphop.attention_forward_planned(plans[0], Q, K, V, scale)
+    assert_close(lse, want[1], 2e-3, 2e-3, "lse")
