@@ -237,6 +237,60 @@ softmax_tile_kernel(const int32_t* __restrict__ erow, const int32_t* __restrict_
   __syncthreads();
   st.warps = s_warps;
 
+  if (st.warps == 0) {
+    // The tile lies inside one node that began before it (most tiles of a skewed graph): two block reductions, no scans, and
+    // nothing to write yet.
+    const int row = r[0];
+    if (row >= 0) {
+      A m[H], l[H];
+#pragma unroll
+      for (int h = 0; h < H; ++h) {
+        m[h] = kBackward ? A(0) : neg_inf<A>();
+#pragma unroll
+        for (int i = 0; i < P; ++i) {
+          if constexpr (kBackward) m[h] += a[i][h] * b[i][h];
+          else m[h] = seg_op<true>(m[h], a[i][h]);
+        }
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) m[h] = seg_op<!kBackward>(m[h], __shfl_xor_sync(kFull, m[h], o));
+        if (st.lane == 0) s_head[0][st.w][h] = m[h];
+      }
+      __syncthreads();
+#pragma unroll
+      for (int h = 0; h < H; ++h) {
+        m[h] = s_head[0][0][h];
+#pragma unroll
+        for (int k = 1; k < kSoftmaxWarps; ++k) m[h] = seg_op<!kBackward>(m[h], s_head[0][k][h]);
+      }
+      if constexpr (!kBackward) {
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+          l[h] = A(0);
+#pragma unroll
+          for (int i = 0; i < P; ++i) l[h] += gk_exp(a[i][h] - m[h]);
+          l[h] = warp_sum(l[h]);
+          if (st.lane == 0) s_head[1][st.w][h] = l[h];
+        }
+        __syncthreads();
+      }
+      if (tid == 0)
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+          slots[2 * t * kSlot + h] = m[h];
+          if constexpr (!kBackward) {
+#pragma unroll
+            for (int k = 1; k < kSoftmaxWarps; ++k) l[h] += s_head[1][k][h];
+            slots[2 * t * kSlot + H + h] = l[h];
+          }
+        }
+    }
+    if (tid == 0) {
+      slot_rows[2 * t] = row;
+      slot_rows[2 * t + 1] = -1;
+    }
+    return;
+  }
+
   A m[P][H];    // maxima (backward: sums)
   A l[kBackward ? 1 : P][H];
   if constexpr (kBackward) {
