@@ -509,26 +509,62 @@ softmax_finish_kernel(const int32_t* __restrict__ erow, const int32_t* __restric
     }
   }
   __syncthreads();
-  const long long j0 = t * kSoftmaxTile, j1 = j0 + kSoftmaxTile < E ? j0 + kSoftmaxTile : E;
+  constexpr int P = kSoftmaxPer;
+  const long long p = t * kSoftmaxTile + tid * P;
+  alignas(16) int r[P];
+  long long e[P];
+  if (p + P <= E) {
+    *reinterpret_cast<int4*>(r) = __ldg(reinterpret_cast<const int4*>(erow + p));
+  } else {
 #pragma unroll
-  for (int i = 0; i < kSoftmaxPer; ++i) {
-    const long long j = j0 + i * kSoftmaxThreads + tid;
-    const int r = j < j1 ? __ldg(erow + j) : -1;
-    if (r < 0 || (r != head_row && r != tail_row)) continue;
-    const long long e = eid ? (long long)__ldg(eid + j) : j;
-    const A* st = s_stat[r == head_row ? 0 : 1];
-    A a[H], y[H];
-    load_heads<T, H, kVec>(a, in0 + e * hs + h0);
-    if constexpr (kBackward) {
-      A b[H];
-      load_heads<T, H, kVec>(b, in1 + e * hs + h0);
+    for (int i = 0; i < P; ++i) r[i] = p + i < E ? __ldg(erow + p + i) : -1;
+  }
+  bool todo[P], all = true, any = false;
 #pragma unroll
-      for (int h = 0; h < H; ++h) y[h] = a[h] * (b[h] - st[h]);
-    } else {
+  for (int i = 0; i < P; ++i) {
+    todo[i] = r[i] >= 0 && (r[i] == head_row || r[i] == tail_row);
+    all = all && todo[i];
+    any = any || todo[i];
+  }
+  if (!any) return;
 #pragma unroll
-      for (int h = 0; h < H; ++h) y[h] = gk_exp(a[h] - st[h]) / st[H + h];
+  for (int i = 0; i < P; ++i) e[i] = eid && todo[i] ? (long long)__ldg(eid + p + i) : p + i;
+  // four consecutive edges are one piece of memory (the tile kernel's case)
+  bool run = kVec && all && e[1] == e[0] + 1 && e[2] == e[0] + 2 && e[3] == e[0] + 3;
+  if constexpr (kVec) {
+    constexpr int kWide = P * H * (int)sizeof(T) < 16 ? P * H * (int)sizeof(T) : 16;
+    run = run && ((uintptr_t)(in0 + e[0] * H) % kWide) == 0 && ((uintptr_t)(out + e[0] * H) % kWide) == 0 &&
+          (!kBackward || ((uintptr_t)(in1 + e[0] * H) % kWide) == 0);
+  }
+  A a[P][H];
+  A b[kBackward ? P : 1][H];
+  if (run) {
+    load_vec<T, P * H>(reinterpret_cast<A(&)[P * H]>(a), in0 + e[0] * H);
+    if constexpr (kBackward) load_vec<T, P * H>(reinterpret_cast<A(&)[P * H]>(b), in1 + e[0] * H);
+  } else {
+#pragma unroll
+    for (int i = 0; i < P; ++i)
+      if (todo[i]) {
+        load_heads<T, H, kVec>(a[i], in0 + e[i] * hs + h0);
+        if constexpr (kBackward) load_heads<T, H, kVec>(b[i], in1 + e[i] * hs + h0);
+      }
+  }
+#pragma unroll
+  for (int i = 0; i < P; ++i) {
+    if (!todo[i]) continue;
+    const A* st = s_stat[r[i] == head_row ? 0 : 1];
+#pragma unroll
+    for (int h = 0; h < H; ++h) {
+      if constexpr (kBackward) a[i][h] = a[i][h] * (b[i][h] - st[h]);
+      else a[i][h] = gk_exp(a[i][h] - st[h]) / st[H + h];
     }
-    store_heads<T, H, kVec>(out + e * hs + h0, y);
+  }
+  if (run) {
+    store_vec<T, P * H>(out + e[0] * H, reinterpret_cast<A(&)[P * H]>(a));
+  } else {
+#pragma unroll
+    for (int i = 0; i < P; ++i)
+      if (todo[i]) store_heads<T, H, kVec>(out + e[i] * hs + h0, a[i]);
   }
 }
 
