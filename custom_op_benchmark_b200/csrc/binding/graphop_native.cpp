@@ -17,6 +17,7 @@
 
 #include <limits>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -155,7 +156,7 @@ GRAPHOP_OVERLOADS(internal_attention_bias_backward)
 struct Tables {
   std::vector<Tensor> t;
   std::vector<uint32_t> versions;
-  GraphPtr rows, cols;
+  GraphPtr rows;
   Tables(std::initializer_list<Tensor> list) : t(list) {
     versions.reserve(t.size());
     for (const Tensor& x : t) versions.push_back(x.defined() && !x.is_inference() ? x._version() : 0);
@@ -198,20 +199,34 @@ Tensor edge_out(const Tensor& node, int64_t n_edges, int H) {
 }
 graphop_stream_t raw(cudaStream_t s) { return (graphop_stream_t)s; }
 
-// what a node of these ops keeps besides its saved tensors
+// What a node of these ops keeps: written when the call is recorded and read-only from then on, but for `saved`, which a
+// backward that does not retain the graph releases.  Two threads may run the backward of one graph: `saved` is touched
+// under the node's mutex, everything else a backward makes is its own.
 struct GraphNode : Node {
   TablesPtr tables;             // chunk-table forms
+  std::vector<SavedVariable> saved;
   std::string name() const override { return "GraphopBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> hold(mutex_);
+    for (SavedVariable& s : saved) s.reset_data();
+  }
+  std::vector<Tensor> unpack_saved() {
+    const std::shared_ptr<Node> self = shared_from_this();   // for a saved output
+    std::lock_guard<std::mutex> hold(mutex_);
+    std::vector<Tensor> t;
+    t.reserve(saved.size());
+    for (const SavedVariable& s : saved) t.push_back(s.unpack(self));
+    return t;
+  }
 };
 
 // ---- SparseSoftmax (wrapper.py:8-18) ------------------------------------------------------
 struct SparseSoftmaxBackward : GraphNode {
-  SavedVariable y_;
-  void release_variables() override { y_.reset_data(); }
   variable_list apply(variable_list&& grads) override {
     if (!grads[0].defined()) return {Tensor()};
     tables->check_unmodified();
-    const Tensor y = y_.unpack(shared_from_this()), dy = upstream(grads, "dy");
+    const std::vector<Tensor> kept = unpack_saved();
+    const Tensor y = kept[0], dy = upstream(grads, "dy");
     const int elem = elem_of({&y, &dy}), H = edge_heads(dy);
     Call c(y);
     Tensor dx = at::empty_like(dy);
@@ -249,36 +264,34 @@ Tensor sparse_softmax(const Tensor& row, const Tensor& indptr, const Tensor& eid
   }
   record<SparseSoftmaxBackward>({x}, y, [&](SparseSoftmaxBackward& n) {
     n.tables = tb;
-    n.y_ = SavedVariable(y, true);
+    n.saved.emplace_back(y, true);
   });
   return y;
 }
 
 // ---- MaskedMMCSR (wrapper.py:20-30) -------------------------------------------------------
 // the view of the other orientation, whose tables start at t[at]
-void column_view(Tables& tb, int at, int64_t e, int64_t n_src, cudaStream_t stream) {
-  if (tb.cols) return;
+GraphPtr column_view(const Tables& tb, int at, int64_t e, int64_t n_src, cudaStream_t stream) {
   const char* names[] = {"col", "indptr", "eid", "indices"};
   for (int i = 0; i < 4; ++i) check_input(tb.t[at + i], names[i]);
   check_chunks(tb.t[at], tb.t[at + 1]);
-  tb.cols = view_of(tb.t[at], tb.t[at + 1], tb.t[at + 2], tb.t[at + 3], e, n_src, stream);
+  return view_of(tb.t[at], tb.t[at + 1], tb.t[at + 2], tb.t[at + 3], e, n_src, stream);
 }
 struct MaskedMMBackward : GraphNode {
-  SavedVariable a_, b_;
-  void release_variables() override { a_.reset_data(); b_.reset_data(); }
   variable_list apply(variable_list&& grads) override {
     if (!grads[0].defined()) return {Tensor(), Tensor()};
     tables->check_unmodified();
-    const Tensor A = a_.unpack(), B = b_.unpack(), dy = upstream(grads, "dy");
+    const std::vector<Tensor> kept = unpack_saved();
+    const Tensor A = kept[0], B = kept[1], dy = upstream(grads, "dy");
     const int elem = elem_of({&A, &B, &dy});
     const NodeShape s = node_shape(A);
     Call c(A);
     const int64_t e = tables->t[2].size(0), nb = B.size(0);
     Tensor dA = at::empty_like(A.detach()), dB = at::empty_like(B.detach());
     if (e == 0) return {dA.zero_(), dB.zero_()};
-    column_view(*tables, 4, e, nb, c.stream);
+    const GraphPtr cols = column_view(*tables, 4, e, nb, c.stream);
     c.workspace(GRAPHOP_OP_MASKEDMM_BWD, e, std::max(s.n, nb), s.H, s.D, A);
-    const graphop_plan_t *pr = &tables->rows->plan, *pc = &tables->cols->plan;
+    const graphop_plan_t *pr = &tables->rows->plan, *pc = &cols->plan;
     check_status(by_elem(elem, [&](auto* k) {
       using E = std::remove_pointer_t<decltype(k)>;
       return maskedmm_csr_backward_planned(k, pr, pc, (const E*)ptr<E>(A), (const E*)ptr<E>(B), (const E*)ptr<E>(dy),
@@ -316,20 +329,19 @@ Tensor maskedmm_csr(const Tensor& row, const Tensor& indptr_r, const Tensor& eid
   record<MaskedMMBackward>({A, B}, y, [&](MaskedMMBackward& n) {
     // the backward reads the column side; wrong tensors are reported there, as its arguments always were
     n.tables = tb;
-    n.a_ = SavedVariable(A, false);
-    n.b_ = SavedVariable(B, false);
+    n.saved.emplace_back(A, false);
+    n.saved.emplace_back(B, false);
   });
   return y;
 }
 
 // ---- NodeMulEdge (wrapper.py:32-42) -------------------------------------------------------
 struct NodeMulEdgeBackward : GraphNode {
-  SavedVariable a_, b_;
-  void release_variables() override { a_.reset_data(); b_.reset_data(); }
   variable_list apply(variable_list&& grads) override {
     if (!grads[0].defined()) return {Tensor(), Tensor()};
     tables->check_unmodified();
-    const Tensor A = a_.unpack(), B = b_.unpack(), dy = upstream(grads, "dy");
+    const std::vector<Tensor> kept = unpack_saved();
+    const Tensor A = kept[0], B = kept[1], dy = upstream(grads, "dy");
     const int elem = elem_of({&A, &B, &dy});
     const NodeShape s = node_shape(A);
     Call c(A);
@@ -370,29 +382,28 @@ Tensor node_mul_edge(const Tensor& row, const Tensor& indptr, const Tensor& eid,
   }
   record<NodeMulEdgeBackward>({A, B}, y, [&](NodeMulEdgeBackward& n) {
     n.tables = tb;
-    n.a_ = SavedVariable(A, false);
-    n.b_ = SavedVariable(B, false);
+    n.saved.emplace_back(A, false);
+    n.saved.emplace_back(B, false);
   });
   return y;
 }
 
 // ---- VectorSPMM (wrapper.py:44-55) --------------------------------------------------------
 struct VectorSPMMBackward : GraphNode {
-  SavedVariable w_, x_;
-  void release_variables() override { w_.reset_data(); x_.reset_data(); }
   variable_list apply(variable_list&& grads) override {
     if (!grads[0].defined()) return {Tensor(), Tensor()};
     tables->check_unmodified();
-    const Tensor w = w_.unpack(), x = x_.unpack(), dy = upstream(grads, "dy");
+    const std::vector<Tensor> kept = unpack_saved();
+    const Tensor w = kept[0], x = kept[1], dy = upstream(grads, "dy");
     const int elem = elem_of({&w, &dy, &x});
     const NodeShape s = node_shape(x);
     Call c(x);
     const int64_t e = tables->t[2].size(0), n_dst = dy.size(0);
     Tensor dw = at::empty_like(w.detach()), dx = at::empty_like(x.detach());
     if (e == 0) return {dw, dx.zero_()};
-    column_view(*tables, 4, e, s.n, c.stream);
+    const GraphPtr cols = column_view(*tables, 4, e, s.n, c.stream);
     c.workspace(GRAPHOP_OP_SPMM_BWD, e, std::max(n_dst, s.n), s.H, s.D, x);
-    const graphop_plan_t *pr = &tables->rows->plan, *pt = &tables->cols->plan;
+    const graphop_plan_t *pr = &tables->rows->plan, *pt = &cols->plan;
     check_status(by_elem(elem, [&](auto* k) {
       using E = std::remove_pointer_t<decltype(k)>;
       return vector_spmm_backward_planned(k, pr, pt, (const E*)ptr<E>(w), (const E*)ptr<E>(dy), (const E*)ptr<E>(x),
@@ -428,27 +439,24 @@ Tensor vector_spmm(const Tensor& row, const Tensor& indptr, const Tensor& eid, c
   }
   record<VectorSPMMBackward>({w, x}, y, [&](VectorSPMMBackward& n) {
     n.tables = tb;
-    n.w_ = SavedVariable(w, false);
-    n.x_ = SavedVariable(x, false);
+    n.saved.emplace_back(w, false);
+    n.saved.emplace_back(x, false);
   });
   return y;
 }
 
 // ---- fused attention on plans, with and without the edge term ------------------------------
 struct AttentionBackward : GraphNode {
-  GraphPtr rows, cols;
-  SavedVariable q_, k_, v_, rel_, o_, lse_;
+  GraphPtr rows, cols;   // cols: null for chunk tables
   double scale = 1.0;
   bool bias = false;
-  void release_variables() override {
-    for (SavedVariable* s : {&q_, &k_, &v_, &rel_, &o_, &lse_}) s->reset_data();
-  }
   variable_list apply(variable_list&& grads) override {
     const size_t n_out = bias ? 4 : 3;
     if (!grads[0].defined()) return variable_list(n_out);
     if (tables) tables->check_unmodified();
-    const Tensor q = q_.unpack(), k = k_.unpack(), v = v_.unpack(), o = o_.unpack(shared_from_this()), lse = lse_.unpack(),
-                 rel = bias ? rel_.unpack() : Tensor(), g = upstream(grads, "d_o");
+    const std::vector<Tensor> kept = unpack_saved();
+    const Tensor q = kept[0], k = kept[1], v = kept[2], o = kept[3], lse = kept[4], rel = bias ? kept[5] : Tensor(),
+                 g = upstream(grads, "d_o");
     const int elem = elem_of({&q, &k, &v, &o, &g});
     const NodeShape s = node_shape(q);
     Call c(q);
@@ -460,11 +468,8 @@ struct AttentionBackward : GraphNode {
       if (bias) out.push_back(drel);
       return out;
     }
-    if (!cols) {
-      column_view(*tables, 3, rows->plan.n_edges, nk, c.stream);
-      cols = tables->cols;
-    }
-    const graphop_plan_t *pr = &rows->plan, *pt = &cols->plan;
+    const GraphPtr other = cols ? cols : column_view(*tables, 3, rows->plan.n_edges, nk, c.stream);
+    const graphop_plan_t *pr = &rows->plan, *pt = &other->plan;
     c.workspace(pt->eid ? GRAPHOP_OP_ATTENTION_BWD_PAIRS : GRAPHOP_OP_ATTENTION_BWD, rows->plan.n_edges, std::max(s.n, nk), s.H,
                 s.D, q);
     check_status(by_elem(elem, [&](auto* e) {
@@ -514,12 +519,10 @@ Tensor attention_common(const GraphPtr& rows, const GraphPtr& cols, const Tables
     n.cols = cols;
     n.scale = scale;
     n.bias = bias;
-    n.q_ = SavedVariable(q, false);
-    n.k_ = SavedVariable(k, false);
-    n.v_ = SavedVariable(v, false);
-    if (bias) n.rel_ = SavedVariable(rel, false);
-    n.o_ = SavedVariable(o, true);
-    n.lse_ = SavedVariable(lse, false);
+    for (const Tensor* t : {&q, &k, &v}) n.saved.emplace_back(*t, false);
+    n.saved.emplace_back(o, true);
+    n.saved.emplace_back(lse, false);
+    if (bias) n.saved.emplace_back(rel, false);
   };
   if (bias) record<AttentionBackward>({q, k, v, rel}, o, save);
   else record<AttentionBackward>({q, k, v}, o, save);

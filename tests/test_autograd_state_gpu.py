@@ -1,0 +1,79 @@
+"""What the native autograd Functions keep, and for how long: device memory beyond the tensors a call was given and
+returned, one graph's backward from several threads."""
+import threading
+
+import pytest
+import torch as th
+
+from helpers import chunked, random_graph
+from custom_op_benchmark_b200 import wrapper
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+N, H, D = 4000, 4, 32
+
+
+@pytest.fixture(scope="module")
+def tables():
+    deg = th.randint(0, 100, (N,), generator=th.Generator().manual_seed(1))
+    g = random_graph(N, N, deg, 2)
+    return ([t.to(DEV) for t in chunked(g, 32, dtype=th.int64)],
+            [t.to(DEV) for t in chunked(g, 32, transposed=True, dtype=th.int64)], g.n_edges)
+
+
+def _normal(*shape, seed):
+    return th.randn(*shape, generator=th.Generator().manual_seed(seed)).to(DEV)
+
+
+def _call(name, tables):
+    """(apply on fresh leaves, the leaves) of each Function that takes chunk tables."""
+    r, c, e = tables
+    node, edge = [_normal(N, H, D, seed=k) for k in range(3)], _normal(e, H, seed=3)
+    if name == "SparseSoftmax":
+        return wrapper.SparseSoftmax, r[:3], [edge]
+    if name == "MaskedMMCSR":
+        return wrapper.MaskedMMCSR, [*r, *c], node[:2]
+    if name == "NodeMulEdge":
+        return wrapper.NodeMulEdge, r[:3], [node[0], _normal(e, D, seed=4)]
+    if name == "VectorSPMM":
+        return wrapper.VectorSPMM, [*r, *c], [edge, node[0]]
+    return wrapper.GraphAttentionBias, [r[0], r[1], r[3], *c], [*node, _normal(e, D, seed=4), D ** -0.5]
+
+
+FUNCTIONS = ["SparseSoftmax", "MaskedMMCSR", "NodeMulEdge", "VectorSPMM", "GraphAttentionBias"]
+
+
+def _leaves(given):
+    return [t.clone().requires_grad_(True) if isinstance(t, th.Tensor) else t for t in given]
+
+
+def _tensors(given):
+    return [t for t in given if isinstance(t, th.Tensor)]
+
+
+@pytest.mark.parametrize("name", FUNCTIONS)
+def test_one_graph_backward_from_several_threads(tables, name):
+    function, tabs, given = _call(name, tables)
+    leaves = _leaves(given)
+    out = function.apply(*tabs, *leaves)
+    grad = _normal(*out.shape, seed=9)
+    want = th.autograd.grad(out, _tensors(leaves), grad, retain_graph=True)
+    out = function.apply(*tabs, *leaves)   # a graph no backward has run on yet
+    th.cuda.synchronize()
+    got, errors, ready = [], [], threading.Barrier(4)
+
+    def work():
+        try:
+            ready.wait()
+            for _ in range(5):
+                got.append(th.autograd.grad(out, _tensors(leaves), grad, retain_graph=True))
+        except Exception as e:   # reported by the main thread
+            errors.append(e)
+    threads = [threading.Thread(target=work) for _ in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    th.cuda.synchronize()
+    assert not errors and len(got) == 20
+    assert all(th.equal(a, b) for grads in got for a, b in zip(grads, want))
