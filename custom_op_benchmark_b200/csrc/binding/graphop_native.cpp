@@ -39,22 +39,29 @@ void check_input(const Tensor& t, const char* name) {
   if (!t.is_cuda()) fail(std::string(name) + " must be a CUDA tensor");
   if (!t.is_contiguous()) fail(std::string(name) + " must be contiguous");
 }
-int index_bytes_of(std::initializer_list<const Tensor*> ts) {
-  at::ScalarType dt = at::ScalarType::Undefined;
+std::string dtype_text(const Tensor& t) {
+  const auto names = c10::getDtypeNames(t.scalar_type());
+  return "torch." + names.first;
+}
+int index_bytes_of(at::ArrayRef<const Tensor*> ts) {
+  const Tensor* first = nullptr;
   for (const Tensor* t : ts) {
     if (!t || !t->defined()) continue;
-    if (dt == at::ScalarType::Undefined) dt = t->scalar_type();
-    if (dt != at::kInt && dt != at::kLong) fail("index tensors must be int32 or int64, got " + std::string(toString(dt)));
-    if (t->scalar_type() != dt) fail("expected all index tensors to share one dtype");
+    if (!first) first = t;
+    if (first->scalar_type() != at::kInt && first->scalar_type() != at::kLong)
+      fail("index tensors must be int32 or int64, got " + dtype_text(*first));
+    if (t->scalar_type() != first->scalar_type())
+      fail("expected all index tensors to share dtype " + dtype_text(*first) + ", got " + dtype_text(*t));
   }
-  return dt == at::kLong ? 8 : 4;
+  return first && first->scalar_type() == at::kLong ? 8 : 4;
 }
 int elem_of(std::initializer_list<const Tensor*> ts) {
   const at::ScalarType dt = (*ts.begin())->scalar_type();
   if (dt != at::kFloat && dt != at::kDouble && dt != at::kBFloat16)
     fail("\"graphop\" not implemented for '" + std::string(toString(dt)) + "'");
   for (const Tensor* t : ts)
-    if (t->scalar_type() != dt) fail("expected all floating tensors to share one dtype");
+    if (t->scalar_type() != dt)
+      fail("expected all floating tensors to share dtype " + dtype_text(**ts.begin()) + ", got " + dtype_text(*t));
   return dt == at::kFloat ? 0 : dt == at::kDouble ? 1 : 2;
 }
 struct NodeShape { int64_t n; int H, D; };
@@ -275,6 +282,9 @@ GraphPtr column_view(const Tables& tb, int at, int64_t e, int64_t n_src, cudaStr
   const char* names[] = {"col", "indptr", "eid", "indices"};
   for (int i = 0; i < 4; ++i) check_input(tb.t[at + i], names[i]);
   check_chunks(tb.t[at], tb.t[at + 1]);
+  std::vector<const Tensor*> all;   // both orientations: one call has one index type
+  for (const Tensor& t : tb.t) all.push_back(&t);
+  index_bytes_of(all);
   return view_of(tb.t[at], tb.t[at + 1], tb.t[at + 2], tb.t[at + 3], e, n_src, stream);
 }
 struct MaskedMMBackward : GraphNode {

@@ -77,3 +77,12 @@ def test_one_graph_backward_from_several_threads(tables, name):
     th.cuda.synchronize()
     assert not errors and len(got) == 20
     assert all(th.equal(a, b) for grads in got for a, b in zip(grads, want))
+
+
+@pytest.mark.parametrize("name", ["MaskedMMCSR", "VectorSPMM", "GraphAttentionBias"])
+def test_index_types_of_the_two_orientations_agree(tables, name):
+    function, tabs, given = _call(name, tables)
+    leaves, half = _leaves(given), len(tabs) - 4
+    out = function.apply(*tabs[:half], *[t.int() for t in tabs[half:]], *leaves)
+    with pytest.raises(RuntimeError, match="expected all index tensors to share dtype torch.int64, got torch.int32"):
+        out.sum().backward()
