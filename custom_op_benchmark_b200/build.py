@@ -54,7 +54,7 @@ def _build_one_module(name, force):
     import torch
     from torch.utils import cpp_extension as ce
     out, src = module_path(name), os.path.join(BINDING_DIR, MODULES[name])
-    deps = [src, LIB, os.path.join(CSRC, "graphop_internal.h"), os.path.join(HERE, "..", "include", "graphop_b200.h"),
+    deps = [src, LIB, os.path.join(HERE, "..", "include", "graphop_b200.h"),
             os.path.join(HERE, "..", "include", "graphop_dlpack.h")]
     if not force and not _stale(out, deps):
         return out

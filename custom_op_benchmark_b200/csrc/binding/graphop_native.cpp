@@ -6,8 +6,9 @@
 // C ABI's planned entry point; the backward runs on autograd's thread without taking the interpreter lock.
 //
 // The chunk-table signatures (row, indptr, eid, indices) of the reference carry the graph on every call.  The owner
-// table, 32-bit index copies and work tiles that the forward makes from them (a "view": a plan without the shape
-// analysis) are saved for the backward of the same call, beside its tensors.
+// table, 32-bit index copies and work tiles that the kernels make from them are workspace of each direction: kept from
+// the forward to the backward (one launch less for MaskedMMCSR and GraphAttentionBias) they held 12 to 18 bytes per edge,
+// and as much again afterwards, as long as the output lived.
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/function.h>
@@ -21,7 +22,7 @@
 #include <string>
 #include <vector>
 
-#include "../graphop_internal.h"
+#include "../../../include/graphop_b200.h"
 
 namespace {
 
@@ -81,36 +82,10 @@ void check_status(int rc, const char* what) {
 }
 
 // ------------------------------------------------------------------------------------------
-// graphs: plans made by Python, views made here
+// calling the C ABI
 // ------------------------------------------------------------------------------------------
-struct Graph {
-  graphop_plan_t plan{};
-  std::vector<Tensor> keep;   // device memory the plan refers to
-};
-using GraphPtr = std::shared_ptr<Graph>;
-
 void check_chunks(const Tensor& row, const Tensor& indptr) {
   if (indptr.size(0) != row.size(0) + 1) fail("indptr must hold row.size(0) + 1 entries");
-}
-
-// The view of a chunk table; eid and indices may be undefined.  n_nodes < 0: for an op that walks no node rows.  clear: an
-// edge output that is zero where no chunk covers it, done on the way.
-GraphPtr view_of(const Tensor& row, const Tensor& indptr, const Tensor& eid, const Tensor& indices, int64_t n_edges,
-                 int64_t n_nodes, cudaStream_t stream, const Tensor& clear = Tensor()) {
-  const int ib = index_bytes_of({&row, &indptr, &eid, &indices});
-  const auto data = [](const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; };
-  auto g = std::make_shared<Graph>();
-  const size_t bytes = graphop_internal_view_bytes(n_edges, n_nodes, ib);
-  const Tensor memory = at::empty({(int64_t)bytes}, row.options().dtype(at::kByte));
-  check_status(graphop_internal_view_build(data(row), data(indptr), data(eid), data(indices), ib, row.size(0), n_edges,
-                                           n_nodes, data(clear), clear.defined() ? clear.nbytes() : 0, memory.data_ptr(), bytes,
-                                           &g->plan, (graphop_stream_t)stream),
-               "view_build");
-  g->keep = {memory};
-  // 32-bit index arrays are used where they are
-  for (const Tensor* t : {&eid, &indices})
-    if (ib == 4 && t->defined()) g->keep.push_back(*t);
-  return g;
 }
 
 // What one op call needs besides its tensors: device guard, stream, workspace.
@@ -121,15 +96,15 @@ struct Call {
   void* ws = nullptr;
   size_t bytes = 0;
   explicit Call(const Tensor& on) : guard(on.device()), stream(at::cuda::getCurrentCUDAStream(on.get_device())) {}
-  void workspace(int op, int64_t n_edges, int64_t n_nodes, int H, int D, const Tensor& like) {
-    bytes = graphop_workspace_bytes(op, n_edges, n_nodes, H, D, (int)like.element_size(), 4);
+  void workspace(int op, int64_t n_edges, int64_t n_nodes, int H, int D, const Tensor& like, int index_bytes = 4) {
+    bytes = graphop_workspace_bytes(op, n_edges, n_nodes, H, D, (int)like.element_size(), index_bytes);
     scratch = at::empty({(int64_t)bytes + 256}, like.options().dtype(at::kByte));
     ws = reinterpret_cast<void*>((reinterpret_cast<uintptr_t>(scratch.data_ptr()) + 255) / 256 * 256);
   }
 };
 
-// a tensor's storage as the element type the entry point wants
-template <typename E> E* ptr(const Tensor& t) { return reinterpret_cast<E*>(t.data_ptr()); }
+// a tensor's storage as the element type the entry point wants; null for an undefined one
+template <typename E> E* ptr(const Tensor& t) { return t.defined() ? reinterpret_cast<E*>(t.data_ptr()) : nullptr; }
 
 // f is called with a null pointer of the element type
 template <class F> auto by_elem(int elem, F&& f) {
@@ -137,46 +112,41 @@ template <class F> auto by_elem(int elem, F&& f) {
   if (elem == 1) return f((double*)nullptr);
   return f((uint16_t*)nullptr);
 }
+// and of the index type
+template <class F> auto by_types(int elem, int index_bytes, F&& f) {
+  return by_elem(elem, [&](auto* e) { return index_bytes == 8 ? f(e, (int64_t*)nullptr) : f(e, (int32_t*)nullptr); });
+}
 
-// one overload set per op over the three element types
+// one overload set per op over the three element types (and the two index types)
+#define GRAPHOP_OVERLOADS(op)                                                                                        \
+  template <class... X> int op(float*, int32_t*, X... x) { return graphop_##op##_f32_i32(x...); }                    \
+  template <class... X> int op(float*, int64_t*, X... x) { return graphop_##op##_f32_i64(x...); }                    \
+  template <class... X> int op(double*, int32_t*, X... x) { return graphop_##op##_f64_i32(x...); }                   \
+  template <class... X> int op(double*, int64_t*, X... x) { return graphop_##op##_f64_i64(x...); }                   \
+  template <class... X> int op(uint16_t*, int32_t*, X... x) { return graphop_##op##_bf16_i32(x...); }                \
+  template <class... X> int op(uint16_t*, int64_t*, X... x) { return graphop_##op##_bf16_i64(x...); }
+GRAPHOP_OVERLOADS(maskedmm_csr_forward)
+GRAPHOP_OVERLOADS(maskedmm_csr_backward)
+GRAPHOP_OVERLOADS(node_mul_edge_forward)
+GRAPHOP_OVERLOADS(node_mul_edge_backward)
+GRAPHOP_OVERLOADS(sparse_softmax_forward)
+GRAPHOP_OVERLOADS(sparse_softmax_backward)
+GRAPHOP_OVERLOADS(vector_spmm_forward)
+GRAPHOP_OVERLOADS(vector_spmm_backward)
+GRAPHOP_OVERLOADS(attention_bias_forward)
+GRAPHOP_OVERLOADS(attention_bias_backward)
+#undef GRAPHOP_OVERLOADS
 #define GRAPHOP_OVERLOADS(op)                                                                                        \
   template <class... X> int op(float*, X... x) { return graphop_##op##_f32(x...); }                                  \
   template <class... X> int op(double*, X... x) { return graphop_##op##_f64(x...); }                                 \
   template <class... X> int op(uint16_t*, X... x) { return graphop_##op##_bf16(x...); }
-GRAPHOP_OVERLOADS(maskedmm_csr_forward_planned)
-GRAPHOP_OVERLOADS(maskedmm_csr_backward_planned)
-GRAPHOP_OVERLOADS(node_mul_edge_forward_planned)
-GRAPHOP_OVERLOADS(node_mul_edge_backward_planned)
-GRAPHOP_OVERLOADS(sparse_softmax_forward_planned)
-GRAPHOP_OVERLOADS(sparse_softmax_backward_planned)
-GRAPHOP_OVERLOADS(vector_spmm_forward_planned)
-GRAPHOP_OVERLOADS(vector_spmm_backward_planned)
 GRAPHOP_OVERLOADS(attention_forward_planned)
 GRAPHOP_OVERLOADS(attention_backward_planned)
-GRAPHOP_OVERLOADS(internal_attention_bias_forward)
-GRAPHOP_OVERLOADS(internal_attention_bias_backward)
 #undef GRAPHOP_OVERLOADS
 
 // ------------------------------------------------------------------------------------------
-// the chunk-table arguments of one Function: views made when needed, versions checked in the backward
+// autograd nodes
 // ------------------------------------------------------------------------------------------
-struct Tables {
-  std::vector<Tensor> t;
-  std::vector<uint32_t> versions;
-  GraphPtr rows;
-  Tables(std::initializer_list<Tensor> list) : t(list) {
-    versions.reserve(t.size());
-    for (const Tensor& x : t) versions.push_back(x.defined() && !x.is_inference() ? x._version() : 0);
-  }
-  void check_unmodified() const {
-    for (size_t i = 0; i < t.size(); ++i)
-      if (t[i].defined() && !t[i].is_inference() && t[i]._version() != versions[i])
-        fail("one of the variables needed for gradient computation has been modified by an inplace operation: an index "
-             "tensor of a graphop function");
-  }
-};
-using TablesPtr = std::shared_ptr<Tables>;
-
 // Links `outputs` to a backward node of type N made from `inputs` (the differentiable ones, in the order of the
 // gradients the node returns) when any of them needs a gradient; `save` stores what the backward reads.
 template <class N, class Save>
@@ -206,106 +176,119 @@ Tensor edge_out(const Tensor& node, int64_t n_edges, int H) {
 }
 graphop_stream_t raw(cudaStream_t s) { return (graphop_stream_t)s; }
 
-// What a node of these ops keeps: written when the call is recorded and read-only from then on, but for `saved`, which a
-// backward that does not retain the graph releases.  Two threads may run the backward of one graph: `saved` is touched
-// under the node's mutex, everything else a backward makes is its own.
+// What a node of these ops keeps from its forward: the tensors of the call, index tensors included, as saved variables
+// (so that hooks see them, in-place changes are found and a backward that does not retain the graph lets go of them), and
+// nothing else: the tables that the kernels make of a chunk table are workspace of either direction.  Two threads may run
+// the backward of one graph: the saved tensors are read and released under the node's mutex.
 struct GraphNode : Node {
-  TablesPtr tables;             // chunk-table forms
-  std::vector<SavedVariable> saved;
   std::string name() const override { return "GraphopBackward"; }
+  void save(const Tensor& t, bool is_output = false) {
+    // an index tensor made in inference mode has no version to check: kept as it is
+    const bool plain = t.defined() && t.is_inference() && !at::isFloatingType(t.scalar_type());
+    saved.emplace_back(plain ? Tensor() : t, is_output);
+    unversioned.push_back(plain ? t : Tensor());
+  }
+  void save_all(std::initializer_list<Tensor> ts) {
+    saved.reserve(ts.size() + 2);
+    unversioned.reserve(ts.size() + 2);
+    for (const Tensor& t : ts) save(t);
+  }
   void release_variables() override {
     std::lock_guard<std::mutex> hold(mutex_);
     for (SavedVariable& s : saved) s.reset_data();
+    for (Tensor& t : unversioned) t = Tensor();
   }
   std::vector<Tensor> unpack_saved() {
     const std::shared_ptr<Node> self = shared_from_this();   // for a saved output
     std::lock_guard<std::mutex> hold(mutex_);
     std::vector<Tensor> t;
     t.reserve(saved.size());
-    for (const SavedVariable& s : saved) t.push_back(s.unpack(self));
+    for (size_t i = 0; i < saved.size(); ++i) t.push_back(unversioned[i].defined() ? unversioned[i] : saved[i].unpack(self));
     return t;
   }
+
+ private:
+  std::vector<SavedVariable> saved;
+  std::vector<Tensor> unversioned;
 };
+
+// The column side's arguments, which only the backward reads: wrong ones are reported there, as they always were.  t: the
+// call's index tensors, the four of the column side from t[at]; n: how many there are.
+int check_columns(const std::vector<Tensor>& t, size_t at, size_t n, const char* const (&names)[4]) {
+  for (int i = 0; i < 4; ++i) check_input(t[at + i], names[i]);
+  std::vector<const Tensor*> all;   // both orientations: one call has one index type
+  for (size_t i = 0; i < n; ++i) all.push_back(&t[i]);
+  const int ib = index_bytes_of(all);
+  check_chunks(t[at], t[at + 1]);
+  return ib;
+}
 
 // ---- SparseSoftmax (wrapper.py:8-18) ------------------------------------------------------
 struct SparseSoftmaxBackward : GraphNode {
   variable_list apply(variable_list&& grads) override {
     if (!grads[0].defined()) return {Tensor()};
-    tables->check_unmodified();
-    const std::vector<Tensor> kept = unpack_saved();
-    const Tensor y = kept[0], dy = upstream(grads, "dy");
-    const int elem = elem_of({&y, &dy}), H = edge_heads(dy);
+    const std::vector<Tensor> t = unpack_saved();   // row, indptr, eid, y
+    const Tensor &y = t[3], dy = upstream(grads, "dy");
+    const int elem = elem_of({&y, &dy}), ib = index_bytes_of({&t[0], &t[1], &t[2]}), H = edge_heads(dy);
     Call c(y);
     Tensor dx = at::empty_like(dy);
-    const int64_t e = tables->t[2].size(0);
+    const int64_t e = t[2].size(0), chunks = t[0].size(0);
     if (e == 0) return {dx};
-    c.workspace(GRAPHOP_OP_SOFTMAX_BWD, e, 0, H, 1, y);
-    const graphop_plan_t* p = &tables->rows->plan;
-    check_status(by_elem(elem, [&](auto* k) {
+    c.workspace(GRAPHOP_OP_SOFTMAX_BWD, e, 0, H, 1, y, ib);
+    check_status(by_types(elem, ib, [&](auto* k, auto* i) {
       using E = std::remove_pointer_t<decltype(k)>;
-      return sparse_softmax_backward_planned(k, p, (const E*)ptr<E>(y), (const E*)ptr<E>(dy), ptr<E>(dx), H, c.ws, c.bytes,
-                                             raw(c.stream));
+      using I = std::remove_pointer_t<decltype(i)>;
+      return sparse_softmax_backward(k, i, (const I*)ptr<I>(t[0]), (const I*)ptr<I>(t[1]), (const I*)ptr<I>(t[2]),
+                                     (const E*)ptr<E>(y), (const E*)ptr<E>(dy), ptr<E>(dx), chunks, e, (int64_t)0, H, c.ws,
+                                     c.bytes, raw(c.stream));
     }), "sparse_softmax_backward");
     return {dx};
   }
 };
 Tensor sparse_softmax(const Tensor& row, const Tensor& indptr, const Tensor& eid, const Tensor& x) {
   check_input(row, "row"); check_input(indptr, "indptr"); check_input(eid, "eid"); check_input(x, "x");
-  const int elem = elem_of({&x}), H = edge_heads(x);
-  index_bytes_of({&row, &indptr, &eid});
+  const int elem = elem_of({&x}), H = edge_heads(x), ib = index_bytes_of({&row, &indptr, &eid});
   check_chunks(row, indptr);
-  auto tb = std::make_shared<Tables>(std::initializer_list<Tensor>{row, indptr, eid});
   Call c(x);
-  const int64_t e = eid.size(0);
+  const int64_t e = eid.size(0), chunks = row.size(0);
   Tensor y = at::empty_like(x.detach());
   if (e > 0) {
-    tb->rows = view_of(row, indptr, eid, Tensor(), e, -1, c.stream, y);
-    c.workspace(GRAPHOP_OP_SOFTMAX_FWD, e, 0, H, 1, x);
-    graphop_plan_t cleared = tb->rows->plan;   // by the view, for this call's output
-    cleared.flags |= GRAPHOP_PLAN_COVERED;
-    const graphop_plan_t* p = &cleared;
-    check_status(by_elem(elem, [&](auto* k) {
+    c.workspace(GRAPHOP_OP_SOFTMAX_FWD, e, 0, H, 1, x, ib);
+    check_status(by_types(elem, ib, [&](auto* k, auto* i) {
       using E = std::remove_pointer_t<decltype(k)>;
-      return sparse_softmax_forward_planned(k, p, (const E*)ptr<E>(x), ptr<E>(y), H, c.ws, c.bytes, raw(c.stream));
+      using I = std::remove_pointer_t<decltype(i)>;
+      return sparse_softmax_forward(k, i, (const I*)ptr<I>(row), (const I*)ptr<I>(indptr), (const I*)ptr<I>(eid),
+                                    (const E*)ptr<E>(x), ptr<E>(y), chunks, e, (int64_t)0, H, c.ws, c.bytes, raw(c.stream));
     }), "sparse_softmax_forward");
   }
   record<SparseSoftmaxBackward>({x}, y, [&](SparseSoftmaxBackward& n) {
-    n.tables = tb;
-    n.saved.emplace_back(y, true);
+    n.save_all({row, indptr, eid});
+    n.save(y, true);
   });
   return y;
 }
 
 // ---- MaskedMMCSR (wrapper.py:20-30) -------------------------------------------------------
-// the view of the other orientation, whose tables start at t[at]
-GraphPtr column_view(const Tables& tb, int at, int64_t e, int64_t n_src, cudaStream_t stream) {
-  const char* names[] = {"col", "indptr", "eid", "indices"};
-  for (int i = 0; i < 4; ++i) check_input(tb.t[at + i], names[i]);
-  check_chunks(tb.t[at], tb.t[at + 1]);
-  std::vector<const Tensor*> all;   // both orientations: one call has one index type
-  for (const Tensor& t : tb.t) all.push_back(&t);
-  index_bytes_of(all);
-  return view_of(tb.t[at], tb.t[at + 1], tb.t[at + 2], tb.t[at + 3], e, n_src, stream);
-}
 struct MaskedMMBackward : GraphNode {
   variable_list apply(variable_list&& grads) override {
     if (!grads[0].defined()) return {Tensor(), Tensor()};
-    tables->check_unmodified();
-    const std::vector<Tensor> kept = unpack_saved();
-    const Tensor A = kept[0], B = kept[1], dy = upstream(grads, "dy");
+    const std::vector<Tensor> t = unpack_saved();   // row, indptr_r, eid_r, indices_r, col, indptr_c, eid_c, indices_c, A, B
+    const Tensor &A = t[8], &B = t[9], dy = upstream(grads, "dy");
     const int elem = elem_of({&A, &B, &dy});
+    const int ib = check_columns(t, 4, 8, {"col", "indptr_c", "eid_c", "indices_c"});
     const NodeShape s = node_shape(A);
     Call c(A);
-    const int64_t e = tables->t[2].size(0), nb = B.size(0);
+    const int64_t e = t[2].size(0), nb = B.size(0), chunks = t[0].size(0), chunks_c = t[4].size(0);
     Tensor dA = at::empty_like(A.detach()), dB = at::empty_like(B.detach());
     if (e == 0) return {dA.zero_(), dB.zero_()};
-    const GraphPtr cols = column_view(*tables, 4, e, nb, c.stream);
-    c.workspace(GRAPHOP_OP_MASKEDMM_BWD, e, std::max(s.n, nb), s.H, s.D, A);
-    const graphop_plan_t *pr = &tables->rows->plan, *pc = &cols->plan;
-    check_status(by_elem(elem, [&](auto* k) {
+    c.workspace(GRAPHOP_OP_MASKEDMM_BWD, e, std::max(s.n, nb), s.H, s.D, A, ib);
+    check_status(by_types(elem, ib, [&](auto* k, auto* i) {
       using E = std::remove_pointer_t<decltype(k)>;
-      return maskedmm_csr_backward_planned(k, pr, pc, (const E*)ptr<E>(A), (const E*)ptr<E>(B), (const E*)ptr<E>(dy),
-                                           ptr<E>(dA), ptr<E>(dB), s.n, nb, s.H, s.D, c.ws, c.bytes, raw(c.stream));
+      using I = std::remove_pointer_t<decltype(i)>;
+      const auto in = [&](int at) { return (const I*)ptr<I>(t[at]); };
+      return maskedmm_csr_backward(k, i, in(0), in(1), in(2), in(3), chunks, in(4), in(5), in(6), in(7), chunks_c,
+                                   (const E*)ptr<E>(A), (const E*)ptr<E>(B), (const E*)ptr<E>(dy), ptr<E>(dA), ptr<E>(dB), e,
+                                   s.n, nb, s.H, s.D, c.ws, c.bytes, raw(c.stream));
     }), "maskedmm_csr_backward");
     return {dA, dB};
   }
@@ -315,32 +298,24 @@ Tensor maskedmm_csr(const Tensor& row, const Tensor& indptr_r, const Tensor& eid
                     const Tensor& A, const Tensor& B) {
   check_input(row, "row"); check_input(indptr_r, "indptr"); check_input(eid_r, "eid"); check_input(indices_r, "indices");
   check_input(A, "A"); check_input(B, "B");
-  const int elem = elem_of({&A, &B});
-  index_bytes_of({&row, &indptr_r, &eid_r, &indices_r});
+  const int elem = elem_of({&A, &B}), ib = index_bytes_of({&row, &indptr_r, &eid_r, &indices_r});
   const NodeShape s = node_shape(A);
   check_chunks(row, indptr_r);
-  auto tb = std::make_shared<Tables>(
-      std::initializer_list<Tensor>{row, indptr_r, eid_r, indices_r, col, indptr_c, eid_c, indices_c});
   Call c(A);
-  const int64_t e = eid_r.size(0), nb = B.size(0);
+  const int64_t e = eid_r.size(0), nb = B.size(0), chunks = row.size(0);
   Tensor y = edge_out(A, e, s.H);
   if (e > 0) {
-    tb->rows = view_of(row, indptr_r, eid_r, indices_r, e, s.n, c.stream, y);
-    c.workspace(GRAPHOP_OP_MASKEDMM_FWD, e, std::max(s.n, nb), s.H, s.D, A);
-    graphop_plan_t cleared = tb->rows->plan;   // by the view, for this call's output
-    cleared.flags |= GRAPHOP_PLAN_COVERED;
-    const graphop_plan_t* p = &cleared;
-    check_status(by_elem(elem, [&](auto* k) {
+    c.workspace(GRAPHOP_OP_MASKEDMM_FWD, e, std::max(s.n, nb), s.H, s.D, A, ib);
+    check_status(by_types(elem, ib, [&](auto* k, auto* i) {
       using E = std::remove_pointer_t<decltype(k)>;
-      return maskedmm_csr_forward_planned(k, p, (const E*)ptr<E>(A), (const E*)ptr<E>(B), ptr<E>(y), s.n, nb, s.H, s.D, c.ws,
-                                          c.bytes, raw(c.stream));
+      using I = std::remove_pointer_t<decltype(i)>;
+      return maskedmm_csr_forward(k, i, (const I*)ptr<I>(row), (const I*)ptr<I>(indptr_r), (const I*)ptr<I>(eid_r),
+                                  (const I*)ptr<I>(indices_r), (const E*)ptr<E>(A), (const E*)ptr<E>(B), ptr<E>(y), chunks, e,
+                                  s.n, nb, s.H, s.D, c.ws, c.bytes, raw(c.stream));
     }), "maskedmm_csr_forward");
   }
   record<MaskedMMBackward>({A, B}, y, [&](MaskedMMBackward& n) {
-    // the backward reads the column side; wrong tensors are reported there, as its arguments always were
-    n.tables = tb;
-    n.saved.emplace_back(A, false);
-    n.saved.emplace_back(B, false);
+    n.save_all({row, indptr_r, eid_r, indices_r, col, indptr_c, eid_c, indices_c, A, B});
   });
   return y;
 }
@@ -349,52 +324,44 @@ Tensor maskedmm_csr(const Tensor& row, const Tensor& indptr_r, const Tensor& eid
 struct NodeMulEdgeBackward : GraphNode {
   variable_list apply(variable_list&& grads) override {
     if (!grads[0].defined()) return {Tensor(), Tensor()};
-    tables->check_unmodified();
-    const std::vector<Tensor> kept = unpack_saved();
-    const Tensor A = kept[0], B = kept[1], dy = upstream(grads, "dy");
-    const int elem = elem_of({&A, &B, &dy});
+    const std::vector<Tensor> t = unpack_saved();   // row, indptr, eid, A, B
+    const Tensor &A = t[3], &B = t[4], dy = upstream(grads, "dy");
+    const int elem = elem_of({&A, &B, &dy}), ib = index_bytes_of({&t[0], &t[1], &t[2]});
     const NodeShape s = node_shape(A);
     Call c(A);
-    const int64_t e = tables->t[2].size(0);
+    const int64_t e = t[2].size(0), chunks = t[0].size(0);
     Tensor dA = at::empty_like(A.detach()), dB = at::empty_like(B.detach());
     if (e == 0) return {dA.zero_(), dB};
-    c.workspace(GRAPHOP_OP_NODE_MUL_EDGE_BWD, e, s.n, s.H, s.D, A);
-    const graphop_plan_t* p = &tables->rows->plan;
-    check_status(by_elem(elem, [&](auto* k) {
+    c.workspace(GRAPHOP_OP_NODE_MUL_EDGE_BWD, e, s.n, s.H, s.D, A, ib);
+    check_status(by_types(elem, ib, [&](auto* k, auto* i) {
       using E = std::remove_pointer_t<decltype(k)>;
-      return node_mul_edge_backward_planned(k, p, (const E*)ptr<E>(A), (const E*)ptr<E>(B), (const E*)ptr<E>(dy), ptr<E>(dA),
-                                            ptr<E>(dB), s.n, s.H, s.D, c.ws, c.bytes, raw(c.stream));
+      using I = std::remove_pointer_t<decltype(i)>;
+      return node_mul_edge_backward(k, i, (const I*)ptr<I>(t[0]), (const I*)ptr<I>(t[1]), (const I*)ptr<I>(t[2]),
+                                    (const E*)ptr<E>(A), (const E*)ptr<E>(B), (const E*)ptr<E>(dy), ptr<E>(dA), ptr<E>(dB),
+                                    chunks, e, s.n, s.H, s.D, c.ws, c.bytes, raw(c.stream));
     }), "node_mul_edge_backward");
     return {dA, dB};
   }
 };
 Tensor node_mul_edge(const Tensor& row, const Tensor& indptr, const Tensor& eid, const Tensor& A, const Tensor& B) {
   check_input(row, "row"); check_input(indptr, "indptr"); check_input(eid, "eid"); check_input(A, "A"); check_input(B, "B");
-  const int elem = elem_of({&A, &B});
-  index_bytes_of({&row, &indptr, &eid});
+  const int elem = elem_of({&A, &B}), ib = index_bytes_of({&row, &indptr, &eid});
   const NodeShape s = node_shape(A);
   check_chunks(row, indptr);
-  auto tb = std::make_shared<Tables>(std::initializer_list<Tensor>{row, indptr, eid});
   Call c(A);
-  const int64_t e = eid.size(0);
+  const int64_t e = eid.size(0), chunks = row.size(0);
   Tensor y = edge_out(A, e, s.H);
   if (e > 0) {
-    tb->rows = view_of(row, indptr, eid, Tensor(), e, s.n, c.stream, y);
-    c.workspace(GRAPHOP_OP_NODE_MUL_EDGE_FWD, e, s.n, s.H, s.D, A);
-    graphop_plan_t cleared = tb->rows->plan;   // by the view, for this call's output
-    cleared.flags |= GRAPHOP_PLAN_COVERED;
-    const graphop_plan_t* p = &cleared;
-    check_status(by_elem(elem, [&](auto* k) {
+    c.workspace(GRAPHOP_OP_NODE_MUL_EDGE_FWD, e, s.n, s.H, s.D, A, ib);
+    check_status(by_types(elem, ib, [&](auto* k, auto* i) {
       using E = std::remove_pointer_t<decltype(k)>;
-      return node_mul_edge_forward_planned(k, p, (const E*)ptr<E>(A), (const E*)ptr<E>(B), ptr<E>(y), s.n, s.H, s.D, c.ws,
-                                           c.bytes, raw(c.stream));
+      using I = std::remove_pointer_t<decltype(i)>;
+      return node_mul_edge_forward(k, i, (const I*)ptr<I>(row), (const I*)ptr<I>(indptr), (const I*)ptr<I>(eid),
+                                   (const E*)ptr<E>(A), (const E*)ptr<E>(B), ptr<E>(y), chunks, e, s.n, s.H, s.D, c.ws, c.bytes,
+                                   raw(c.stream));
     }), "node_mul_edge_forward");
   }
-  record<NodeMulEdgeBackward>({A, B}, y, [&](NodeMulEdgeBackward& n) {
-    n.tables = tb;
-    n.saved.emplace_back(A, false);
-    n.saved.emplace_back(B, false);
-  });
+  record<NodeMulEdgeBackward>({A, B}, y, [&](NodeMulEdgeBackward& n) { n.save_all({row, indptr, eid, A, B}); });
   return y;
 }
 
@@ -402,22 +369,23 @@ Tensor node_mul_edge(const Tensor& row, const Tensor& indptr, const Tensor& eid,
 struct VectorSPMMBackward : GraphNode {
   variable_list apply(variable_list&& grads) override {
     if (!grads[0].defined()) return {Tensor(), Tensor()};
-    tables->check_unmodified();
-    const std::vector<Tensor> kept = unpack_saved();
-    const Tensor w = kept[0], x = kept[1], dy = upstream(grads, "dy");
+    const std::vector<Tensor> t = unpack_saved();   // row, indptr, eid, indices, col, indptr_t, eid_t, indices_t, w, x
+    const Tensor &w = t[8], &x = t[9], dy = upstream(grads, "dy");
     const int elem = elem_of({&w, &dy, &x});
+    const int ib = check_columns(t, 4, 8, {"col", "indptr_t", "eid_t", "indices_t"});
     const NodeShape s = node_shape(x);
     Call c(x);
-    const int64_t e = tables->t[2].size(0), n_dst = dy.size(0);
+    const int64_t e = t[2].size(0), n_dst = dy.size(0), chunks = t[0].size(0), chunks_t = t[4].size(0);
     Tensor dw = at::empty_like(w.detach()), dx = at::empty_like(x.detach());
     if (e == 0) return {dw, dx.zero_()};
-    const GraphPtr cols = column_view(*tables, 4, e, s.n, c.stream);
-    c.workspace(GRAPHOP_OP_SPMM_BWD, e, std::max(n_dst, s.n), s.H, s.D, x);
-    const graphop_plan_t *pr = &tables->rows->plan, *pt = &cols->plan;
-    check_status(by_elem(elem, [&](auto* k) {
+    c.workspace(GRAPHOP_OP_SPMM_BWD, e, std::max(n_dst, s.n), s.H, s.D, x, ib);
+    check_status(by_types(elem, ib, [&](auto* k, auto* i) {
       using E = std::remove_pointer_t<decltype(k)>;
-      return vector_spmm_backward_planned(k, pr, pt, (const E*)ptr<E>(w), (const E*)ptr<E>(dy), (const E*)ptr<E>(x),
-                                          ptr<E>(dw), ptr<E>(dx), n_dst, s.n, s.H, s.D, c.ws, c.bytes, raw(c.stream));
+      using I = std::remove_pointer_t<decltype(i)>;
+      const auto in = [&](int at) { return (const I*)ptr<I>(t[at]); };
+      return vector_spmm_backward(k, i, in(0), in(1), in(2), in(3), chunks, in(4), in(5), in(6), in(7), chunks_t,
+                                  (const E*)ptr<E>(w), (const E*)ptr<E>(dy), (const E*)ptr<E>(x), ptr<E>(dw), ptr<E>(dx), e,
+                                  n_dst, s.n, s.H, s.D, c.ws, c.bytes, raw(c.stream));
     }), "vector_spmm_backward");
     return {dw, dx};
   }
@@ -426,148 +394,165 @@ Tensor vector_spmm(const Tensor& row, const Tensor& indptr, const Tensor& eid, c
                    const Tensor& indptr_t, const Tensor& eid_t, const Tensor& indices_t, const Tensor& w, const Tensor& x) {
   check_input(row, "row"); check_input(indptr, "indptr"); check_input(eid, "eid"); check_input(indices, "indices");
   check_input(w, "edata"); check_input(x, "x");
-  const int elem = elem_of({&w, &x});
-  index_bytes_of({&row, &indptr, &eid, &indices});
+  const int elem = elem_of({&w, &x}), ib = index_bytes_of({&row, &indptr, &eid, &indices});
   const NodeShape s = node_shape(x);
   if (edge_heads(w) != s.H) fail("edata and x disagree on the number of heads");
   check_chunks(row, indptr);
-  auto tb = std::make_shared<Tables>(std::initializer_list<Tensor>{row, indptr, eid, indices, col, indptr_t, eid_t, indices_t});
   Call c(x);
-  const int64_t e = eid.size(0);
+  const int64_t e = eid.size(0), chunks = row.size(0);
   Tensor y = at::empty(x.sizes(), x.options());
   if (e == 0) {
     y.zero_();
   } else {
-    tb->rows = view_of(row, indptr, eid, indices, e, s.n, c.stream);
-    c.workspace(GRAPHOP_OP_SPMM_FWD, e, s.n, s.H, s.D, x);
-    const graphop_plan_t* p = &tb->rows->plan;
-    check_status(by_elem(elem, [&](auto* k) {
+    c.workspace(GRAPHOP_OP_SPMM_FWD, e, s.n, s.H, s.D, x, ib);
+    check_status(by_types(elem, ib, [&](auto* k, auto* i) {
       using E = std::remove_pointer_t<decltype(k)>;
-      return vector_spmm_forward_planned(k, p, (const E*)ptr<E>(w), (const E*)ptr<E>(x), ptr<E>(y), s.n, s.n, s.H, s.D, c.ws,
-                                         c.bytes, raw(c.stream));
+      using I = std::remove_pointer_t<decltype(i)>;
+      return vector_spmm_forward(k, i, (const I*)ptr<I>(row), (const I*)ptr<I>(indptr), (const I*)ptr<I>(eid),
+                                 (const I*)ptr<I>(indices), (const E*)ptr<E>(w), (const E*)ptr<E>(x), ptr<E>(y), chunks, e, s.n,
+                                 s.n, s.H, s.D, c.ws, c.bytes, raw(c.stream));
     }), "vector_spmm_forward");
   }
   record<VectorSPMMBackward>({w, x}, y, [&](VectorSPMMBackward& n) {
-    n.tables = tb;
-    n.saved.emplace_back(w, false);
-    n.saved.emplace_back(x, false);
+    n.save_all({row, indptr, eid, indices, col, indptr_t, eid_t, indices_t, w, x});
   });
   return y;
 }
 
-// ---- fused attention on plans, with and without the edge term ------------------------------
-struct AttentionBackward : GraphNode {
-  GraphPtr rows, cols;   // cols: null for chunk tables
-  double scale = 1.0;
-  bool bias = false;
-  variable_list apply(variable_list&& grads) override {
-    const size_t n_out = bias ? 4 : 3;
-    if (!grads[0].defined()) return variable_list(n_out);
-    if (tables) tables->check_unmodified();
-    const std::vector<Tensor> kept = unpack_saved();
-    const Tensor q = kept[0], k = kept[1], v = kept[2], o = kept[3], lse = kept[4], rel = bias ? kept[5] : Tensor(),
-                 g = upstream(grads, "d_o");
-    const int elem = elem_of({&q, &k, &v, &o, &g});
-    const NodeShape s = node_shape(q);
-    Call c(q);
-    Tensor dq = at::empty_like(q.detach()), dk = at::empty_like(k.detach()), dv = at::empty_like(v.detach());
-    Tensor drel = bias ? at::empty_like(rel.detach()) : Tensor();
-    const int64_t nk = k.size(0);
-    if (rows->plan.n_edges == 0) {
-      variable_list out{dq.zero_(), dk.zero_(), dv.zero_()};
-      if (bias) out.push_back(drel);
-      return out;
-    }
-    const GraphPtr other = cols ? cols : column_view(*tables, 3, rows->plan.n_edges, nk, c.stream);
-    const graphop_plan_t *pr = &rows->plan, *pt = &other->plan;
-    c.workspace(pt->eid ? GRAPHOP_OP_ATTENTION_BWD_PAIRS : GRAPHOP_OP_ATTENTION_BWD, rows->plan.n_edges, std::max(s.n, nk), s.H,
-                s.D, q);
-    check_status(by_elem(elem, [&](auto* e) {
-      using E = std::remove_pointer_t<decltype(e)>;
-      if (bias)
-        return internal_attention_bias_backward(
-            e, pr, pt, (const void*)ptr<E>(q), (const void*)ptr<E>(k), (const void*)ptr<E>(v), (const void*)ptr<E>(rel),
-            (const void*)ptr<E>(o), (const void*)lse.data_ptr(), (const void*)ptr<E>(g), scale, (void*)ptr<E>(dq),
-            (void*)ptr<E>(dk), (void*)ptr<E>(dv), (void*)ptr<E>(drel), s.n, nk, s.H, s.D, c.ws, c.bytes, raw(c.stream));
-      return attention_backward_planned(e, pr, pt, (const E*)ptr<E>(q), (const E*)ptr<E>(k), (const E*)ptr<E>(v),
-                                        (const E*)ptr<E>(o), (const void*)lse.data_ptr(), (const E*)ptr<E>(g), scale,
-                                        ptr<E>(dq), ptr<E>(dk), ptr<E>(dv), s.n, nk, s.H, s.D, c.ws, c.bytes, raw(c.stream));
-    }), bias ? "attention_bias_backward" : "attention_backward");
-    variable_list out{dq, dk, dv};
-    if (bias) out.push_back(drel);
-    return out;
-  }
-};
-
-Tensor attention_common(const GraphPtr& rows, const GraphPtr& cols, const TablesPtr& tables, Call& c, const Tensor& q,
-                        const Tensor& k, const Tensor& v, const Tensor& rel, double scale) {
-  const bool bias = rel.defined();
-  const int elem = elem_of({&q, &k, &v});
-  const NodeShape s = node_shape(q);
-  const int64_t nk = k.size(0);
-  Tensor o = at::empty_like(q.detach());
-  Tensor lse = at::empty({s.n, s.H}, q.options().dtype(elem == 1 ? at::kDouble : at::kFloat));
-  if (rows->plan.n_edges == 0) {
-    o.zero_();
-    lse.fill_(-std::numeric_limits<double>::infinity());
-  } else {
-    c.workspace(GRAPHOP_OP_ATTENTION_FWD, rows->plan.n_edges, std::max(s.n, nk), s.H, s.D, q);
-    const graphop_plan_t* p = &rows->plan;
-    check_status(by_elem(elem, [&](auto* e) {
-      using E = std::remove_pointer_t<decltype(e)>;
-      if (bias)
-        return internal_attention_bias_forward(e, p, (const void*)ptr<E>(q), (const void*)ptr<E>(k), (const void*)ptr<E>(v),
-                                               (const void*)ptr<E>(rel), scale, (void*)ptr<E>(o), (void*)lse.data_ptr(),
-                                               s.n, nk, s.H, s.D, c.ws, c.bytes, raw(c.stream));
-      return attention_forward_planned(e, p, (const E*)ptr<E>(q), (const E*)ptr<E>(k), (const E*)ptr<E>(v), scale, ptr<E>(o),
-                                       (void*)lse.data_ptr(), s.n, nk, s.H, s.D, c.ws, c.bytes, raw(c.stream));
-    }), bias ? "attention_bias_forward" : "attention_forward");
-  }
-  auto save = [&](AttentionBackward& n) {
-    n.tables = tables;
-    n.rows = rows;
-    n.cols = cols;
-    n.scale = scale;
-    n.bias = bias;
-    for (const Tensor* t : {&q, &k, &v}) n.saved.emplace_back(*t, false);
-    n.saved.emplace_back(o, true);
-    n.saved.emplace_back(lse, false);
-    if (bias) n.saved.emplace_back(rel, false);
-  };
-  if (bias) record<AttentionBackward>({q, k, v, rel}, o, save);
-  else record<AttentionBackward>({q, k, v}, o, save);
-  return o;
-}
-
+// ---- fused attention on plans --------------------------------------------------------------
 // A plan built by graphop.GraphPlan: the struct is copied, the memory it refers to kept alive.
+struct Graph {
+  graphop_plan_t plan{};
+  std::vector<Tensor> keep;
+};
+using GraphPtr = std::shared_ptr<Graph>;
 struct PlanHandle {
   GraphPtr graph;
   PlanHandle(uintptr_t address, std::vector<Tensor> keep) : graph(std::make_shared<Graph>()) {
     graph->plan = *reinterpret_cast<const graphop_plan_t*>(address);
     graph->keep = std::move(keep);
-      }
+  }
+};
+Tensor lse_like(const Tensor& q, const NodeShape& s, int elem) {
+  return at::empty({s.n, s.H}, q.options().dtype(elem == 1 ? at::kDouble : at::kFloat));
+}
+void no_edges(Tensor& o, Tensor& lse) {
+  o.zero_();
+  lse.fill_(-std::numeric_limits<double>::infinity());
+}
+
+struct AttentionBackward : GraphNode {
+  GraphPtr rows, cols;
+  double scale = 1.0;
+  variable_list apply(variable_list&& grads) override {
+    if (!grads[0].defined()) return variable_list(3);
+    const std::vector<Tensor> t = unpack_saved();   // q, k, v, lse, o
+    const Tensor &q = t[0], &k = t[1], &v = t[2], &lse = t[3], &o = t[4], g = upstream(grads, "d_o");
+    const int elem = elem_of({&q, &k, &v, &o, &g});
+    const NodeShape s = node_shape(q);
+    Call c(q);
+    Tensor dq = at::empty_like(q.detach()), dk = at::empty_like(k.detach()), dv = at::empty_like(v.detach());
+    const int64_t nk = k.size(0);
+    const graphop_plan_t *pr = &rows->plan, *pt = &cols->plan;
+    if (pr->n_edges == 0) return {dq.zero_(), dk.zero_(), dv.zero_()};
+    c.workspace(pt->eid ? GRAPHOP_OP_ATTENTION_BWD_PAIRS : GRAPHOP_OP_ATTENTION_BWD, pr->n_edges, std::max(s.n, nk), s.H, s.D, q);
+    check_status(by_elem(elem, [&](auto* e) {
+      using E = std::remove_pointer_t<decltype(e)>;
+      return attention_backward_planned(e, pr, pt, (const E*)ptr<E>(q), (const E*)ptr<E>(k), (const E*)ptr<E>(v),
+                                        (const E*)ptr<E>(o), (const void*)lse.data_ptr(), (const E*)ptr<E>(g), scale,
+                                        ptr<E>(dq), ptr<E>(dk), ptr<E>(dv), s.n, nk, s.H, s.D, c.ws, c.bytes, raw(c.stream));
+    }), "attention_backward");
+    return {dq, dk, dv};
+  }
 };
 Tensor attention_planned(const PlanHandle& plan_r, const PlanHandle& plan_t, const Tensor& q, const Tensor& k,
                          const Tensor& v, double scale) {
   check_input(q, "q"); check_input(k, "k"); check_input(v, "v");
+  const int elem = elem_of({&q, &k, &v});
+  const NodeShape s = node_shape(q);
+  const int64_t nk = k.size(0);
   Call c(q);
-  return attention_common(plan_r.graph, plan_t.graph, nullptr, c, q, k, v, Tensor(), scale);
+  Tensor o = at::empty_like(q.detach()), lse = lse_like(q, s, elem);
+  const graphop_plan_t* p = &plan_r.graph->plan;
+  if (p->n_edges == 0) {
+    no_edges(o, lse);
+  } else {
+    c.workspace(GRAPHOP_OP_ATTENTION_FWD, p->n_edges, std::max(s.n, nk), s.H, s.D, q);
+    check_status(by_elem(elem, [&](auto* e) {
+      using E = std::remove_pointer_t<decltype(e)>;
+      return attention_forward_planned(e, p, (const E*)ptr<E>(q), (const E*)ptr<E>(k), (const E*)ptr<E>(v), scale, ptr<E>(o),
+                                       (void*)lse.data_ptr(), s.n, nk, s.H, s.D, c.ws, c.bytes, raw(c.stream));
+    }), "attention_forward");
+  }
+  record<AttentionBackward>({q, k, v}, o, [&](AttentionBackward& n) {
+    n.rows = plan_r.graph;
+    n.cols = plan_t.graph;
+    n.scale = scale;
+    n.save_all({q, k, v, lse});
+    n.save(o, true);
+  });
+  return o;
 }
+
+// ---- fused attention with an edge term on chunk tables --------------------------------------
+struct AttentionBiasBackward : GraphNode {
+  double scale = 1.0;
+  variable_list apply(variable_list&& grads) override {
+    if (!grads[0].defined()) return variable_list(4);
+    // row, indptr, indices, col, indptr_t, eid_t, indices_t, q, k, v, rel, lse, o
+    const std::vector<Tensor> t = unpack_saved();
+    const Tensor &q = t[7], &k = t[8], &v = t[9], &rel = t[10], &lse = t[11], &o = t[12], g = upstream(grads, "d_o");
+    const int ib = check_columns(t, 3, 7, {"col", "indptr_t", "eid_t", "indices_t"});
+    const int elem = elem_of({&q, &k, &v, &rel, &o, &g});
+    const NodeShape s = node_shape(q);
+    Call c(q);
+    const int64_t e = t[2].size(0), nk = k.size(0), chunks = t[0].size(0), chunks_t = t[3].size(0);
+    Tensor dq = at::empty_like(q.detach()), dk = at::empty_like(k.detach()), dv = at::empty_like(v.detach()),
+           drel = at::empty_like(rel.detach());
+    if (e == 0) return {dq.zero_(), dk.zero_(), dv.zero_(), drel};
+    c.workspace(GRAPHOP_OP_ATTENTION_BWD_PAIRS, e, std::max(s.n, nk), s.H, s.D, q, ib);
+    check_status(by_types(elem, ib, [&](auto* x, auto* i) {
+      using E = std::remove_pointer_t<decltype(x)>;
+      using I = std::remove_pointer_t<decltype(i)>;
+      const auto in = [&](int at) { return (const I*)ptr<I>(t[at]); };
+      return attention_bias_backward(x, i, in(0), in(1), in(2), chunks, in(3), in(4), in(5), in(6), chunks_t,
+                                     (const E*)ptr<E>(q), (const E*)ptr<E>(k), (const E*)ptr<E>(v), (const E*)ptr<E>(rel),
+                                     (const E*)ptr<E>(o), (const void*)lse.data_ptr(), (const E*)ptr<E>(g), scale, ptr<E>(dq),
+                                     ptr<E>(dk), ptr<E>(dv), ptr<E>(drel), e, s.n, nk, s.H, s.D, c.ws, c.bytes, raw(c.stream));
+    }), "attention_bias_backward");
+    return {dq, dk, dv, drel};
+  }
+};
 Tensor attention_bias(const Tensor& row, const Tensor& indptr, const Tensor& indices, const Tensor& col,
                       const Tensor& indptr_t, const Tensor& eid_t, const Tensor& indices_t, const Tensor& q,
                       const Tensor& k, const Tensor& v, const Tensor& rel, double scale) {
   check_input(row, "row"); check_input(indptr, "indptr"); check_input(indices, "indices");
   check_input(q, "q"); check_input(k, "k"); check_input(v, "v"); check_input(rel, "rel");
-  elem_of({&q, &k, &v, &rel});
-  index_bytes_of({&row, &indptr, &indices});
+  const int elem = elem_of({&q, &k, &v, &rel}), ib = index_bytes_of({&row, &indptr, &indices});
   const NodeShape s = node_shape(q);
   check_chunks(row, indptr);
-  const int64_t e = indices.size(0);
+  const int64_t e = indices.size(0), nk = k.size(0), chunks = row.size(0);
   if (rel.dim() != 2 || rel.size(0) != e || rel.size(1) != s.D) fail("rel must be (e, d)");
-  auto tb = std::make_shared<Tables>(std::initializer_list<Tensor>{row, indptr, indices, col, indptr_t, eid_t, indices_t});
   Call c(q);
-  GraphPtr rows = e > 0 ? view_of(row, indptr, Tensor(), indices, e, s.n, c.stream) : std::make_shared<Graph>();
-  return attention_common(rows, nullptr, tb, c, q, k, v, rel, scale);
+  Tensor o = at::empty_like(q.detach()), lse = lse_like(q, s, elem);
+  if (e == 0) {
+    no_edges(o, lse);
+  } else {
+    c.workspace(GRAPHOP_OP_ATTENTION_FWD, e, std::max(s.n, nk), s.H, s.D, q, ib);
+    check_status(by_types(elem, ib, [&](auto* x, auto* i) {
+      using E = std::remove_pointer_t<decltype(x)>;
+      using I = std::remove_pointer_t<decltype(i)>;
+      return attention_bias_forward(x, i, (const I*)ptr<I>(row), (const I*)ptr<I>(indptr), (const I*)ptr<I>(indices), chunks,
+                                    (const E*)ptr<E>(q), (const E*)ptr<E>(k), (const E*)ptr<E>(v), (const E*)ptr<E>(rel), scale,
+                                    ptr<E>(o), (void*)lse.data_ptr(), e, s.n, nk, s.H, s.D, c.ws, c.bytes, raw(c.stream));
+    }), "attention_bias_forward");
+  }
+  record<AttentionBiasBackward>({q, k, v, rel}, o, [&](AttentionBiasBackward& n) {
+    n.scale = scale;
+    n.save_all({row, indptr, indices, col, indptr_t, eid_t, indices_t, q, k, v, rel, lse});
+    n.save(o, true);
+  });
+  return o;
 }
 
 // ---- graph preparation: graphop.py's functions of the same names ---------------------------

@@ -853,25 +853,6 @@ inline int attention_bias_backward(const GS& gs_r, const GS& gs_c, bool has_eid_
 }
 
 template <typename T>
-inline int attention_bias_forward_planned(const graphop_plan_t* plan, const T* q, const T* k, const T* v, const T* rel,
-                                          double scale, T* o, void* lse, long long n_dst, long long n_src, int H, int D,
-                                          void* ws, size_t wsb, cudaStream_t st) {
-  if (!plan) return GRAPHOP_ERR_INVALID_ARGUMENT;
-  return attention_bias_forward<T>(FromPlan{plan}, plan->n_chunks, q, k, v, rel, scale, o, lse, plan->n_edges, n_dst,
-                                   n_src, H, D, ws, wsb, st);
-}
-template <typename T>
-inline int attention_bias_backward_planned(const graphop_plan_t* plan_r, const graphop_plan_t* plan_t, const T* q,
-                                           const T* k, const T* v, const T* rel, const T* o, const void* lse,
-                                           const T* dout, double scale, T* dq, T* dk, T* dv, T* d_rel, long long n_dst,
-                                           long long n_src, int H, int D, void* ws, size_t wsb, cudaStream_t st) {
-  if (!plan_r || !plan_t) return GRAPHOP_ERR_INVALID_ARGUMENT;
-  return attention_bias_backward<T>(FromPlan{plan_r}, FromPlan{plan_t}, plan_t->eid != nullptr, plan_r->n_chunks,
-                                    plan_t->n_chunks, q, k, v, rel, o, lse, dout, scale, dq, dk, dv, d_rel,
-                                    plan_r->n_edges, n_dst, n_src, H, D, ws, wsb, st);
-}
-
-template <typename T>
 inline int attention_backward_planned(const graphop_plan_t* plan_r, const graphop_plan_t* plan_t, const T* q,
                                       const T* k, const T* v, const T* o, const void* lse, const T* dout, double scale,
                                       T* dq, T* dk, T* dv, long long n_dst, long long n_src, int H, int D, void* ws,

@@ -6,7 +6,6 @@
 #include <climits>
 
 #include "gk_host.cuh"
-#include "graphop_internal.h"
 
 namespace gk {
 
@@ -202,35 +201,6 @@ inline int plan_build(const I* row, const I* indptr, const I* eid, const I* indi
   plan->flags |= GRAPHOP_PLAN_ROW_TILES;
   if (!host.row_crosses) plan->flags |= GRAPHOP_PLAN_NO_CARRY;
   if (back.cover.cover_hi - back.cover.cover_lo >= E) plan->flags |= GRAPHOP_PLAN_COVERED;
-  return GRAPHOP_OK;
-}
-
-// A plan without the shape analysis, built without waiting (graphop_internal.h).
-inline size_t view_bytes(long long E, long long n_nodes, int index_bytes) {
-  size_t b = align_up((size_t)E * 4) + align_up(sizeof(PlanHeader));
-  if (n_nodes >= 0) b += align_up((size_t)(tile_count(E, n_nodes, tile_cost(E, n_nodes)) + 1) * 4);
-  if (index_bytes == 8) b += 2 * align_up((size_t)E * 4);
-  return b + kAlign;
-}
-template <typename I>
-inline int view_build(const I* row, const I* indptr, const I* eid, const I* indices, long long C, long long E,
-                      long long n_nodes, Clear clear, void* memory, size_t bytes, graphop_plan_t* plan, cudaStream_t st) {
-  *plan = graphop_plan_t{};
-  if (C < 0 || E < 1 || E >= (1LL << 31) || n_nodes >= (1LL << 31)) return GRAPHOP_ERR_INVALID_ARGUMENT;
-  if (!indptr || (C > 0 && !row)) return GRAPHOP_ERR_INVALID_ARGUMENT;
-  GK_TRY(check_ws(memory));
-  Arena ar(memory, bytes);
-  GraphView g{};
-  GK_TRY(prepare_graph<I>(ar, row, indptr, eid, indices, C, E, n_nodes, st, &g, clear));
-  plan->n_chunks = C;
-  plan->n_edges = E;
-  plan->n_nodes = n_nodes > 0 ? n_nodes : 0;
-  plan->header = g.hdr;
-  plan->erow = g.erow;
-  plan->other = g.other;
-  plan->eid = g.eid;
-  plan->tile = g.tile;
-  plan->tile_start = g.tile_start;
   return GRAPHOP_OK;
 }
 

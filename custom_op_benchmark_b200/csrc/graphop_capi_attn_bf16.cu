@@ -6,4 +6,3 @@ GRAPHOP_DEFINE_ATTENTION(bf16_i64, uint16_t, __nv_bfloat16, int64_t)
 GRAPHOP_DEFINE_ATTENTION_BIAS(bf16_i32, uint16_t, __nv_bfloat16, int32_t)
 GRAPHOP_DEFINE_ATTENTION_BIAS(bf16_i64, uint16_t, __nv_bfloat16, int64_t)
 GRAPHOP_DEFINE_PLANNED_ATTENTION(bf16, uint16_t, __nv_bfloat16)
-GRAPHOP_DEFINE_PLANNED_ATTENTION_BIAS(bf16, __nv_bfloat16)

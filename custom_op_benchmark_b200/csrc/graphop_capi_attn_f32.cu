@@ -5,4 +5,3 @@ GRAPHOP_DEFINE_ATTENTION(f32_i64, float, float, int64_t)
 GRAPHOP_DEFINE_ATTENTION_BIAS(f32_i32, float, float, int32_t)
 GRAPHOP_DEFINE_ATTENTION_BIAS(f32_i64, float, float, int64_t)
 GRAPHOP_DEFINE_PLANNED_ATTENTION(f32, float, float)
-GRAPHOP_DEFINE_PLANNED_ATTENTION_BIAS(f32, float)

@@ -5,4 +5,3 @@ GRAPHOP_DEFINE_ATTENTION(f64_i64, double, double, int64_t)
 GRAPHOP_DEFINE_ATTENTION_BIAS(f64_i32, double, double, int32_t)
 GRAPHOP_DEFINE_ATTENTION_BIAS(f64_i64, double, double, int64_t)
 GRAPHOP_DEFINE_PLANNED_ATTENTION(f64, double, double)
-GRAPHOP_DEFINE_PLANNED_ATTENTION_BIAS(f64, double)

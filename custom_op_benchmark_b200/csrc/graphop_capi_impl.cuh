@@ -195,21 +195,3 @@
                                              lse, (const T*)d_o, scale, (T*)dq, (T*)dk, (T*)dv, n_dst, n_src, H, D,  \
                                              ws, wsb, GK_ST);                                                        \
   }
-
-// Plan forms of the edge-term attention, for the library's own binding (graphop_internal.h).
-#define GRAPHOP_DEFINE_PLANNED_ATTENTION_BIAS(SUF, T)                                                                \
-  extern "C" int graphop_internal_attention_bias_forward_##SUF(                                                      \
-      const graphop_plan_t* plan, const void* q, const void* k, const void* v, const void* rel, double scale,        \
-      void* o, void* lse, int64_t n_dst, int64_t n_src, int H, int D, void* ws, size_t wsb,                          \
-      graphop_stream_t stream) {                                                                                     \
-    return gk::attention_bias_forward_planned<T>(plan, (const T*)q, (const T*)k, (const T*)v, (const T*)rel, scale,  \
-                                                 (T*)o, lse, n_dst, n_src, H, D, ws, wsb, GK_ST);                    \
-  }                                                                                                                  \
-  extern "C" int graphop_internal_attention_bias_backward_##SUF(                                                     \
-      const graphop_plan_t* plan_r, const graphop_plan_t* plan_t, const void* q, const void* k, const void* v,       \
-      const void* rel, const void* o, const void* lse, const void* d_o, double scale, void* dq, void* dk, void* dv,  \
-      void* d_rel, int64_t n_dst, int64_t n_src, int H, int D, void* ws, size_t wsb, graphop_stream_t stream) {      \
-    return gk::attention_bias_backward_planned<T>(plan_r, plan_t, (const T*)q, (const T*)k, (const T*)v,             \
-                                                  (const T*)rel, (const T*)o, lse, (const T*)d_o, scale, (T*)dq,     \
-                                                  (T*)dk, (T*)dv, (T*)d_rel, n_dst, n_src, H, D, ws, wsb, GK_ST);    \
-  }

@@ -284,18 +284,3 @@ extern "C" int graphop_plan_build_i64(const int64_t* row, const int64_t* indptr,
   return gk::plan_build<int64_t>(row, indptr, eid, indices, n_chunks, n_edges, n_nodes, memory, memory_bytes, plan,
                                  (cudaStream_t)stream);
 }
-
-extern "C" size_t graphop_internal_view_bytes(int64_t n_edges, int64_t n_nodes, int index_bytes) {
-  return gk::view_bytes(n_edges, n_nodes, index_bytes);
-}
-extern "C" int graphop_internal_view_build(const void* row, const void* indptr, const void* eid, const void* indices,
-                                           int index_bytes, int64_t n_chunks, int64_t n_edges, int64_t n_nodes,
-                                           void* clear, size_t clear_bytes, void* memory, size_t memory_bytes, graphop_plan_t* plan,
-                                           graphop_stream_t stream) {
-  const auto st = (cudaStream_t)stream;
-  if (index_bytes == 8)
-    return gk::view_build<int64_t>((const int64_t*)row, (const int64_t*)indptr, (const int64_t*)eid, (const int64_t*)indices,
-                                   n_chunks, n_edges, n_nodes, gk::Clear{clear, clear_bytes}, memory, memory_bytes, plan, st);
-  return gk::view_build<int32_t>((const int32_t*)row, (const int32_t*)indptr, (const int32_t*)eid, (const int32_t*)indices,
-                                 n_chunks, n_edges, n_nodes, gk::Clear{clear, clear_bytes}, memory, memory_bytes, plan, st);
-}

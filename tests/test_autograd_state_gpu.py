@@ -86,3 +86,61 @@ def test_index_types_of_the_two_orientations_agree(tables, name):
     out = function.apply(*tabs[:half], *[t.int() for t in tabs[half:]], *leaves)
     with pytest.raises(RuntimeError, match="expected all index tensors to share dtype torch.int64, got torch.int32"):
         out.sum().backward()
+
+
+@pytest.mark.parametrize("name", FUNCTIONS)
+def test_nothing_but_the_tensors_of_the_call_is_held(tables, name):
+    """Between the directions: the output (and the attention's log-sum, 4 bytes per node and head). After the backward: the
+    output alone, and not the call's own index tensors."""
+    function, tabs, given = _call(name, tables)
+    leaves = _leaves(given)
+
+    def asked():   # what was asked for: blocks handed out may be larger
+        return th.cuda.memory_stats()["requested_bytes.all.current"]
+    before = asked()
+    own = [t.clone() for t in tabs]
+    indices = asked() - before
+    out = function.apply(*own, *leaves)
+    lse = N * H * 4 if name == "GraphAttentionBias" else 0
+    assert asked() - before == indices + out.numel() * 4 + lse
+    del own
+    ones = th.ones_like(out)
+    grads = th.autograd.grad(out, _tensors(leaves), ones)
+    assert asked() - before == sum(t.numel() * 4 for t in (out, ones, *grads))
+    del ones, grads, out
+    assert asked() == before
+
+
+@pytest.mark.parametrize("name", FUNCTIONS)
+def test_saved_tensor_hooks_see_all_that_is_saved(tables, name):
+    """Offloading: what the hooks move to the host leaves the device, and the backward runs on what they bring back."""
+    function, tabs, given = _call(name, tables)
+    leaves = _leaves(given)
+    want = function.apply(*tabs, *leaves)
+    grad = _normal(*want.shape, seed=9)
+    want_grads = th.autograd.grad(want, _tensors(leaves), grad)
+    packed = []
+
+    def pack(t):
+        packed.append(t.data_ptr())
+        return t.cpu()
+    with th.autograd.graph.saved_tensors_hooks(pack, lambda t: t.to(DEV)):
+        out = function.apply(*[t.clone() for t in tabs], *leaves)
+    extra = {"SparseSoftmax": 0, "GraphAttentionBias": 2}.get(name, 0)   # the softmax saves its output for its input
+    assert len(packed) == len(tabs) + len(_tensors(given)) + extra
+    th.empty(1 << 20, device=DEV).fill_(7)   # over what the clones held
+    assert all(th.equal(a, b) for a, b in zip(th.autograd.grad(out, _tensors(leaves), grad), want_grads))
+
+
+def test_index_tensors_are_checked_and_may_come_from_inference_mode(tables):
+    function, tabs, given = _call("MaskedMMCSR", tables)
+    with th.inference_mode():
+        tabs = [t.clone() for t in tabs]
+    leaves = _leaves(given)
+    out = function.apply(*tabs, *leaves)
+    th.autograd.grad(out, _tensors(leaves), th.ones_like(out))
+    tabs = [t.clone() for t in tabs]
+    out = function.apply(*tabs, *leaves)
+    tabs[5].add_(0)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        out.sum().backward()
