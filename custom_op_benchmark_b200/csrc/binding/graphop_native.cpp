@@ -31,6 +31,20 @@ using torch::autograd::Node;
 using torch::autograd::SavedVariable;
 using torch::autograd::variable_list;
 
+// Calls that the code below does not carry are left to torch.autograd.Function (an empty result; wrapper.py goes on there):
+// a trace being recorded, a transform of torch.func or a dispatch mode at work, a tangent of forward-mode differentiation,
+// tensors that wrap others.
+using Result = c10::optional<Tensor>;
+bool left_to_python(std::initializer_list<const Tensor*> ts) {
+  using c10::DispatchKey;
+  constexpr c10::DispatchKeySet modes({DispatchKey::Tracer, DispatchKey::Python, DispatchKey::FuncTorchDynamicLayerFrontMode,
+                                       DispatchKey::FuncTorchDynamicLayerBackMode});
+  if (c10::impl::tls_local_dispatch_key_set().included_.has_any(modes)) return true;
+  for (const Tensor* t : ts)
+    if (t->defined() && (t->key_set().has(DispatchKey::Python) || !t->has_storage() || t->_fw_grad(0).defined())) return true;
+  return false;
+}
+
 // ------------------------------------------------------------------------------------------
 // checks: the texts and exception types of graphop.py
 // ------------------------------------------------------------------------------------------
@@ -245,7 +259,8 @@ struct SparseSoftmaxBackward : GraphNode {
     return {dx};
   }
 };
-Tensor sparse_softmax(const Tensor& row, const Tensor& indptr, const Tensor& eid, const Tensor& x) {
+Result sparse_softmax(const Tensor& row, const Tensor& indptr, const Tensor& eid, const Tensor& x) {
+  if (left_to_python({&row, &indptr, &eid, &x})) return c10::nullopt;
   check_input(row, "row"); check_input(indptr, "indptr"); check_input(eid, "eid"); check_input(x, "x");
   const int elem = elem_of({&x}), H = edge_heads(x), ib = index_bytes_of({&row, &indptr, &eid});
   check_chunks(row, indptr);
@@ -293,9 +308,10 @@ struct MaskedMMBackward : GraphNode {
     return {dA, dB};
   }
 };
-Tensor maskedmm_csr(const Tensor& row, const Tensor& indptr_r, const Tensor& eid_r, const Tensor& indices_r,
+Result maskedmm_csr(const Tensor& row, const Tensor& indptr_r, const Tensor& eid_r, const Tensor& indices_r,
                     const Tensor& col, const Tensor& indptr_c, const Tensor& eid_c, const Tensor& indices_c,
                     const Tensor& A, const Tensor& B) {
+  if (left_to_python({&row, &indptr_r, &eid_r, &indices_r, &col, &indptr_c, &eid_c, &indices_c, &A, &B})) return c10::nullopt;
   check_input(row, "row"); check_input(indptr_r, "indptr"); check_input(eid_r, "eid"); check_input(indices_r, "indices");
   check_input(A, "A"); check_input(B, "B");
   const int elem = elem_of({&A, &B}), ib = index_bytes_of({&row, &indptr_r, &eid_r, &indices_r});
@@ -343,7 +359,8 @@ struct NodeMulEdgeBackward : GraphNode {
     return {dA, dB};
   }
 };
-Tensor node_mul_edge(const Tensor& row, const Tensor& indptr, const Tensor& eid, const Tensor& A, const Tensor& B) {
+Result node_mul_edge(const Tensor& row, const Tensor& indptr, const Tensor& eid, const Tensor& A, const Tensor& B) {
+  if (left_to_python({&row, &indptr, &eid, &A, &B})) return c10::nullopt;
   check_input(row, "row"); check_input(indptr, "indptr"); check_input(eid, "eid"); check_input(A, "A"); check_input(B, "B");
   const int elem = elem_of({&A, &B}), ib = index_bytes_of({&row, &indptr, &eid});
   const NodeShape s = node_shape(A);
@@ -390,8 +407,9 @@ struct VectorSPMMBackward : GraphNode {
     return {dw, dx};
   }
 };
-Tensor vector_spmm(const Tensor& row, const Tensor& indptr, const Tensor& eid, const Tensor& indices, const Tensor& col,
+Result vector_spmm(const Tensor& row, const Tensor& indptr, const Tensor& eid, const Tensor& indices, const Tensor& col,
                    const Tensor& indptr_t, const Tensor& eid_t, const Tensor& indices_t, const Tensor& w, const Tensor& x) {
+  if (left_to_python({&row, &indptr, &eid, &indices, &col, &indptr_t, &eid_t, &indices_t, &w, &x})) return c10::nullopt;
   check_input(row, "row"); check_input(indptr, "indptr"); check_input(eid, "eid"); check_input(indices, "indices");
   check_input(w, "edata"); check_input(x, "x");
   const int elem = elem_of({&w, &x}), ib = index_bytes_of({&row, &indptr, &eid, &indices});
@@ -465,8 +483,9 @@ struct AttentionBackward : GraphNode {
     return {dq, dk, dv};
   }
 };
-Tensor attention_planned(const PlanHandle& plan_r, const PlanHandle& plan_t, const Tensor& q, const Tensor& k,
+Result attention_planned(const PlanHandle& plan_r, const PlanHandle& plan_t, const Tensor& q, const Tensor& k,
                          const Tensor& v, double scale) {
+  if (left_to_python({&q, &k, &v})) return c10::nullopt;
   check_input(q, "q"); check_input(k, "k"); check_input(v, "v");
   const int elem = elem_of({&q, &k, &v});
   const NodeShape s = node_shape(q);
@@ -523,9 +542,10 @@ struct AttentionBiasBackward : GraphNode {
     return {dq, dk, dv, drel};
   }
 };
-Tensor attention_bias(const Tensor& row, const Tensor& indptr, const Tensor& indices, const Tensor& col,
+Result attention_bias(const Tensor& row, const Tensor& indptr, const Tensor& indices, const Tensor& col,
                       const Tensor& indptr_t, const Tensor& eid_t, const Tensor& indices_t, const Tensor& q,
                       const Tensor& k, const Tensor& v, const Tensor& rel, double scale) {
+  if (left_to_python({&row, &indptr, &indices, &col, &indptr_t, &eid_t, &indices_t, &q, &k, &v, &rel})) return c10::nullopt;
   check_input(row, "row"); check_input(indptr, "indptr"); check_input(indices, "indices");
   check_input(q, "q"); check_input(k, "k"); check_input(v, "v"); check_input(rel, "rel");
   const int elem = elem_of({&q, &k, &v, &rel}), ib = index_bytes_of({&row, &indptr, &indices});

@@ -4,7 +4,9 @@ the same `None` gradients for every index argument, plus `GraphAttention`, the f
 
 `apply` of these classes runs the same Function in native code (csrc/binding/graphop_native.cpp): on small graphs the
 Python forward and backward below took several times as long as the kernels.  They are what `apply` runs when `_g` is
-another module with the ops of `graphop` (the compiled module of that name, say).
+another module with the ops of `graphop` (the compiled module of that name, say), and where torch.autograd.Function does
+more than the native node: while torch.jit.trace records, under torch.func's transforms and dispatch modes, on tensors
+with a forward-mode tangent.
 """
 import torch as th
 from torch.autograd import Function
@@ -20,14 +22,21 @@ __all__ = ["SparseSoftmax", "MaskedMMCSR", "NodeMulEdge", "VectorSPMM", "GraphAt
 chunk_size = 32  # wrapper.py:6
 
 
+def _run(function, name, *args):
+    """`function` on `args`: `name` of the native module, or, where that leaves the call to it (see above), the Function."""
+    if _g is _graphop:
+        out = getattr(_native(), name)(*args)
+        if out is not None:
+            return out
+    return super(function, function).apply(*args)
+
+
 class SparseSoftmax(Function):
     """wrapper.py:8-18"""
 
     @staticmethod
     def apply(row, indptr, eid, x):
-        if _g is not _graphop:
-            return super(SparseSoftmax, SparseSoftmax).apply(row, indptr, eid, x)
-        return _native().sparse_softmax(row, indptr, eid, x)
+        return _run(SparseSoftmax, "sparse_softmax", row, indptr, eid, x)
 
     @staticmethod
     def forward(ctx, row, indptr, eid, x):
@@ -46,9 +55,7 @@ class MaskedMMCSR(Function):
 
     @staticmethod
     def apply(row, indptr_r, eid_r, indices_r, col, indptr_c, eid_c, indices_c, A, B):
-        if _g is not _graphop:
-            return super(MaskedMMCSR, MaskedMMCSR).apply(row, indptr_r, eid_r, indices_r, col, indptr_c, eid_c, indices_c, A, B)
-        return _native().maskedmm_csr(row, indptr_r, eid_r, indices_r, col, indptr_c, eid_c, indices_c, A, B)
+        return _run(MaskedMMCSR, "maskedmm_csr", row, indptr_r, eid_r, indices_r, col, indptr_c, eid_c, indices_c, A, B)
 
     @staticmethod
     def forward(ctx, row, indptr_r, eid_r, indices_r, col, indptr_c, eid_c, indices_c, A, B):
@@ -68,9 +75,7 @@ class NodeMulEdge(Function):
 
     @staticmethod
     def apply(row, indptr, eid, A, B):
-        if _g is not _graphop:
-            return super(NodeMulEdge, NodeMulEdge).apply(row, indptr, eid, A, B)
-        return _native().node_mul_edge(row, indptr, eid, A, B)
+        return _run(NodeMulEdge, "node_mul_edge", row, indptr, eid, A, B)
 
     @staticmethod
     def forward(ctx, row, indptr, eid, A, B):
@@ -89,9 +94,7 @@ class VectorSPMM(Function):
 
     @staticmethod
     def apply(row, indptr, eid, indices, col, ptr_t, eid_t, indices_t, edata, x):
-        if _g is not _graphop:
-            return super(VectorSPMM, VectorSPMM).apply(row, indptr, eid, indices, col, ptr_t, eid_t, indices_t, edata, x)
-        return _native().vector_spmm(row, indptr, eid, indices, col, ptr_t, eid_t, indices_t, edata, x)
+        return _run(VectorSPMM, "vector_spmm", row, indptr, eid, indices, col, ptr_t, eid_t, indices_t, edata, x)
 
     @staticmethod
     def forward(ctx, row, indptr, eid, indices, col, ptr_t, eid_t, indices_t, edata, x):
@@ -117,14 +120,14 @@ class GraphAttention(Function):
 
     @staticmethod
     def apply(row, indptr, indices, col, indptr_t, indices_t, Q, K, V, scale, eid_t=None):
-        if _g is not _graphop:
-            return super(GraphAttention, GraphAttention).apply(row, indptr, indices, col, indptr_t, indices_t, Q, K, V, scale, eid_t)
         # the same graph tensors come back every step: their plans are built once and looked up here, so this per-call
         # signature runs the planned kernels (and, on a dense band in bfloat16, the tensor-core ones)
-        if _g.plan_cache_size > 0 and indices.numel() > 0:
+        if _g is _graphop and _g.plan_cache_size > 0 and indices.numel() > 0:
             plans = _g.cached_plan(row, indptr, None, indices, Q.size(0)), _g.cached_plan(col, indptr_t, eid_t, indices_t,
                                                                                          K.size(0))
-            return _native().attention_planned(plans[0].native(), plans[1].native(), Q, K, V, scale)
+            out = _native().attention_planned(plans[0].native(), plans[1].native(), Q, K, V, scale)
+            if out is not None:
+                return out
         return super(GraphAttention, GraphAttention).apply(row, indptr, indices, col, indptr_t, indices_t, Q, K, V, scale,
                                                            eid_t)
 
@@ -166,9 +169,8 @@ class GraphAttentionBias(Function):
 
     @staticmethod
     def apply(row, indptr, indices, col, indptr_t, eid_t, indices_t, Q, K, V, rel, scale):
-        if _g is not _graphop:
-            return super(GraphAttentionBias, GraphAttentionBias).apply(row, indptr, indices, col, indptr_t, eid_t, indices_t, Q, K, V, rel, scale)
-        return _native().attention_bias(row, indptr, indices, col, indptr_t, eid_t, indices_t, Q, K, V, rel, scale)
+        return _run(GraphAttentionBias, "attention_bias", row, indptr, indices, col, indptr_t,
+                    eid_t, indices_t, Q, K, V, rel, scale)
 
     @staticmethod
     def forward(ctx, row, indptr, indices, col, indptr_t, eid_t, indices_t, Q, K, V, rel, scale):
@@ -192,9 +194,11 @@ class GraphAttentionPlanned(Function):
 
     @staticmethod
     def apply(plan_r, plan_t, Q, K, V, scale):
-        if _g is not _graphop:
-            return super(GraphAttentionPlanned, GraphAttentionPlanned).apply(plan_r, plan_t, Q, K, V, scale)
-        return _native().attention_planned(plan_r.native(), plan_t.native(), Q, K, V, scale)
+        if _g is _graphop:
+            out = _native().attention_planned(plan_r.native(), plan_t.native(), Q, K, V, scale)
+            if out is not None:
+                return out
+        return super(GraphAttentionPlanned, GraphAttentionPlanned).apply(plan_r, plan_t, Q, K, V, scale)
 
     @staticmethod
     def forward(ctx, plan_r, plan_t, Q, K, V, scale):
