@@ -51,7 +51,7 @@ bool left_to_python(std::initializer_list<const Tensor*> ts) {
 [[noreturn]] void fail(const std::string& text) { throw std::runtime_error(text); }
 
 void check_input(const Tensor& t, const char* name) {
-  if (!t.is_cuda()) fail(std::string(name) + " must be a CUDA tensor");
+  if (!t.defined() || !t.is_cuda()) fail(std::string(name) + " must be a CUDA tensor");
   if (!t.is_contiguous()) fail(std::string(name) + " must be contiguous");
 }
 std::string dtype_text(const Tensor& t) {
@@ -119,6 +119,10 @@ struct Call {
 
 // a tensor's storage as the element type the entry point wants; null for an undefined one
 template <typename E> E* ptr(const Tensor& t) { return t.defined() ? reinterpret_cast<E*>(t.data_ptr()) : nullptr; }
+
+// An argument that only the backward reads: a call without one may leave it out.
+using Later = c10::optional<Tensor>;
+Tensor given(const Later& t) { return t.value_or(Tensor()); }
 
 // f is called with a null pointer of the element type
 template <class F> auto by_elem(int elem, F&& f) {
@@ -309,8 +313,9 @@ struct MaskedMMBackward : GraphNode {
   }
 };
 Result maskedmm_csr(const Tensor& row, const Tensor& indptr_r, const Tensor& eid_r, const Tensor& indices_r,
-                    const Tensor& col, const Tensor& indptr_c, const Tensor& eid_c, const Tensor& indices_c,
+                    const Later& col_in, const Later& indptr_c_in, const Later& eid_c_in, const Later& indices_c_in,
                     const Tensor& A, const Tensor& B) {
+  const Tensor col = given(col_in), indptr_c = given(indptr_c_in), eid_c = given(eid_c_in), indices_c = given(indices_c_in);
   if (left_to_python({&row, &indptr_r, &eid_r, &indices_r, &col, &indptr_c, &eid_c, &indices_c, &A, &B})) return c10::nullopt;
   check_input(row, "row"); check_input(indptr_r, "indptr"); check_input(eid_r, "eid"); check_input(indices_r, "indices");
   check_input(A, "A"); check_input(B, "B");
@@ -407,8 +412,10 @@ struct VectorSPMMBackward : GraphNode {
     return {dw, dx};
   }
 };
-Result vector_spmm(const Tensor& row, const Tensor& indptr, const Tensor& eid, const Tensor& indices, const Tensor& col,
-                   const Tensor& indptr_t, const Tensor& eid_t, const Tensor& indices_t, const Tensor& w, const Tensor& x) {
+Result vector_spmm(const Tensor& row, const Tensor& indptr, const Tensor& eid, const Tensor& indices, const Later& col_in,
+                   const Later& indptr_t_in, const Later& eid_t_in, const Later& indices_t_in, const Tensor& w,
+                   const Tensor& x) {
+  const Tensor col = given(col_in), indptr_t = given(indptr_t_in), eid_t = given(eid_t_in), indices_t = given(indices_t_in);
   if (left_to_python({&row, &indptr, &eid, &indices, &col, &indptr_t, &eid_t, &indices_t, &w, &x})) return c10::nullopt;
   check_input(row, "row"); check_input(indptr, "indptr"); check_input(eid, "eid"); check_input(indices, "indices");
   check_input(w, "edata"); check_input(x, "x");
@@ -542,9 +549,10 @@ struct AttentionBiasBackward : GraphNode {
     return {dq, dk, dv, drel};
   }
 };
-Result attention_bias(const Tensor& row, const Tensor& indptr, const Tensor& indices, const Tensor& col,
-                      const Tensor& indptr_t, const Tensor& eid_t, const Tensor& indices_t, const Tensor& q,
+Result attention_bias(const Tensor& row, const Tensor& indptr, const Tensor& indices, const Later& col_in,
+                      const Later& indptr_t_in, const Later& eid_t_in, const Later& indices_t_in, const Tensor& q,
                       const Tensor& k, const Tensor& v, const Tensor& rel, double scale) {
+  const Tensor col = given(col_in), indptr_t = given(indptr_t_in), eid_t = given(eid_t_in), indices_t = given(indices_t_in);
   if (left_to_python({&row, &indptr, &indices, &col, &indptr_t, &eid_t, &indices_t, &q, &k, &v, &rel})) return c10::nullopt;
   check_input(row, "row"); check_input(indptr, "indptr"); check_input(indices, "indices");
   check_input(q, "q"); check_input(k, "k"); check_input(v, "v"); check_input(rel, "rel");

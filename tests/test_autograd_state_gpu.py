@@ -144,3 +144,15 @@ def test_index_tensors_are_checked_and_may_come_from_inference_mode(tables):
     tabs[5].add_(0)
     with pytest.raises(RuntimeError, match="modified by an inplace operation"):
         out.sum().backward()
+
+
+@pytest.mark.parametrize("name", ["MaskedMMCSR", "VectorSPMM", "GraphAttentionBias"])
+def test_inference_without_the_column_side(tables, name):
+    """Only the backward reads the column CSR: a call without a gradient may leave it out, a backward says what is missing."""
+    function, tabs, given = _call(name, tables)
+    half = len(tabs) - 4
+    with th.no_grad():
+        assert th.equal(function.apply(*tabs[:half], None, None, None, None, *given), function.apply(*tabs, *given))
+    out = function.apply(*tabs[:half], None, None, None, None, *_leaves(given))
+    with pytest.raises(RuntimeError, match="col must be a CUDA tensor"):
+        out.sum().backward()
