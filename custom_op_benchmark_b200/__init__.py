@@ -41,6 +41,16 @@ def native_functions():
 _NATIVE = None
 
 
+def native_functions_if_built():
+    """native_functions(), or None where the package was built without the compiled modules (``build.py --no-module``, which
+    needs neither torch's headers nor g++): the same calls then go to the same kernels from Python, through ctypes."""
+    from . import build as _build
+    import os
+    if _NATIVE is None and not os.path.exists(_build.module_path("graphop_native")):
+        return None
+    return native_functions()
+
+
 def _load_compiled(name):
     import importlib.util
     import os

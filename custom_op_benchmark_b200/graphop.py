@@ -18,7 +18,7 @@ import weakref
 
 import torch as th
 
-from . import _capi, native_functions
+from . import _capi, native_functions_if_built
 
 __all__ = [
     "maskedmm_csr_forward", "maskedmm_csr_backward", "node_mul_edge_forward", "node_mul_edge_backward",
@@ -89,6 +89,17 @@ def _heads(t, node):
 
 def _p(t):
     return None if t is None else t.data_ptr()
+
+
+def _scratch(need, device):
+    """(the tensor, its first 256-byte aligned address, need): `need` bytes of device memory."""
+    t = th.empty(need + 256, dtype=th.uint8, device=device)
+    return t, (t.data_ptr() + 255) // 256 * 256, need
+
+
+def _check(rc, name):
+    if rc != _capi.OK:
+        raise RuntimeError("graphop_%s: %s" % (name, _capi.error_message(rc)))
 
 
 def _call(name, elem, index, op_id, n_edges, n_nodes, h, d, device, args):
@@ -381,14 +392,35 @@ def pull_rows(tables, seg, idx, row_bytes, out):
 
 def partition_csr(indptr, chunk_size=32):
     """partition_csr of the reference (part_csr.py:13-27) for an int32 / int64 indptr on a CUDA device, by the
-    library's kernels (graphop_partition_csr_count / _fill): (row, indptr_) as int64 tensors on that device."""
+    library's kernels (graphop_partition_csr_count / _fill): (row, indptr_) as int64 tensors on that device.
+
+    This function, transpose_csr and GraphPlan run in native code (csrc/binding/graphop_native.cpp); the ctypes code below is
+    for a package built without the compiled modules."""
+    import ctypes
     if chunk_size <= 0:
         raise ValueError("chunk_size must be positive")
     if not indptr.is_cuda or indptr.dtype not in (th.int32, th.int64) or indptr.dim() != 1:
         raise RuntimeError("indptr must be a one-dimensional int32 or int64 CUDA tensor")
     if indptr.numel() < 1:
         raise IndexError("indptr must hold at least one element")
-    return native_functions().partition_csr(indptr, int(chunk_size))
+    native = native_functions_if_built()
+    if native is not None:
+        return native.partition_csr(indptr, int(chunk_size))
+    ip = indptr.contiguous()
+    n = ip.numel() - 1
+    suffix = "i32" if ip.dtype == th.int32 else "i64"
+    lib = _capi.lib()
+    with th.cuda.device(ip.device):
+        stream = th.cuda.current_stream(ip.device).cuda_stream
+        _ws, base, need = _scratch(lib.graphop_partition_csr_workspace_bytes(n), ip.device)
+        count = ctypes.c_int64(0)
+        _check(getattr(lib, "graphop_partition_csr_count_" + suffix)(
+            _p(ip), n, int(chunk_size), base, need, ctypes.byref(count), stream), "partition_csr_count")
+        row = th.empty(count.value, dtype=th.int64, device=ip.device)
+        ptr = th.empty(count.value + 1, dtype=th.int64, device=ip.device)
+        _check(getattr(lib, "graphop_partition_csr_fill_" + suffix)(
+            _p(ip), n, int(chunk_size), base, count.value, _p(row), _p(ptr), stream), "partition_csr_fill")
+    return row, ptr
 
 
 def transpose_csr(indptr, indices, n_src):
@@ -400,7 +432,21 @@ def transpose_csr(indptr, indices, n_src):
         raise RuntimeError("indptr and indices must be one-dimensional CUDA tensors of the same type, int32 or int64")
     if indptr.numel() < 1:
         raise IndexError("indptr must hold at least one element")
-    return native_functions().transpose_csr(indptr, indices, int(n_src))
+    native = native_functions_if_built()
+    if native is not None:
+        return native.transpose_csr(indptr, indices, int(n_src))
+    ip, idx = indptr.contiguous(), indices.contiguous()
+    n_dst, e, n_src = ip.numel() - 1, idx.numel(), int(n_src)
+    suffix, width = ("i32", 4) if ip.dtype == th.int32 else ("i64", 8)
+    lib = _capi.lib()
+    with th.cuda.device(ip.device):
+        _ws, base, need = _scratch(lib.graphop_transpose_csr_workspace_bytes(e, width), ip.device)
+        ptr_t = th.empty(n_src + 1, dtype=ip.dtype, device=ip.device)
+        idx_t, eid_t = th.empty_like(idx), th.empty_like(idx)
+        _check(getattr(lib, "graphop_transpose_csr_" + suffix)(
+            _p(ip), _p(idx), n_dst, n_src, e, _p(ptr_t), _p(idx_t), _p(eid_t), base, need,
+            th.cuda.current_stream(ip.device).cuda_stream), "transpose_csr")
+    return ptr_t, idx_t, eid_t
 
 
 def check_graph(row, indptr, eid, indices, n_nodes, n_other):
@@ -442,7 +488,7 @@ class GraphPlan:
         if indices is not None:
             given["indices"] = indices
         _check_all(**given)
-        _index(*given.values())
+        index = _index(*given.values())
         self.n_chunks, self.n_nodes = _chunks(row, indptr), int(n_nodes)
         self.n_edges = int(indices.size(0) if indices is not None else (eid.size(0) if eid is not None else 0))
         if eid is not None and indices is not None and eid.size(0) != indices.size(0):
@@ -451,8 +497,17 @@ class GraphPlan:
         self._keep = (row, indptr, eid, indices)
         self._native = None
         self.c = _capi.Plan()
-        self._memory = native_functions().plan_build(row, indptr, eid, indices, self.n_edges, self.n_nodes,
-                                                     ctypes.addressof(self.c))
+        native = native_functions_if_built()
+        if native is not None:
+            self._memory = native.plan_build(row, indptr, eid, indices, self.n_edges, self.n_nodes, ctypes.addressof(self.c))
+            return
+        lib = _capi.lib()
+        with th.cuda.device(self.device):
+            self._memory, base, need = _scratch(lib.graphop_plan_bytes(self.n_chunks, self.n_edges, self.n_nodes, index[1]),
+                                                self.device)
+            _check(getattr(lib, "graphop_plan_build_" + index[0])(
+                _p(row), _p(indptr), _p(eid), _p(indices), self.n_chunks, self.n_edges, self.n_nodes, base, need,
+                ctypes.byref(self.c), th.cuda.current_stream(self.device).cuda_stream), "plan_build")
 
     @property
     def dense_band(self):
@@ -477,7 +532,7 @@ class GraphPlan:
         if self._native is None:
             import ctypes
             keep = [self._memory] + [t for t in self._keep if t is not None]
-            self._native = native_functions().PlanHandle(ctypes.addressof(self.c), keep)
+            self._native = native_functions_if_built().PlanHandle(ctypes.addressof(self.c), keep)
         return self._native
 
 

@@ -6,14 +6,14 @@ the same `None` gradients for every index argument, plus `GraphAttention`, the f
 Python forward and backward below took several times as long as the kernels.  They are what `apply` runs when `_g` is
 another module with the ops of `graphop` (the compiled module of that name, say), and where torch.autograd.Function does
 more than the native node: while torch.jit.trace records, under torch.func's transforms and dispatch modes, on tensors
-with a forward-mode tangent.
+with a forward-mode tangent; and all there is in a package built without the compiled modules.
 """
 import torch as th
 from torch.autograd import Function
 
 from . import graphop as _g
 from . import graphop as _graphop
-from . import native_functions as _native
+from . import native_functions_if_built
 from .part_csr import partition_csr  # noqa: F401  (the reference wrapper re-exports it, wrapper.py:4)
 
 __all__ = ["SparseSoftmax", "MaskedMMCSR", "NodeMulEdge", "VectorSPMM", "GraphAttention", "GraphAttentionBias", "GraphAttentionPlanned",
@@ -22,12 +22,17 @@ __all__ = ["SparseSoftmax", "MaskedMMCSR", "NodeMulEdge", "VectorSPMM", "GraphAt
 chunk_size = 32  # wrapper.py:6
 
 
+def _native():
+    """The native module where `apply` goes through it."""
+    return native_functions_if_built() if _g is _graphop else None
+
+
 def _run(function, name, *args):
     """`function` on `args`: `name` of the native module, or, where that leaves the call to it (see above), the Function."""
-    if _g is _graphop:
-        out = getattr(_native(), name)(*args)
-        if out is not None:
-            return out
+    native = _native()
+    out = getattr(native, name)(*args) if native is not None else None
+    if out is not None:
+        return out
     return super(function, function).apply(*args)
 
 
@@ -122,10 +127,11 @@ class GraphAttention(Function):
     def apply(row, indptr, indices, col, indptr_t, indices_t, Q, K, V, scale, eid_t=None):
         # the same graph tensors come back every step: their plans are built once and looked up here, so this per-call
         # signature runs the planned kernels (and, on a dense band in bfloat16, the tensor-core ones)
-        if _g is _graphop and _g.plan_cache_size > 0 and indices.numel() > 0:
+        native = _native()
+        if native is not None and _g.plan_cache_size > 0 and indices.numel() > 0:
             plans = _g.cached_plan(row, indptr, None, indices, Q.size(0)), _g.cached_plan(col, indptr_t, eid_t, indices_t,
                                                                                          K.size(0))
-            out = _native().attention_planned(plans[0].native(), plans[1].native(), Q, K, V, scale)
+            out = native.attention_planned(plans[0].native(), plans[1].native(), Q, K, V, scale)
             if out is not None:
                 return out
         return super(GraphAttention, GraphAttention).apply(row, indptr, indices, col, indptr_t, indices_t, Q, K, V, scale,
@@ -194,8 +200,9 @@ class GraphAttentionPlanned(Function):
 
     @staticmethod
     def apply(plan_r, plan_t, Q, K, V, scale):
-        if _g is _graphop:
-            out = _native().attention_planned(plan_r.native(), plan_t.native(), Q, K, V, scale)
+        native = _native()
+        if native is not None:
+            out = native.attention_planned(plan_r.native(), plan_t.native(), Q, K, V, scale)
             if out is not None:
                 return out
         return super(GraphAttentionPlanned, GraphAttentionPlanned).apply(plan_r, plan_t, Q, K, V, scale)
