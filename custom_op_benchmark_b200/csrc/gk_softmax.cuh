@@ -69,6 +69,9 @@ __device__ __forceinline__ void store_heads(T* __restrict__ p, const typename Ac
 template <bool kMax, typename A> __device__ __forceinline__ A seg_op(A a, A b) {
   return kMax ? (b > a ? b : a) : a + b;
 }
+// What the exponents of a part of a row are relative to: its maximum, or 0 where all of the part is masked (scores of -inf,
+// maximum -inf).  Such a part's sum is 0 and has no weight in the row's; -inf - -inf would make it, and with it the row, NaN.
+template <typename A> __device__ __forceinline__ A exp_ref(A m) { return m == neg_inf<A>() ? A(0) : m; }
 template <bool kMax, typename A> __device__ __forceinline__ A seg_identity() { return kMax ? neg_inf<A>() : A(0); }
 
 // Where the segments of a thread's positions begin.
@@ -267,7 +270,7 @@ softmax_tile_kernel(const int32_t* __restrict__ erow, const int32_t* __restrict_
         for (int h = 0; h < H; ++h) {
           l[h] = A(0);
 #pragma unroll
-          for (int i = 0; i < P; ++i) l[h] += gk_exp(a[i][h] - m[h]);
+          for (int i = 0; i < P; ++i) l[h] += gk_exp(a[i][h] - exp_ref(m[h]));
           l[h] = warp_sum(l[h]);
           if (st.lane == 0) s_head[1][st.w][h] = l[h];
         }
@@ -308,7 +311,7 @@ softmax_tile_kernel(const int32_t* __restrict__ erow, const int32_t* __restrict_
 #pragma unroll
     for (int i = 0; i < P; ++i)
 #pragma unroll
-      for (int h = 0; h < H; ++h) l[i][h] = a[i][h] = r[i] >= 0 ? gk_exp(a[i][h] - m[i][h]) : A(0);
+      for (int h = 0; h < H; ++h) l[i][h] = a[i][h] = r[i] >= 0 ? gk_exp(a[i][h] - exp_ref(m[i][h])) : A(0);
     segment_totals<A, H, false>(l, st, s_head[1], s_tail[1]);
   }
 
