@@ -794,8 +794,8 @@ struct GroupEdgeDot : GEO, Shape<GEO, 1, 0, 1, 1, 0, 2> {
 };
 
 // Fused attention forward: o[node] = sum_k softmax_k(scale q.k) v.  Scores in base-2 units (q is multiplied by
-// scale * log2 e when a node starts).  The accumulators are rescaled only in steps in which some group's running maximum
-// grows (a vote), which is rare after a node's first edges.
+// scale * log2 e when a node starts).  The accumulators are rescaled in every step: with several groups per warp some group's
+// running maximum grows in most of them.
 // kBias: the score's key row gets the edge's row of rel added (one D-vector per edge, shared by the heads).
 template <class GEO, bool kBias>
 struct GroupAttnFwd : GEO, Shape<GEO, kBias ? 3 : 2, 0, 2, 1, 0, 2> {
@@ -858,15 +858,15 @@ struct GroupAttnFwd : GEO, Shape<GEO, kBias ? 3 : 2, 0, 2, 1, 0, 2> {
       if (!active[v]) s[v] = neg_inf<A>();
       mn = s[v] > mn ? s[v] : mn;
     }
-    // no branch on "the maximum grows": with several groups per warp some group's does in most steps
     const A corr = st.m == mn ? A(1) : gk_exp2(st.m - mn);   // m = -inf before a node's first edge: 2^-inf = 0
+    const A ref = mn == neg_inf<A>() ? A(0) : mn;            // nothing but masked scores (-inf) so far: they add 2^-inf
     st.m = mn;
     st.l *= corr;
 #pragma unroll
     for (int i = 0; i < W; ++i) st.acc[i].scale(corr);
 #pragma unroll
     for (int v = 0; v < N; ++v) {
-      p[v] = active[v] ? gk_exp2(s[v] - mn) : A(0);
+      p[v] = active[v] ? gk_exp2(s[v] - ref) : A(0);
       st.l += p[v];
       F f[W];
       this->load_staged(f, slot + v * this->kStepBytes + kRow);

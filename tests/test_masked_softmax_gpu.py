@@ -4,7 +4,8 @@ import pytest
 import torch as th
 
 from helpers import chunked, random_graph
-from custom_op_benchmark_b200 import wrapper
+from custom_op_benchmark_b200 import graphop, wrapper
+from oracle import edge_list_f64 as ref
 from oracle import graphop_oracle as orc
 
 pytestmark = pytest.mark.gpu
@@ -69,3 +70,27 @@ def test_what_has_no_value_stays_nan(what):
     bad = th.zeros(g.n_edges, dtype=th.bool)
     bad[middle] = True
     assert bool(th.isnan(y[bad]).all()) and bool(th.isfinite(y[~bad]).all())
+
+
+@pytest.mark.parametrize("h,d,dtype", [(4, 32, th.float32), (8, 64, th.float32), (1, 16, th.float32), (2, 64, th.bfloat16)])
+def test_scores_that_overflow_in_the_fused_layer(h, d, dtype):
+    """Finite queries and keys whose product is -inf in float: such an edge has probability 0, also where a node's first
+    edges are all of that kind (half of the sources are, in runs of any length)."""
+    g = random_graph(300, 200, [40] * 299 + [3000], 11)
+    gen = th.Generator().manual_seed(12)
+    q, k, v, do = (th.randn(n, h, d, generator=gen) for n in (300, 200, 200, 300))
+    q[..., 0], k[..., 0] = 1e20, 0.0
+    k[::2, :, 0] = -1e20
+    q, k, v, do = (t.to(dtype).to(DEV) for t in (q, k, v, do))
+    r, c = [t.to(DEV) for t in chunked(g, 32)], [t.to(DEV) for t in chunked(g, 32, transposed=True)]
+    plans = graphop.GraphPlan(*r, 300), graphop.GraphPlan(*c, 200)
+    leaves = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    scale = d ** -0.5
+    o = wrapper.GraphAttentionPlanned.apply(*plans, *leaves, scale)
+    got = [o, *th.autograd.grad(o, leaves, do)]
+    want = ref.attention_f64(g.indptr.to(DEV), g.indices.to(DEV), q, k, v, scale, do)
+    tol = 3e-5 if dtype == th.float32 else 2e-2
+    for name, a, b in zip(("o", "dq", "dk", "dv"), got, (want[0], *want[2:])):
+        assert bool(th.isfinite(a).all()), name
+        a, b = a.double()[..., 1:], b[..., 1:]   # feature 0 of dk is a sum of terms of 1e20 that cancel
+        assert bool(((a - b).abs() <= tol * (b.abs() + max(1.0, float(b.abs().max())))).all()), name
