@@ -312,42 +312,48 @@ expand_rows_kernel(const I* __restrict__ row, const I* __restrict__ indptr, long
     for (int k = w - 1; k >= 0 && before == kNone; --k) before = s_last[k];
 #pragma unroll
     for (int i = 0; i < kExpandPer; ++i) r[i] = r[i] == kNone ? before : r[i];
-    const int p = q0 + tid * kExpandPer;
-    const bool whole = p >= at && p + kExpandPer <= stop;
+    // relative to the step: E may be 2^31 - 1, and positions of threads past the last one do not fit 32 bits then
+    const int o = tid * kExpandPer, from_o = at - q0, to_o = stop - q0;
+    const bool whole = o >= from_o && o + kExpandPer <= to_o;
+    int32_t* const out = erow + q0;
     if (whole) {
 #pragma unroll
-      for (int i = 0; i < kExpandPer; i += 4) *reinterpret_cast<int4*>(erow + p + i) = *reinterpret_cast<int4*>(r + i);
+      for (int i = 0; i < kExpandPer; i += 4) *reinterpret_cast<int4*>(out + o + i) = *reinterpret_cast<int4*>(r + i);
     } else {
 #pragma unroll
       for (int i = 0; i < kExpandPer; ++i)
-        if (p + i >= at && p + i < stop) erow[p + i] = r[i];
+        if (o + i >= from_o && o + i < to_o) out[o + i] = r[i];
     }
     if (cut.start) {
       const auto node = [&](int rr, int pp) { return rr >= 0 ? rr : pp < base ? 0 : tail; };
-      // the first thread's predecessor lies in the step before
-      const int was_node = p <= at ? prev : node(before, p - 1);
-      long long was = tile_at(cut, (p > at ? p : at) - 1, was_node);
-      const long long mine = tile_at(cut, p + kExpandPer - 1, r[kExpandPer - 1]);
-      if (whole && !bare && was <= mine && p + kExpandPer < E) {
-        // nodes do not decrease: boundary t lies at the first of these positions whose cost reaches it
-        for (long long t = was + 1; t <= mine && t <= cut.n; ++t) {
-          const long long reach = t << cut.shift;
-          int below = 0;
+      if (o < to_o) {
+        const int p = q0 + o;
+        // the first thread's predecessor lies in the step before
+        const int was_node = p <= at ? prev : node(before, p - 1);
+        long long was = tile_at(cut, (p > at ? p : at) - 1, was_node);
+        const bool quick = whole && !bare && o + kExpandPer < E - q0;
+        const long long mine = quick ? tile_at(cut, p + kExpandPer - 1, r[kExpandPer - 1]) : -1;
+        if (quick && was <= mine) {
+          // nodes do not decrease: boundary t lies at the first of these positions whose cost reaches it
+          for (long long t = was + 1; t <= mine && t <= cut.n; ++t) {
+            const long long reach = t << cut.shift;
+            int below = 0;
 #pragma unroll
-          for (int i = 0; i < kExpandPer; ++i) below += p + i + (long long)kRowCost * r[i] < reach;
-          cut.start[t] = p + (below < kExpandPer ? below : kExpandPer - 1);
-        }
-      } else {
+            for (int i = 0; i < kExpandPer; ++i) below += p + i + (long long)kRowCost * r[i] < reach;
+            cut.start[t] = p + (below < kExpandPer ? below : kExpandPer - 1);
+          }
+        } else {
 #pragma unroll 1
-        for (int i = 0; i < kExpandPer; ++i) {
-          const int q = p + i;
-          int rr = r[0];   // selected, not indexed: r stays in registers
+          for (int i = 0; i < kExpandPer && o + i < to_o; ++i) {
+            const int q = p + i;
+            int rr = r[0];   // selected, not indexed: r stays in registers
 #pragma unroll
-          for (int k = 1; k < kExpandPer; ++k) rr = k == i ? r[k] : rr;
-          if (q >= at && q < stop) {
-            const long long mine = tile_at(cut, q, node(rr, q));
-            if (mine != was || q == E - 1) cut_tiles(cut, q, E, was, mine);
-            was = mine;
+            for (int k = 1; k < kExpandPer; ++k) rr = k == i ? r[k] : rr;
+            if (q >= at) {
+              const long long mine = tile_at(cut, q, node(rr, q));
+              if (mine != was || q == E - 1) cut_tiles(cut, q, E, was, mine);
+              was = mine;
+            }
           }
         }
       }

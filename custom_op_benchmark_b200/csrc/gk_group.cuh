@@ -433,7 +433,7 @@ group_walk_kernel(const __grid_constant__ Op op, const __grid_constant__ WalkArg
             act[v] = p + v < lim;
             ed[v] = Op::kFoldsEid ? __shfl_sync(kFull, e0, i + v, G) : 0;
           }
-          op.template fold<U>(st, slot, tab0 + i * ENTRY, act, (int)j0 + p, ed);
+          op.template fold<U>(st, slot, tab0 + i * ENTRY, act, (unsigned)j0 + p, ed);
         } else {
           [[maybe_unused]] bool taken = false;   // the iteration's room for a node held an earlier one
 #pragma unroll 1
@@ -479,7 +479,7 @@ group_walk_kernel(const __grid_constant__ Op op, const __grid_constant__ WalkArg
             }
             const bool act[1] = {p + v < lim};
             const int ed[1] = {Op::kFoldsEid ? __shfl_sync(kFull, e0, i + v, G) : 0};
-            op.template fold<1>(st, slot + v * STEP, tab0 + (i + v) * ENTRY, act, (int)j0 + p + v, ed);
+            op.template fold<1>(st, slot + v * STEP, tab0 + (i + v) * ENTRY, act, (unsigned)j0 + p + v, ed);
           }
         }
         stage_some(slot, i + ahead, rs, os, es, ss);
@@ -640,7 +640,7 @@ struct GroupAggregate : GEO, Shape<GEO, 1, (int)sizeof(typename GEO::T), 1, 0, 0
     return w + ((unsigned long long)(unsigned)e * (unsigned)this->H + h);
   }
   template <int N>
-  __device__ __forceinline__ void fold(State& st, unsigned slot, unsigned tab, const bool (&)[N], int,
+  __device__ __forceinline__ void fold(State& st, unsigned slot, unsigned tab, const bool (&)[N], unsigned,
                                        const int (&)[N]) const {
     // positions without an edge have rows and weights of zeros
 #pragma unroll
@@ -701,7 +701,7 @@ struct GroupFeatAggregate : GEO, Shape<GEO, 1, (int)sizeof(typename GEO::T), 1, 
     return w + ((unsigned long long)(unsigned)e * (unsigned)W + h);
   }
   template <int N>
-  __device__ __forceinline__ void fold(State& st, unsigned slot, unsigned tab, const bool (&)[N], int,
+  __device__ __forceinline__ void fold(State& st, unsigned slot, unsigned tab, const bool (&)[N], unsigned,
                                        const int (&)[N]) const {
 #pragma unroll
     for (int v = 0; v < N; ++v) {
@@ -765,7 +765,7 @@ struct GroupEdgeDot : GEO, Shape<GEO, 1, 0, 1, 1, 0, 2> {
   }
   __device__ __forceinline__ const void* scalar_of(int, int, int) const { return nullptr; }
   template <int N>
-  __device__ __forceinline__ void fold(State& st, unsigned slot, unsigned, const bool (&active)[N], int,
+  __device__ __forceinline__ void fold(State& st, unsigned slot, unsigned, const bool (&active)[N], unsigned,
                                        const int (&e)[N]) const {
     A s[N];
 #pragma unroll
@@ -836,7 +836,7 @@ struct GroupAttnFwd : GEO, Shape<GEO, kBias ? 3 : 2, 0, 2, 1, 0, 2> {
   }
   __device__ __forceinline__ const void* scalar_of(int, int, int) const { return nullptr; }
   template <int N>
-  __device__ __forceinline__ void fold(State& st, unsigned slot, unsigned, const bool (&active)[N], int,
+  __device__ __forceinline__ void fold(State& st, unsigned slot, unsigned, const bool (&active)[N], unsigned,
                                        const int (&)[N]) const {
     A s[N], p[N];
     A mn = st.m;
@@ -977,7 +977,7 @@ struct GroupAttnBwdDst : GEO, Shape<GEO, kBias ? 3 : 2, 0, 4, 3, (int)sizeof(typ
   }
   __device__ __forceinline__ const void* scalar_of(int, int, int) const { return nullptr; }
   template <int N>
-  __device__ __forceinline__ void fold(State& st, unsigned slot, unsigned, const bool (&active)[N], int pos,
+  __device__ __forceinline__ void fold(State& st, unsigned slot, unsigned, const bool (&active)[N], unsigned pos,
                                        const int (&)[N]) const {
     A s[N], dp[N];
     F f[N][W];
@@ -1005,7 +1005,7 @@ struct GroupAttnBwdDst : GEO, Shape<GEO, kBias ? 3 : 2, 0, 4, 3, (int)sizeof(typ
       A ds = p * (dp[v] - st.delta) * scale;
       if (!active[v]) ds = A(0);
       if (active[v] && pd && st.ln.first)
-        pd[(unsigned long long)(unsigned)(pos + v) * (unsigned)Hp + st.ln.head] = EdgePair<A>{p, ds};
+        pd[(unsigned long long)(pos + v) * (unsigned)Hp + st.ln.head] = EdgePair<A>{p, ds};
 #pragma unroll
       for (int i = 0; i < W; ++i) st.acc[i].axpy(ds, f[v][i]);
     }
@@ -1104,7 +1104,7 @@ struct GroupAttnBwdSrc : GEO, Shape<GEO, 2, 2 * (int)sizeof(typename GEO::A), kP
     else return stat + ((unsigned long long)(unsigned)id * (unsigned)Hp + h);
   }
   template <int N>
-  __device__ __forceinline__ void fold(State& st, unsigned slot, unsigned tab, const bool (&active)[N], int,
+  __device__ __forceinline__ void fold(State& st, unsigned slot, unsigned tab, const bool (&active)[N], unsigned,
                                        const int (&)[N]) const {
     // positions without an edge have rows and pairs of zeros
 #pragma unroll

@@ -51,7 +51,7 @@ __device__ __forceinline__ void band_positions(const int32_t* __restrict__ erow,
     const int r = erow[j];
     if (r < 0) continue;
     const int f = first[r];
-    if (other[j] != other[f] + (int)(j - f)) bad = 1;
+    if (other[j] != other[f] + (j - f)) bad = 1;   // in 64 bits: on any other graph the sum may pass 2^31
   }
   // one atomic per block, none once the verdict is known (one per thread serialised: 14 us on 0.6M edges)
   if (__syncthreads_or(bad) && threadIdx.x == 0 && !*(volatile const int*)&verdict->not_contiguous)
@@ -70,7 +70,8 @@ __device__ __forceinline__ void band_tiles(const int32_t* __restrict__ other, co
     const int d = deg[r];
     const int l = d > 0 ? other[first[r]] : 0;
     node_lo[r] = l;
-    if (d > 0) { lo = l; hi = l + d - 1; }
+    // (the end of a run of d neighbours from l; where they are no run the graph is no band, and the clamp says nothing)
+    if (d > 0) { lo = l; hi = (int)min((long long)l + d - 1, (long long)INT_MAX - 1); }
   }
 #pragma unroll
   for (int o = 16; o; o >>= 1) {
@@ -81,7 +82,8 @@ __device__ __forceinline__ void band_tiles(const int32_t* __restrict__ other, co
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int w = 1; w < kBandTileRows / 32; ++w) { lo = min(lo, s_lo[w]); hi = max(hi, s_hi[w]); }
-    if (hi >= lo && hi - lo + 1 > *(volatile const int*)&verdict->max_span) atomicMax(&verdict->max_span, hi - lo + 1);
+    const int span = hi >= lo ? hi - lo + 1 : 0;
+    if (span > *(volatile const int*)&verdict->max_span) atomicMax(&verdict->max_span, span);
   }
 }
 
