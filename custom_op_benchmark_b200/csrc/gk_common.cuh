@@ -40,8 +40,6 @@ template <> __device__ __forceinline__ __nv_bfloat16 from_acc<__nv_bfloat16>(flo
 
 __device__ __forceinline__ float gk_exp(float x) { return expf(x); }
 __device__ __forceinline__ double gk_exp(double x) { return exp(x); }
-__device__ __forceinline__ float gk_log(float x) { return logf(x); }
-__device__ __forceinline__ double gk_log(double x) { return log(x); }
 template <typename A> __device__ __forceinline__ A neg_inf();
 template <> __device__ __forceinline__ float neg_inf<float>() { return -INFINITY; }
 template <> __device__ __forceinline__ double neg_inf<double>() { return -(double)INFINITY; }
@@ -94,14 +92,6 @@ template <typename A> __device__ __forceinline__ A warp_sum(A v) {
   return v;
 }
 
-// One value per lane summed over the LPH lanes of a head, lane distances 1, 2, 4, ... in that order.
-template <int LPH, typename A>
-__device__ __forceinline__ A reduce_ascending(A v) {
-#pragma unroll
-  for (int o = 1; o < LPH; o <<= 1) v += __shfl_xor_sync(kFull, v, o);
-  return v;
-}
-
 // Per-lane view of a node's feature row: lane owns slots lane, lane+32, ..., each V elements.
 template <int R> struct SlotMap {
   int head[R];  // head index of the slot
@@ -120,33 +110,6 @@ template <int R> struct SlotMap {
     }
   }
 };
-
-// Sums the per-register partial dot products over the lanes (and registers) that hold the
-// same head; afterwards every lane holds the head's total in each of its registers.
-// lph = lanes (vector slots) per head, a power of two.
-template <typename A, int R>
-__device__ __forceinline__ void reduce_heads(A (&p)[R], int lph) {
-  if (lph >= 32) {
-    const int rph = lph >> 5;  // registers per head
-#pragma unroll
-    for (int s = 1; s < R; s <<= 1) {
-      if (s < rph) {
-        A t[R];
-#pragma unroll
-        for (int i = 0; i < R; ++i) t[i] = p[i ^ s];
-#pragma unroll
-        for (int i = 0; i < R; ++i) p[i] += t[i];
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < R; ++i) p[i] = warp_sum(p[i]);
-  } else {
-    for (int o = 1; o < lph; o <<= 1) {
-#pragma unroll
-      for (int i = 0; i < R; ++i) p[i] += __shfl_xor_sync(kFull, p[i], o);
-    }
-  }
-}
 
 // ---------------------------------------------------------------------------------------
 // expansion: chunk table -> erow[], optional int64 -> int32 copies of indices / eid

@@ -97,15 +97,6 @@ template <int V> struct Frag<float, V> {
 #pragma unroll
     for (int i = 0; i < P; ++i) p[i] = fma2(x.p[i], bb, mul2(p[i], aa));
   }
-  __device__ __forceinline__ void add_xor(int lanes) {
-#pragma unroll
-    for (int i = 0; i < P; ++i) {
-      float a, b;
-      unpack2(a, b, p[i]);
-      const float ta = __shfl_xor_sync(kFull, a, lanes), tb = V == 1 ? 0.f : __shfl_xor_sync(kFull, b, lanes);
-      p[i] = add2(p[i], pack2(ta, tb));
-    }
-  }
 };
 
 template <int V> struct Frag<double, V> {
@@ -137,10 +128,6 @@ template <int V> struct Frag<double, V> {
   __device__ __forceinline__ void blend(double wa, const Frag& x, double wb) {
 #pragma unroll
     for (int i = 0; i < V; ++i) p[i] = p[i] * wa + x.p[i] * wb;
-  }
-  __device__ __forceinline__ void add_xor(int lanes) {
-#pragma unroll
-    for (int i = 0; i < V; ++i) p[i] += __shfl_xor_sync(kFull, p[i], lanes);
   }
 };
 
@@ -213,7 +200,7 @@ __device__ __forceinline__ void lds2(float& a, float& b, unsigned at) {
 __device__ __forceinline__ void lds2(double& a, double& b, unsigned at) {
   asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(a), "=d"(b) : "r"(at));
 }
-// raw slot bytes -> fragment, from shared memory / from global memory (read-only data)
+// raw slot bytes -> fragment, from shared memory
 template <typename T, int SB>
 __device__ __forceinline__ void frag_lds(Frag<typename AccOf<T>::type, SB / (int)sizeof(T)>& f, unsigned at) {
   if constexpr (sizeof(T) == 4 && SB == 16) {
@@ -228,10 +215,6 @@ __device__ __forceinline__ void frag_lds(Frag<typename AccOf<T>::type, SB / (int
     lds(w, at);
     frag_unpack<T, SB>(f, w);
   }
-}
-template <typename T, int SB>
-__device__ __forceinline__ void frag_ldg(Frag<typename AccOf<T>::type, SB / (int)sizeof(T)>& f, const void* p) {
-  frag_unpack<T, SB>(f, __ldg(reinterpret_cast<const typename SlotWord<SB>::type*>(p)));
 }
 // fragment -> V elements of T, one store of SB bytes
 template <typename T, int SB>

@@ -14,7 +14,6 @@ and float64; ``dy`` is made contiguous instead of being read unchecked
 (graphop.cpp:120-130, 148-153); the source and destination node counts may differ.
 """
 import collections
-import weakref
 
 import torch as th
 

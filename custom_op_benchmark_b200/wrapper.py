@@ -8,7 +8,6 @@ another module with the ops of `graphop` (the compiled module of that name, say)
 more than the native node: while torch.jit.trace records, under torch.func's transforms and dispatch modes, on tensors
 with a forward-mode tangent; and all there is in a package built without the compiled modules.
 """
-import torch as th
 from torch.autograd import Function
 
 from . import graphop as _g
