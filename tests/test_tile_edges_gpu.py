@@ -1,6 +1,6 @@
 """The kernels' tiles at their edges: rows one short of, as long as and one longer than a work tile, a softmax tile and an
-expansion step, a row over many of them, empty rows between; head sizes and counts on both sides of every dispatch
-line.  Against the float64 oracle."""
+expansion step, a row over many of them, empty rows between; head sizes and counts of every kind (each geometry the walker
+is compiled for: test_geometries_gpu.py).  Against the float64 oracle."""
 import threading
 
 import pytest
