@@ -17,8 +17,10 @@ time, against the measured HBM copy bandwidth), `cpu_baseline` (the torch CPU ch
 sample), `kernels` (per-kernel mean milliseconds of one step), `phases` (forward / backward ms).
 """
 import argparse
+import hashlib
 import json
 import os
+import re
 import statistics
 import subprocess
 import sys
@@ -902,12 +904,27 @@ def measured_peak():
     return 6650.0, "fallback"
 
 
-def traffic_for(kernel, workload):
-    """DRAM bytes per launch of `kernel` on `workload` from the committed ncu summary, if any."""
-    path = os.path.join(ROOT, "profiles", "dram_traffic.json")
-    if os.path.exists(path):
-        return json.load(open(path)).get(workload, {}).get(kernel)
-    return None
+def code_digest(names, root=None):
+    """Digest of kernel sources without their comments and white space: what a captured figure was measured on."""
+    digest = hashlib.sha256()
+    for name in names:
+        with open(os.path.join(root or ROOT, "custom_op_benchmark_b200", "csrc", name)) as f:
+            text = re.sub(r"//[^\n]*|/\*.*?\*/", "", f.read(), flags=re.S)
+        digest.update(re.sub(r"\s+", "", text).encode())
+    return digest.hexdigest()[:16]
+
+
+def traffic_for(kernel, workload, scale=None, root=None):
+    """DRAM bytes per launch of `kernel` on `workload` from the committed ncu summary; None where there is none, where the
+    kernels have changed since it was captured, or for another graph size than the workload's own."""
+    path = os.path.join(root or ROOT, "profiles", "dram_traffic.json")
+    if scale or not os.path.exists(path):
+        return None
+    with open(path) as f:
+        captured = json.load(f).get(workload)
+    if not captured or code_digest(captured["sources"], root) != captured["digest"]:
+        return None
+    return captured["bytes"].get(kernel)
 
 
 def build_workload(args, spec, rank, dev, world):
@@ -1189,13 +1206,13 @@ def run_gpu(args):
             "roofline": {"bound": "hbm", "kernel": top, "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "peak_source": peak_kind, "algorithmic_bytes": alg[top],
                          "frac_of_spec_8000": achieved / 8000.0,
-                         "ms": top_ms, "traffic": traffic_for(top, args.workload),
+                         "ms": top_ms, "traffic": traffic_for(top, args.workload, args.scale),
                          "gather_bytes": wl.gather_bytes(top) if hasattr(wl, "gather_bytes") else None,
                          "step_algorithmic_bytes": wl.alg_step,
                          "step_frac": wl.alg_step / (ms_per_step * 1e-3) / 1e9 / peak},
             "kernels": kernels,
         }
-        traffic_step = sum(traffic_for(k, args.workload) or 0 for k in kernels)
+        traffic_step = sum(traffic_for(k, args.workload, args.scale) or 0 for k in kernels)
         if traffic_step:
             out["roofline"]["step_dram_traffic"] = traffic_step
             out["roofline"]["step_dram_frac"] = traffic_step / (ms_per_step * 1e-3) / 1e9 / peak
