@@ -199,7 +199,6 @@ graphop_stream_t raw(cudaStream_t s) { return (graphop_stream_t)s; }
 // nothing else: the tables that the kernels make of a chunk table are workspace of either direction.  Two threads may run
 // the backward of one graph: the saved tensors are read and released under the node's mutex.
 struct GraphNode : Node {
-  std::string name() const override { return "GraphopBackward"; }
   void save(const Tensor& t, bool is_output = false) {
     // an index tensor made in inference mode has no version to check: kept as it is
     const bool plain = t.defined() && t.is_inference() && !at::isFloatingType(t.scalar_type());
@@ -243,6 +242,7 @@ int check_columns(const std::vector<Tensor>& t, size_t at, size_t n, const char*
 
 // ---- SparseSoftmax (wrapper.py:8-18) ------------------------------------------------------
 struct SparseSoftmaxBackward : GraphNode {
+  std::string name() const override { return "SparseSoftmaxBackward"; }
   variable_list apply(variable_list&& grads) override {
     if (!grads[0].defined()) return {Tensor()};
     const std::vector<Tensor> t = unpack_saved();   // row, indptr, eid, y
@@ -289,6 +289,7 @@ Result sparse_softmax(const Tensor& row, const Tensor& indptr, const Tensor& eid
 
 // ---- MaskedMMCSR (wrapper.py:20-30) -------------------------------------------------------
 struct MaskedMMBackward : GraphNode {
+  std::string name() const override { return "MaskedMMCSRBackward"; }
   variable_list apply(variable_list&& grads) override {
     if (!grads[0].defined()) return {Tensor(), Tensor()};
     const std::vector<Tensor> t = unpack_saved();   // row, indptr_r, eid_r, indices_r, col, indptr_c, eid_c, indices_c, A, B
@@ -343,6 +344,7 @@ Result maskedmm_csr(const Tensor& row, const Tensor& indptr_r, const Tensor& eid
 
 // ---- NodeMulEdge (wrapper.py:32-42) -------------------------------------------------------
 struct NodeMulEdgeBackward : GraphNode {
+  std::string name() const override { return "NodeMulEdgeBackward"; }
   variable_list apply(variable_list&& grads) override {
     if (!grads[0].defined()) return {Tensor(), Tensor()};
     const std::vector<Tensor> t = unpack_saved();   // row, indptr, eid, A, B
@@ -389,6 +391,7 @@ Result node_mul_edge(const Tensor& row, const Tensor& indptr, const Tensor& eid,
 
 // ---- VectorSPMM (wrapper.py:44-55) --------------------------------------------------------
 struct VectorSPMMBackward : GraphNode {
+  std::string name() const override { return "VectorSPMMBackward"; }
   variable_list apply(variable_list&& grads) override {
     if (!grads[0].defined()) return {Tensor(), Tensor()};
     const std::vector<Tensor> t = unpack_saved();   // row, indptr, eid, indices, col, indptr_t, eid_t, indices_t, w, x
@@ -467,6 +470,7 @@ void no_edges(Tensor& o, Tensor& lse) {
 }
 
 struct AttentionBackward : GraphNode {
+  std::string name() const override { return "GraphAttentionPlannedBackward"; }
   GraphPtr rows, cols;
   double scale = 1.0;
   variable_list apply(variable_list&& grads) override {
@@ -522,6 +526,7 @@ Result attention_planned(const PlanHandle& plan_r, const PlanHandle& plan_t, con
 
 // ---- fused attention with an edge term on chunk tables --------------------------------------
 struct AttentionBiasBackward : GraphNode {
+  std::string name() const override { return "GraphAttentionBiasBackward"; }
   double scale = 1.0;
   variable_list apply(variable_list&& grads) override {
     if (!grads[0].defined()) return variable_list(4);

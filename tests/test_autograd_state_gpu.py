@@ -156,3 +156,13 @@ def test_inference_without_the_column_side(tables, name):
     out = function.apply(*tabs[:half], None, None, None, None, *_leaves(given))
     with pytest.raises(RuntimeError, match="col must be a CUDA tensor"):
         out.sum().backward()
+
+
+@pytest.mark.parametrize("name", FUNCTIONS)
+def test_nodes_have_the_names_of_their_functions(tables, name):
+    function, tabs, given = _call(name, tables)
+    leaves = _leaves(given)
+    with th.autograd.set_detect_anomaly(True):   # which reports nodes by these names
+        out = function.apply(*tabs, *leaves)
+        assert out.grad_fn.name() == name + "Backward"
+        th.autograd.grad(out, _tensors(leaves), th.ones_like(out))
