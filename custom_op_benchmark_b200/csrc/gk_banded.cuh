@@ -225,7 +225,7 @@ __device__ __forceinline__ void store_stage_row(unsigned char* row_at, int c, in
 }
 // One block per (tile of 128 nodes, head).  Bound by the chain load - scores - softmax - output of a block of the band; three
 // tiles per SM overlap theirs.  With one tile of 512 threads per SM and the whole band in shared memory, four sequences of
-// 8192, 8 heads, window 128, took 121 us.
+// 8192, 8 heads, window 128, took 121 us instead of 86.
 __global__ void __launch_bounds__(kThreads, 3)
 attention_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                          const __grid_constant__ CUtensorMap map_v, const Params p) {
@@ -450,8 +450,8 @@ attention_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
 // A tile takes the blocks its band reaches, two of them in shared memory at a time: the next but one is asked for when the
 // gradient products that read its slot are done.  85 KB (destination side) or 101 KB (source side) of shared memory and
 // 256 tensor-memory columns, so that two tiles share an SM and one's products and loads run under the other's
-// element-wise stage: with the whole band and 128 x 128 staging tiles (one tile per SM) the tensor pipe was busy 9 to 13 %
-// of the time and every wait was exposed.
+// element-wise stage: with the whole band and 128 x 128 staging tiles (one tile per SM) the tensor pipe was busy 11 to 14 %
+// of the time and every wait was exposed; now 16 to 17 %.
 // ---------------------------------------------------------------------------------------------------------
 struct BwdParams {
   const __nv_bfloat16* o;     // (n_dst, H, 64): destination side only

@@ -373,7 +373,7 @@ __global__ void zero_uncovered_kernel(const PlanHeader* __restrict__ hdr, long l
 // wholly inside one node writes its partial to slot 2t and a neutral partial to 2t+1, so
 // the slots of one node are always consecutive.  Level k+1 (kCarryLevel = true) walks that
 // slot stream with the same code, merging partials instead of edges, stores the nodes whose
-// slots end inside one of its tiles and emits the next, 128-times shorter stream, until a
+// slots end inside one of its tiles and emits the next stream, of two slots per tile, until a
 // level fits one tile.  Every merge order is a function of (E, tile sizes) only.
 template <class Op, bool kCarryLevel>
 __global__ void __launch_bounds__(kWarpsPerCta * 32)

@@ -1,7 +1,7 @@
 // The gathering walker: row-owned reductions and per-edge products over a CSR position stream.
 //
-// Decomposition (as in gk_common.cuh): the positions 0..E-1 are cut into tiles of equal length, so the work of a tile does
-// not depend on the degrees.  A warp is NE = 32 / G groups of G lanes and every group walks a tile of its own:
+// Decomposition (as in gk_common.cuh): the positions 0..E-1 are cut into tiles of equal cost (cut_tiles), so the work of a
+// tile does not depend on the degrees.  A warp is NE = 32 / G groups of G lanes and every group walks a tile of its own:
 //   * A step folds one position per group.  A lane owns W slots (16, 8 or 4 bytes each) of one head of the row, a row of
 //     128 bytes is 8 lanes: four edges per step share the address arithmetic, shuffles, exponentials and loop work that one
 //     edge spread over 32 lanes would need alone.  Groups never exchange partial results: a node's edges are folded by the

@@ -1,7 +1,7 @@
-// The per-edge bodies ("ops") that the tile walker of gk_common.cuh drives, one per
-// reference kernel family.  Each op cites the reference kernel whose arithmetic it computes
-// (graphop/graphop_kernel.cu); none of them shares its scheduling: no transposed copies of
-// the node tensors, no atomics, 128-bit loads of whole feature rows.
+// The ops of walk_kernel (gk_common.cuh), for the row shapes that the gathering walker (gk_group.cuh) has no slot width
+// for, and the kernels over edge feature rows that all heads of a node share.  Each cites the reference kernel whose
+// arithmetic it computes (graphop/graphop_kernel.cu); none of them shares its scheduling: no transposed copies of the node
+// tensors, no atomics.
 #pragma once
 #include "gk_common.cuh"
 
