@@ -120,6 +120,12 @@ struct Call {
 // a tensor's storage as the element type the entry point wants; null for an undefined one
 template <typename E> E* ptr(const Tensor& t) { return t.defined() ? reinterpret_cast<E*>(t.data_ptr()) : nullptr; }
 
+// The owner nodes of a chunk table.  One without chunks is a table like any other (every edge output is zero), but has no
+// memory, and the entry points refuse a null pointer: nothing is read through this one.
+template <typename I> const I* owners(const Tensor& row, const Tensor& indptr) {
+  return row.size(0) ? ptr<I>(row) : ptr<I>(indptr);
+}
+
 // An argument that only the backward reads: a call without one may leave it out.
 using Later = c10::optional<Tensor>;
 Tensor given(const Later& t) { return t.value_or(Tensor()); }
@@ -256,7 +262,7 @@ struct SparseSoftmaxBackward : GraphNode {
     check_status(by_types(elem, ib, [&](auto* k, auto* i) {
       using E = std::remove_pointer_t<decltype(k)>;
       using I = std::remove_pointer_t<decltype(i)>;
-      return sparse_softmax_backward(k, i, (const I*)ptr<I>(t[0]), (const I*)ptr<I>(t[1]), (const I*)ptr<I>(t[2]),
+      return sparse_softmax_backward(k, i, owners<I>(t[0], t[1]), (const I*)ptr<I>(t[1]), (const I*)ptr<I>(t[2]),
                                      (const E*)ptr<E>(y), (const E*)ptr<E>(dy), ptr<E>(dx), chunks, e, (int64_t)0, H, c.ws,
                                      c.bytes, raw(c.stream));
     }), "sparse_softmax_backward");
@@ -276,7 +282,7 @@ Result sparse_softmax(const Tensor& row, const Tensor& indptr, const Tensor& eid
     check_status(by_types(elem, ib, [&](auto* k, auto* i) {
       using E = std::remove_pointer_t<decltype(k)>;
       using I = std::remove_pointer_t<decltype(i)>;
-      return sparse_softmax_forward(k, i, (const I*)ptr<I>(row), (const I*)ptr<I>(indptr), (const I*)ptr<I>(eid),
+      return sparse_softmax_forward(k, i, owners<I>(row, indptr), (const I*)ptr<I>(indptr), (const I*)ptr<I>(eid),
                                     (const E*)ptr<E>(x), ptr<E>(y), chunks, e, (int64_t)0, H, c.ws, c.bytes, raw(c.stream));
     }), "sparse_softmax_forward");
   }
@@ -306,7 +312,7 @@ struct MaskedMMBackward : GraphNode {
       using E = std::remove_pointer_t<decltype(k)>;
       using I = std::remove_pointer_t<decltype(i)>;
       const auto in = [&](int at) { return (const I*)ptr<I>(t[at]); };
-      return maskedmm_csr_backward(k, i, in(0), in(1), in(2), in(3), chunks, in(4), in(5), in(6), in(7), chunks_c,
+      return maskedmm_csr_backward(k, i, owners<I>(t[0], t[1]), in(1), in(2), in(3), chunks, owners<I>(t[4], t[5]), in(5), in(6), in(7), chunks_c,
                                    (const E*)ptr<E>(A), (const E*)ptr<E>(B), (const E*)ptr<E>(dy), ptr<E>(dA), ptr<E>(dB), e,
                                    s.n, nb, s.H, s.D, c.ws, c.bytes, raw(c.stream));
     }), "maskedmm_csr_backward");
@@ -331,7 +337,7 @@ Result maskedmm_csr(const Tensor& row, const Tensor& indptr_r, const Tensor& eid
     check_status(by_types(elem, ib, [&](auto* k, auto* i) {
       using E = std::remove_pointer_t<decltype(k)>;
       using I = std::remove_pointer_t<decltype(i)>;
-      return maskedmm_csr_forward(k, i, (const I*)ptr<I>(row), (const I*)ptr<I>(indptr_r), (const I*)ptr<I>(eid_r),
+      return maskedmm_csr_forward(k, i, owners<I>(row, indptr_r), (const I*)ptr<I>(indptr_r), (const I*)ptr<I>(eid_r),
                                   (const I*)ptr<I>(indices_r), (const E*)ptr<E>(A), (const E*)ptr<E>(B), ptr<E>(y), chunks, e,
                                   s.n, nb, s.H, s.D, c.ws, c.bytes, raw(c.stream));
     }), "maskedmm_csr_forward");
@@ -359,7 +365,7 @@ struct NodeMulEdgeBackward : GraphNode {
     check_status(by_types(elem, ib, [&](auto* k, auto* i) {
       using E = std::remove_pointer_t<decltype(k)>;
       using I = std::remove_pointer_t<decltype(i)>;
-      return node_mul_edge_backward(k, i, (const I*)ptr<I>(t[0]), (const I*)ptr<I>(t[1]), (const I*)ptr<I>(t[2]),
+      return node_mul_edge_backward(k, i, owners<I>(t[0], t[1]), (const I*)ptr<I>(t[1]), (const I*)ptr<I>(t[2]),
                                     (const E*)ptr<E>(A), (const E*)ptr<E>(B), (const E*)ptr<E>(dy), ptr<E>(dA), ptr<E>(dB),
                                     chunks, e, s.n, s.H, s.D, c.ws, c.bytes, raw(c.stream));
     }), "node_mul_edge_backward");
@@ -380,7 +386,7 @@ Result node_mul_edge(const Tensor& row, const Tensor& indptr, const Tensor& eid,
     check_status(by_types(elem, ib, [&](auto* k, auto* i) {
       using E = std::remove_pointer_t<decltype(k)>;
       using I = std::remove_pointer_t<decltype(i)>;
-      return node_mul_edge_forward(k, i, (const I*)ptr<I>(row), (const I*)ptr<I>(indptr), (const I*)ptr<I>(eid),
+      return node_mul_edge_forward(k, i, owners<I>(row, indptr), (const I*)ptr<I>(indptr), (const I*)ptr<I>(eid),
                                    (const E*)ptr<E>(A), (const E*)ptr<E>(B), ptr<E>(y), chunks, e, s.n, s.H, s.D, c.ws, c.bytes,
                                    raw(c.stream));
     }), "node_mul_edge_forward");
@@ -408,7 +414,7 @@ struct VectorSPMMBackward : GraphNode {
       using E = std::remove_pointer_t<decltype(k)>;
       using I = std::remove_pointer_t<decltype(i)>;
       const auto in = [&](int at) { return (const I*)ptr<I>(t[at]); };
-      return vector_spmm_backward(k, i, in(0), in(1), in(2), in(3), chunks, in(4), in(5), in(6), in(7), chunks_t,
+      return vector_spmm_backward(k, i, owners<I>(t[0], t[1]), in(1), in(2), in(3), chunks, owners<I>(t[4], t[5]), in(5), in(6), in(7), chunks_t,
                                   (const E*)ptr<E>(w), (const E*)ptr<E>(dy), (const E*)ptr<E>(x), ptr<E>(dw), ptr<E>(dx), e,
                                   n_dst, s.n, s.H, s.D, c.ws, c.bytes, raw(c.stream));
     }), "vector_spmm_backward");
@@ -436,7 +442,7 @@ Result vector_spmm(const Tensor& row, const Tensor& indptr, const Tensor& eid, c
     check_status(by_types(elem, ib, [&](auto* k, auto* i) {
       using E = std::remove_pointer_t<decltype(k)>;
       using I = std::remove_pointer_t<decltype(i)>;
-      return vector_spmm_forward(k, i, (const I*)ptr<I>(row), (const I*)ptr<I>(indptr), (const I*)ptr<I>(eid),
+      return vector_spmm_forward(k, i, owners<I>(row, indptr), (const I*)ptr<I>(indptr), (const I*)ptr<I>(eid),
                                  (const I*)ptr<I>(indices), (const E*)ptr<E>(w), (const E*)ptr<E>(x), ptr<E>(y), chunks, e, s.n,
                                  s.n, s.H, s.D, c.ws, c.bytes, raw(c.stream));
     }), "vector_spmm_forward");
@@ -546,7 +552,7 @@ struct AttentionBiasBackward : GraphNode {
       using E = std::remove_pointer_t<decltype(x)>;
       using I = std::remove_pointer_t<decltype(i)>;
       const auto in = [&](int at) { return (const I*)ptr<I>(t[at]); };
-      return attention_bias_backward(x, i, in(0), in(1), in(2), chunks, in(3), in(4), in(5), in(6), chunks_t,
+      return attention_bias_backward(x, i, owners<I>(t[0], t[1]), in(1), in(2), chunks, owners<I>(t[3], t[4]), in(4), in(5), in(6), chunks_t,
                                      (const E*)ptr<E>(q), (const E*)ptr<E>(k), (const E*)ptr<E>(v), (const E*)ptr<E>(rel),
                                      (const E*)ptr<E>(o), (const void*)lse.data_ptr(), (const E*)ptr<E>(g), scale, ptr<E>(dq),
                                      ptr<E>(dk), ptr<E>(dv), ptr<E>(drel), e, s.n, nk, s.H, s.D, c.ws, c.bytes, raw(c.stream));
@@ -575,7 +581,7 @@ Result attention_bias(const Tensor& row, const Tensor& indptr, const Tensor& ind
     check_status(by_types(elem, ib, [&](auto* x, auto* i) {
       using E = std::remove_pointer_t<decltype(x)>;
       using I = std::remove_pointer_t<decltype(i)>;
-      return attention_bias_forward(x, i, (const I*)ptr<I>(row), (const I*)ptr<I>(indptr), (const I*)ptr<I>(indices), chunks,
+      return attention_bias_forward(x, i, owners<I>(row, indptr), (const I*)ptr<I>(indptr), (const I*)ptr<I>(indices), chunks,
                                     (const E*)ptr<E>(q), (const E*)ptr<E>(k), (const E*)ptr<E>(v), (const E*)ptr<E>(rel), scale,
                                     ptr<E>(o), (void*)lse.data_ptr(), e, s.n, nk, s.H, s.D, c.ws, c.bytes, raw(c.stream));
     }), "attention_bias_forward");

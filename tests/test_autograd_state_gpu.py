@@ -166,3 +166,20 @@ def test_nodes_have_the_names_of_their_functions(tables, name):
         out = function.apply(*tabs, *leaves)
         assert out.grad_fn.name() == name + "Backward"
         th.autograd.grad(out, _tensors(leaves), th.ones_like(out))
+
+
+@pytest.mark.parametrize("name", FUNCTIONS)
+@pytest.mark.parametrize("start", [0, 3])
+def test_chunk_tables_without_chunks(name, start):
+    """No chunk, seven edges: outputs and gradients are zero, whatever position the table stops at."""
+    empty, stop = th.zeros(0, dtype=th.int64, device=DEV), th.full((1,), start, dtype=th.int64, device=DEV)
+    ids = th.arange(7, device=DEV) % 5
+    table = [empty, stop, th.arange(7, device=DEV), ids]
+    node, edge, rel = _normal(5, H, D, seed=1), _normal(7, H, seed=2), _normal(7, D, seed=3)
+    tabs, given = {"SparseSoftmax": (table[:3], [edge]), "MaskedMMCSR": (table * 2, [node, node]),
+                   "NodeMulEdge": (table[:3], [node, rel]), "VectorSPMM": (table * 2, [edge, node]),
+                   "GraphAttentionBias": ([empty, stop, ids, *table], [node, node, node, rel, 0.25])}[name]
+    leaves = _leaves(given)
+    out = getattr(wrapper, name).apply(*tabs, *leaves)
+    assert not out.any()
+    assert not any(g.any() for g in th.autograd.grad(out, _tensors(leaves), th.ones_like(out)))
