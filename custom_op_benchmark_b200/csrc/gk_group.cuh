@@ -51,11 +51,12 @@ struct WalkArgs {
   const int32_t* erow;
   const int32_t* other;
   const int32_t* eid;          // null: an edge's id is its position
-  const int32_t* tile_start;   // (ntiles[0] + 1) boundaries
+  const int32_t* tile_start;   // (cut_tiles + 1) boundaries
   long long E, n_rows;
   int tile;                    // nominal cost of a tile; rows at least this long may be cut
   int aligned;                 // the boundaries are row starts already wherever a row can be kept whole
-  unsigned n_tiles;
+  unsigned cut_tiles, span;    // tiles the graph was cut into; `span` consecutive ones are one tile of this launch
+  unsigned n_tiles;            // tiles of this launch
   void* carry;                 // (head blocks, 2 * n_tiles) partial records; null: no row crosses a tile boundary
   uint32_t* rows;              // what each record stands for: 2 * node + 1, 2 * node where the slot holds nothing (its tile
                                // lies inside one node that goes on), kNoRow: unused
@@ -281,7 +282,8 @@ group_walk_kernel(const __grid_constant__ Op op, const __grid_constant__ WalkArg
   const bool here = t < a.n_tiles;
   // A nominal boundary moves up to the first row start within the following `tile` positions, so that only rows longer
   // than a tile are ever cut (in a plan's boundaries that is done; else every group looks for its own).
-  long long j0 = __ldg(a.tile_start + (here ? t : 0u)), j1 = __ldg(a.tile_start + (here ? t + 1 : 0u));
+  const unsigned cut0 = here ? t * a.span : 0u, cut1 = here ? min(cut0 + a.span, a.cut_tiles) : 0u;
+  long long j0 = __ldg(a.tile_start + cut0), j1 = __ldg(a.tile_start + cut1);
   if (!a.aligned) {
     auto move_up = [&](long long x) {
       long long found = x <= 0 ? 0 : x >= a.E ? a.E : -1;

@@ -176,6 +176,20 @@ inline int allow_smem(Kernel kernel, int bytes, std::atomic<bool> (&configured)[
   return GRAPHOP_OK;
 }
 
+// How many of the graph's tiles a lane group walks as one.  A tile begins with a chain of dependent loads (boundaries, nodes
+// and endpoints, the first rows) and ends in carry records; with the head blocks of a wide row the smallest tiles make far
+// more warps than it takes to fill the chip.  About kWarpsWanted warps leave every SM six rounds or more of them.  Step times
+// with a tile each and with about 16 K, 20 K and 40 K warps: 15360 nodes of 30 edges, 8 x 64 fp32, three Functions 811 / 747 /
+// - / 811 us; R-MAT 18 with an edge term, 4 x 64 bf16, 2.79 / 2.58 / 2.59 / 2.79 ms; R-MAT 20, 4 x 32, multiply and aggregate
+// 5.84 / - / 5.70 / 5.84; R-MAT 22, 1 x 128, aggregate 13.5 / - / 12.7 / 12.5; with 4 K the chip is not filled evenly (R-MAT
+// 18: 3.0 ms).
+constexpr long long kWarpsWanted = 20480;
+inline unsigned tile_span(long long n_tiles, int nhb, int per_warp) {
+  const long long warps = n_tiles * nhb / per_warp;
+  const long long span = (warps + kWarpsWanted / 2) / kWarpsWanted;
+  return span < 1 ? 1 : span < n_tiles ? (unsigned)span : (unsigned)n_tiles;
+}
+
 // The op over every position and head block, and the merge of the rows that tiles had to cut.
 template <class Op>
 inline int launch_walk(Arena& ar, const GraphView& g, const GeoPick& p, const Op& op, long long n_rows, cudaStream_t st) {
@@ -183,10 +197,12 @@ inline int launch_walk(Arena& ar, const GraphView& g, const GeoPick& p, const Op
   a.hdr = g.hdr; a.erow = g.erow; a.other = g.other; a.eid = g.eid;
   a.tile_start = g.tile_start;
   a.E = g.E; a.n_rows = n_rows; a.tile = g.tile; a.aligned = g.aligned;
-  a.n_tiles = (unsigned)g.n_tiles;
+  a.cut_tiles = (unsigned)g.n_tiles;
+  a.span = tile_span(g.n_tiles, p.nhb, Op::NE);
+  a.n_tiles = (a.cut_tiles + a.span - 1) / a.span;
   const bool cuts = Op::kRowOut && !g.no_carry;
   if (cuts) {
-    const size_t slots = (size_t)p.nhb * 2 * g.n_tiles;
+    const size_t slots = (size_t)p.nhb * 2 * a.n_tiles;
     a.carry = ar.take(slots * Op::kCarryElems * sizeof(typename Op::A));
     a.rows = (uint32_t*)ar.take(slots * 4);
   }
@@ -197,7 +213,7 @@ inline int launch_walk(Arena& ar, const GraphView& g, const GeoPick& p, const Op
     constexpr int smem = Op::kWarps * Op::kWarpBytes;
     GK_TRY(allow_smem(group_walk_kernel<Op>, smem, configured));
     constexpr int per_block = Op::kWarps * Op::NE;   // one tile per lane group
-    const dim3 grid((unsigned)((g.n_tiles + per_block - 1) / per_block), (unsigned)p.nhb);
+    const dim3 grid((a.n_tiles + per_block - 1) / per_block, (unsigned)p.nhb);
     group_walk_kernel<Op><<<grid, Op::kWarps * 32, smem, st>>>(op, a);
     GK_LAUNCHED(Op::kName);
   }
@@ -206,7 +222,7 @@ inline int launch_walk(Arena& ar, const GraphView& g, const GeoPick& p, const Op
       static std::atomic<bool> configured[64];
       constexpr int threads = kCarryThreads<Op>, smem = threads / Op::G * Op::kCarryElems * (int)sizeof(typename Op::A);
       GK_TRY(allow_smem(carry_rows_kernel<Op>, smem, configured));
-      const dim3 grid((unsigned)((2 * g.n_tiles + threads - 1) / threads), (unsigned)p.nhb);
+      const dim3 grid((2 * a.n_tiles + threads - 1) / threads, (unsigned)p.nhb);
       carry_rows_kernel<Op><<<grid, threads, smem, st>>>(op, a);
       GK_LAUNCHED("carry_rows");
     }
