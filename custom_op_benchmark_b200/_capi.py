@@ -48,7 +48,7 @@ class Plan(ctypes.Structure):
                 ("tile", ctypes.c_int32), ("reserved", ctypes.c_int32)]
 
 
-PLAN_DENSE_BAND, PLAN_ROW_TILES, PLAN_NO_CARRY = 1, 2, 4
+PLAN_DENSE_BAND, PLAN_ROW_TILES, PLAN_NO_CARRY, PLAN_COVERED, PLAN_SKEWED = 1, 2, 4, 8, 16
 _PP = ctypes.POINTER(Plan)
 
 # argument lists of the plan forms (one per element type), in the order of include/graphop_b200.h

@@ -179,6 +179,15 @@ __device__ __forceinline__ void frag_unpack(Frag<typename AccOf<T>::type, SB / (
     for (int i = 0; i < V; ++i) f.p[i] = to_acc<T>(u.t[i]);
   }
 }
+// Loads of gathered rows.  volatile: a slot is refilled where it was last read, not before.
+__device__ __forceinline__ void ldg_word(uint4& v, const void* p) {
+  asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+}
+__device__ __forceinline__ void ldg_word(uint2& v, const void* p) {
+  asm volatile("ld.global.nc.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+}
+__device__ __forceinline__ void ldg_word(uint32_t& v, const void* p) { asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p)); }
+
 // Shared memory by its 32-bit address.  volatile: these loads stay behind the waits for the asynchronous copies.
 __device__ __forceinline__ void lds(uint4& v, unsigned at) {
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(at));

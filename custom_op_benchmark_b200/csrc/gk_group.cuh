@@ -58,6 +58,7 @@ struct WalkArgs {
   unsigned cut_tiles, span;    // tiles the graph was cut into; `span` consecutive ones are one tile of this launch
   unsigned n_tiles;            // tiles of this launch
   void* carry;                 // (head blocks, 2 * n_tiles) partial records; null: no row crosses a tile boundary
+  int only;                    // 0 / 1: nothing is done unless hdr->skewed is that; -1: always
   uint32_t* rows;              // what each record stands for: 2 * node + 1, 2 * node where the slot holds nothing (its tile
                                // lies inside one node that goes on), kNoRow: unused
 };
@@ -73,6 +74,7 @@ struct Geo {
   using A = typename AccOf<T>::type;
   static constexpr int SB = SB_, G = G_, W = W_, LT = LT_, V = SB / (int)sizeof(T), NE = 32 / G;
   using F = Frag<A, V>;
+  using Word = typename SlotWord<SB>::type;
   static constexpr int kAccs = W * V * G;   // accumulators of one row of a head block
   static constexpr int kRow = W * 32 * SB;  // ring bytes of one operand row per group
   static constexpr int kHeads = LT > 0 ? G / LT : (G < kMaxBlockHeads ? G : kMaxBlockHeads);   // heads (or pieces) per block at most
@@ -165,6 +167,11 @@ struct Geo {
     for (int i = 0; i < W; ++i)
       cp_async_slot<SB>(dst + i * 32 * SB, p + (size_t)(i * slot_step()) * sizeof(T), live && has(ln, i));
   }
+  // the lane's first slot of a row, as it lies in memory; zeros where it does not exist
+  __device__ __forceinline__ void fetch_slot(const Lane& ln, Word& w, const unsigned char* base, int id, unsigned rowb) const {
+    if (LT == 0 && !has(ln, 0)) w = Word{};
+    else ldg_word(w, base + (unsigned long long)(unsigned)id * rowb);
+  }
   __device__ __forceinline__ void load_staged(F (&f)[W], unsigned src) const {
 #pragma unroll
     for (int i = 0; i < W; ++i) frag_lds<T, SB>(f[i], src + i * 32 * SB);
@@ -229,6 +236,7 @@ struct FeatGeo : Geo<T_, 16, G_, W_, G_> {
 // one edge, is fetched when its turn comes), where a room per step would leave too few warps.  kScalar bytes per edge and head wait in a table; kState fragments of W slots live in a lane's registers.
 template <class GEO, int kRows, int kScalar, int kState, int kNode, int kNodeScalar, int kU, bool kShare = false>
 struct Shape {
+  static constexpr bool kSums = false;
   static constexpr int kWarps = 1;
   static constexpr int kStepBytes = kRows * GEO::kRow;
   static constexpr int kNodeScalarAt = kNode * GEO::kRow;                  // from the node's room
@@ -265,6 +273,37 @@ struct Shape {
 //   began(st, node, mine)                         the part of begin that needs the whole warp
 //   store_row(st, node), zero_row(st, node)
 //   begin_merge(st), merge(st, Carry), load_carry, save_carry, kCarryElems
+// Two walkers are launched where the better one is known on the device alone: one of them has nothing to do.
+__device__ __forceinline__ bool not_asked(const WalkArgs& a) { return a.only >= 0 && a.hdr->skewed != a.only; }
+
+// The positions of tile t of a launch, for the lane group that walks it (called by the whole warp; here: the tile exists).  A
+// nominal boundary moves up to the first row start within the following `tile` positions, so that only rows longer than a
+// tile are ever cut (in a plan's boundaries that is done; else every group looks for its own).
+template <int G>
+__device__ __forceinline__ void tile_of(const WalkArgs& a, unsigned t, bool here, int& begin, int& n) {
+  const int lane = threadIdx.x & 31, g = lane / G, gl = lane & (G - 1);
+  const unsigned cut0 = here ? t * a.span : 0u, cut1 = here ? min(cut0 + a.span, a.cut_tiles) : 0u;
+  begin = __ldg(a.tile_start + cut0);
+  int end = __ldg(a.tile_start + cut1);
+  if (!a.aligned) {
+    const int E = (int)a.E;
+    const auto move_up = [&](int x) {
+      int found = x <= 0 ? 0 : x >= E ? E : -1;
+      for (int s = 0; s < a.tile; s += G) {
+        if (__all_sync(kFull, found >= 0)) break;
+        const bool in = found < 0 && s + gl < a.tile && s + gl < E - x;
+        const bool starts = in && __ldg(a.erow + x + s + gl) != __ldg(a.erow + x + s + gl - 1);
+        const unsigned m = (__ballot_sync(kFull, starts) >> (g * G)) & (kFull >> (32 - G));
+        if (found < 0 && m) found = x + s + __ffs(m) - 1;
+      }
+      return found >= 0 ? found : x;
+    };
+    begin = move_up(begin);
+    end = move_up(end);
+  }
+  n = here ? end - begin : 0;
+}
+
 template <class Op>
 __global__ void __launch_bounds__(Op::kWarps * 32, Op::kMinCtas)
 group_walk_kernel(const __grid_constant__ Op op, const __grid_constant__ WalkArgs a) {
@@ -277,30 +316,12 @@ group_walk_kernel(const __grid_constant__ Op op, const __grid_constant__ WalkArg
   const int g = lane / G, gl = lane & (G - 1);
   const int hb = blockIdx.y;
   const unsigned t0 = (blockIdx.x * Op::kWarps + w) * NE;   // the warp's first tile
-  if (t0 >= a.n_tiles) return;
+  if (t0 >= a.n_tiles || not_asked(a)) return;
   const unsigned t = t0 + g;
   const bool here = t < a.n_tiles;
-  // A nominal boundary moves up to the first row start within the following `tile` positions, so that only rows longer
-  // than a tile are ever cut (in a plan's boundaries that is done; else every group looks for its own).
-  const unsigned cut0 = here ? t * a.span : 0u, cut1 = here ? min(cut0 + a.span, a.cut_tiles) : 0u;
-  long long j0 = __ldg(a.tile_start + cut0), j1 = __ldg(a.tile_start + cut1);
-  if (!a.aligned) {
-    auto move_up = [&](long long x) {
-      long long found = x <= 0 ? 0 : x >= a.E ? a.E : -1;
-      for (int s = 0; s < a.tile; s += G) {
-        if (__all_sync(kFull, found >= 0)) break;
-        const long long q = x + s + gl;
-        const bool in = found < 0 && s + gl < a.tile && q < a.E;
-        const bool starts = in && __ldg(a.erow + q) != __ldg(a.erow + q - 1);
-        const unsigned m = (__ballot_sync(kFull, starts) >> (g * G)) & (kFull >> (32 - G));
-        if (found < 0 && m) found = x + s + __ffs(m) - 1;
-      }
-      return found >= 0 ? found : x;
-    };
-    j0 = move_up(j0);
-    j1 = move_up(j1);
-  }
-  const int n = here ? (int)(j1 - j0) : 0;
+  int begin, n;   // the group's first position and their number
+  tile_of<G>(a, t, here, begin, n);
+  const long long j0 = begin, j1 = j0 + n;
   int longest = n;
 #pragma unroll
   for (int o = G; o < 32; o <<= 1) {
@@ -532,6 +553,7 @@ carry_rows_kernel(const __grid_constant__ Op op, const __grid_constant__ WalkArg
   A* part = reinterpret_cast<A*>(gk_ring);   // UNITS records
   __shared__ unsigned s_start[THREADS / 2], s_long[THREADS / 2];
   __shared__ int s_n, s_nlong, s_end;
+  if (not_asked(a)) return;
   const int tid = threadIdx.x, u = tid / G, gl = tid & (G - 1), hb = blockIdx.y;
   const uint32_t* ids = a.rows + (size_t)hb * 2 * a.n_tiles;
   const A* rec = reinterpret_cast<const A*>(a.carry) + (size_t)hb * 2 * a.n_tiles * CE;

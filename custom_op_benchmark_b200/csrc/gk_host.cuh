@@ -109,9 +109,10 @@ inline int pick_tile(long long n_edges) {
 // (attention step, 4 heads x 32 fp32: R-MAT 15 with tiles of 256 / 128 / 64 / 32 355 / 274 / 265 / 256 us, R-MAT 18
 // 1480 / 1437 / 1462 / 1545 us, R-MAT 21 12.97 / 12.95 / 13.00 / 14.06 ms).
 constexpr long long kTilesWanted = 49152;
+constexpr int kSmallestTile = 32;
 inline int tile_cost(long long E, long long n_nodes) {
   const long long total = E + kRowCost * n_nodes;
-  int t = 32;
+  int t = kSmallestTile;
   while (t < 256 && total / t > kTilesWanted) t <<= 1;
   return t;
 }
@@ -120,7 +121,7 @@ inline long long tile_count(long long E, long long n_nodes, int tile) { return (
 inline long long tile_bound(long long E, long long n_nodes) {
   const int t = tile_cost(E, n_nodes);
   const long long n = tile_count(E, n_nodes, t);
-  return t > 32 && n < kTilesWanted + 2 ? kTilesWanted + 2 : n;
+  return t > kSmallestTile && n < kTilesWanted + 2 ? kTilesWanted + 2 : n;
 }
 
 struct Levels {
@@ -164,6 +165,7 @@ struct GraphView {
   long long n_tiles = 0;
   int tile = 0;
   bool aligned = false, no_carry = false;
+  int skewed = -1;   // few rows are gathered by many positions: 0 / 1, a plan's finding; -1: hdr->skewed has it once asked for
 };
 
 // an edge output that starts from zero when some position belongs to no chunk
@@ -246,6 +248,7 @@ struct FromPlan {
     g->n_tiles = p->tile ? tile_count(p->n_edges, p->n_nodes, p->tile) : 0;
     g->aligned = (p->flags & GRAPHOP_PLAN_ROW_TILES) != 0;
     g->no_carry = (p->flags & GRAPHOP_PLAN_NO_CARRY) != 0;
+    g->skewed = (p->flags & GRAPHOP_PLAN_SKEWED) != 0;
     const long long words = (long long)(clear.bytes / 2);
     if (words && !(p->flags & GRAPHOP_PLAN_COVERED)) {
       zero_uncovered_kernel<uint16_t><<<(unsigned)((words + 1023) / 1024 < 2048 ? (words + 1023) / 1024 : 2048), 256, 0, st>>>(
@@ -331,11 +334,33 @@ inline int dispatch_feat(int H, int ds, F&& f) {
   return heads(std::integral_constant<int, 32>{});
 }
 
+// Which sums of gathered rows go to the summing walker (gk_sum.cuh has what either side of the lines measures): elements of 4
+// and 8 bytes; tables that fit the L2; larger ones, up to kSumTableBytes each, where few of their rows are gathered by many
+// edges.  f(sums, only, most) launches the summing or the gathering walker: where the graph's skew is known to the device alone
+// both are, and the one that it does not ask for returns at once (a few microseconds beside kernels that take hundreds).
+template <typename T> constexpr bool kSumsByRegister = sizeof(T) >= 4;
+constexpr long long kSumTableBytes = 3ll << 29;
+template <class F>
+inline int choose_walker(Arena& ar, const GraphView& g, int tables, long long table, cudaStream_t st, F&& f) {
+  if (tables * table <= kL2Table) return f(true, -1, 0);
+  if (table > kSumTableBytes) return f(false, -1, tiles_near(table));
+  if (g.skewed >= 0) return g.skewed ? f(true, -1, 0) : f(false, -1, tiles_near(table));
+  if (ar.base && !ar.overflow) {
+    skew_kernel<1024><<<1, 1024, 0, st>>>(g.other, g.E, const_cast<PlanHeader*>(g.hdr));
+    GK_LAUNCHED("skew");
+  }
+  const size_t mark = ar.used;
+  GK_TRY(f(true, 1, 0));
+  ar.used = mark;   // one of the two does the work: the same scratch
+  return f(false, 0, tiles_near(table));
+}
+
 // out[node] = sum_k w[eid[k]] * feat(k)
 template <typename T, bool kEdgeFeat>
-inline int run_aggregate(Arena& ar, const GraphView& g, const T* w, const T* x, T* y, long long n_rows, int H, int D,
-                         cudaStream_t st) {
+inline int run_aggregate(Arena& ar, const GraphView& g, const T* w, const T* x, T* y, long long n_rows, long long n_gathered,
+                         int H, int D, cudaStream_t st) {
   using A = typename AccOf<T>::type;
+  const long long table = n_gathered * H * D * (long long)sizeof(T);   // 0: the edges' own rows
   if constexpr (kEdgeFeat) {
     if (const int ds = feat_slots<T>(H, D, {x, y}))
       return dispatch_feat<T>(H, ds, [&](auto heads, auto slots) -> int {
@@ -344,7 +369,27 @@ inline int run_aggregate(Arena& ar, const GraphView& g, const T* w, const T* x, 
         GroupFeatAggregate<FeatGeo<T, decltype(slots)::value, decltype(heads)::value>> op;
         fill_geo(op, p, H, D);
         op.w = w; op.x = x; op.y = y;
-        return launch_walk(ar, g, p, op, n_rows, st);
+        return launch_walk(ar, g, p, op, n_rows, tiles_near(table), st);
+      });
+  }
+  if constexpr (!kEdgeFeat && kSumsByRegister<T>) {
+    const GeoPick p = pick_sum_geo(H, D, sizeof(T), slot_align_of({x, y})), ring = pick_geo(H, D, sizeof(T), slot_align_of({x, y}), true);
+    if (p.SB && p.nhb <= kMaxHeadBlocks)
+      return choose_walker(ar, g, 1, table, st, [&](bool sums, int only, int most) -> int {
+        if (sums)
+          return dispatch_sum_geo<T, true>(p, [&](auto tag) -> int {
+            SumAggregate<typename decltype(tag)::type> op;
+            fill_geo(op, p, H, D);
+            op.w = w; op.x = x; op.y = y;
+            op.wide_scalars = wide_scalars(p, w, H, sizeof(T));
+            return launch_walk(ar, g, p, op, n_rows, most, st, only);
+          });
+        return dispatch_geo<T, true, false>(ring, [&](auto tag) -> int {
+          GroupAggregate<typename decltype(tag)::type, false> op;
+          fill_geo(op, ring, H, D);
+          op.w = w; op.x = x; op.y = y;
+          return launch_walk(ar, g, ring, op, n_rows, most, st, only);
+        });
       });
   }
   const GeoPick p = pick_geo(H, D, sizeof(T), slot_align_of({x, y}), true);
@@ -353,7 +398,7 @@ inline int run_aggregate(Arena& ar, const GraphView& g, const T* w, const T* x, 
       GroupAggregate<typename decltype(tag)::type, kEdgeFeat> op;
       fill_geo(op, p, H, D);
       op.w = w; op.x = x; op.y = y;
-      return launch_walk(ar, g, p, op, n_rows, st);
+      return launch_walk(ar, g, p, op, n_rows, tiles_near(table), st);
     });
   // 2-byte elements with an odd D: one element per slot, feature blocks of 256
   const int HD = H * D, tile0 = pick_tile(g.E);
@@ -373,7 +418,8 @@ inline int run_aggregate(Arena& ar, const GraphView& g, const T* w, const T* x, 
 
 // y[eid[k], h] = a[node(k), h, :] . feat(k)[h, :]
 template <typename T, bool kEdgeFeat>
-inline int run_edge_dot(Arena& ar, const GraphView& g, const T* a, const T* b, T* y, int H, int D, cudaStream_t st) {
+inline int run_edge_dot(Arena& ar, const GraphView& g, const T* a, const T* b, T* y, long long n_gathered, int H, int D,
+                        cudaStream_t st) {
   if constexpr (kEdgeFeat) {
     const size_t row = (size_t)H * sizeof(T);
     const int ds = (uintptr_t)y % (row < 16 ? row : 16) == 0 ? feat_slots<T>(H, D, {a, b}) : 0;
@@ -394,7 +440,7 @@ inline int run_edge_dot(Arena& ar, const GraphView& g, const T* a, const T* b, T
       GroupEdgeDot<typename decltype(tag)::type, kEdgeFeat> op;
       fill_geo(op, p, H, D);
       op.a = a; op.b = b; op.y = y;
-      return launch_walk(ar, g, p, op, 0, st);
+      return launch_walk(ar, g, p, op, 0, tiles_near(n_gathered * H * D * (long long)sizeof(T)), st);
     });
   const int tile0 = pick_tile(g.E);
   EdgeDotAnyOp<T, kEdgeFeat> op;
@@ -512,7 +558,7 @@ inline int maskedmm_forward(const GS& gs, const T* A_, const T* B_, T* y, long l
   Arena ar(ws, wsb);
   GraphView g;
   GK_TRY(gs(ar, n_dst, st, &g, Clear{y, (size_t)E * H * sizeof(T)}));
-  return run_edge_dot<T, false>(ar, g, A_, B_, y, H, D, st);
+  return run_edge_dot<T, false>(ar, g, A_, B_, y, n_src, H, D, st);
 }
 
 template <typename T, class GS>
@@ -533,12 +579,12 @@ inline int maskedmm_backward(const GS& gs_r, const GS& gs_c, long long Cr, long 
   {
     GraphView g;
     GK_TRY(gs_r(ar, n_dst, st, &g));
-    GK_TRY((run_aggregate<T, false>(ar, g, dy, B_, dA, n_dst, H, D, st)));
+    GK_TRY((run_aggregate<T, false>(ar, g, dy, B_, dA, n_dst, n_src, H, D, st)));
   }
   ar.used = 0;  // the second pass runs after the first on the same stream: reuse the scratch
   GraphView g;
   GK_TRY(gs_c(ar, n_src, st, &g));
-  return run_aggregate<T, false>(ar, g, dy, A_, dB, n_src, H, D, st);
+  return run_aggregate<T, false>(ar, g, dy, A_, dB, n_src, n_dst, H, D, st);
 }
 
 template <typename T, class GS>
@@ -551,7 +597,7 @@ inline int node_mul_edge_forward(const GS& gs, const T* A_, const T* B_, T* y, l
   Arena ar(ws, wsb);
   GraphView g;
   GK_TRY(gs(ar, n_dst, st, &g, Clear{y, (size_t)E * H * sizeof(T)}));
-  return run_edge_dot<T, true>(ar, g, A_, B_, y, H, D, st);
+  return run_edge_dot<T, true>(ar, g, A_, B_, y, 0, H, D, st);
 }
 
 template <typename T, class GS>
@@ -567,7 +613,7 @@ inline int node_mul_edge_backward(const GS& gs, const T* A_, const T* B_, const 
   Arena ar(ws, wsb);
   GraphView g;
   GK_TRY(gs(ar, n_dst, st, &g, Clear{dB, (size_t)E * D * sizeof(T)}));
-  GK_TRY((run_aggregate<T, true>(ar, g, dy, B_, dA, n_dst, H, D, st)));
+  GK_TRY((run_aggregate<T, true>(ar, g, dy, B_, dA, n_dst, 0, H, D, st)));
   if (!ar.base) return GRAPHOP_OK;
   return run_edge_mix<T, false>(g, dy, nullptr, 0, A_, dB, H, D, st);
 }
@@ -599,7 +645,7 @@ inline int spmm_forward(const GS& gs, const T* edata, const T* x, T* y, long lon
   Arena ar(ws, wsb);
   GraphView g;
   GK_TRY(gs(ar, n_dst, st, &g));
-  return run_aggregate<T, false>(ar, g, edata, x, y, n_dst, H, D, st);
+  return run_aggregate<T, false>(ar, g, edata, x, y, n_dst, n_src, H, D, st);
 }
 
 template <typename T, class GS>
@@ -618,12 +664,12 @@ inline int spmm_backward(const GS& gs_r, const GS& gs_c, long long C, long long 
   {
     GraphView g;
     GK_TRY(gs_r(ar, n_dst, st, &g, Clear{dedata, (size_t)E * H * sizeof(T)}));
-    if (ar.base) GK_TRY((run_edge_dot<T, false>(ar, g, dy, x, dedata, H, D, st)));
+    if (ar.base) GK_TRY((run_edge_dot<T, false>(ar, g, dy, x, dedata, n_src, H, D, st)));
   }
   ar.used = 0;
   GraphView g;
   GK_TRY(gs_c(ar, n_src, st, &g));
-  return run_aggregate<T, false>(ar, g, edata, dy, dx, n_src, H, D, st);
+  return run_aggregate<T, false>(ar, g, edata, dy, dx, n_src, n_dst, H, D, st);
 }
 
 template <typename A>
@@ -646,39 +692,65 @@ inline bool attention_shape_ok(int H, int D, bool al, GeoPick* p) {
 
 template <typename T, bool kBias>
 inline int run_attn_forward(Arena& ar, const GraphView& g, const GeoPick& s, const T* q, const T* k, const T* v,
-                            const T* rel, double scale, T* o, void* lse, long long n_dst, int H, int D,
-                            cudaStream_t st) {
+                            const T* rel, double scale, T* o, void* lse, long long n_dst, long long n_src, int H,
+                            int D, cudaStream_t st) {
   return dispatch_geo<T, false, true>(s, [&](auto tag) -> int {
     GroupAttnFwd<typename decltype(tag)::type, kBias> op;
     using A = typename decltype(op)::A;
     fill_geo(op, s, H, D);
     op.q = q; op.k = k; op.v = v; op.rel = rel; op.o = o; op.lse = (A*)lse; op.scale = (A)scale;
-    return launch_walk(ar, g, s, op, n_dst, st);
+    return launch_walk(ar, g, s, op, n_dst, tiles_near(2 * n_src * H * D * (long long)sizeof(T)), st);
   });
 }
 template <typename T, bool kBias, class A>
 inline int run_attn_bwd_dst(Arena& ar, const GraphView& g, const GeoPick& s, const T* q, const T* k, const T* v,
                             const T* rel, const T* o, const T* dout, const void* lse, StatPair<A>* stat,
-                            EdgePair<A>* pd, double scale, T* dq, long long n_dst, int H, int D, cudaStream_t st) {
+                            EdgePair<A>* pd, double scale, T* dq, long long n_dst, long long n_src, int H, int D,
+                            cudaStream_t st) {
   return dispatch_geo<T, false, true>(s, [&](auto tag) -> int {
     GroupAttnBwdDst<typename decltype(tag)::type, kBias> op;
     fill_geo(op, s, H, D);
     op.q = q; op.k = k; op.v = v; op.rel = rel; op.o = o; op.dout = dout; op.lse = (const A*)lse; op.stat = stat;
     op.pd = pd; op.dq = dq; op.scale = (A)scale; op.Hp = stat_heads(H, (int)sizeof(A));
-    return launch_walk(ar, g, s, op, n_dst, st);
+    return launch_walk(ar, g, s, op, n_dst, tiles_near(2 * n_src * H * D * (long long)sizeof(T)), st);
   });
 }
 template <typename T, bool kPairs, class A>
 inline int run_attn_bwd_src(Arena& ar, const GraphView& g, const GeoPick& s, const T* q, const T* k, const T* v,
                             const T* dout, const StatPair<A>* stat, const EdgePair<A>* pd, double scale, T* dk, T* dv,
-                            long long n_src, int H, int D, cudaStream_t st) {
+                            long long n_src, int H, int D, cudaStream_t st, int most, int only = -1) {
   return dispatch_geo<T, false, true>(s, [&](auto tag) -> int {
     GroupAttnBwdSrc<typename decltype(tag)::type, kPairs> op;
     fill_geo(op, s, H, D);
     op.q = q; op.k = k; op.v = v; op.dout = dout; op.stat = stat; op.pd = pd; op.dk = dk; op.dv = dv;
     op.scale = (A)scale; op.Hp = stat_heads(H, (int)sizeof(A));
-    return launch_walk(ar, g, s, op, n_src, st);
+    return launch_walk(ar, g, s, op, n_src, most, st, only);
   });
+}
+
+// from the pairs that the destination side left
+template <typename T, class A>
+inline int run_attn_bwd_pairs(Arena& ar, const GraphView& g, const GeoPick& s, const T* q, const T* k, const T* v,
+                              const T* dout, const StatPair<A>* stat, const EdgePair<A>* pd, double scale, T* dk, T* dv,
+                              long long n_dst, long long n_src, int H, int D, cudaStream_t st) {
+  if constexpr (kSumsByRegister<T>) {
+    const long long table = n_dst * H * D * (long long)sizeof(T);
+    return choose_walker(ar, g, 2, table, st, [&](bool sums, int only, int most) -> int {
+      if (!sums) return run_attn_bwd_src<T, true>(ar, g, s, q, k, v, dout, stat, pd, scale, dk, dv, n_src, H, D, st, most, only);
+      const GeoPick p = pick_sum_geo(H, D, sizeof(T), 16);
+      return dispatch_sum_geo<T, false>(p, [&](auto tag) -> int {
+        SumAttnPairs<typename decltype(tag)::type> op;
+        fill_geo(op, p, H, D);
+        op.q = q; op.dout = dout; op.pd = pd; op.dk = dk; op.dv = dv;
+        op.Hp = stat_heads(H, (int)sizeof(A));
+        op.wide_scalars = wide_scalars(p, pd, op.Hp, 2 * (int)sizeof(A));
+        return launch_walk(ar, g, p, op, n_src, most, st, only);
+      });
+    });
+  } else {
+    return run_attn_bwd_src<T, true>(ar, g, s, q, k, v, dout, stat, pd, scale, dk, dv, n_src, H, D, st,
+                                     tiles_near(2 * n_dst * H * D * (long long)sizeof(T)));
+  }
 }
 
 template <typename T, class GS>
@@ -707,7 +779,7 @@ inline int attention_forward(const GS& gs, long long C, const T* q, const T* k, 
   }
   if (!gs.valid(true)) return GRAPHOP_ERR_INVALID_ARGUMENT;
   GK_TRY(gs(ar, n_dst, st, &g));
-  return run_attn_forward<T, false>(ar, g, s, q, k, v, (const T*)nullptr, scale, o, lse, n_dst, H, D, st);
+  return run_attn_forward<T, false>(ar, g, s, q, k, v, (const T*)nullptr, scale, o, lse, n_dst, n_src, H, D, st);
 }
 
 // Defined in gk_banded.cuh for bfloat16: the tensor-core kernel for dense-band graphs.  Returns
@@ -779,13 +851,14 @@ inline int attention_backward(const GS& gs_r, const GS& gs_c, bool has_eid_t, lo
     GraphView g;
     GK_TRY(gs_r(ar, n_dst, st, &g));
     GK_TRY((run_attn_bwd_dst<T, false>(ar, g, s, q, k, v, (const T*)nullptr, o, dout, lse, stat, pd, scale, dq, n_dst,
-                                       H, D, st)));
+                                       n_src, H, D, st)));
   }
   ar.used = mark;
   GraphView g;
   GK_TRY(gs_c(ar, n_src, st, &g));
-  if (pd) return run_attn_bwd_src<T, true>(ar, g, s, q, k, v, dout, stat, pd, scale, dk, dv, n_src, H, D, st);
-  return run_attn_bwd_src<T, false>(ar, g, s, q, k, v, dout, stat, pd, scale, dk, dv, n_src, H, D, st);
+  if (pd) return run_attn_bwd_pairs<T>(ar, g, s, q, k, v, dout, stat, pd, scale, dk, dv, n_dst, n_src, H, D, st);
+  return run_attn_bwd_src<T, false>(ar, g, s, q, k, v, dout, stat, pd, scale, dk, dv, n_src, H, D, st,
+                                    tiles_near(2 * n_dst * H * D * (long long)sizeof(T)));
 }
 
 // ---------------------------------------------------------------------------------------
@@ -810,7 +883,7 @@ inline int attention_bias_forward(const GS& gs, long long C, const T* q, const T
   Arena ar(ws, wsb);
   GraphView g;
   GK_TRY(gs(ar, n_dst, st, &g));
-  return run_attn_forward<T, true>(ar, g, s, q, k, v, rel, scale, o, lse, n_dst, H, D, st);
+  return run_attn_forward<T, true>(ar, g, s, q, k, v, rel, scale, o, lse, n_dst, n_src, H, D, st);
 }
 
 // Gradients of the above.  The transposed CSR must carry eid_t (for each of its positions the row-CSR position of
@@ -844,13 +917,14 @@ inline int attention_bias_backward(const GS& gs_r, const GS& gs_c, bool has_eid_
   {
     GraphView g;
     GK_TRY(gs_r(ar, n_dst, st, &g));
-    GK_TRY((run_attn_bwd_dst<T, true>(ar, g, s, q, k, v, rel, o, dout, lse, stat, pd, scale, dq, n_dst, H, D, st)));
+    GK_TRY((run_attn_bwd_dst<T, true>(ar, g, s, q, k, v, rel, o, dout, lse, stat, pd, scale, dq, n_dst, n_src, H,
+                                      D, st)));
     GK_TRY((run_edge_mix<T, true>(g, nullptr, pd, Hp, q, d_rel, H, D, st)));
   }
   ar.used = mark;
   GraphView g;
   GK_TRY(gs_c(ar, n_src, st, &g));
-  return run_attn_bwd_src<T, true>(ar, g, s, q, k, v, dout, stat, pd, scale, dk, dv, n_src, H, D, st);
+  return run_attn_bwd_pairs<T>(ar, g, s, q, k, v, dout, stat, pd, scale, dk, dv, n_dst, n_src, H, D, st);
 }
 
 template <typename T>

@@ -1,6 +1,7 @@
 // Launching the gathering walker (gk_group.cuh): which geometry a row shape gets, the carry records, the launch.
 #pragma once
 #include "gk_group.cuh"
+#include "gk_sum.cuh"
 
 namespace gk {
 
@@ -22,7 +23,7 @@ struct GeoPick {
 // 512 / 256 / 128 bytes 3.5 / 3.7 / 5.3 ms): every block walks the nodes again.  Four slots per lane touch 32 bytes of
 // four heads per copy instruction: 6.3 ms.  2-byte elements have twice the accumulators per slot: one slot per lane and
 // blocks of 16 slots (16 lanes x 2 slots spilled and ran half as fast).
-inline GeoPick pick_geo(int H, int D, int elem, int slot_align, bool split) {
+inline GeoPick pick_geo(int H, int D, int elem, int slot_align, bool split, bool one_slot = false) {
   GeoPick g;
   const int target = elem == 2 ? 16 : 32;
   const long long db = (long long)D * elem;
@@ -32,7 +33,7 @@ inline GeoPick pick_geo(int H, int D, int elem, int slot_align, bool split) {
   int ds = (int)(db / sb);   // slots per head
   const auto pow2 = [](int v) { int p = 1; while (p < v) p <<= 1; return p; };
   bool exact = (ds & (ds - 1)) == 0;
-  const bool two_byte = elem == 2;
+  const bool two_byte = elem == 2 || one_slot;
   if (split && ds > target) {
     g.parts = (ds + target - 1) / target;
     exact = exact && ds % target == 0;
@@ -65,6 +66,16 @@ inline int slot_align_of(std::initializer_list<const void*> ptrs) {
   uintptr_t bits = 16;
   for (const void* p : ptrs) bits |= (uintptr_t)p;
   return (bits & 3) ? 1 : (bits & 7) ? 4 : (bits & 15) ? 8 : 16;
+}
+
+// The summing walker's: one slot per lane, and no head is too wide, it is walked piece by piece.  With rows of 512 bytes as
+// 16 lanes x 2 slots a load instruction touches 64 bytes of every head: 15360 nodes of 30 edges, 8 x 64 fp32, 61 us for a
+// table's rows alone against 44.
+inline GeoPick pick_sum_geo(int H, int D, int elem, int slot_align) { return pick_geo(H, D, elem, slot_align, true, true); }
+
+// Whether an edge's scalars (per_edge of them, elem bytes each) are whole 16-byte pieces for every block of heads
+inline bool wide_scalars(const GeoPick& p, const void* base, int per_edge, int elem) {
+  return p.LT > 0 && p.parts == 1 && ((uintptr_t)base & 15) == 0 && (long long)per_edge * elem % 16 == 0;
 }
 
 constexpr int kMaxHeadBlocks = 65535;   // grid.y
@@ -143,6 +154,41 @@ inline int dispatch_geo(const GeoPick& p, F&& f) {
 #undef GK_GEO
   return GRAPHOP_ERR_UNSUPPORTED;
 }
+// The same for the summing walker.
+template <typename T, bool kNarrowSlots, class F>
+inline int dispatch_sum_geo(const GeoPick& p, F&& f) {
+#define GK_GEO(SB_, G_, LT_) \
+  if (p.SB == SB_ && p.G == G_ && p.W == 1 && (LT_ == 0 || p.LT == LT_)) return f(TypeTag<Geo<T, SB_, G_, 1, LT_>>{});
+  if constexpr (sizeof(T) == 4) {
+    GK_GEO(16, 32, 4)
+    GK_GEO(16, 32, 8)
+    GK_GEO(16, 32, 16)
+    GK_GEO(16, 32, 32)
+    GK_GEO(16, 16, 4)
+    GK_GEO(16, 16, 8)
+    GK_GEO(16, 16, 16)
+    GK_GEO(16, 8, 4)
+    GK_GEO(16, 8, 8)
+  }
+  GK_GEO(16, 32, 0)
+  GK_GEO(16, 16, 0)
+  GK_GEO(16, 8, 0)
+  GK_GEO(16, 4, 0)
+  if constexpr (kNarrowSlots) {
+    GK_GEO(8, 32, 0)
+    GK_GEO(8, 16, 0)
+    GK_GEO(8, 8, 0)
+    GK_GEO(8, 4, 0)
+    if constexpr (sizeof(T) == 4) {
+      GK_GEO(4, 32, 0)
+      GK_GEO(4, 16, 0)
+      GK_GEO(4, 8, 0)
+      GK_GEO(4, 4, 0)
+    }
+  }
+#undef GK_GEO
+  return GRAPHOP_ERR_UNSUPPORTED;
+}
 // the narrow-slot set has no 32 x 4: such rows take 32 x 8
 inline GeoPick narrow_fix(GeoPick p) {
   if (p.SB && p.SB < 16 && p.G == 32 && p.W == 4) p.W = 8;
@@ -183,22 +229,42 @@ inline int allow_smem(Kernel kernel, int bytes, std::atomic<bool> (&configured)[
 // - / 811 us; R-MAT 18 with an edge term, 4 x 64 bf16, 2.79 / 2.58 / 2.59 / 2.79 ms; R-MAT 20, 4 x 32, multiply and aggregate
 // 5.84 / - / 5.70 / 5.84; R-MAT 22, 1 x 128, aggregate 13.5 / - / 12.7 / 12.5; with 4 K the chip is not filled evenly (R-MAT
 // 18: 3.0 ms).
+//
+// The summing walker's warps run in step on a small graph, and its resident warps (`slots`) are what a round of them is: one
+// round, or two where that would make long ones, beat any other number.  Its kernels by rounds: 4096 nodes of 16 edges, 8 x 64
+// fp32, 2.9 / 0.96 rounds 25 / 21 us; 150 thousand edges, 3 x 20, 1.7 / 0.9 17 / 14 us; 15360 nodes of 30 edges, 8 x 64,
+// 15.8 / 5.3 / 3.2 / 2.0 / 1.2 / 0.75 82 / 81 / 78 / 66 / 84 / 72 us.  Larger graphs get tiles of more than kSmallestTile.
+//
+// The nodes of neighbouring tiles often gather the same rows (blocks, bands).  Where the tables do not fit the L2 as they are
+// and the graph is not known to be skewed, the warps at work had better lie close together: `most` (0: any number) is two.  331
+// thousand nodes in blocks of 47, 4 x 64 fp32, backward: 2.36 + 1.95 ms with a tile each, 2.83 + 2.37 with three; a row of 7M
+// edges on 1M nodes, 2 x 64: its records take 326 us to merge with a tile each, 168 with two.
 constexpr long long kWarpsWanted = 20480;
-inline unsigned tile_span(long long n_tiles, int nhb, int per_warp) {
-  const long long warps = n_tiles * nhb / per_warp;
-  const long long span = (warps + kWarpsWanted / 2) / kWarpsWanted;
+constexpr long long kL2Table = 64ll << 20;
+inline int tiles_near(long long table) { return table > kL2Table ? 2 : 0; }
+inline unsigned tile_span(long long n_tiles, int nhb, int per_warp, int tile, long long slots, int most) {
+  const long long warps = (n_tiles * nhb + per_warp - 1) / per_warp;
+  long long span = (warps + kWarpsWanted / 2) / kWarpsWanted;
+  if (most) {
+    span = span < most ? span : most;
+  } else if (slots && tile == kSmallestTile) {
+    const long long round = warps <= 4 * slots ? slots : 2 * slots;
+    span = (warps + round - 1) / round;
+  }
   return span < 1 ? 1 : span < n_tiles ? (unsigned)span : (unsigned)n_tiles;
 }
 
-// The op over every position and head block, and the merge of the rows that tiles had to cut.
+// The op over every position and head block, and the merge of the rows that tiles had to cut.  most: see tile_span; only: see
+// WalkArgs.
 template <class Op>
-inline int launch_walk(Arena& ar, const GraphView& g, const GeoPick& p, const Op& op, long long n_rows, cudaStream_t st) {
+inline int launch_walk(Arena& ar, const GraphView& g, const GeoPick& p, const Op& op, long long n_rows, int most,
+                       cudaStream_t st, int only = -1) {
   WalkArgs a{};
   a.hdr = g.hdr; a.erow = g.erow; a.other = g.other; a.eid = g.eid;
   a.tile_start = g.tile_start;
-  a.E = g.E; a.n_rows = n_rows; a.tile = g.tile; a.aligned = g.aligned;
+  a.E = g.E; a.n_rows = n_rows; a.tile = g.tile; a.aligned = g.aligned; a.only = only;
   a.cut_tiles = (unsigned)g.n_tiles;
-  a.span = tile_span(g.n_tiles, p.nhb, Op::NE);
+  a.span = tile_span(g.n_tiles, p.nhb, Op::NE, g.tile, Op::kSums ? 148ll * Op::kMinCtas * Op::kWarps : 0, most);
   a.n_tiles = (a.cut_tiles + a.span - 1) / a.span;
   const bool cuts = Op::kRowOut && !g.no_carry;
   if (cuts) {
@@ -211,10 +277,13 @@ inline int launch_walk(Arena& ar, const GraphView& g, const GeoPick& p, const Op
   {
     static std::atomic<bool> configured[64];
     constexpr int smem = Op::kWarps * Op::kWarpBytes;
-    GK_TRY(allow_smem(group_walk_kernel<Op>, smem, configured));
+    void (*kernel)(const Op, const WalkArgs);
+    if constexpr (Op::kSums) kernel = sum_walk_kernel<Op>;
+    else kernel = group_walk_kernel<Op>;
+    GK_TRY(allow_smem(kernel, smem, configured));
     constexpr int per_block = Op::kWarps * Op::NE;   // one tile per lane group
     const dim3 grid((a.n_tiles + per_block - 1) / per_block, (unsigned)p.nhb);
-    group_walk_kernel<Op><<<grid, Op::kWarps * 32, smem, st>>>(op, a);
+    kernel<<<grid, Op::kWarps * 32, smem, st>>>(op, a);
     GK_LAUNCHED(Op::kName);
   }
   if constexpr (Op::kRowOut) {

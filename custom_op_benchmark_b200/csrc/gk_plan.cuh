@@ -113,14 +113,22 @@ __device__ __forceinline__ void align_tiles(const int32_t* __restrict__ erow, lo
   if (crosses) atomicOr(&verdict->row_crosses, 1);
 }
 
-// What follows the expansion: the first `aligning` blocks move the tile boundaries, the others find the nodes' ranges.
+// What follows the expansion: the first block looks for skew, the next `aligning` ones move the tile boundaries, the others
+// find the nodes' ranges.
 template <typename I>
 __global__ void __launch_bounds__(256)
 plan_nodes_kernel(const I* __restrict__ row, const I* __restrict__ indptr, long long C, long long n_nodes,
                   int32_t* __restrict__ first, int32_t* __restrict__ deg, const int32_t* __restrict__ erow, long long E, int tile,
-                  long long n_tiles, int32_t* __restrict__ tile_start, BandVerdict* __restrict__ verdict, unsigned aligning) {
-  if (blockIdx.x < aligning) align_tiles(erow, E, tile, n_tiles, tile_start, verdict, blockIdx.x, aligning);
-  else node_ranges<I>(row, indptr, C, n_nodes, first, deg, blockIdx.x - aligning, gridDim.x - aligning);
+                  long long n_tiles, int32_t* __restrict__ tile_start, BandVerdict* __restrict__ verdict, unsigned aligning,
+                  const int32_t* __restrict__ other, PlanHeader* __restrict__ hdr) {
+  if (blockIdx.x == 0) {
+    const bool skewed = other && skewed_gather<256>(other, E);
+    if (threadIdx.x == 0) hdr->skewed = skewed;
+    return;
+  }
+  const unsigned block = blockIdx.x - 1;
+  if (block < aligning) align_tiles(erow, E, tile, n_tiles, tile_start, verdict, block, aligning);
+  else node_ranges<I>(row, indptr, C, n_nodes, first, deg, block - aligning, gridDim.x - 1 - aligning);
 }
 // The shape analysis, on the nodes' ranges: a block per 128 nodes, the others go over the positions.
 template <int kThreads>
@@ -179,8 +187,9 @@ inline int plan_build(const I* row, const I* indptr, const I* eid, const I* indi
   {
     const unsigned aligning = (unsigned)((g.n_tiles + 256) / 256 < 4096 ? (g.n_tiles + 256) / 256 : 4096);
     const unsigned ranging = n_nodes > 0 && C > 0 ? (unsigned)((C + 255) / 256 < 8192 ? (C + 255) / 256 : 8192) : 0;
-    plan_nodes_kernel<I><<<aligning + ranging, 256, 0, st>>>(row, indptr, C, n_nodes, first, deg, g.erow, E, g.tile, g.n_tiles,
-                                                             const_cast<int32_t*>(g.tile_start), verdict, aligning);
+    plan_nodes_kernel<I><<<1 + aligning + ranging, 256, 0, st>>>(row, indptr, C, n_nodes, first, deg, g.erow, E, g.tile, g.n_tiles,
+                                                             const_cast<int32_t*>(g.tile_start), verdict, aligning, g.other,
+                                                             &facts->cover);
     GK_LAUNCHED("plan_nodes");
   }
   if (g.other && n_nodes > 0) {
@@ -202,6 +211,7 @@ inline int plan_build(const I* row, const I* indptr, const I* eid, const I* indi
   plan->tile_start = g.tile_start;
   plan->flags |= GRAPHOP_PLAN_ROW_TILES;
   if (!host.row_crosses) plan->flags |= GRAPHOP_PLAN_NO_CARRY;
+  if (back.cover.skewed) plan->flags |= GRAPHOP_PLAN_SKEWED;
   if (back.cover.cover_hi - back.cover.cover_lo >= E) plan->flags |= GRAPHOP_PLAN_COVERED;
   return GRAPHOP_OK;
 }

@@ -25,10 +25,11 @@ size_t walk_bytes(long long E, long long n_nodes, int H, int D, int elem, bool s
   const int tile = pick_tile(E);
   size_t most = split ? levels_bytes(E, tile, (size_t)H * D * acc) : 0;
   for (int align = 16; align >= 4; align >>= 1) {
-    const GeoPick p = pick_geo(H, D, elem, align, split);
-    if (!p.SB) continue;
-    const size_t b = carry_bytes(tile_bound(E, n_nodes), p.nhb, (long long)accs * p.accs(elem) + stats * p.G, acc);
-    most = b > most ? b : most;
+    for (const GeoPick& p : {pick_geo(H, D, elem, align, split), pick_sum_geo(H, D, elem, align)}) {
+      if (!p.SB) continue;
+      const size_t b = carry_bytes(tile_bound(E, n_nodes), p.nhb, (long long)accs * p.accs(elem) + stats * p.G, acc);
+      most = b > most ? b : most;
+    }
   }
   return most;
 }

@@ -164,7 +164,8 @@ enum {
   GRAPHOP_PLAN_DENSE_BAND = 1,
   GRAPHOP_PLAN_ROW_TILES = 2, /* tile_start holds the work tiles' boundaries, moved up to row starts, ... */
   GRAPHOP_PLAN_NO_CARRY = 4,  /* ... and no node's positions cross one: row reductions finish in one launch */
-  GRAPHOP_PLAN_COVERED = 8    /* every position belongs to some chunk: no edge output needs clearing first */
+  GRAPHOP_PLAN_COVERED = 8,   /* every position belongs to some chunk: no edge output needs clearing first */
+  GRAPHOP_PLAN_SKEWED = 16    /* few of the gathered rows are gathered by many edges: which kernels suit it */
 };
 #define GRAPHOP_BAND_MAX_SPAN 384
 
