@@ -51,7 +51,7 @@ struct SumShape {
 //   fold(st, rows, tab)                add a position's rows; tab: the table's entry of the position and this lane's head
 //   flush(st)                          a block of positions is done: its sums join those of the node's blocks before it, so that
 //                                      a long run is summed in two levels (in one, a tile's hundreds of edges one after the
-//                                      other, R-MAT 18's dv is 1.16e-7 off float64 instead of 0.83e-7)
+//                                      other, R-MAT 18's dv is 1.16e-7 off float64 instead of 0.83e-7); sum_span bounds the second
 //   store_row(st, node), zero_row(st, node), begin_merge(st), merge(st, Carry), load_carry, save_carry, kCarryElems
 template <class Op>
 __global__ void __launch_bounds__(Op::kWarps * 32, Op::kMinCtas)
