@@ -45,7 +45,7 @@ class Plan(ctypes.Structure):
                 ("header", ctypes.c_void_p), ("erow", ctypes.c_void_p), ("other", ctypes.c_void_p),
                 ("eid", ctypes.c_void_p), ("node_lo", ctypes.c_void_p), ("node_deg", ctypes.c_void_p),
                 ("flags", ctypes.c_int32), ("band_span", ctypes.c_int32), ("tile_start", ctypes.c_void_p),
-                ("tile", ctypes.c_int32), ("reserved", ctypes.c_int32)]
+                ("tile", ctypes.c_int32), ("gather_repeats", ctypes.c_int32)]
 
 
 PLAN_DENSE_BAND, PLAN_ROW_TILES, PLAN_NO_CARRY, PLAN_COVERED, PLAN_SKEWED = 1, 2, 4, 8, 16

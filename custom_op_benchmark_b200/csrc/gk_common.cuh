@@ -24,8 +24,8 @@ constexpr unsigned kFull = 0xffffffffu;
 struct PlanHeader {
   long long cover_lo;  // first CSR position any chunk covers  (= indptr[0])
   long long cover_hi;  // one past the last covered position   (= indptr[C])
-  int skewed;          // few rows are gathered by many edges (skewed_gather); set where an op or a plan asks for it
-  int unused;
+  int skewed;          // few rows are gathered by many edges; set by skew_kernel where an op asks for it
+  int repeats;         // gather_repeats, set where a plan is built
 };
 
 // ---------------------------------------------------------------------------------------
@@ -137,13 +137,14 @@ __device__ __forceinline__ void cut_tiles(const TileCut& cut, long long p, long 
     for (long long t = hi + 1; t <= cut.n; ++t) cut.start[t] = (int32_t)E;
 }
 
-// Whether few of the rows that the positions gather are gathered by many: among kSkewSamples evenly spaced positions more than
-// kSkewRepeats name a row that another one named, as far as a table of kSkewBits bits tells (8 of different rows share one).
-// Uniform sources on 100 thousand nodes repeat 5 times, neighbours that follow the nodes not at all, R-MAT 20 about 50 times
-// and a hub that has a tenth of the edges 100 times.  For one block of THREADS; the answer is every thread's.
-constexpr int kSkewSamples = 1024, kSkewRepeats = 24, kSkewBits = 65536;
+// How many of kSkewSamples evenly spaced positions gather a row that another one of them gathers, as far as a table of kSkewBits
+// bits tells.  Many where few rows are gathered by many edges (R-MAT 20: 37 to 48, R-MAT 16: 141 to 166, a hub that has a tenth of
+// the edges: 100), none where the neighbours follow the nodes, and as many as chance has it where the sources are uniform: 8 of
+// different rows that share a bit, and more of the same row the fewer rows there are (skew_allowed).  For one block of THREADS;
+// the answer is every thread's.
+constexpr int kSkewSamples = 1024, kSkewBits = 65536;
 template <int THREADS>
-__device__ __forceinline__ bool skewed_gather(const int32_t* __restrict__ other, long long E) {
+__device__ __forceinline__ int gather_repeats(const int32_t* __restrict__ other, long long E) {
   __shared__ __align__(16) unsigned s_seen[kSkewBits / 32];
   const int tid = threadIdx.x, n = E < kSkewSamples ? (int)E : kSkewSamples;
   int key[kSkewSamples / THREADS], repeats = 0;   // all asked for before any is looked at
@@ -166,12 +167,12 @@ __device__ __forceinline__ bool skewed_gather(const int32_t* __restrict__ other,
   __syncthreads();
   if ((tid & 31) == 0) atomicAdd(s_seen, (unsigned)repeats);
   __syncthreads();
-  return s_seen[0] > (unsigned)kSkewRepeats;
+  return (int)s_seen[0];
 }
 template <int THREADS>
-__global__ void __launch_bounds__(THREADS) skew_kernel(const int32_t* __restrict__ other, long long E, PlanHeader* __restrict__ hdr) {
-  const bool skewed = skewed_gather<THREADS>(other, E);
-  if (threadIdx.x == 0) hdr->skewed = skewed;
+__global__ void __launch_bounds__(THREADS) skew_kernel(const int32_t* __restrict__ other, long long E, int allowed, PlanHeader* __restrict__ hdr) {
+  const int repeats = gather_repeats<THREADS>(other, E);
+  if (threadIdx.x == 0) hdr->skewed = repeats > allowed;
 }
 
 // What an op wants done on the way: 32-bit copies of up to two 64-bit index arrays (a null source is skipped), and an

@@ -2,6 +2,7 @@
 // launch sequences.  Everything here enqueues on the caller's stream and never synchronises.
 #pragma once
 #include <atomic>
+#include <cmath>
 #include <cstdio>
 #include <initializer_list>
 #include <mutex>
@@ -165,7 +166,7 @@ struct GraphView {
   long long n_tiles = 0;
   int tile = 0;
   bool aligned = false, no_carry = false;
-  int skewed = -1;   // few rows are gathered by many positions: 0 / 1, a plan's finding; -1: hdr->skewed has it once asked for
+  int repeats = -1;   // gather_repeats, a plan's finding; -1: skew_kernel counts them
 };
 
 // an edge output that starts from zero when some position belongs to no chunk
@@ -248,7 +249,7 @@ struct FromPlan {
     g->n_tiles = p->tile ? tile_count(p->n_edges, p->n_nodes, p->tile) : 0;
     g->aligned = (p->flags & GRAPHOP_PLAN_ROW_TILES) != 0;
     g->no_carry = (p->flags & GRAPHOP_PLAN_NO_CARRY) != 0;
-    g->skewed = (p->flags & GRAPHOP_PLAN_SKEWED) != 0;
+    g->repeats = p->gather_repeats;
     const long long words = (long long)(clear.bytes / 2);
     if (words && !(p->flags & GRAPHOP_PLAN_COVERED)) {
       zero_uncovered_kernel<uint16_t><<<(unsigned)((words + 1023) / 1024 < 2048 ? (words + 1023) / 1024 : 2048), 256, 0, st>>>(
@@ -334,19 +335,39 @@ inline int dispatch_feat(int H, int ds, F&& f) {
   return heads(std::integral_constant<int, 32>{});
 }
 
+// The most repeats among the samples (gather_repeats) that chance explains where E positions gather n rows uniformly: their mean
+// and four standard deviations, at least 16 (24 for many rows, 36 for 49 thousand, 88 for 10 thousand; seen on 200 uniform draws
+// each: 16, 23, 69 at most).
+inline int skew_allowed(long long n, long long E) {
+  const double s = E < kSkewSamples ? (double)E : kSkewSamples, bits = kSkewBits, rows = n > 1 ? (double)n : 1;
+  const double distinct = n > 1 ? -rows * std::expm1(s * std::log1p(-1 / rows)) : 1;
+  const double chance = s + bits * std::expm1(distinct * std::log1p(-1 / bits)), spread = 4 * std::sqrt(chance > 0 ? chance : 0);
+  return (int)std::ceil(chance + (spread > 16 ? spread : 16));
+}
+
 // Which sums of gathered rows go to the summing walker (gk_sum.cuh has what either side of the lines measures): elements of 4
-// and 8 bytes; tables that fit the L2; larger ones, up to kSumTableBytes each, where few of their rows are gathered by many
-// edges.  f(sums, only, most) launches the summing or the gathering walker: where the graph's skew is known to the device alone
-// both are, and the one that it does not ask for returns at once (a few microseconds beside kernels that take hundreds).
+// and 8 bytes.  Tables that fit the L2, which for `nhb` blocks of heads, walked one after the other, is up to twice as much if
+// a block's share is not large: 33 thousand nodes of 30 edges, 16 x 64 fp32 (129 MB, blocks of 16), 320 against 405 us; 60
+// thousand of 16, 8 x 64 (117 MB, blocks of 29), 177 to 207 against 202 to 214; 80 thousand (156 MB, blocks of 39) 266 against 248.
+// Any larger one of so few rows that several blocks' shares fit, as long as the walks stay short enough for the blocks to follow
+// one another: 4000 nodes of 30 edges, 128 x 128 (250 MB, blocks of 2), 632 against 726 us, but 926 in walks of any length; 20
+// thousand of 16, 16 x 128 (156 MB, blocks of 10), 234 against 246.  Other larger ones, up to kSumTableBytes each, where few of
+// their rows are gathered by many edges.  f(sums, only, most) launches the summing or the gathering walker: where the graph's skew
+// is known to the device alone both are, and the one that it does not ask for returns at once (14 us a call, with the question:
+// 98 -> 112 us on 1.4M uniform edges, 358 -> 379 on 6M; hubs 284 -> 112 and 541 -> 193).
 template <typename T> constexpr bool kSumsByRegister = sizeof(T) >= 4;
-constexpr long long kSumTableBytes = 3ll << 29;
+constexpr long long kSumTableBytes = 3ll << 29, kSumShare = 32ll << 20, kSumFewRows = 8ll << 20;
 template <class F>
-inline int choose_walker(Arena& ar, const GraphView& g, int tables, long long table, cudaStream_t st, F&& f) {
-  if (tables * table <= kL2Table) return f(true, -1, 0);
+inline int choose_walker(Arena& ar, const GraphView& g, int tables, long long table, int nhb, long long n_gathered, cudaStream_t st,
+                         F&& f) {
+  const long long all = tables * table, share = all / nhb;
+  if (all <= kL2Table || (all <= 2 * kL2Table && share <= kSumShare)) return f(true, -1, 0);
   if (table > kSumTableBytes) return f(false, -1, tiles_near(table));
-  if (g.skewed >= 0) return g.skewed ? f(true, -1, 0) : f(false, -1, tiles_near(table));
+  if (share <= kSumFewRows) return f(true, -1, tiles_near(table));
+  const int allowed = skew_allowed(n_gathered, g.E);
+  if (g.repeats >= 0) return g.repeats > allowed ? f(true, -1, 0) : f(false, -1, tiles_near(table));
   if (ar.base && !ar.overflow) {
-    skew_kernel<1024><<<1, 1024, 0, st>>>(g.other, g.E, const_cast<PlanHeader*>(g.hdr));
+    skew_kernel<1024><<<1, 1024, 0, st>>>(g.other, g.E, allowed, const_cast<PlanHeader*>(g.hdr));
     GK_LAUNCHED("skew");
   }
   const size_t mark = ar.used;
@@ -375,7 +396,7 @@ inline int run_aggregate(Arena& ar, const GraphView& g, const T* w, const T* x, 
   if constexpr (!kEdgeFeat && kSumsByRegister<T>) {
     const GeoPick p = pick_sum_geo(H, D, sizeof(T), slot_align_of({x, y})), ring = pick_geo(H, D, sizeof(T), slot_align_of({x, y}), true);
     if (p.SB && p.nhb <= kMaxHeadBlocks)
-      return choose_walker(ar, g, 1, table, st, [&](bool sums, int only, int most) -> int {
+      return choose_walker(ar, g, 1, table, p.nhb, n_gathered, st, [&](bool sums, int only, int most) -> int {
         if (sums)
           return dispatch_sum_geo<T, true>(p, [&](auto tag) -> int {
             SumAggregate<typename decltype(tag)::type> op;
@@ -735,9 +756,9 @@ inline int run_attn_bwd_pairs(Arena& ar, const GraphView& g, const GeoPick& s, c
                               long long n_dst, long long n_src, int H, int D, cudaStream_t st) {
   if constexpr (kSumsByRegister<T>) {
     const long long table = n_dst * H * D * (long long)sizeof(T);
-    return choose_walker(ar, g, 2, table, st, [&](bool sums, int only, int most) -> int {
+    const GeoPick p = pick_sum_geo(H, D, sizeof(T), 16);
+    return choose_walker(ar, g, 2, table, p.nhb, n_dst, st, [&](bool sums, int only, int most) -> int {
       if (!sums) return run_attn_bwd_src<T, true>(ar, g, s, q, k, v, dout, stat, pd, scale, dk, dv, n_src, H, D, st, most, only);
-      const GeoPick p = pick_sum_geo(H, D, sizeof(T), 16);
       return dispatch_sum_geo<T, false>(p, [&](auto tag) -> int {
         SumAttnPairs<typename decltype(tag)::type> op;
         fill_geo(op, p, H, D);

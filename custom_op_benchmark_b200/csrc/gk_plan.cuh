@@ -113,7 +113,7 @@ __device__ __forceinline__ void align_tiles(const int32_t* __restrict__ erow, lo
   if (crosses) atomicOr(&verdict->row_crosses, 1);
 }
 
-// What follows the expansion: the first block looks for skew, the next `aligning` ones move the tile boundaries, the others
+// What follows the expansion: the first block looks for rows gathered repeatedly, the next `aligning` ones move the tile boundaries, the others
 // find the nodes' ranges.
 template <typename I>
 __global__ void __launch_bounds__(256)
@@ -122,8 +122,8 @@ plan_nodes_kernel(const I* __restrict__ row, const I* __restrict__ indptr, long 
                   long long n_tiles, int32_t* __restrict__ tile_start, BandVerdict* __restrict__ verdict, unsigned aligning,
                   const int32_t* __restrict__ other, PlanHeader* __restrict__ hdr) {
   if (blockIdx.x == 0) {
-    const bool skewed = other && skewed_gather<256>(other, E);
-    if (threadIdx.x == 0) hdr->skewed = skewed;
+    const int repeats = other ? gather_repeats<256>(other, E) : 0;
+    if (threadIdx.x == 0) hdr->repeats = repeats;
     return;
   }
   const unsigned block = blockIdx.x - 1;
@@ -211,7 +211,8 @@ inline int plan_build(const I* row, const I* indptr, const I* eid, const I* indi
   plan->tile_start = g.tile_start;
   plan->flags |= GRAPHOP_PLAN_ROW_TILES;
   if (!host.row_crosses) plan->flags |= GRAPHOP_PLAN_NO_CARRY;
-  if (back.cover.skewed) plan->flags |= GRAPHOP_PLAN_SKEWED;
+  plan->gather_repeats = back.cover.repeats;
+  if (back.cover.repeats > skew_allowed(LLONG_MAX, E)) plan->flags |= GRAPHOP_PLAN_SKEWED;
   if (back.cover.cover_hi - back.cover.cover_lo >= E) plan->flags |= GRAPHOP_PLAN_COVERED;
   return GRAPHOP_OK;
 }

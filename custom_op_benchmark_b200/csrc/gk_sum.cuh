@@ -10,11 +10,11 @@
 // Against the gathering walker, B200.  Tables that fit the L2: 15360 nodes of 30 edges, 8 x 64 fp32, 94 -> 67 us (13.9 TB/s
 // of rows); 800 thousand skewed edges, 4 x 50, 180 -> 126 us; the source side of 4096 nodes of 16 edges, 8 x 64, 34 -> 23 us.
 // Larger ones with hubs: 50M edges to hubs, 2 x 64, 2.85 -> 1.85 ms; R-MAT 20, 4 x 32, 0.96 + 1.12 -> 0.87 + 0.99 ms; the
-// source side of R-MAT 21, 4 x 32, 4.40 -> 4.12 ms.  It loses, and the gathering walker stays, on larger tables without hubs
-// (321 thousand nodes, 6.3M edges, 2 x 64: 347 + 438 against 410 + 474 us; blocks of 47, 4 x 64: 1.95 against 3.6 ms: fewer
-// rows are on their way, and the L1 has nothing to add), on tables of 2 GB, which the DRAM bounds whatever the L1 holds (R-MAT
-// 22, 1 x 128: 3.46 + 4.28 against 4.00 + 4.75 ms), and for 2-byte elements, whose accumulators are twice as many registers
-// per slot (R-MAT 18, 2 x 64 bf16: 215 against 236 us; pairs, 4 x 64: 541 against 595 us).
+// source side of R-MAT 21, 4 x 32, 4.40 -> 4.12 ms.  Wide rows of few nodes: choose_walker.  It loses, and the gathering walker
+// stays, on larger tables without hubs (321 thousand nodes, 6.3M edges, 2 x 64: 347 + 438 against 410 + 474 us; blocks of 47,
+// 4 x 64: 1.95 against 3.6 ms: fewer rows are on their way, and the L1 has nothing to add), on tables of 2 GB, which the DRAM
+// bounds whatever the L1 holds (R-MAT 22, 1 x 128: 3.46 + 4.28 against 4.00 + 4.75 ms), and for 2-byte elements, whose
+// accumulators are twice as many registers per slot (R-MAT 18, 2 x 64 bf16: 215 against 236 us; pairs, 4 x 64: 541 against 595 us).
 #pragma once
 #include "gk_group.cuh"
 

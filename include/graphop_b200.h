@@ -165,7 +165,7 @@ enum {
   GRAPHOP_PLAN_ROW_TILES = 2, /* tile_start holds the work tiles' boundaries, moved up to row starts, ... */
   GRAPHOP_PLAN_NO_CARRY = 4,  /* ... and no node's positions cross one: row reductions finish in one launch */
   GRAPHOP_PLAN_COVERED = 8,   /* every position belongs to some chunk: no edge output needs clearing first */
-  GRAPHOP_PLAN_SKEWED = 16    /* few of the gathered rows are gathered by many edges: which kernels suit it */
+  GRAPHOP_PLAN_SKEWED = 16    /* few of the gathered rows are gathered by many edges, however many rows there are */
 };
 #define GRAPHOP_BAND_MAX_SPAN 384
 
@@ -183,7 +183,7 @@ typedef struct graphop_plan {
   int32_t band_span;       /* most different neighbours any 128 consecutive nodes reach (dense-band graphs) */
   const int32_t* tile_start; /* device, n_tiles + 1: first position of every work tile (GRAPHOP_PLAN_ROW_TILES) */
   int32_t tile;            /* cost per work tile the boundaries were made for */
-  int32_t reserved;
+  int32_t gather_repeats;  /* of up to 1024 evenly spaced positions, how many gather a row that another one gathers */
 } graphop_plan_t;
 
 /* Bytes of device memory (256-byte aligned) a plan of these sizes needs. */
