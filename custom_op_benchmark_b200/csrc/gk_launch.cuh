@@ -230,16 +230,22 @@ inline int allow_smem(Kernel kernel, int bytes, std::atomic<bool> (&configured)[
 // 5.84 / - / 5.70 / 5.84; R-MAT 22, 1 x 128, aggregate 13.5 / - / 12.7 / 12.5; with 4 K the chip is not filled evenly (R-MAT
 // 18: 3.0 ms).
 //
-// The summing walker's warps run in step on a small graph, and its resident warps (`slots`) are what a round of them is: one
-// round, or two where that would make long ones, beat any other number.  Its kernels by rounds: 4096 nodes of 16 edges, 8 x 64
-// fp32, 2.9 / 0.96 rounds 25 / 21 us; 150 thousand edges, 3 x 20, 1.7 / 0.9 17 / 14 us; 15360 nodes of 30 edges, 8 x 64,
-// 15.8 / 5.3 / 3.2 / 2.0 / 1.2 / 0.75 82 / 81 / 78 / 66 / 84 / 72 us.  Larger graphs get tiles of more than kSmallestTile.
+// The summing walker's warps run in step on a small graph, and what counts is how many rounds of the resident ones (`slots`: what
+// the launch bounds of its kernels allow, which use their registers up) they are.  Whole rounds are best, and a part of one just
+// above a whole one is worst: kernel times by rounds, 15360 nodes of 30 edges, 8 x 64 fp32, 15.8 / 3.9 / 3.2 / 2.6 / 2.0 / 1.6 / 1.3 /
+// 0.98 / 0.66 108 / 69 / 73 / 69 / 63 / 69 / 77 / 62 / 75 us.  So the warps are cut to one round, and to two where one round would
+// make them long (a warp inside hubs then ends last).  441 graphs of 1.1 to 25 rounds (blocks of 30, 16 and 50 random sources per
+// node, uniform, skewed; 1 to 8 blocks of heads), time over the best of the spans tried, mean and worst: a tile each 1.28, 1.90;
+// one round up to 4 and else two 1.03, 1.19 (at 4.1 rounds: 1.4 are left); up to 8 1.015, 1.12; up to 12 1.008, 1.12; always one
+// 1.006, 1.19 (skewed, 15 rounds).  The source side alone, 100 graphs: the same order.  Larger graphs get tiles of more than
+// kSmallestTile.
 //
 // The nodes of neighbouring tiles often gather the same rows (blocks, bands).  Where the tables do not fit the L2 as they are
 // and the graph is not known to be skewed, the warps at work had better lie close together: `most` (0: any number) is two.  331
 // thousand nodes in blocks of 47, 4 x 64 fp32, backward: 2.36 + 1.95 ms with a tile each, 2.83 + 2.37 with three; a row of 7M
 // edges on 1M nodes, 2 x 64: its records take 326 us to merge with a tile each, 168 with two.
 constexpr long long kWarpsWanted = 20480;
+constexpr int kOneRound = 12;
 constexpr long long kL2Table = 64ll << 20;
 inline int tiles_near(long long table) { return table > kL2Table ? 2 : 0; }
 inline unsigned tile_span(long long n_tiles, int nhb, int per_warp, int tile, long long slots, int most) {
@@ -248,7 +254,7 @@ inline unsigned tile_span(long long n_tiles, int nhb, int per_warp, int tile, lo
   if (most) {
     span = span < most ? span : most;
   } else if (slots && tile == kSmallestTile) {
-    const long long round = warps <= 4 * slots ? slots : 2 * slots;
+    const long long round = warps <= kOneRound * slots ? slots : 2 * slots;
     span = (warps + round - 1) / round;
   }
   return span < 1 ? 1 : span < n_tiles ? (unsigned)span : (unsigned)n_tiles;

@@ -41,6 +41,7 @@ struct SumShape {
   static constexpr int kRegs = 44 + kRows * (kUnroll * GEO::SB / 4 + 2 * kWords);   // fewer spill in the loop
   static constexpr int kRegsRounded = (kRegs + 7) / 8 * 8;
   static constexpr int kMinCtas = 65536 / (32 * kWarps * kRegsRounded);
+  static_assert(kMinCtas * (kWarps * kWarpBytes + 1024) <= 226 * 1024, "the registers say how many blocks are resident");
 };
 
 // Op interface (all members __device__), on top of its Geo and SumShape:
