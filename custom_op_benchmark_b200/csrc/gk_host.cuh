@@ -361,6 +361,8 @@ template <class F>
 inline int choose_walker(Arena& ar, const GraphView& g, int tables, long long table, int nhb, long long n_gathered, cudaStream_t st,
                          F&& f) {
   const long long all = tables * table, share = all / nhb;
+  // No row to gather, so no position has an edge: the summing walker loads row 0 in the place of one that is not there.
+  if (all == 0) return f(false, -1, 0);
   if (all <= kL2Table || (all <= 2 * kL2Table && share <= kSumShare)) return f(true, -1, 0);
   if (table > kSumTableBytes) return f(false, -1, tiles_near(table));
   if (share <= kSumFewRows) return f(true, -1, tiles_near(table));

@@ -106,3 +106,30 @@ def test_uncovered_positions(lead, tail):
     dst = th.repeat_interleave(th.arange(50), g.indptr[1:] - g.indptr[:-1]).to(DEV)
     keep = slice(lead, lead + e)
     _close(y, _sums(w[keep], x[:49], dst, src[keep].to(DEV), 50), th.float32, "y")
+
+
+# A caller of the C interface may pass edges that no chunk covers and a gathered table without rows.  Nothing of the table may be
+# read then; the pointers here lie in live allocations, and the kernels' names tell who ran.
+@pytest.mark.parametrize("op", ["vector_spmm_forward", "attention_backward"])
+def test_gathered_table_without_rows(op):
+    lib, e, n, h, d = _capi.lib(), 40, 5, 4, 32
+    none = th.zeros(2, dtype=th.int32, device=DEV)   # one chunk, of node 0, from position 0 to position 0
+    ids, w = th.arange(e, dtype=th.int32, device=DEV), _draw(th.float32, e, h, seed=1)
+    table = th.full((n, h, d), float("nan"), device=DEV)
+    out = th.full((3, n, h, d), float("nan"), device=DEV)
+    query = _capi.OP_SPMM_FWD if op == "vector_spmm_forward" else _capi.OP_ATTENTION_BWD_PAIRS
+    ws = th.empty(lib.graphop_workspace_bytes(query, e, n, h, d, 4, 4), dtype=th.uint8, device=DEV)
+    tail = [h, d, ws.data_ptr(), ws.numel(), th.cuda.current_stream().cuda_stream]
+    p = [t.data_ptr() for t in (none, none, ids, ids, w, table)]
+    if op == "vector_spmm_forward":
+        args, written = p + [out[0].data_ptr(), 1, e, n, 0] + tail, out[:1]
+    else:
+        rows = [table.data_ptr()] * 4 + [w.data_ptr(), table.data_ptr()]   # q, k, v, o, lse, d_o
+        args = p[:2] + [p[2], 1] + p[:4] + [1] + rows + [1.0] + [t.data_ptr() for t in out] + [e, 0, n] + tail
+        written = out[1:]
+    with th.profiler.profile(activities=[th.profiler.ProfilerActivity.CUDA]) as seen:
+        assert getattr(lib, "graphop_%s_f32_i32" % op)(*args) == _capi.OK
+        th.cuda.synchronize()
+    ran = [x.name for x in seen.events()]
+    assert any("group_walk_kernel" in x for x in ran) and not any("sum_walk_kernel" in x for x in ran), ran
+    assert bool((written == 0).all())
