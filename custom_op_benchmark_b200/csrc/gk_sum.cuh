@@ -217,6 +217,7 @@ sum_walk_kernel(const __grid_constant__ Op op, const __grid_constant__ WalkArgs 
     r0 = r1;
     starts0 = starts1; gaps0 = gaps1;
   }
+  cp_async_commit();   // what the last block published past the end, too: no copy is under way when the warp leaves
   cp_async_wait<0>();
 
   uint32_t tail_id = kNoRow;
