@@ -15,17 +15,26 @@ DEV = "cuda:0"
 TOL = {th.float32: 3e-5, th.bfloat16: 2e-2}
 
 
-@pytest.fixture(scope="module")
-def graph():
+def _graph(nodes, most):
     gen = th.Generator().manual_seed(5)
-    deg = th.randint(0, 12, (30_000,), generator=gen)
+    deg = th.randint(0, most, (nodes,), generator=gen)
     deg[th.rand(deg.numel(), generator=gen) < 0.2] = 0
-    deg[[7, 9_000, 9_001, 29_000]] = th.tensor([3_000, 40, 700, 131])
+    deg[[7, 3 * nodes // 10, 3 * nodes // 10 + 1, nodes - 1_000]] = th.tensor([3_000, 40, 700, 131])
     g = random_graph(deg.numel(), deg.numel(), deg, 6)
     row, ptr = partition_csr(g.indptr, 32)
     col, ptr_t = partition_csr(g.indptr_t, 32)
     tables = [[t.int().to(DEV) for t in o] for o in ((row, ptr, g.eid, g.indices), (col, ptr_t, g.eid_t, g.indices_t))]
     return g, tables
+
+
+@pytest.fixture(scope="module")
+def graph():
+    return _graph(30_000, 12)
+
+
+@pytest.fixture(scope="module")
+def long_rows():
+    return _graph(5_003, 240)
 
 
 def _draw(dtype, *shape, seed=0):
@@ -38,10 +47,23 @@ def _close(got, want, tol, what):
     assert err <= tol * max(1.0, float(want.abs().max())), (what, err)
 
 
-# 8 head blocks of 512 bytes and 150 thousand positions: three tiles per walk
+# 8 head blocks of 512 bytes or 16 of 256, K and V beyond the L2: two tiles per walk, for the forward and the destination side
 @pytest.mark.parametrize("dtype,h,d", [(th.float32, 8, 128), (th.bfloat16, 16, 128)])
 @pytest.mark.parametrize("planned", [False, True])
 def test_attention(graph, dtype, h, d, planned):
+    _attention(graph, dtype, h, d, planned)
+
+
+# K and V of 41 MB together, 15697 tiles: walks of any length, of three tiles in 4-byte elements and of six in bfloat16
+@pytest.mark.parametrize("dtype,h,d", [(th.float32, 8, 128), (th.bfloat16, 16, 128)])
+@pytest.mark.parametrize("planned", [False, True])
+def test_attention_in_long_walks(long_rows, dtype, h, d, planned):
+    g = long_rows[0]
+    assert ((g.n_edges + 4 * g.n_dst) // 32 + 1) % 3 != 0   # the last walk is shorter in both
+    _attention(long_rows, dtype, h, d, planned)
+
+
+def _attention(graph, dtype, h, d, planned):
     g, (r, c) = graph
     q, k, v = (_draw(dtype, g.n_dst, h, d, seed=i) for i in range(3))
     grad = _draw(dtype, g.n_dst, h, d, seed=3).detach()
@@ -55,7 +77,7 @@ def test_attention(graph, dtype, h, d, planned):
         _close(a, b, TOL[dtype], name)
 
 
-# one head in 64 pieces: a few dozen tiles per walk
+# one head in 64 or 128 pieces: ten tiles per walk of the 4-byte sums, two in bfloat16
 @pytest.mark.parametrize("dtype,d", [(th.float32, 8192), (th.float32, 8188), (th.bfloat16, 16384)])
 def test_aggregate_and_dot(graph, dtype, d):
     g, (r, c) = graph
