@@ -265,18 +265,6 @@ struct Shape {
   static constexpr int kMinCtas = kFit < kRegFit ? kFit : kRegFit;
 };
 
-// Op interface (all members __device__), on top of its Geo and Shape; `slot` is the ring step's memory at this lane:
-//   kRowOut, kUsesOther, kUsesEid, kFoldsEid; State, Carry
-//   setup(st, gl, hb)
-//   stage(st, slot, id, edge, live)               copy the rows of (other endpoint, edge) into the ring
-//   scalar_of(h, id, edge)                        where the edge's scalars of head h are
-//   fold<N>(st, slot, tab, active, pos, edge)     fold N = 1 or 2 positions per group (called by the whole warp); tab: the
-//                                                 table's entry of the first position and this lane's head
-//   stage_node(st, buf, lane, node)               copy what begin(node) will read into the node buffer
-//   begin(st, buf, lane)                          a node begins (called by the groups concerned)
-//   began(st, node, mine)                         the part of begin that needs the whole warp
-//   store_row(st, node), zero_row(st, node)
-//   begin_merge(st), merge(st, Carry), load_carry, save_carry, kCarryElems
 // Two walkers are launched where the better one is known on the device alone: one of them has nothing to do.
 __device__ __forceinline__ bool not_asked(const WalkArgs& a) { return a.only >= 0 && a.hdr->skewed != a.only; }
 
@@ -316,6 +304,19 @@ __device__ __forceinline__ bool cut_inside(const WalkArgs& a, unsigned j, int r)
   return __ldg(a.erow + (last < E ? last : E - 1)) == r;
 }
 
+// Op interface (all members __device__), on top of its Geo and Shape; `slot` is the ring step's memory at this lane:
+//   kRowOut, kUsesOther, kUsesEid, kFoldsEid; State, Carry
+//   setup(st, gl, hb)
+//   stage(st, slot, id, edge, live)               copy the rows of (other endpoint, edge) into the ring
+//   scalar_of(h, id, edge)                        where the edge's scalars of head h are
+//   fold<N>(st, slot, tab, active, pos, edge)     fold N = 1 or 2 positions per group (called by the whole warp); tab: the
+//                                                 table's entry of the first position and this lane's head
+//   stage_node(st, buf, lane, node)               copy what begin(node) will read into the node buffer
+//   begin(st, buf, lane)                          a node begins (called by the groups concerned)
+//   began(st, node, mine)                         the part of begin that needs the whole warp
+//   store_row(st, node), zero_row(st, node)
+//   begin_merge(st), merge(st, Carry), load_carry, save_carry, kCarryElems
+//
 // kPieces: walks of several tiles on a graph whose rows the tiles may cut.  A kernel of its own, because the few instructions
 // per block and per node that it has more cost 2 to 5 % where there is nothing to cut (the loop is bound by issue and its code
 // by the instruction cache; the same tests behind a flag cost as much).

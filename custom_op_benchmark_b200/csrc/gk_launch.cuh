@@ -240,8 +240,10 @@ inline int allow_smem(Kernel kernel, int bytes, std::atomic<bool> (&configured)[
 // 1.006, 1.19 (skewed, 15 rounds).  The source side alone, 100 graphs: the same order.  Larger graphs get tiles of more than
 // kSmallestTile.
 //
-// The nodes of neighbouring tiles often gather the same rows (blocks, bands).  Where the tables do not fit the L2 as they are
-// and the graph is not known to be skewed, the warps at work had better lie close together: `most` (0: any number) is two.  331
+// The nodes of neighbouring tiles often gather the same rows (blocks, bands).  Where the tables do not fit the L2 as they are,
+// the warps at work had better lie close together: `most` (0: any number) is two.  That goes by the tables' size alone for the
+// gathering walker, skewed or not; the summing walker has no limit on skewed graphs and two on tables of few rows
+// (choose_walker).  331
 // thousand nodes in blocks of 47, 4 x 64 fp32, backward: 2.36 + 1.95 ms with a tile each, 2.83 + 2.37 with three; a row of 7M
 // edges on 1M nodes, 2 x 64: its records take 326 us to merge with a tile each, 168 with two.
 constexpr long long kWarpsWanted = 20480;

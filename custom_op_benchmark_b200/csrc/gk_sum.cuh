@@ -1,16 +1,17 @@
 // The summing walker: sums of gathered rows with per-edge weights that are known beforehand (aggregation, the source side of
-// the attention backward from stored pairs), for elements of 4 and 8 bytes.  The decomposition, the carry records and the
-// order of the sums are the gathering walker's (gk_group.cuh); what differs is how rows arrive.  Nothing but multiply-adds is
+// the attention backward from stored pairs), for elements of 4 and 8 bytes.  The decomposition and the carry records are the
+// gathering walker's (gk_group.cuh); what differs is how rows arrive and in which groups a row's edges are added up: blocks of
+// G positions (the lanes of a group, 4 to 32), then their totals (flush).  Nothing but multiply-adds is
 // done with a row, so a lane holds its slot of kUnroll positions' rows in registers and loads the slot of the position kUnroll
 // on where it was used: kUnroll rows per lane group are on their way whatever the lengths of the nodes.  The loads go through
 // the L1, which serves the nodes that many edges share (the ring's copies pass it by), and shared memory holds the indices
 // and weights of two blocks of positions alone, so that most of the 256 KB are L1.  Bound by the L2's answers to what misses
 // there, and by issue slots on short rows.
 //
-// Against the gathering walker, B200.  Tables that fit the L2: 15360 nodes of 30 edges, 8 x 64 fp32, 94 -> 67 us (13.9 TB/s
+// Against the gathering walker, B200.  Tables that fit the L2: 15360 nodes of 30 edges, 8 x 64 fp32, 94 -> 70 us (13.5 TB/s
 // of rows); 800 thousand skewed edges, 4 x 50, 180 -> 126 us; the source side of 4096 nodes of 16 edges, 8 x 64, 34 -> 23 us.
-// Larger ones with hubs: 50M edges to hubs, 2 x 64, 2.85 -> 1.85 ms; R-MAT 20, 4 x 32, 0.96 + 1.12 -> 0.87 + 0.99 ms; the
-// source side of R-MAT 21, 4 x 32, 4.40 -> 4.12 ms.  Wide rows of few nodes: choose_walker.  It loses, and the gathering walker
+// Larger ones with hubs: 50M edges to hubs, 2 x 64, 2.85 -> 1.85 ms; R-MAT 20, 4 x 32, 0.96 + 1.12 -> 0.90 + 1.06 ms; the
+// source side of R-MAT 21, 4 x 32, 4.40 -> 4.09 ms.  Wide rows of few nodes: choose_walker.  It loses, and the gathering walker
 // stays, on larger tables without hubs (321 thousand nodes, 6.3M edges, 2 x 64: 347 + 438 against 410 + 474 us; blocks of 47,
 // 4 x 64: 1.95 against 3.6 ms: fewer rows are on their way, and the L1 has nothing to add), on tables of 2 GB, which the DRAM
 // bounds whatever the L1 holds (R-MAT 22, 1 x 128: 3.46 + 4.28 against 4.00 + 4.75 ms), and for 2-byte elements, whose
