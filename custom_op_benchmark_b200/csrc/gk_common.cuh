@@ -141,11 +141,11 @@ __device__ __forceinline__ void cut_tiles(const TileCut& cut, long long p, long 
 // bits tells.  Many where few rows are gathered by many edges (R-MAT 20: 37 to 48, R-MAT 16: 141 to 166, a hub that has a tenth of
 // the edges: 100), none where the neighbours follow the nodes, and as many as chance has it where the sources are uniform: 8 of
 // different rows that share a bit, and more of the same row the fewer rows there are (skew_allowed).  For one block of THREADS;
-// the answer is every thread's.
+// the answer is every thread's.  seen: the table, in shared or device memory, nobody else's meanwhile.
 constexpr int kSkewSamples = 1024, kSkewBits = 65536;
 template <int THREADS>
-__device__ __forceinline__ int gather_repeats(const int32_t* __restrict__ other, long long E) {
-  __shared__ __align__(16) unsigned s_seen[kSkewBits / 32];
+__device__ __forceinline__ int gather_repeats(const int32_t* __restrict__ other, long long E, unsigned* seen) {
+  __shared__ int s_repeats;
   const int tid = threadIdx.x, n = E < kSkewSamples ? (int)E : kSkewSamples;
   int key[kSkewSamples / THREADS], repeats = 0;   // all asked for before any is looked at
 #pragma unroll
@@ -153,25 +153,24 @@ __device__ __forceinline__ int gather_repeats(const int32_t* __restrict__ other,
     const int k = tid + i * THREADS;
     key[i] = k < n ? __ldg(other + E * k / n) : -1;
   }
-  for (int i = tid; i < kSkewBits / 128; i += THREADS) reinterpret_cast<uint4*>(s_seen)[i] = make_uint4(0, 0, 0, 0);
+  for (int i = tid; i < kSkewBits / 128; i += THREADS) reinterpret_cast<uint4*>(seen)[i] = make_uint4(0, 0, 0, 0);
+  if (tid == 0) s_repeats = 0;
   __syncthreads();
 #pragma unroll
   for (int i = 0; i < kSkewSamples / THREADS; ++i) {
     const unsigned at = (unsigned)key[i] * 2654435761u >> 16, bit = 1u << (at & 31);
-    if (key[i] >= 0 && (atomicOr(s_seen + (at >> 5), bit) & bit)) ++repeats;
+    if (key[i] >= 0 && (atomicOr(seen + (at >> 5), bit) & bit)) ++repeats;
   }
 #pragma unroll
   for (int o = 16; o; o >>= 1) repeats += __shfl_xor_sync(kFull, repeats, o);
+  if ((tid & 31) == 0) atomicAdd(&s_repeats, repeats);
   __syncthreads();
-  if (tid == 0) s_seen[0] = 0;
-  __syncthreads();
-  if ((tid & 31) == 0) atomicAdd(s_seen, (unsigned)repeats);
-  __syncthreads();
-  return (int)s_seen[0];
+  return s_repeats;
 }
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS) skew_kernel(const int32_t* __restrict__ other, long long E, int allowed, PlanHeader* __restrict__ hdr) {
-  const int repeats = gather_repeats<THREADS>(other, E);
+  __shared__ __align__(16) unsigned s_seen[kSkewBits / 32];
+  const int repeats = gather_repeats<THREADS>(other, E, s_seen);
   if (threadIdx.x == 0) hdr->skewed = repeats > allowed;
 }
 
