@@ -241,6 +241,7 @@ struct FeatGeo : Geo<T_, 16, G_, W_, G_> {
 template <class GEO, int kRows, int kScalar, int kState, int kNode, int kNodeScalar, int kU, bool kShare = false>
 struct Shape {
   static constexpr bool kSums = false;
+  static constexpr bool kOptional = false;   // may be one of two walkers launched for the same sums
   static constexpr int kWarps = 1;
   static constexpr int kStepBytes = kRows * GEO::kRow;
   static constexpr int kNodeScalarAt = kNode * GEO::kRow;                  // from the node's room
@@ -265,8 +266,11 @@ struct Shape {
   static constexpr int kMinCtas = kFit < kRegFit ? kFit : kRegFit;
 };
 
-// Two walkers are launched where the better one is known on the device alone: one of them has nothing to do.
-__device__ __forceinline__ bool not_asked(const WalkArgs& a) { return a.only >= 0 && a.hdr->skewed != a.only; }
+// Two walkers are launched where the better one is known on the device alone: one of them has nothing to do.  Ops that are never
+// one of two do not ask (in their merge kernel the question alone took the loads of records apart: 17804 nodes, 82 thousand skewed
+// edges, 8 x 64 bf16, destination side, 8.9 -> 15.6 us).
+template <class Op>
+__device__ __forceinline__ bool not_asked(const WalkArgs& a) { return Op::kOptional && a.only >= 0 && a.hdr->skewed != a.only; }
 
 // The positions of tile t of a launch, for the lane group that walks it (called by the whole warp; here: the tile exists).  A
 // nominal boundary moves up to the first row start within the following `tile` positions, so that only rows longer than a
@@ -332,7 +336,7 @@ group_walk_kernel(const __grid_constant__ Op op, const __grid_constant__ WalkArg
   const int g = lane / G, gl = lane & (G - 1);
   const int hb = blockIdx.y;
   const unsigned t0 = (blockIdx.x * Op::kWarps + w) * NE;   // the warp's first tile
-  if (t0 >= a.n_tiles || not_asked(a)) return;
+  if (t0 >= a.n_tiles || not_asked<Op>(a)) return;
   const unsigned t = t0 + g;
   const bool here = t < a.n_tiles;
   int begin, n;   // the group's first position and their number
@@ -589,7 +593,7 @@ carry_rows_kernel(const __grid_constant__ Op op, const __grid_constant__ WalkArg
   A* part = reinterpret_cast<A*>(gk_ring);   // UNITS records
   __shared__ unsigned s_start[THREADS / 2], s_long[THREADS / 2];
   __shared__ int s_n, s_nlong, s_end;
-  if (not_asked(a)) return;
+  if (not_asked<Op>(a)) return;
   const int tid = threadIdx.x, u = tid / G, gl = tid & (G - 1), hb = blockIdx.y;
   const uint32_t* ids = a.rows + (size_t)hb * 2 * a.n_tiles;
   const A* rec = reinterpret_cast<const A*>(a.carry) + (size_t)hb * 2 * a.n_tiles * CE;
@@ -681,7 +685,7 @@ struct GroupAggregate : GEO, Shape<GEO, 1, (int)sizeof(typename GEO::T), 1, 0, 0
   using F = typename GEO::F;
   static constexpr const char* kName = kEdgeFeat ? "aggregate_edge_feat" : "aggregate";
   static constexpr bool kRowOut = true, kUsesOther = !kEdgeFeat, kUsesEid = true,
-                        kFoldsEid = false;
+                        kFoldsEid = false, kOptional = !kEdgeFeat && sizeof(T) >= 4;
   static constexpr int W = GEO::W;
   const T* __restrict__ w;
   const T* __restrict__ x;
@@ -1129,7 +1133,7 @@ struct GroupAttnBwdSrc : GEO, Shape<GEO, 2, 2 * (int)sizeof(typename GEO::A), kP
   static constexpr int W = GEO::W, V = GEO::V, kRow = GEO::kRow;   // rows of a ring step: q, dO
   static constexpr const char* kName = "attention_bwd_src";
   static constexpr bool kRowOut = true, kUsesOther = true, kUsesEid = kPairs,
-                        kFoldsEid = false;
+                        kFoldsEid = false, kOptional = kPairs && sizeof(T) >= 4;
   const T* __restrict__ q;
   const T* __restrict__ k;
   const T* __restrict__ v;

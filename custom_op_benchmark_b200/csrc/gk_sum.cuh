@@ -30,7 +30,7 @@ __device__ __forceinline__ void sts_int(unsigned at, int v) { asm volatile("st.s
 // block: with one, the 32 blocks an SM takes are too few warps; with more, a block holds its place until the slowest is done.
 template <class GEO, int kRows, int kScalar>
 struct SumShape {
-  static constexpr bool kSums = true;
+  static constexpr bool kSums = true, kOptional = true;
   static constexpr int kWarps = 2;
   static constexpr int kUnroll = 4;
   static constexpr int kIdsBytes = 32 * 4;                                 // the gathered rows' ids of a block of positions
@@ -66,7 +66,7 @@ sum_walk_kernel(const __grid_constant__ Op op, const __grid_constant__ WalkArgs 
   const int g = lane / G, gl = lane & (G - 1);
   const int hb = blockIdx.y;
   const unsigned t0 = (blockIdx.x * Op::kWarps + w) * NE;   // the warp's first tile
-  if (t0 >= a.n_tiles || not_asked(a)) return;
+  if (t0 >= a.n_tiles || not_asked<Op>(a)) return;
   const unsigned t = t0 + g;
   const bool here = t < a.n_tiles;
   int j0, n;   // the group's first position and their number
