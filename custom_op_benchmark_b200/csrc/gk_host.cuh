@@ -351,12 +351,13 @@ inline int skew_allowed(long long n, long long E) {
 // thousand of 16, 8 x 64 (117 MB, blocks of 29), 177 to 207 against 202 to 214; 80 thousand (156 MB, blocks of 39) 266 against 248.
 // Any larger one of so few rows that several blocks' shares fit, as long as the walks stay short enough for the blocks to follow
 // one another: 4000 nodes of 30 edges, 128 x 128 (250 MB, blocks of 2), 632 against 726 us, but 926 in walks of any length; 20
-// thousand of 16, 16 x 128 (156 MB, blocks of 10), 234 against 246.  Other larger ones, up to kSumTableBytes each, where few of
-// their rows are gathered by many edges.  f(sums, only, most) launches the summing or the gathering walker: where the graph's skew
+// thousand of 16, 16 x 128 (156 MB, blocks of 10), 234 against 246.  Other larger ones, up to kSumTableBytes each and
+// kSumAllBytes together, where few of their rows are gathered by many edges (two tables, 2.1 GB, R-MAT 21: 4.40 -> 4.09 ms; 3.0 GB,
+// 6.2M skewed edges on 1.47M nodes, 4 x 64: 1.41 against 1.64 ms).  f(sums, only, most) launches the summing or the gathering walker: where the graph's skew
 // is known to the device alone both are, and the one that it does not ask for returns at once (14 us a call, with the question:
 // 98 -> 112 us on 1.4M uniform edges, 358 -> 379 on 6M; hubs 284 -> 112 and 541 -> 193).
 template <typename T> constexpr bool kSumsByRegister = sizeof(T) >= 4;
-constexpr long long kSumTableBytes = 3ll << 29, kSumShare = 32ll << 20, kSumFewRows = 8ll << 20;
+constexpr long long kSumTableBytes = 3ll << 29, kSumAllBytes = 5ll << 29, kSumShare = 32ll << 20, kSumFewRows = 8ll << 20;
 template <class F>
 inline int choose_walker(Arena& ar, const GraphView& g, int tables, long long table, int nhb, long long n_gathered, cudaStream_t st,
                          F&& f) {
@@ -364,7 +365,7 @@ inline int choose_walker(Arena& ar, const GraphView& g, int tables, long long ta
   // No row to gather, so no position has an edge: the summing walker loads row 0 in the place of one that is not there.
   if (all == 0) return f(false, -1, 0);
   if (all <= kL2Table || (all <= 2 * kL2Table && share <= kSumShare)) return f(true, -1, 0);
-  if (table > kSumTableBytes) return f(false, -1, tiles_near(table));
+  if (table > kSumTableBytes || all > kSumAllBytes) return f(false, -1, tiles_near(table));
   if (share <= kSumFewRows) return f(true, -1, tiles_near(table));
   const int allowed = skew_allowed(n_gathered, g.E);
   if (g.repeats >= 0) return g.repeats > allowed ? f(true, -1, 0) : f(false, -1, tiles_near(table));
