@@ -243,7 +243,9 @@ inline int allow_smem(Kernel kernel, int bytes, std::atomic<bool> (&configured)[
 // The nodes of neighbouring tiles often gather the same rows (blocks, bands).  Where the tables do not fit the L2 as they are,
 // the warps at work had better lie close together: `most` (0: any number) is two.  That goes by the tables' size alone for the
 // gathering walker, skewed or not; the summing walker has no limit on skewed graphs and two on tables of few rows
-// (choose_walker).  331
+// (choose_walker).  Where a plan says that no row is cut there are no records to save, and the gathering walker stays with a tile
+// each: 900 thousand nodes in blocks of 50, 1 x 64 fp32, backward 1.84 + 1.66 ms, with two 1.93 + 2.17; 9.6M uniform edges on 2M
+// nodes, 2 x 64, 1.71 + 2.07 + 1.98 ms against 1.75 + 2.09 + 2.01.  331
 // thousand nodes in blocks of 47, 4 x 64 fp32, backward: 2.36 + 1.95 ms with a tile each, 2.83 + 2.37 with three; a row of 7M
 // edges on 1M nodes, 2 x 64: its records take 326 us to merge with a tile each, 168 with two.
 constexpr long long kWarpsWanted = 20480;
@@ -283,7 +285,8 @@ inline int launch_walk(Arena& ar, const GraphView& g, const GeoPick& p, const Op
   a.tile_start = g.tile_start;
   a.E = g.E; a.n_rows = n_rows; a.tile = g.tile; a.aligned = g.aligned; a.only = only;
   a.cut_tiles = (unsigned)g.n_tiles;
-  a.span = tile_span(g.n_tiles, p.nhb, Op::NE, g.tile, Op::kSums ? 148ll * Op::kMinCtas * Op::kWarps : 0, most);
+  a.span = tile_span(g.n_tiles, p.nhb, Op::NE, g.tile, Op::kSums ? 148ll * Op::kMinCtas * Op::kWarps : 0,
+                     most && g.no_carry && !Op::kSums ? 1 : most);
   if (Op::kSums) a.span = a.span < sum_span(g.tile, Op::G) ? a.span : sum_span(g.tile, Op::G);
   a.n_tiles = (a.cut_tiles + a.span - 1) / a.span;
   const bool cuts = Op::kRowOut && !g.no_carry;
